@@ -18,15 +18,17 @@
 
 namespace sray {
 
-/* photon map on the device: photons in Morton order of their grid cell,
- * a dense table of (first, count) per cell */
+/* photon map on the device: photons in the order of their grid cell (x
+ * fastest, so that a row of cells is one run of photons), and the photons
+ * before every cell */
 struct DPhotonMap {
 	const DevPhoton *ph;
-	const uint2 *cells;       /* per linear cell: first photon, count */
+	const unsigned *start;    /* per linear cell and one past the last: the photons in the cells before it */
 	int n;
 	int dims[3];
 	float org[3];
-	float cell;
+	float cell, inv_cell;
+	float reach;              /* the radius in cells, rounded up */
 	int k;                    /* 0 = fixed-radius range gather, >0 = k nearest */
 	double range;             /* query radius as the kd-tree sees it (float-rounded) */
 	float inv_area;           /* range mode: 1 / (pi r^2) of the unrounded radius */

@@ -8,13 +8,12 @@
  *                   (src/scene.cc:571-760), one interaction per pass; the
  *                   renderer's k_trace finds the hits in between
  *   compaction      keeps stored photons in emission order
- *   k_rs_*          stable LSD radix sort of the photons by the Morton code of
- *                   their grid cell
- *   k_cells         (first, end) of every occupied cell
+ *   k_rs_*          stable LSD radix sort of the photons by their grid cell
+ *   k_starts        the photons before every cell
  * PhotonMap::add_photon / scale_photon_power (src/pmap.cc:73-100) become the
  * per-light power scale applied at store time.  The kd-tree of the reference
- * (kd_insert3f, kd_nearest_range3f) is replaced by the Morton-ordered grid:
- * a range query visits the cells overlapping the query cube and tests every
+ * (kd_insert3f, kd_nearest_range3f) is replaced by the grid: a range
+ * query visits the rows of cells that its sphere reaches and tests every
  * photon in them with the kd-tree's distance rule, so the photon set of each
  * gather is the same.
  */
@@ -518,18 +517,22 @@ __device__ __forceinline__ unsigned spread3(unsigned v)
 	return v;
 }
 
-__global__ void k_keys(const DevPhoton *ph, int n, DPhotonMap M, int morton, unsigned *keys, unsigned *vals, unsigned *lin)
+__device__ __forceinline__ unsigned cell_key(const DevPhoton &p, const DPhotonMap &M, int morton)
+{
+	int c[3];
+	for(int a = 0; a < 3; a++) {
+		double v = floor(((double)p.p[a] - (double)M.org[a]) / (double)M.cell);
+		c[a] = v < 0.0 ? 0 : (v > (double)(M.dims[a] - 1) ? M.dims[a] - 1 : (int)v);
+	}
+	return morton ? (spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2))
+		: (unsigned)(((size_t)c[2] * M.dims[1] + c[1]) * M.dims[0] + c[0]);
+}
+
+__global__ void k_keys(const DevPhoton *ph, int n, DPhotonMap M, int morton, unsigned *keys, unsigned *vals)
 {
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		int c[3];
-		for(int a = 0; a < 3; a++) {
-			double v = floor(((double)ph[i].p[a] - (double)M.org[a]) / (double)M.cell);
-			c[a] = v < 0.0 ? 0 : (v > (double)(M.dims[a] - 1) ? M.dims[a] - 1 : (int)v);
-		}
-		unsigned l = (unsigned)(((size_t)c[2] * M.dims[1] + c[1]) * M.dims[0] + c[0]);
-		keys[i] = morton ? (spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2)) : l;
+		keys[i] = cell_key(ph[i], M, morton);
 		vals[i] = (unsigned)i;
-		lin[i] = l;
 	}
 }
 
@@ -581,22 +584,69 @@ __global__ void k_rs_scatter(const unsigned *keys, const unsigned *vals, int n, 
 	}
 }
 
-__global__ void k_permute(const DevPhoton *in, const unsigned *vals, const unsigned *lin_in, int n, DevPhoton *out, unsigned *lin_out)
+__global__ void k_permute(const DevPhoton *in, const unsigned *vals, int n, DevPhoton *out)
 {
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		unsigned v = vals[i];
-		out[i] = in[v];
-		lin_out[i] = lin_in[v];
-	}
+	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = in[vals[i]];
 }
 
-__global__ void k_cells(const unsigned *lin, int n, uint2 *cells)
+/* the first of keys[lo, hi) (ascending) that is at least k */
+__device__ __forceinline__ unsigned lower_key(const unsigned *keys, unsigned lo, unsigned hi, unsigned k)
 {
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		unsigned l = lin[i];
-		if(i == 0 || lin[i - 1] != l) cells[l].x = (unsigned)i;
-		if(i == n - 1 || lin[i + 1] != l) cells[l].y = (unsigned)(i + 1);
+	while(lo < hi) {
+		unsigned mid = (lo + hi) >> 1;
+		if(__ldg(keys + mid) < k) lo = mid + 1;
+		else hi = mid;
 	}
+	return lo;
+}
+
+/* A map's cell table from the sorted cell keys of its photons [i0, i1):
+ * start[c] = its photons (counted from i0) in cells before c, for every cell
+ * and one past the last.  A block takes START_CELLS cells: two searches find
+ * its photons, counters in shared memory their cells, a scan the starts;
+ * what bounds it is the table's own write (4 bytes a cell). */
+#define START_CELLS 2048
+__device__ __forceinline__ void cell_starts(const unsigned *keys, unsigned i0, unsigned i1, size_t ncells, unsigned *start)
+{
+	__shared__ unsigned cnt[START_CELLS];
+	__shared__ unsigned range[2];
+	__shared__ unsigned wsum[8];
+	const size_t c0 = (size_t)blockIdx.x * START_CELLS;
+	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+	if(t < 2) range[t] = lower_key(keys, i0, i1, (unsigned)min(c0 + (size_t)t * START_CELLS, (size_t)0xffffffffu));
+	for(int i = t; i < START_CELLS; i += 256) cnt[i] = 0;
+	__syncthreads();
+	const unsigned b = range[0], e = range[1];
+	for(unsigned i = b + t; i < e; i += 256) atomicAdd(&cnt[__ldg(keys + i) - (unsigned)c0], 1u);
+	__syncthreads();
+	/* eight cells per thread, scanned over the block */
+	unsigned v[8], s = 0;
+	#pragma unroll
+	for(int k = 0; k < 8; k++) {
+		v[k] = cnt[t * 8 + k];
+		s += v[k];
+	}
+	unsigned incl = s;
+	for(int o = 1; o < 32; o <<= 1) {
+		unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+		if(lane >= o) incl += u;
+	}
+	if(lane == 31) wsum[w] = incl;
+	__syncthreads();
+	unsigned run = b - i0 + incl - s;
+	for(int k = 0; k < w; k++) run += wsum[k];
+	#pragma unroll
+	for(int k = 0; k < 8; k++) {
+		cnt[t * 8 + k] = run;
+		run += v[k];
+	}
+	__syncthreads();
+	for(int i = t; i < START_CELLS && c0 + i <= ncells; i += 256) start[c0 + i] = cnt[i];
+}
+
+__global__ void __launch_bounds__(256) k_starts(const unsigned *keys, int n, size_t ncells, unsigned *start)
+{
+	cell_starts(keys, 0, (unsigned)n, ncells, start);
 }
 
 /* Photon launches run beside the frame's higher-priority stream: a block
@@ -828,30 +878,58 @@ int photon_shoot_maps(Renderer &R, const DScene &base, const std::vector<uint32_
 	return photon_finalize(R, 1, valid + o1, ph + o1, out[0].total[1], s, ng);
 }
 
-/* A map's grid over box rb for gathers of radius rad (k nearest, or all
- * within rad when k = 0): cells twice the radius, so that a query cube
- * overlaps at most 2x2x2, at most 2^26 of them; the map's range constants.
- * Morton keys when every dimension fits 10 bits. */
-static void map_grid(int k, double rad, const Box &rb, DPhotonMap &M, bool *morton, size_t *ncells)
+/* A map's grid over box rb: cells of the given width, at most 2^26 of them;
+ * returns their number */
+static size_t map_cells(double width, const Box &rb, DPhotonMap &M)
 {
-	double cell = rad > 0.0 ? 2.0 * rad : 1.0;
+	double cell = width;
 	double ext[3];
 	for(int a = 0; a < 3; a++) ext[a] = rb.mx[a] - rb.mn[a];
 	int dims[3];
 	for(;;) {
 		double total_cells = 1.0;
 		for(int a = 0; a < 3; a++) {
-			dims[a] = (int)floor(ext[a] / cell) + 1;
-			total_cells *= dims[a];
+			double d = floor(ext[a] / cell) + 1.0;
+			dims[a] = d < 67108864.0 ? (int)d : 67108864;
+			total_cells *= d;
 		}
 		if(total_cells <= (double)(1 << 26)) break;
 		cell *= 1.25;
 	}
-	M.k = k;
 	M.cell = (float)cell;
 	while((double)M.cell < cell) M.cell = nextafterf(M.cell, INFINITY);
 	for(int a = 0; a < 3; a++) { M.dims[a] = dims[a]; M.org[a] = (float)rb.mn[a]; }
 	for(int a = 0; a < 3; a++) while((double)M.org[a] > rb.mn[a]) M.org[a] = nextafterf(M.org[a], -INFINITY);
+	return (size_t)dims[0] * dims[1] * dims[2];
+}
+
+/* The map of n photons over box rb for gathers of radius rad (k nearest, or
+ * all within rad when k = 0): its range constants and the grid that queries
+ * walk.  A query reads the photons of whole cells; on a surface, the cells
+ * that the range reaches cover 1.7 times its disc when they are half the
+ * radius wide, 2.6 times at the radius and 4.8 times at twice the radius.
+ * Measured, 500,009 points of a map of 500k emitted photons: 1.17 ms at half
+ * the radius, 1.25 at the radius, 1.43 at twice, and 1.28 at a third, where
+ * the rows to look up outweigh the photons saved.  A finer grid costs its
+ * table, 4 bytes a cell to write at every build: the finest of the three
+ * widths whose table has at most 32 cells per photon (and 65,536) is taken,
+ * so that the table stays small beside the photons (48 bytes each, moved
+ * several times by the sort). */
+static size_t map_grid(int k, double rad, const Box &rb, int n, DPhotonMap &M)
+{
+	const double most = 32.0 * n + 65536.0;
+	size_t ncells = 0;
+	const double f[3] = {0.5, 1.0, 2.0};
+	for(int i = 0; i < 3; i++) {
+		double w = rad > 0.0 ? f[i] * rad : 1.0;
+		double cells = 1.0;
+		for(int a = 0; a < 3; a++) cells *= floor((rb.mx[a] - rb.mn[a]) / w) + 1.0;
+		if(cells > most && i < 2) continue;
+		ncells = map_cells(w, rb, M);
+		break;
+	}
+	M.n = n;
+	M.k = k;
 	M.range = (double)(float)rad;
 	M.inv_area = (float)(1.0 / (M_PI * (rad * rad)));
 	M.range_f = (float)rad;
@@ -861,11 +939,21 @@ static void map_grid(int k, double rad, const Box &rb, DPhotonMap &M, bool *mort
 		M.r2_lo = (float)(r2 - (double)M.r2_hi);
 		M.screen = (float)(r2 * (1.0 + 1.0 / 1048576.0));
 	}
-	*morton = dims[0] <= 1024 && dims[1] <= 1024 && dims[2] <= 1024;
-	*ncells = (size_t)dims[0] * dims[1] * dims[2];
+	M.inv_cell = (float)(1.0 / (double)M.cell);
+	M.reach = (float)((double)M.range_f / (double)M.cell * (1.0 + 1e-6));
+	return ncells;
 }
 
-/* the map over the n photons in P.ph: grid, Morton sort, cell table */
+static int key_bits(unsigned maxkey)
+{
+	int bits = 0;
+	while(bits < 32 && (maxkey >> bits)) bits++;
+	return bits;
+}
+
+/* the map over the n photons in P.ph: grid, sort by cell, cell table.  The
+ * photons as given stay in P.tmp_ph (photon_map_read's order starts from
+ * them). */
 int photon_map_build(Renderer &R, int global, int n, cudaStream_t s)
 {
 	PhotonBufs &P = global ? R.gi : R.caust;
@@ -877,43 +965,57 @@ int photon_map_build(Renderer &R, int global, int n, cudaStream_t s)
 	int k = global ? opt.gi_k : opt.caust_k;
 	/* a job of a batch gathers with the radius of its own interval */
 	double rad = k > 0 ? (double)opt.gather_rcap : (R.map_gather_dist >= 0.0 ? R.map_gather_dist : R.sc.gather_dist);
-	DPhotonMap &M = P.map;
-	bool morton;
-	size_t ncells;
-	map_grid(k, rad, rb, M, &morton, &ncells);
-	M.n = n;
+	DPhotonMap M = DPhotonMap();
+	const size_t ncells = map_grid(k, rad, rb, n, M);
+	map_cells(rad > 0.0 ? 2.0 * rad : 1.0, rb, P.order);
 	PCK(P.keys.ensure((size_t)n * 4), "keys");
 	PCK(P.keys2.ensure((size_t)n * 4), "keys");
 	PCK(P.vals.ensure((size_t)n * 4), "vals");
 	PCK(P.vals2.ensure((size_t)n * 4), "vals");
-	PCK(P.lin.ensure((size_t)n * 8), "cell ids");
-	PCK(P.cells.ensure(ncells * sizeof(uint2)), "cell table");
-	unsigned *keys = P.keys.as<unsigned>(), *keys2 = P.keys2.as<unsigned>();
-	unsigned *vals = P.vals.as<unsigned>(), *vals2 = P.vals2.as<unsigned>();
-	unsigned *lin = P.lin.as<unsigned>(), *lin2 = lin + n;
-	LAUNCH(R, "photon_sort", s, k_keys<<<grid_n(n, 256), 256, 0, s>>>(P.ph.as<DevPhoton>(), n, M, morton ? 1 : 0, keys, vals, lin));
-	unsigned maxkey = morton ? (1u << 30) - 1u : (unsigned)(ncells - 1);
-	int bits = 0;
-	while(bits < 32 && (maxkey >> bits)) bits++;
-	int passes = (bits + 7) / 8;
-	int nbr = (n + TILE - 1) / TILE;
-	PCK(P.hist.ensure((size_t)256 * nbr * sizeof(unsigned) + 16), "radix histogram");
-	for(int ps = 0; ps < passes; ps++) {
-		int shift = ps * 8;
-		LAUNCH(R, "photon_sort", s, k_rs_hist<<<nbr, RS_THREADS, 0, s>>>(keys, n, shift, P.hist.as<unsigned>(), nbr));
-		LAUNCH(R, "photon_sort", s, k_scan_excl<<<1, 1024, 0, s>>>(P.hist.as<unsigned>(), 256 * nbr, nullptr));
-		LAUNCH(R, "photon_sort", s, k_rs_scatter<<<nbr, RS_THREADS, 0, s>>>(keys, vals, n, shift, P.hist.as<unsigned>(), nbr, keys2, vals2));
-		std::swap(keys, keys2);
-		std::swap(vals, vals2);
-	}
+	PCK(P.starts.ensure((ncells + 1) * sizeof(unsigned)), "cell table");
 	PCK(P.tmp_ph.ensure((size_t)n * sizeof(DevPhoton)), "photon buffer");
-	LAUNCH(R, "photon_sort", s, k_permute<<<grid_n(n, 256), 256, 0, s>>>(P.ph.as<DevPhoton>(), vals, lin, n, P.tmp_ph.as<DevPhoton>(), lin2));
-	PCK(cudaMemsetAsync(P.cells.p, 0, ncells * sizeof(uint2), s), "cell table");
-	LAUNCH(R, "photon_sort", s, k_cells<<<grid_n(n, 256), 256, 0, s>>>(lin2, n, P.cells.as<uint2>()));
+	unsigned *keys = P.keys.as<unsigned>(), *vals = P.vals.as<unsigned>();
+	LAUNCH(R, "photon_sort", s, k_keys<<<grid_n(n, 256), 256, 0, s>>>(P.ph.as<DevPhoton>(), n, M, 0, keys, vals));
+	if(int r = sort_pairs(R, keys, vals, P.keys2.as<unsigned>(), P.vals2.as<unsigned>(), n, key_bits((unsigned)(ncells - 1)), P.hist, P.scan,
+			"photon_sort", s, &keys, &vals))
+		return r;
+	LAUNCH(R, "photon_sort", s, k_permute<<<grid_n(n, 256), 256, 0, s>>>(P.ph.as<DevPhoton>(), vals, n, P.tmp_ph.as<DevPhoton>()));
+	LAUNCH(R, "photon_sort", s, k_starts<<<(unsigned)((ncells + START_CELLS) / START_CELLS), 256, 0, s>>>(keys, n, ncells,
+			P.starts.as<unsigned>()));
 	std::swap(P.ph, P.tmp_ph);
 	M.ph = P.ph.as<DevPhoton>();
-	M.cells = P.cells.as<uint2>();
+	M.start = P.starts.as<unsigned>();
+	P.map = M;
 	PCK(cudaStreamSynchronize(s), "photon map build");
+	R.prof_collect();
+	return 0;
+}
+
+/* The photons of map `global` as programs see them (sray_gpu_get_photons,
+ * dumps): in Morton order of cells twice the gather radius (linear order
+ * where a dimension passes 10 bits), ties in emission order, into h. */
+int photon_map_read(Renderer &R, int global, std::vector<DevPhoton> &h, cudaStream_t s)
+{
+	PhotonBufs &P = global ? R.gi : R.caust;
+	const int n = P.map.n;
+	h.resize(n > 0 ? n : 0);
+	if(n <= 0) return 0;
+	const DPhotonMap &M = P.order;
+	const int morton = M.dims[0] <= 1024 && M.dims[1] <= 1024 && M.dims[2] <= 1024;
+	const size_t ncells = (size_t)M.dims[0] * M.dims[1] * M.dims[2];
+	struct Scratch {
+		DevBuf b;
+		~Scratch() { b.release(); }
+	} out;
+	PCK(out.b.ensure((size_t)n * sizeof(DevPhoton)), "photon buffer");
+	unsigned *keys = P.keys.as<unsigned>(), *vals = P.vals.as<unsigned>();
+	LAUNCH(R, "photon_sort", s, k_keys<<<grid_n(n, 256), 256, 0, s>>>(P.tmp_ph.as<DevPhoton>(), n, M, morton, keys, vals));
+	if(int r = sort_pairs(R, keys, vals, P.keys2.as<unsigned>(), P.vals2.as<unsigned>(), n, morton ? 30 : key_bits((unsigned)(ncells - 1)),
+			P.hist, P.scan, "photon_sort", s, &keys, &vals))
+		return r;
+	LAUNCH(R, "photon_sort", s, k_permute<<<grid_n(n, 256), 256, 0, s>>>(P.tmp_ph.as<DevPhoton>(), vals, n, out.b.as<DevPhoton>()));
+	PCK(cudaMemcpyAsync(h.data(), out.b.p, (size_t)n * sizeof(DevPhoton), cudaMemcpyDeviceToHost, s), "read photons");
+	PCK(cudaStreamSynchronize(s), "read photons");
 	R.prof_collect();
 	return 0;
 }
@@ -994,21 +1096,26 @@ __global__ void k_seg_offsets(const int *valid, const unsigned *tile_offs, const
 	if(threadIdx.x == 0) offs[blockIdx.x] = tile_offs[tile] + (unsigned)red[0];
 }
 
-/* cell keys of the compacted photons, each in its segment's grid */
-__global__ void k_keys_seg(const DevPhoton *ph, int n, const DPhotonMap *grids, const int *morton, const unsigned *offs, int nseg,
-		unsigned *keys, unsigned *vals, unsigned *lin)
+/* cell keys of the compacted photons, each in its segment's grid; kept in
+ * `lin` too, for the cell tables */
+__global__ void k_keys_seg(const DevPhoton *ph, int n, const DPhotonMap *grids, const unsigned *offs, int nseg, unsigned *keys,
+		unsigned *vals, unsigned *lin)
 {
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		const DPhotonMap &M = grids[seg_of(offs, nseg, (unsigned)i)];
-		int c[3];
-		for(int a = 0; a < 3; a++) {
-			double v = floor(((double)ph[i].p[a] - (double)M.org[a]) / (double)M.cell);
-			c[a] = v < 0.0 ? 0 : (v > (double)(M.dims[a] - 1) ? M.dims[a] - 1 : (int)v);
-		}
-		unsigned l = (unsigned)(((size_t)c[2] * M.dims[1] + c[1]) * M.dims[0] + c[0]);
-		keys[i] = morton[seg_of(offs, nseg, (unsigned)i)] ? (spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2)) : l;
+		unsigned l = cell_key(ph[i], grids[seg_of(offs, nseg, (unsigned)i)], 0);
+		keys[i] = l;
 		vals[i] = (unsigned)i;
 		lin[i] = l;
+	}
+}
+
+/* the photons and their cells in sorted order */
+__global__ void k_permute_seg(const DevPhoton *in, const unsigned *vals, const unsigned *lin_in, int n, DevPhoton *out, unsigned *lin_out)
+{
+	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+		unsigned v = vals[i];
+		out[i] = in[v];
+		lin_out[i] = lin_in[v];
 	}
 }
 
@@ -1018,18 +1125,14 @@ __global__ void k_seg_keys(const unsigned *vals, int n, const unsigned *offs, in
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) keys[i] = (unsigned)seg_of(offs, nseg, vals[i]);
 }
 
-/* (first, end) of every occupied cell of every segment, relative to the
- * segment's first photon, in the segment's own cell table */
-__global__ void k_cells_seg(const unsigned *lin, int n, const unsigned *offs, int nseg, const unsigned long long *cell_base, uint2 *cells)
+/* every segment's cell table (block row y: segment y) */
+__global__ void __launch_bounds__(256) k_starts_seg(const unsigned *lin, const unsigned *offs, const unsigned long long *cell_base,
+		unsigned *starts)
 {
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		int sg = seg_of(offs, nseg, (unsigned)i);
-		unsigned i0 = offs[sg], i1 = offs[sg + 1];
-		unsigned l = lin[i];
-		uint2 *c = cells + cell_base[sg];
-		if((unsigned)i == i0 || lin[i - 1] != l) c[l].x = (unsigned)i - i0;
-		if((unsigned)i + 1 == i1 || lin[i + 1] != l) c[l].y = (unsigned)i + 1 - i0;
-	}
+	const int sg = blockIdx.y;
+	const size_t ncells = (size_t)(cell_base[sg + 1] - cell_base[sg]) - 1;
+	if((size_t)blockIdx.x * START_CELLS > ncells) return;
+	cell_starts(lin, offs[sg], offs[sg + 1], ncells, starts + cell_base[sg]);
 }
 
 /* exclusive scan of m entries (scratch `part` for the parts' totals); the
@@ -1050,10 +1153,10 @@ static int scan_long(Renderer &R, unsigned *data, int m, unsigned *total, DevBuf
 }
 
 /* stable LSD radix sort of n (key, value) pairs over the low `bits` bits of
- * the keys, ping-ponging with keys2 / vals2; *vals_out is the buffer that
- * holds the sorted values (scratch: hist, part) */
+ * the keys, ping-ponging with keys2 / vals2; *keys_out and *vals_out are the
+ * buffers that hold the sorted pairs (scratch: hist, part) */
 int sort_pairs(Renderer &R, unsigned *keys, unsigned *vals, unsigned *keys2, unsigned *vals2, int n, int bits, DevBuf &hist,
-		DevBuf &part, const char *name, cudaStream_t s, unsigned **vals_out)
+		DevBuf &part, const char *name, cudaStream_t s, unsigned **keys_out, unsigned **vals_out)
 {
 	int nbr = (n + TILE - 1) / TILE;
 	PCK(hist.ensure((size_t)256 * nbr * sizeof(unsigned) + 16), "radix histogram");
@@ -1065,13 +1168,14 @@ int sort_pairs(Renderer &R, unsigned *keys, unsigned *vals, unsigned *keys2, uns
 		std::swap(keys, keys2);
 		std::swap(vals, vals2);
 	}
+	*keys_out = keys;
 	*vals_out = vals;
 	return 0;
 }
 
 /* every job's two maps from the wavefront's output: maps[2j] caustic,
  * maps[2j + 1] global, over the boxes and range radii of the jobs' own
- * frames.  Returns 1 (nothing done) when the maps' cell tables together
+ * frames.  Returns 1 (no map built) when the maps' cell tables together
  * would pass 2^28 cells, for the map-by-map build to take over. */
 int photon_finalize_jobs(Renderer &R, const std::vector<PJobOut> &jobs, const std::vector<Box> &boxes,
 		const std::vector<double> &gather_dist, std::vector<DPhotonMap> &maps, cudaStream_t s)
@@ -1079,18 +1183,6 @@ int photon_finalize_jobs(Renderer &R, const std::vector<PJobOut> &jobs, const st
 	const sray_opts &opt = R.opt;
 	int nj = (int)jobs.size(), nseg = 2 * nj;
 	maps.assign(nseg, DPhotonMap());
-	std::vector<int> morton(nseg);
-	std::vector<unsigned long long> cell_base(nseg + 1, 0);
-	for(int sg = 0; sg < nseg; sg++) {
-		int k = (sg & 1) ? opt.gi_k : opt.caust_k;
-		double rad = k > 0 ? (double)opt.gather_rcap : gather_dist[sg >> 1];
-		bool mo;
-		size_t nc;
-		map_grid(k, rad, boxes[sg >> 1], maps[sg], &mo, &nc);
-		morton[sg] = mo ? 1 : 0;
-		cell_base[sg + 1] = cell_base[sg] + nc;
-	}
-	if(cell_base[nseg] > (1ull << 28)) return 1;
 	const PJobOut &last = jobs[nj - 1];
 	int total = last.base + last.total[0] + last.total[1];
 	if(total == 0) return 0;
@@ -1117,53 +1209,50 @@ int photon_finalize_jobs(Renderer &R, const std::vector<PJobOut> &jobs, const st
 	R.h2d += (int64_t)bounds.size() * sizeof(int);
 	R.prof_collect();
 	int n = (int)h_offs[nseg];
-	for(int sg = 0; sg < nseg; sg++) maps[sg].n = (int)(h_offs[sg + 1] - h_offs[sg]);
+	/* a table per map: its cells and one entry more */
+	std::vector<unsigned long long> cell_base(nseg + 1, 0);
+	unsigned long long most_cells = 0;
+	for(int sg = 0; sg < nseg; sg++) {
+		int k = (sg & 1) ? opt.gi_k : opt.caust_k;
+		double rad = k > 0 ? (double)opt.gather_rcap : gather_dist[sg >> 1];
+		unsigned long long nc = map_grid(k, rad, boxes[sg >> 1], (int)(h_offs[sg + 1] - h_offs[sg]), maps[sg]);
+		cell_base[sg + 1] = cell_base[sg] + nc + 1;
+		most_cells = std::max(most_cells, nc);
+	}
+	if(cell_base[nseg] > (1ull << 28)) return 1;
 	if(n == 0) return 0;
 	PCK(R.pw_ph.ensure((size_t)n * sizeof(DevPhoton)), "photon maps");
 	PCK(R.pw_sorted.ensure((size_t)n * sizeof(DevPhoton)), "photon maps");
 	LAUNCH(R, "photon_compact", s, k_compact<<<nb, 256, 0, s>>>(valid, R.pw_out.as<DevPhoton>(), total, bc, R.pw_ph.as<DevPhoton>()));
 	PCK(R.pw_grids.upload(maps, s), "map grids");
-	PCK(R.pw_morton.upload(morton, s), "map keys");
 	PCK(R.pw_cellbase.upload(cell_base, s), "cell tables");
-	R.h2d += (int64_t)(maps.size() * sizeof(DPhotonMap) + morton.size() * 4 + cell_base.size() * 8);
+	R.h2d += (int64_t)(maps.size() * sizeof(DPhotonMap) + cell_base.size() * 8);
 	PCK(R.pw_keys.ensure((size_t)n * 16), "keys");
 	PCK(R.pw_lin.ensure((size_t)n * 8), "cell ids");
-	PCK(R.pw_cells.ensure((size_t)cell_base[nseg] * sizeof(uint2) + 16), "cell tables");
+	PCK(R.pw_starts.ensure((size_t)cell_base[nseg] * sizeof(unsigned)), "cell tables");
 	unsigned *keys = R.pw_keys.as<unsigned>(), *vals = keys + n, *keys2 = keys + 2 * (size_t)n, *vals2 = keys + 3 * (size_t)n;
 	unsigned *lin = R.pw_lin.as<unsigned>(), *lin2 = lin + n;
-	LAUNCH(R, "photon_sort", s, k_keys_seg<<<grid_n(n, 256), 256, 0, s>>>(R.pw_ph.as<DevPhoton>(), n, R.pw_grids.as<DPhotonMap>(),
-			R.pw_morton.as<int>(), offs, nseg, keys, vals, lin));
-	int key_bits = 0;
-	for(int sg = 0; sg < nseg; sg++) {
-		unsigned long long maxkey = morton[sg] ? (1ull << 30) - 1ull : cell_base[sg + 1] - cell_base[sg] - 1ull;
-		int b = 0;
-		while(b < 32 && (maxkey >> b)) b++;
-		key_bits = std::max(key_bits, b);
-	}
-	int seg_bits = 0;
-	while(seg_bits < 32 && ((unsigned)(nseg - 1) >> seg_bits)) seg_bits++;
-	int nbr = (n + TILE - 1) / TILE;
-	PCK(R.pw_hist.ensure((size_t)256 * nbr * sizeof(unsigned) + 16), "radix histogram");
-	unsigned *hist = R.pw_hist.as<unsigned>();
-	int key_passes = (key_bits + 7) / 8, seg_passes = (seg_bits + 7) / 8;
-	for(int ps = 0; ps < key_passes + seg_passes; ps++) {
-		if(ps == key_passes)
-			LAUNCH(R, "photon_sort", s, k_seg_keys<<<grid_n(n, 256), 256, 0, s>>>(vals, n, offs, nseg, keys));
-		int shift = (ps < key_passes ? ps : ps - key_passes) * 8;
-		LAUNCH(R, "photon_sort", s, k_rs_hist<<<nbr, RS_THREADS, 0, s>>>(keys, n, shift, hist, nbr));
-		if(scan_long(R, hist, 256 * nbr, nullptr, R.pw_part, "photon_sort", s)) return SRAY_ECUDA;
-		LAUNCH(R, "photon_sort", s, k_rs_scatter<<<nbr, RS_THREADS, 0, s>>>(keys, vals, n, shift, hist, nbr, keys2, vals2));
+	LAUNCH(R, "photon_sort", s, k_keys_seg<<<grid_n(n, 256), 256, 0, s>>>(R.pw_ph.as<DevPhoton>(), n, R.pw_grids.as<DPhotonMap>(), offs,
+			nseg, keys, vals, lin));
+	/* by cell, then by segment (keys and values back in the first halves or the second) */
+	unsigned *ks = nullptr, *vs = nullptr;
+	if(int r = sort_pairs(R, keys, vals, keys2, vals2, n, key_bits((unsigned)(most_cells - 1)), R.pw_hist, R.pw_part, "photon_sort", s,
+			&ks, &vs))
+		return r;
+	if(ks != keys) {
 		std::swap(keys, keys2);
 		std::swap(vals, vals2);
 	}
-	LAUNCH(R, "photon_sort", s, k_permute<<<grid_n(n, 256), 256, 0, s>>>(R.pw_ph.as<DevPhoton>(), vals, lin, n, R.pw_sorted.as<DevPhoton>(),
-			lin2));
-	PCK(cudaMemsetAsync(R.pw_cells.p, 0, (size_t)cell_base[nseg] * sizeof(uint2), s), "cell tables");
-	LAUNCH(R, "photon_sort", s, k_cells_seg<<<grid_n(n, 256), 256, 0, s>>>(lin2, n, offs, nseg, R.pw_cellbase.as<unsigned long long>(),
-			R.pw_cells.as<uint2>()));
+	LAUNCH(R, "photon_sort", s, k_seg_keys<<<grid_n(n, 256), 256, 0, s>>>(vals, n, offs, nseg, keys));
+	if(int r = sort_pairs(R, keys, vals, keys2, vals2, n, key_bits((unsigned)(nseg - 1)), R.pw_hist, R.pw_part, "photon_sort", s, &ks, &vs))
+		return r;
+	LAUNCH(R, "photon_sort", s, k_permute_seg<<<grid_n(n, 256), 256, 0, s>>>(R.pw_ph.as<DevPhoton>(), vs, lin, n,
+			R.pw_sorted.as<DevPhoton>(), lin2));
+	LAUNCH(R, "photon_sort", s, k_starts_seg<<<dim3((unsigned)((most_cells + START_CELLS) / START_CELLS), nseg), 256, 0, s>>>(lin2, offs,
+			R.pw_cellbase.as<unsigned long long>(), R.pw_starts.as<unsigned>()));
 	for(int sg = 0; sg < nseg; sg++) {
 		maps[sg].ph = R.pw_sorted.as<DevPhoton>() + h_offs[sg];
-		maps[sg].cells = R.pw_cells.as<uint2>() + cell_base[sg];
+		maps[sg].start = R.pw_starts.as<unsigned>() + cell_base[sg];
 	}
 	PCK(cudaStreamSynchronize(s), "photon map build");
 	R.prof_collect();

@@ -1255,29 +1255,61 @@ __global__ void __launch_bounds__(128) k_shadow_warp(DScene S, const ShadowReq *
 #define GATHER_WARPS 8
 #define KEY_CAP 512
 
+/* The rows of cells (along x) that a query must visit: every cell that can
+ * hold a photon within the radius.  Photons were binned with floor((p - org)
+ * / cell) in double; the window is computed in float, in units of cells, and
+ * widened by a slack that covers the float rounding (four operations, each
+ * within 2^-24 of its operands), so it always contains the exact window and
+ * at most grows by one cell where the sphere's edge lies within the slack of
+ * a cell boundary.  A photon outside the grid was binned into its border
+ * cells, which therefore reach out to infinity. */
 struct GatherCells {
-	int lo[3], hi[3];
+	float u[3], slack[3];     /* the query in units of cells */
+	int ylo, zlo, ny, nrow;
 };
 
-/* The grid cells a query must visit: every cell that can hold a photon
- * within the radius.  Photons were binned with floor((p - org) / cell) in
- * double; the window is computed in float and widened by a slack that covers
- * the float rounding (three operations, each within 2^-24 of its operands),
- * so it always contains the exact window and at most grows by one cell where
- * the query's edge lies within the slack of a cell boundary. */
 __device__ __forceinline__ void gather_cells(const DPhotonMap &M, V3 q, GatherCells &gc)
 {
 	float qa[3] = {q.x, q.y, q.z};
+	int lo[3], hi[3];
+	#pragma unroll
 	for(int a = 0; a < 3; a++) {
-		float base = qa[a] - M.org[a];
-		float lo = (base - M.range_f) / M.cell, hi = (base + M.range_f) / M.cell;
-		float slack = 1e-3f + (fabsf(base) + M.range_f) / M.cell * 1e-6f;
-		lo = floorf(lo - slack);
-		hi = floorf(hi + slack);
+		gc.u[a] = (qa[a] - M.org[a]) * M.inv_cell;
+		gc.slack[a] = 1e-3f + (fabsf(gc.u[a]) + M.reach) * 1e-6f;
+		float l = floorf(gc.u[a] - M.reach - gc.slack[a]), h = floorf(gc.u[a] + M.reach + gc.slack[a]);
 		float top = (float)(M.dims[a] - 1);
-		gc.lo[a] = lo >= 0.0f ? (lo > top ? M.dims[a] - 1 : (int)lo) : 0;
-		gc.hi[a] = hi >= 0.0f ? (hi > top ? M.dims[a] - 1 : (int)hi) : 0;
+		lo[a] = l >= 0.0f ? (l > top ? M.dims[a] - 1 : (int)l) : 0;
+		hi[a] = h >= 0.0f ? (h > top ? M.dims[a] - 1 : (int)h) : 0;
 	}
+	gc.ylo = lo[1];
+	gc.zlo = lo[2];
+	gc.ny = hi[1] - lo[1] + 1;
+	gc.nrow = gc.ny * (hi[2] - lo[2] + 1);
+}
+
+/* how far the query is from row c of axis a, in cells and at most (0 inside) */
+__device__ __forceinline__ float gather_off(const DPhotonMap &M, const GatherCells &gc, int a, int c)
+{
+	float below = c > 0 ? (float)c - gc.u[a] : 0.0f;
+	float above = c < M.dims[a] - 1 ? gc.u[a] - (float)(c + 1) : 0.0f;
+	return fmaxf(fmaxf(below, above) - gc.slack[a], 0.0f);
+}
+
+/* the photons [first, end) of row r of the window: its cells within the
+ * sphere's reach along x at the row's distance */
+__device__ __forceinline__ uint2 gather_row(const DPhotonMap &M, const GatherCells &gc, int r)
+{
+	int z = r / gc.ny, y = gc.ylo + r - z * gc.ny;
+	z += gc.zlo;
+	float dy = gather_off(M, gc, 1, y), dz = gather_off(M, gc, 2, z);
+	float h2 = M.reach * M.reach * (1.0f + 1e-6f) - dy * dy - dz * dz;
+	if(!(h2 >= 0.0f)) return make_uint2(0u, 0u);
+	float half = sqrtf(h2) + gc.slack[0];
+	float l = floorf(gc.u[0] - half), h = floorf(gc.u[0] + half);
+	float top = (float)(M.dims[0] - 1);
+	int x0 = l >= 0.0f ? (l > top ? M.dims[0] - 1 : (int)l) : 0, x1 = h >= 0.0f ? (h > top ? M.dims[0] - 1 : (int)h) : 0;
+	const unsigned *row = M.start + ((size_t)z * M.dims[1] + y) * M.dims[0];
+	return make_uint2(__ldg(row + x0), __ldg(row + x1 + 1));
 }
 
 /* squared distance in double between a float photon position and the
@@ -1334,8 +1366,8 @@ __device__ __forceinline__ bool gather_exact(const DPhotonMap &M, const float4 &
 	return in;
 }
 
-/* The cells overlapping the query cube (at most 2x2x2: cells are twice the
- * gather radius) are looked up by the first lanes, their non-empty runs of
+/* The rows of cells that the query's sphere reaches (25 where the cells are
+ * half the radius wide) are looked up a lane each, their non-empty runs of
  * photons listed in shared memory, and the warp strides over the
  * concatenation of the runs, two photons per lane and step (both loads in
  * flight together), whatever the cell occupancy; a lane's run only moves
@@ -1347,20 +1379,11 @@ template <class F>
 __device__ __forceinline__ void for_range(const DPhotonMap &M, const GatherCells &gc, V3 q, int lane, GatherMem &gm, F f)
 {
 	const unsigned FULL = 0xffffffffu;
-	int nx = gc.hi[0] - gc.lo[0] + 1, ny = gc.hi[1] - gc.lo[1] + 1, nz = gc.hi[2] - gc.lo[2] + 1;
-	int ncell = nx * ny * nz;
 	const float thr = M.screen, sure = gather_below(M.r2_hi);
-	for(int c0 = 0; c0 < ncell; c0 += 32) {
-		int c = c0 + lane;
-		unsigned first = 0, cnt = 0;
-		if(c < ncell) {
-			int cx = c % nx, t = c / nx;
-			int cy = t % ny, cz = t / ny;
-			uint2 cr = __ldg(reinterpret_cast<const uint2 *>(M.cells) +
-					((size_t)(gc.lo[2] + cz) * M.dims[1] + (gc.lo[1] + cy)) * M.dims[0] + (gc.lo[0] + cx));
-			first = cr.x;
-			cnt = cr.y - cr.x;
-		}
+	for(int r0 = 0; r0 < gc.nrow; r0 += 32) {
+		uint2 run_ = make_uint2(0u, 0u);
+		if(r0 + lane < gc.nrow) run_ = gather_row(M, gc, r0 + lane);
+		const unsigned first = run_.x, cnt = run_.y - run_.x;
 		unsigned nonempty = __ballot_sync(FULL, cnt > 0);
 		if(!nonempty) continue;
 		/* inclusive prefix of the run lengths over the lanes */
@@ -1595,9 +1618,10 @@ __device__ __noinline__ unsigned gather_unlisted(const DPhotonMap &M, const Gath
  * within its bin) splits the list into photons that are surely among the k
  * nearest, photons that surely are not, and the few within the margin, for
  * which the exact keys decide.  The kernel is bound by instruction issue:
- * 1.51 ms for 500,009 points of a map of 500k emitted photons (k = 100)
- * against 2.33 ms with the exact key of every photon and a 32-step search
- * over all of them. */
+ * 1.15 ms for 500,009 points of a map of 500k emitted photons (k = 100)
+ * against 2.33 ms with the exact key of every photon, a 32-step search over
+ * all of them and cells of twice the radius (1.51 ms with those cells
+ * alone). */
 __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V3 n, GatherMem &gm, GatherWork &gw)
 {
 	const unsigned FULL = 0xffffffffu;
@@ -2654,13 +2678,13 @@ int Renderer::photon_job(DScene base)
 				if(copy_out && M.n > 0) {
 					/* out of the wavefront's buffers into the job's own */
 					PhotonBufs &P = (k & 1) ? job_maps[a + k / 2].gi : job_maps[a + k / 2].caust;
-					size_t ncells = (size_t)M.dims[0] * M.dims[1] * M.dims[2];
+					size_t entries = (size_t)M.dims[0] * M.dims[1] * M.dims[2] + 1;
 					CK(P.ph.ensure((size_t)M.n * sizeof(DevPhoton)), "job photon map");
-					CK(P.cells.ensure(ncells * sizeof(uint2)), "job cell table");
+					CK(P.starts.ensure(entries * sizeof(unsigned)), "job cell table");
 					CK(cudaMemcpyAsync(P.ph.p, M.ph, (size_t)M.n * sizeof(DevPhoton), cudaMemcpyDeviceToDevice, ps), "job photon map");
-					CK(cudaMemcpyAsync(P.cells.p, M.cells, ncells * sizeof(uint2), cudaMemcpyDeviceToDevice, ps), "job cell table");
+					CK(cudaMemcpyAsync(P.starts.p, M.start, entries * sizeof(unsigned), cudaMemcpyDeviceToDevice, ps), "job cell table");
 					M.ph = P.ph.as<DevPhoton>();
-					M.cells = P.cells.as<uint2>();
+					M.start = P.starts.as<unsigned>();
 				}
 				hm[2 * a + k] = M;
 			}
@@ -2796,7 +2820,7 @@ int Renderer::sort_queue(RayQueue &Q, DevBuf &Qbuf, int &Qcap, RayQueue &T, DevB
 	LAUNCH(*this, name, s, k_ray_keys<<<grid_for(n, 256), 256, 0, s>>>(Q, n, lo[0], lo[1], lo[2], ext[0], ext[1], ext[2],
 			24 - bits, keys, vals));
 	unsigned *sorted = nullptr;
-	if(int r = sort_pairs(*this, keys, vals, keys2, vals2, n, bits, hist, part, name, s, &sorted)) return r;
+	if(int r = sort_pairs(*this, keys, vals, keys2, vals2, n, bits, hist, part, name, s, &keys, &sorted)) return r;
 	LAUNCH(*this, name, s, k_ray_permute<<<grid_for(n, 256), 256, 0, s>>>(Q, sorted, n, T));
 	int *count = Q.count;
 	std::swap(Q, T);
@@ -4392,9 +4416,8 @@ int sray_gpu_get_photons(int which, float *out, int cap, int *n_out)
 	if(n_out) *n_out = n;
 	if(!out || cap <= 0 || n == 0) return 0;
 	int m = n < cap ? n : cap;
-	std::vector<DevPhoton> h(m);
-	cudaError_t e = cudaMemcpy(h.data(), P.ph.p, (size_t)m * sizeof(DevPhoton), cudaMemcpyDeviceToHost);
-	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
+	std::vector<DevPhoton> h;
+	if(int r = photon_map_read(R, which ? 1 : 0, h, 0)) { g_err = R.err; return r; }
 	for(int i = 0; i < m; i++) {
 		float *f = out + (size_t)i * 16;
 		f[0] = h[i].p[0]; f[1] = h[i].p[1]; f[2] = h[i].p[2];
@@ -4413,13 +4436,8 @@ int sray_gpu_dump_photons(int which, const char *path)
 	NEED_CTX();
 	Renderer &R = *g_R;
 	if(!path || (which != 0 && which != 1)) { g_err = "bad arguments"; return SRAY_EINVAL; }
-	const PhotonBufs &P = which ? R.gi : R.caust;
-	int n = P.map.n;
-	std::vector<DevPhoton> h(n > 0 ? n : 0);
-	if(n > 0) {
-		cudaError_t e = cudaMemcpy(h.data(), P.ph.p, (size_t)n * sizeof(DevPhoton), cudaMemcpyDeviceToHost);
-		if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
-	}
+	std::vector<DevPhoton> h;
+	if(int r = photon_map_read(R, which, h, 0)) { g_err = R.err; return r; }
 	FILE *fp = fopen(path, "w");
 	if(!fp) { g_err = std::string("failed to dump photon map: ") + path; return SRAY_EIO; }
 	fprintf(fp, "energy %f\n", R.opt.photon_energy);
@@ -4594,7 +4612,7 @@ void sray_gpu_shutdown(void)
 	for(Renderer::JobMaps &jm : R.job_maps) {
 		PhotonBufs *jp[] = {&jm.caust, &jm.gi};
 		for(PhotonBufs *p : jp) {
-			DevBuf *pbufs[] = {&p->ph, &p->cells, &p->tmp_ph, &p->keys, &p->keys2, &p->vals, &p->vals2, &p->lin, &p->hist, &p->scan};
+			DevBuf *pbufs[] = {&p->ph, &p->starts, &p->tmp_ph, &p->keys, &p->keys2, &p->vals, &p->vals2, &p->hist, &p->scan};
 			for(DevBuf *b : pbufs) b->release();
 		}
 	}
@@ -4607,8 +4625,8 @@ void sray_gpu_shutdown(void)
 		&R.active[0], &R.active[1], &R.spp, &R.fbdev, &R.ctr, &R.counts, &R.bnodes, &R.btris, &R.bprim, &R.bhome,
 		&R.fbl, &R.tnodes, &R.ohome, &R.pool_ready, &R.pqbuf[0], &R.pqbuf[1], &R.phits, &R.pfbl, &R.pcounts, &R.pctr,
 		&R.pw_jobs, &R.pw_prefix, &R.pw_scale, &R.pw_bits, &R.pw_cov, &R.pw_pix, &R.pw_out, &R.pw_valid,
-		&R.pw_part, &R.pw_tiles, &R.pw_bounds, &R.pw_offs, &R.pw_ph, &R.pw_sorted, &R.pw_grids, &R.pw_morton, &R.pw_cellbase,
-		&R.pw_keys, &R.pw_lin, &R.pw_cells, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1],
+		&R.pw_part, &R.pw_tiles, &R.pw_bounds, &R.pw_offs, &R.pw_ph, &R.pw_sorted, &R.pw_grids, &R.pw_cellbase,
+		&R.pw_keys, &R.pw_lin, &R.pw_starts, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1],
 		&R.pqsbuf, &R.ps_keys, &R.ps_hist, &R.ps_part,
 		&R.nrc_qx, &R.nrc_qw, &R.nrc_rx, &R.nrc_rt, &R.nrc_ry, &R.nrc_regions};
 	if(R.ps) cudaStreamSynchronize(R.ps);
@@ -4616,7 +4634,7 @@ void sray_gpu_shutdown(void)
 	for(DevBuf *b : bufs) b->release();
 	PhotonBufs *pb[] = {&R.caust, &R.gi};
 	for(PhotonBufs *p : pb) {
-		DevBuf *pbufs[] = {&p->ph, &p->cells, &p->tmp_ph, &p->keys, &p->keys2, &p->vals, &p->vals2, &p->lin, &p->hist, &p->scan};
+		DevBuf *pbufs[] = {&p->ph, &p->starts, &p->tmp_ph, &p->keys, &p->keys2, &p->vals, &p->vals2, &p->hist, &p->scan};
 		for(DevBuf *b : pbufs) b->release();
 	}
 	if(R.pin) cudaFreeHost(R.pin);

@@ -117,8 +117,9 @@ struct NrcRegionStats {
 };
 
 struct PhotonBufs {
-	DevBuf ph, cells, tmp_ph, keys, keys2, vals, vals2, lin, hist, scan;
-	DPhotonMap map;
+	DevBuf ph, starts, tmp_ph, keys, keys2, vals, vals2, hist, scan;
+	DPhotonMap map = DPhotonMap();
+	DPhotonMap order = DPhotonMap();   /* the grid of the order programs see the photons in */
 	int n = 0;
 };
 
@@ -239,7 +240,7 @@ struct Renderer {
 	/* a batch's maps built together (photon_finalize_jobs): scan scratch,
 	 * segment bounds and offsets, compacted and sorted photons, grids, keys,
 	 * cell tables */
-	DevBuf pw_part, pw_tiles, pw_bounds, pw_offs, pw_ph, pw_sorted, pw_grids, pw_morton, pw_cellbase, pw_keys, pw_lin, pw_cells, pw_hist;
+	DevBuf pw_part, pw_tiles, pw_bounds, pw_offs, pw_ph, pw_sorted, pw_grids, pw_cellbase, pw_keys, pw_lin, pw_starts, pw_hist;
 	std::vector<int> batch_scene, batch_caust, batch_gi;   /* jobs' scenes and photon counts (0: the options') */
 	/* a scene set: its scene descriptors on the device */
 	DevBuf dscenes;
@@ -340,13 +341,14 @@ int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJ
 		cudaStream_t s);
 int photon_finalize(Renderer &R, int global, const int *valid, const DevPhoton *in, int total, cudaStream_t s, int *stored);
 int sort_pairs(Renderer &R, unsigned *keys, unsigned *vals, unsigned *keys2, unsigned *vals2, int n, int bits, DevBuf &hist,
-		DevBuf &part, const char *name, cudaStream_t s, unsigned **vals_out);
+		DevBuf &part, const char *name, cudaStream_t s, unsigned **keys_out, unsigned **vals_out);
 int photon_finalize_jobs(Renderer &R, const std::vector<PJobOut> &jobs, const std::vector<Box> &boxes,
 		const std::vector<double> &gather_dist, std::vector<DPhotonMap> &maps, cudaStream_t s);
 int photon_shoot_maps(Renderer &R, const DScene &base, const std::vector<uint32_t> &bits, const std::vector<float> &cov,
 		cudaStream_t s, int *caust_stored, int *gi_stored);
 /* photon.cu: map `global` (0 caustic, 1 global) over the n photons in its buffer / from host photons */
 int photon_map_build(Renderer &R, int global, int n, cudaStream_t s);
+int photon_map_read(Renderer &R, int global, std::vector<DevPhoton> &h, cudaStream_t s);
 int photon_map_restore(Renderer &R, int global, const std::vector<DevPhoton> &h, cudaStream_t s);
 
 }  // namespace sray

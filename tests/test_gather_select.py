@@ -126,3 +126,56 @@ def test_gather_selects_the_k_nearest(gpu_lib, dump, which, k):
             continue
         err = np.abs(got[i] - want) / np.maximum(np.abs(want), 1e-9)
         assert (err <= BOUND).all(), (name, got[i], want)
+
+
+def _spread3(v):
+    r = np.zeros_like(v)
+    for b in range(10):
+        r |= ((v >> b) & 1) << (3 * b)
+    return r
+
+
+@pytest.mark.parametrize("n", [40, 3000, 60000])
+@pytest.mark.parametrize("k", [0, 20])
+def test_gather_grid(gpu_lib, tmp_path, n, k):
+    """Random maps of sizes that take each cell width, photons and queries
+    inside, on the border of and outside the scene's box, every query against
+    all photons in double; and the order programs read the photons in: Morton
+    order of cells twice the radius, ties as given."""
+    rng = np.random.default_rng(n + k)
+    frac = np.float32(0.5 / np.sqrt(40.0 ** 2 + 4.0 ** 2 + 40.0 ** 2))
+    rad = np.sqrt(40.0 ** 2 + 4.0 ** 2 + 40.0 ** 2) * float(frac) if k == 0 else 0.5
+    pos = rng.uniform((-20.5, -0.4, -20.5), (20.5, 4.4, 20.5), (n, 3))
+    pos[: n // 4] = rng.uniform((-1, 1, -1), (1, 1.2, 1), (n // 4, 3))
+    pos[n // 4: n // 3, 0] = rng.choice([-20.0, 20.0], n // 3 - n // 4)
+    power = rng.uniform(0.5, 2.0, (n, 3))
+    path = str(tmp_path / "photons")
+    with open(path, "w") as f:
+        f.write("energy 300.0\n")
+        for p, c in zip(pos, power):
+            f.write("<%.6f %.6f %.6f> <0.0 -1.0 0.0> <0.0 1.0 0.0> <%.6f %.6f %.6f>\n" % (*p, *c))
+    pos, power = [np.array([[float("%.6f" % v) for v in row] for row in a]).astype(np.float32) for a in (pos, power)]
+    g = gpu_lib.GpuRenderer(width=64, height=64, caust_k=k, gi_k=k, gather_rcap=0.5, gather_dist=float(frac), caust_photons=1000,
+                            gi_photons=1000)
+    g.load_xml(SCENE)
+    g.build(0, 0)
+    assert g.restore_photons(1, path) == n
+    near = pos[rng.integers(0, n, 300)] + rng.uniform(-0.3, 0.3, (300, 3))
+    far = rng.uniform((-21, -1, -21), (21, 5, 21), (100, 3))
+    q = np.concatenate([near, far, [[-20, 0, -20], [20, 4, 20], [1000, 0, 0], [0, -1000, 0]]]).astype(np.float32)
+    out = torch.empty((len(q), 3), device="cuda")
+    g.photon_gather(1, torch.tensor(q, device="cuda"), torch.tensor([[0.0, 1.0, 0.0]] * len(q), device="cuda"), out)
+    got = out.cpu().numpy().astype(np.float64)
+    want = np.stack([_expected(pos, power, p, k, 1, rad) for p in q])
+    assert (want > 0).any()
+    assert (np.abs(got - want) <= BOUND * np.maximum(np.abs(want), 1e-9)).all()
+    ph = g.photons(1)
+    g.close()
+    lo = np.float64([-20, 0, -20])
+    cell = float(np.float32(2.0 * rad))
+    while cell < 2.0 * rad:
+        cell = float(np.nextafter(np.float32(cell), np.float32(np.inf)))
+    dims = np.floor(np.float64([40, 4, 40]) / (2.0 * rad)).astype(np.int64) + 1
+    c = np.clip(np.floor((pos.astype(np.float64) - lo) / cell).astype(np.int64), 0, dims - 1)
+    order = np.argsort(_spread3(c[:, 0]) | _spread3(c[:, 1]) << 1 | _spread3(c[:, 2]) << 2, kind="stable")
+    assert np.array_equal(ph[:, 0:3], pos[order]) and np.array_equal(ph[:, 9:12], power[order])
