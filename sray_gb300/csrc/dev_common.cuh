@@ -860,137 +860,143 @@ __device__ __forceinline__ RayT object_ray(const DScene &S, int o, int ti, V3 wo
 	return make_ray(mul_pt(inv, wo), mul_dir(inv, wd));
 }
 
-/* ANY = false: closest hit into h, returns false when the octrees must
- * decide.  ANY = true: returns 1 when a hit the octrees reach exists, 0 when
- * no hit exists, 2 when the octrees must decide.  SORT: a node's hit
- * children are visited nearest first (always for closest hits); an any-hit
- * query may visit them in the node's order instead. */
+/* One ray's walk through the two hierarchies, a step at a time.  ANY =
+ * false: the closest hit; ANY = true: some hit on the segment [eps, 1].
+ * SORT: a node's hit children are visited nearest first (always for closest
+ * hits); an any-hit query may visit them in the node's order instead.
+ *
+ * cur is the next entry to visit: a node (of the object hierarchy, or of the
+ * mesh inside an instance), ~leaf inside an instance, ~object outside one,
+ * or BVH_NONE when the walk has ended.  Each step ends by taking the next
+ * entry from the stack. */
+enum { WALK_GOES = 0, WALK_HIT = 1, WALK_UNDECIDED = 2, WALK_OVERFLOW = 3 };
+enum { WALK_NODE = 0, WALK_LEAF = 1, WALK_OBJECT = 2, WALK_END = 3 };
+
 template <bool COUNT, bool ANY, bool SORT = true>
-__device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, int time, Hit &h, TraceCounters *tc, int *overflow,
-		int scene = -1)
-{
-	h.t = FLT_MAX;
-	h.obj = -1;
-	h.prim = -1;
-	h.tie = 0;
-	const int2 roots = scene_roots(S, scene);
-	if(roots.x < 0) return ANY ? 0 : 1;
-	if(roots.y < 0) return ANY ? 2 : 0;
-	int ti = time_index(S, time);
-	RayT wr = make_ray(wo, wd);
-	const DevNode &sroot = S.snodes[roots.x];
-	RayC wc = make_rayc(wr, box_bound(sroot.mn, sroot.mx));
-	RayT r = wr;
-	RayC rc = wc;
-	TStack st;
-	float best = ANY ? 1.0f : FLT_MAX;
-	int bobj = -1, bprim = -1, bslot = -1;
-	bool eq = false;
-	int sp = 0, inst_base = 0, iobj = -1;
-	bool inst = false;
-	int cur = roots.y;   /* the object hierarchy's root */
-	for(;;) {
-		if(cur == BVH_NONE) {
-			bool found = false;
-			while(sp > 0) {
-				int k = sp - 1;
-				if(inst && k < inst_base) {   /* the instance's entries are done */
-					inst = false;
-					iobj = -1;
-					r = wr;
-					rc = wc;
-				}
-				sp = k;
-				if(ANY || st.te[k] <= best) {
-					cur = st.node[k];
-					found = true;
-					break;
-				}
+struct Walk {
+	V3 wo, wd;            /* the ray */
+	RayT r, wr;           /* in the current space, in world space */
+	RayC rc, wc;
+	float best;
+	int ti;
+	int bobj, bprim, bslot;
+	int sp, inst_base, iobj, cur;
+	bool eq, inst;
+
+	__device__ __forceinline__ void start(const DScene &S, V3 o, V3 d, int time, int2 roots)
+	{
+		wo = o;
+		wd = d;
+		ti = time_index(S, time);
+		wr = make_ray(wo, wd);
+		const DevNode &sroot = S.snodes[roots.x];
+		wc = make_rayc(wr, box_bound(sroot.mn, sroot.mx));
+		r = wr;
+		rc = wc;
+		best = ANY ? 1.0f : FLT_MAX;
+		bobj = bprim = bslot = -1;
+		eq = false;
+		sp = 0;
+		inst_base = 0;
+		iobj = -1;
+		inst = false;
+		cur = roots.y;   /* the object hierarchy's root */
+	}
+
+	__device__ __forceinline__ int kind() const { return cur == BVH_NONE ? WALK_END : (cur >= 0 ? WALK_NODE : (inst ? WALK_LEAF : WALK_OBJECT)); }
+
+	/* the next entry that can hold a closer hit */
+	__device__ __forceinline__ void pop(const TStack &st)
+	{
+		cur = BVH_NONE;
+		while(sp > 0) {
+			int k = sp - 1;
+			if(inst && k < inst_base) {   /* the instance's entries are done */
+				inst = false;
+				iobj = -1;
+				r = wr;
+				rc = wc;
 			}
-			if(!found) break;
+			sp = k;
+			if(ANY || st.te[k] <= best) {
+				cur = st.node[k];
+				break;
+			}
 		}
-		if(!inst && cur < 0) {
-			/* enter object ~cur */
-			int o = ~cur;
-			cur = BVH_NONE;
-			const DevObj ob = S.objs[o];
-			RayT orr = object_ray(S, o, ti, wo, wd);
-			if(ob.type != 2) {
-				if(COUNT) tc->prims++;
-				float t;
-				bool hit = ob.type == 0 ? sphere_hit(orr, ob.rad, S.eps, t) : cylinder_hit(orr, ob.rad, ob.start, ob.end, S.eps, t);
-				if(hit && t <= best) {
-					if(ANY) {
-						bobj = o;
-						bprim = 0;
-						best = t;
-						break;
-					}
-					if(t < best) {
-						best = t;
-						bobj = o;
-						bprim = 0;
-						bslot = -1;
-						eq = false;
-					} else if(o != bobj || bprim != 0) {
-						eq = true;
-					}
-				}
-				continue;
+	}
+
+	/* a candidate at t <= best */
+	__device__ __forceinline__ void candidate(float t, int obj, int prim, int slot)
+	{
+		if(ANY || t < best) {
+			best = t;
+			bobj = obj;
+			bprim = prim;
+			bslot = slot;
+			eq = false;
+		} else if(obj != bobj || prim != bprim) {
+			eq = true;
+		}
+	}
+
+	/* enter object ~cur, or test it where it is a quadric */
+	__device__ __forceinline__ int step_object(const DScene &S, const TStack &st, TraceCounters *tc)
+	{
+		int o = ~cur;
+		const DevObj ob = S.objs[o];
+		RayT orr = object_ray(S, o, ti, wo, wd);
+		if(ob.type != 2) {
+			if(COUNT) tc->prims++;
+			float t;
+			bool hit = ob.type == 0 ? sphere_hit(orr, ob.rad, S.eps, t) : cylinder_hit(orr, ob.rad, ob.start, ob.end, S.eps, t);
+			if(hit && t <= best) {
+				candidate(t, o, 0, -1);
+				if(ANY) return WALK_HIT;
 			}
-			if(ob.mesh_root < 0) continue;
-			if(ob.bvh_root < 0) return ANY ? 2 : 0;
+		} else if(ob.mesh_root >= 0) {
+			if(ob.bvh_root < 0) return WALK_UNDECIDED;
 			/* the mesh octree's entry test: a mesh it would not enter gives
 			 * no candidates (nor one beating the best, when pruned) */
 			float te;
 			const DevNode &rn = S.mnodes[ob.mesh_root];
-			if(!box_hit(rn.mn, rn.mx, orr, te) || (!ANY && SRAY_PRUNE(te, best))) continue;
-			r = orr;
-			rc = make_rayc(orr, box_bound(rn.mn, rn.mx));
-			inst = true;
-			inst_base = sp;
-			iobj = o;
-			cur = ob.bvh_root;
-			continue;
-		}
-		if(inst && cur < 0) {
-			/* a leaf of the mesh hierarchy: its faces */
-			unsigned v = ~(unsigned)cur;
-			cur = BVH_NONE;
-			int start = (int)(v >> 4), cnt = (int)(v & 15u);
-			const float4 *tp = reinterpret_cast<const float4 *>(S.btris + start);
-			bool done = false;
-			for(int k = 0; k < cnt; k++) {
-				float4 a = __ldg(tp + 3 * k), b = __ldg(tp + 3 * k + 1), c = __ldg(tp + 3 * k + 2);
-				if(COUNT) tc->prims++;
-				float t;
-				if(!tri_hit(a, b, c, r, S.eps, best, t)) continue;
-				int prim = __ldg(S.bprim + start + k);
-				if(ANY) {
-					bobj = iobj;
-					bprim = prim;
-					bslot = start + k;
-					best = t;
-					done = true;
-					break;
-				}
-				if(t < best) {
-					best = t;
-					bobj = iobj;
-					bprim = prim;
-					bslot = start + k;
-					eq = false;
-				} else if(iobj != bobj || prim != bprim) {
-					eq = true;
-				}
+			if(box_hit(rn.mn, rn.mx, orr, te) && (ANY || !SRAY_PRUNE(te, best))) {
+				r = orr;
+				rc = make_rayc(orr, box_bound(rn.mn, rn.mx));
+				inst = true;
+				inst_base = sp;
+				iobj = o;
+				cur = ob.bvh_root;
+				return WALK_GOES;
 			}
-			if(ANY && done) break;
-			continue;
 		}
-		/* a node of the object hierarchy (world space) or of a mesh's: up to
-		 * four children in one 128-byte line; the hit ones (nodes, leaves, or
-		 * objects) are visited nearest first, each leaf and object in an
-		 * iteration of its own so that the lanes of a warp stay together */
+		pop(st);
+		return WALK_GOES;
+	}
+
+	/* a leaf of the mesh hierarchy: its faces */
+	__device__ __forceinline__ int step_leaf(const DScene &S, const TStack &st, TraceCounters *tc)
+	{
+		unsigned v = ~(unsigned)cur;
+		int start = (int)(v >> 4), cnt = (int)(v & 15u);
+		const float4 *tp = reinterpret_cast<const float4 *>(S.btris + start);
+		for(int k = 0; k < cnt; k++) {
+			float4 a = __ldg(tp + 3 * k), b = __ldg(tp + 3 * k + 1), c = __ldg(tp + 3 * k + 2);
+			if(COUNT) tc->prims++;
+			float t;
+			if(!tri_hit(a, b, c, r, S.eps, best, t)) continue;
+			candidate(t, iobj, __ldg(S.bprim + start + k), start + k);
+			if(ANY) return WALK_HIT;
+		}
+		pop(st);
+		return WALK_GOES;
+	}
+
+	/* a node of the object hierarchy (world space) or of a mesh's: up to
+	 * four children in one 128-byte line; the hit ones (nodes, leaves, or
+	 * objects) are visited nearest first, each leaf and object in a step of
+	 * its own so that the lanes of a warp stay together */
+	__device__ __forceinline__ int step_node(const DScene &S, TStack &st, TraceCounters *tc)
+	{
 		const float4 *np = reinterpret_cast<const float4 *>((inst ? S.bnodes : S.tnodes) + cur);
 		const NodePlanes pl = node_planes(np, rc);
 		const float4 &nx = pl.nx, &ny = pl.ny, &nz = pl.nz, &fx = pl.fx, &fy = pl.fy, &fz = pl.fz;
@@ -1012,13 +1018,14 @@ __device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, in
 			for(int k = 3; k >= 0; k--) {
 				if(key[k] == INFINITY) continue;
 				if(nxt != BVH_NONE) {
-					if(sp >= SRAY_STACK) { *overflow = 1; return 0; }
+					if(sp >= SRAY_STACK) return WALK_OVERFLOW;
 					st.node[sp++] = nxt;
 				}
 				nxt = ref[k];
 			}
 			cur = nxt;
-			continue;
+			if(nxt == BVH_NONE) pop(st);
+			return WALK_GOES;
 		}
 #define SRAY_CSWAP(i, j) do { if(key[j] < key[i]) { float tk = key[i]; key[i] = key[j]; key[j] = tk; int tr_ = ref[i]; ref[i] = ref[j]; ref[j] = tr_; } } while(0)
 		SRAY_CSWAP(0, 1);
@@ -1028,31 +1035,145 @@ __device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, in
 		SRAY_CSWAP(1, 2);
 #undef SRAY_CSWAP
 		if(key[0] == INFINITY) {
-			cur = BVH_NONE;
-			continue;
+			pop(st);
+			return WALK_GOES;
 		}
 		#pragma unroll
 		for(int k = 3; k >= 1; k--) {
 			if(key[k] == INFINITY) continue;
-			if(sp >= SRAY_STACK) { *overflow = 1; return ANY ? 0 : 1; }
+			if(sp >= SRAY_STACK) return WALK_OVERFLOW;
 			st.node[sp] = ref[k];
 			if(!ANY) st.te[sp] = key[k];   /* any hit visits every entry */
 			sp++;
 		}
 		cur = ref[0];
+		return WALK_GOES;
 	}
-	if(bobj < 0) return ANY ? 0 : 1;
-	if(!ANY && eq) return 0;
-	/* confirm against the octrees */
-	if(bslot >= 0 && !octree_reaches(S.mnodes, S.mprim, __ldg(S.bhome + bslot), object_ray(S, bobj, ti, wo, wd), bprim, best, !ANY))
-		return ANY ? 2 : 0;
-	if(!octree_reaches(S.snodes, S.sslots, __ldg(S.ohome + bobj), wr, bobj, best, !ANY)) return ANY ? 2 : 0;
-	if(ANY) return 1;
-	h.t = best;
-	h.obj = bobj;
-	h.prim = bprim;
+
+	/* after the walk: whether the octrees confirm what it found (no hit
+	 * needs no confirmation; a tie never has it) */
+	__device__ __forceinline__ bool confirmed(const DScene &S) const
+	{
+		if(bobj < 0) return true;
+		if(!ANY && eq) return false;
+		if(bslot >= 0 && !octree_reaches(S.mnodes, S.mprim, __ldg(S.bhome + bslot), object_ray(S, bobj, ti, wo, wd), bprim, best, !ANY))
+			return false;
+		return octree_reaches(S.snodes, S.sslots, __ldg(S.ohome + bobj), make_ray(wo, wd), bobj, best, !ANY);
+	}
+};
+
+/* ANY = false: closest hit into h, returns false when the octrees must
+ * decide.  ANY = true: returns 1 when a hit the octrees reach exists, 0 when
+ * no hit exists, 2 when the octrees must decide.  One ray per thread, every
+ * lane at its own step. */
+template <bool COUNT, bool ANY, bool SORT = true>
+__device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, int time, Hit &h, TraceCounters *tc, int *overflow,
+		int scene = -1)
+{
+	h.t = FLT_MAX;
+	h.obj = -1;
+	h.prim = -1;
 	h.tie = 0;
+	const int2 roots = scene_roots(S, scene);
+	if(roots.x < 0) return ANY ? 0 : 1;
+	if(roots.y < 0) return ANY ? 2 : 0;
+	Walk<COUNT, ANY, SORT> w;
+	TStack st;
+	w.start(S, wo, wd, time, roots);
+	while(w.cur != BVH_NONE) {
+		int res;
+		if(w.cur < 0) res = w.inst ? w.step_leaf(S, st, tc) : w.step_object(S, st, tc);
+		else res = w.step_node(S, st, tc);
+		if(res == WALK_GOES) continue;
+		if(res == WALK_HIT) break;
+		if(res == WALK_OVERFLOW) { *overflow = 1; return ANY ? 0 : 1; }
+		return ANY ? 2 : 0;
+	}
+	if(!w.confirmed(S)) return ANY ? 2 : 0;
+	if(ANY) return w.bobj >= 0 ? 1 : 0;
+	if(w.bobj < 0) return 1;
+	h.t = w.best;
+	h.obj = w.bobj;
+	h.prim = w.bprim;
 	return 1;
+}
+
+/* The rays [*next, end) of a block (next in shared memory), walked by its
+ * warps.  Rays of one warp need very different numbers of steps, and a step
+ * is a node, a leaf or an object: with a ray per thread and every lane at
+ * its own kind of step, 4 of 32 lanes were active per instruction on
+ * incoherent rays (33,500 instructions per warp).  Here a warp takes the
+ * kind of step that most of its lanes wait for, all of them together, and
+ * once REFILL lanes have finished, writes their results and takes new rays
+ * for them.  Each ray's own sequence of steps is that of trace_two_level, so
+ * the results are the same.  load(i, o, d, time, scene) gives ray i (and its
+ * number for done), done(i, result, walk) takes its result as
+ * trace_two_level returns it.  1,000,003 rays from random points in random
+ * directions over the 1.26M-triangle terrain: 1.19 ms, against 1.89 with a
+ * ray per thread. */
+template <int REFILL, bool COUNT, bool ANY, bool SORT, class Load, class Done>
+__device__ __forceinline__ void walk_stream(const DScene &S, int *next, int end, Load load, Done done, TraceCounters *tc, int *overflow)
+{
+	const unsigned FULL = 0xffffffffu;
+	const int lane = threadIdx.x & 31;
+	Walk<COUNT, ANY, SORT> w;
+	TStack st;
+	w.cur = BVH_NONE;
+	int ri = -1;                 /* the lane's ray */
+	int res = WALK_GOES;
+	bool more = true;            /* the block's rays may not have run out */
+	for(;;) {
+		const int kind = ri < 0 ? WALK_END : (res != WALK_GOES ? WALK_END : w.kind());
+		const unsigned mn = __ballot_sync(FULL, kind == WALK_NODE);
+		const unsigned ml = __ballot_sync(FULL, kind == WALK_LEAF);
+		const unsigned mo = __ballot_sync(FULL, kind == WALK_OBJECT);
+		const int nn = __popc(mn), nl = __popc(ml), no = __popc(mo);
+		const int idle = 32 - nn - nl - no;
+		if(idle == 32 || (more && idle >= REFILL)) {
+			/* the finished rays' results, then new rays for the idle lanes */
+			if(kind == WALK_END && ri >= 0) {
+				int out;
+				if(res == WALK_OVERFLOW) { *overflow = 1; out = ANY ? 0 : 1; w.bobj = -1; }
+				else if(res == WALK_UNDECIDED || !w.confirmed(S)) out = ANY ? 2 : 0;
+				else out = ANY ? (w.bobj >= 0 ? 1 : 0) : 1;
+				done(ri, out, w);
+				ri = -1;
+			}
+			if(!more) break;
+			int base = 0;
+			if(lane == 0) base = atomicAdd(next, idle);
+			base = __shfl_sync(FULL, base, 0);
+			more = base + idle < end;
+			const unsigned mi = ~(mn | ml | mo);
+			if(kind == WALK_END) {
+				int i = base + __popc(mi & ((1u << lane) - 1u));
+				if(i < end) {
+					V3 o, d;
+					int time, scene;
+					ri = load(i, o, d, time, scene);
+					const int2 roots = scene_roots(S, scene);
+					res = WALK_GOES;
+					if(roots.x < 0) {
+						w.bobj = -1;
+						w.cur = BVH_NONE;
+					} else if(roots.y < 0) {
+						res = WALK_UNDECIDED;
+					} else {
+						w.start(S, o, d, time, roots);
+					}
+				}
+			}
+			continue;
+		}
+		/* the step most lanes are at */
+		if(nn >= nl && nn >= no) {
+			if(kind == WALK_NODE) res = w.step_node(S, st, tc);
+		} else if(nl >= no) {
+			if(kind == WALK_LEAF) res = w.step_leaf(S, st, tc);
+		} else {
+			if(kind == WALK_OBJECT) res = w.step_object(S, st, tc);
+		}
+	}
 }
 
 /* the octrees alone, kept out of line so that the hierarchy traversal's

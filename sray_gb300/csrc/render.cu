@@ -138,30 +138,65 @@ __global__ void k_ray_permute(RayQueue in, const unsigned *vals, int n, RayQueue
 	}
 }
 
-/* Closest hits.  HYB = true traces through the mesh hierarchies and lists
- * the rays whose result the octree must decide in fb (count in fb[0], ray
- * indices from fb + 1); HYB = false traces the listed rays with the octree
- * alone.  Keeping the two in separate kernels keeps the octree code out of
- * the hierarchy traversal's register allocation. */
-template <bool COUNT, bool HYB>
-__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQueue q, int4 *hits, DevCounters *ctr, int *fb)
+/* idle lanes at which a warp takes new rays: light samples and secondary
+ * rays stay in the order of the pixels they come from, and a refill mixes
+ * early and late ones, so that they wait longer than a program's own rays
+ * (frame of 1920x1080, 4 samples: 27.8 ms at 16 / 24, 28.5 at 12 / 32 and
+ * at 24 / 32, 29.0 at 32 / 32, 30.1 at 4 / 4; a million random rays: 1.19 ms
+ * at 8 to 12, 1.25 at 20) */
+#define TRACE_REFILL 16
+#define SHADOW_REFILL 24
+#define CAST_REFILL 10
+/* Closest hits through the hierarchies, a chunk of the pass's rays per
+ * block (walk_stream); the rays whose result the octrees must decide are
+ * listed in fb (count in fb[0], ray indices from fb + 1), which
+ * k_trace_octree traces with the octrees alone.  Keeping the two in separate
+ * kernels keeps the octree code out of the hierarchy traversal's register
+ * allocation. */
+template <bool COUNT>
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQueue q, int chunk, int4 *hits, DevCounters *ctr, int *fb)
 {
-	int n = HYB ? *q.count : fb[0];
+	__shared__ int next;
+	const int n = *q.count;
+	const int first = blockIdx.x * chunk;
+	if(first >= n) return;
+	if(threadIdx.x == 0) next = first;
+	__syncthreads();
+	TraceCounters tc = {0, 0};
+	int overflow = 0;
+	walk_stream<TRACE_REFILL, COUNT, false, true>(S, &next, min(first + chunk, n),
+			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
+				float4 o4 = q.o[i], d4 = q.d[i];
+				o = mk(o4.x, o4.y, o4.z);
+				d = mk(d4.x, d4.y, d4.z);
+				time = q.meta[i].w;
+				scene = S.nscenes > 1 ? pixel_scene(S, __float_as_int(q.w[i].w)) : -1;
+				return i;
+			},
+			[&](int i, int sure, const Walk<COUNT, false, true> &w) {
+				if(!sure) fb[1 + atomicAdd(fb, 1)] = i;
+				else hits[i] = w.bobj >= 0 ? make_int4(__float_as_int(w.best), w.bobj, w.bprim, 0) : make_int4(__float_as_int(FLT_MAX), -1, -1, 0);
+			}, &tc, &overflow);
+	if(overflow) atomicOr(&ctr->overflow, 1);
+	if(COUNT) {
+		atomicAdd(&ctr->nodes, tc.nodes);
+		atomicAdd(&ctr->prims, tc.prims);
+	}
+}
+
+/* the listed rays, octrees only */
+template <bool COUNT>
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace_octree(DScene S, RayQueue q, int4 *hits, DevCounters *ctr, const int *fb)
+{
+	const int n = fb[0];
 	TraceCounters tc = {0, 0};
 	int overflow = 0;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		int ri = HYB ? i : fb[1 + i];
+		int ri = fb[1 + i];
 		float4 o = q.o[ri], d = q.d[ri];
-		int time = q.meta[ri].w;
 		int scene = S.nscenes > 1 ? pixel_scene(S, __float_as_int(q.w[ri].w)) : -1;
 		Hit h;
-		bool sure = true;
-		if(HYB) sure = trace_two_level<COUNT, false>(S, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), time, h, &tc, &overflow, scene) != 0;
-		else trace_closest_octree_impl<COUNT>(S, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), time, h, &tc, &overflow, scene);
-		if(HYB && !sure) {
-			fb[1 + atomicAdd(fb, 1)] = ri;
-			continue;
-		}
+		trace_closest_octree_impl<COUNT>(S, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), q.meta[ri].w, h, &tc, &overflow, scene);
 		hits[ri] = make_int4(__float_as_int(h.t), h.obj, h.prim, h.tie);
 	}
 	if(overflow) atomicOr(&ctr->overflow, 1);
@@ -169,7 +204,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQu
 		atomicAdd(&ctr->nodes, tc.nodes);
 		atomicAdd(&ctr->prims, tc.prims);
 	}
-	if(!HYB && n > 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->bvh_fallbacks, (unsigned long long)n);
+	if(n > 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->bvh_fallbacks, (unsigned long long)n);
 }
 
 /* Closest hits of coherent rays -- a pass of camera rays, the 32 of a warp
@@ -1186,42 +1221,58 @@ __global__ void __launch_bounds__(128) k_render_pool(DScene S, RayQueue pool, in
 
 /* shadow rays: the reference tests visibility with cast_ray(shadow_ray)
  * (src/shader.cc:266), a hit anywhere on the segment [eps, 1] blocks */
-/* shadow rays; HYB and fb as for k_trace */
-template <bool HYB, bool SORT = true, bool COUNT = false>
-__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow(DScene S, const ShadowReq *sq, const int *sq_count, float4 *acc,
+/* shadow rays; chunks and fb as for k_trace */
+template <bool SORT = true, bool COUNT = false>
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow(DScene S, const ShadowReq *sq, const int *sq_count, int chunk, float4 *acc,
 		DevCounters *ctr, int *fb)
 {
-	int n = HYB ? *sq_count : fb[0];
-	int overflow = 0;
+	__shared__ int next;
+	const int n = *sq_count;
+	if(blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->rays[2], (unsigned long long)n);
+	const int first = blockIdx.x * chunk;
+	if(first >= n) return;
+	if(threadIdx.x == 0) next = first;
+	__syncthreads();
 	TraceCounters tc = {0, 0};
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		int ri = HYB ? i : fb[1 + i];
-		ShadowReq r = sq[ri];
-		int time = __float_as_int(r.a.w), pixel = __float_as_int(r.b.w);
-		int res;
-		int scene = S.nscenes > 1 ? __float_as_int(r.w.w) : -1;
-		if(HYB) {
-			Hit h;
-			res = trace_two_level<COUNT, true, SORT>(S, mk(r.a.x, r.a.y, r.a.z), mk(r.b.x, r.b.y, r.b.z), time, h, &tc, &overflow,
-					scene);
-		} else {
-			res = trace_any_octree_impl(S, mk(r.a.x, r.a.y, r.a.z), mk(r.b.x, r.b.y, r.b.z), time, &overflow, scene) ? 1 : 0;
-		}
-		if(HYB && res == 2) {
-			fb[1 + atomicAdd(fb, 1)] = ri;
-			continue;
-		}
-		if(res == 0) acc_add(acc, pixel, r.w.x, r.w.y, r.w.z);
-	}
+	int overflow = 0;
+	walk_stream<SHADOW_REFILL, COUNT, true, SORT>(S, &next, min(first + chunk, n),
+			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
+				float4 a = sq[i].a, b = sq[i].b;
+				o = mk(a.x, a.y, a.z);
+				d = mk(b.x, b.y, b.z);
+				time = __float_as_int(a.w);
+				scene = S.nscenes > 1 ? __float_as_int(sq[i].w.w) : -1;
+				return i;
+			},
+			[&](int i, int res, const Walk<COUNT, true, SORT> &) {
+				if(res == 2) {
+					fb[1 + atomicAdd(fb, 1)] = i;
+				} else if(res == 0) {
+					float4 w = sq[i].w;
+					acc_add(acc, __float_as_int(sq[i].b.w), w.x, w.y, w.z);
+				}
+			}, &tc, &overflow);
 	if(overflow) atomicOr(&ctr->overflow, 1);
 	if(COUNT) {
 		atomicAdd(&ctr->snodes, tc.nodes);
 		atomicAdd(&ctr->sprims, tc.prims);
 	}
-	if(blockIdx.x == 0 && threadIdx.x == 0) {
-		if(HYB) atomicAdd(&ctr->rays[2], (unsigned long long)n);
-		else if(n > 0) atomicAdd(&ctr->bvh_fallbacks, (unsigned long long)n);
+}
+
+/* the listed segments, octrees only */
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow_octree(DScene S, const ShadowReq *sq, float4 *acc, DevCounters *ctr,
+		const int *fb)
+{
+	const int n = fb[0];
+	int overflow = 0;
+	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+		ShadowReq r = sq[fb[1 + i]];
+		int scene = S.nscenes > 1 ? __float_as_int(r.w.w) : -1;
+		if(!trace_any_octree_impl(S, mk(r.a.x, r.a.y, r.a.z), mk(r.b.x, r.b.y, r.b.z), __float_as_int(r.a.w), &overflow, scene))
+			acc_add(acc, __float_as_int(r.b.w), r.w.x, r.w.y, r.w.z);
 	}
+	if(overflow) atomicOr(&ctr->overflow, 1);
+	if(n > 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->bvh_fallbacks, (unsigned long long)n);
 }
 
 /* light samples with one warp per segment (as k_trace_warp), for passes of
@@ -1894,19 +1945,76 @@ __global__ void k_finish(const int *active, int tw, int th, const int *n_active_
 	}
 }
 
-/* closest hits of caller-supplied world rays (sray_gpu_cast_rays) */
-__global__ void __launch_bounds__(SRAY_TRACE_THREADS) k_cast(DScene S, int n, const float *orig, const float *dir, const int *time, int *obj, int *prim, float *t,
-		unsigned char *tie, DevCounters *ctr)
+/* closest hits of caller-supplied world rays (sray_gpu_cast_rays), as the
+ * frame's passes: chunks of rays per block, or one warp per ray; then the
+ * listed rays by the octrees */
+struct CastRays {
+	const float *orig, *dir;
+	const int *time;          /* may be null: the frame's */
+	int *obj, *prim;
+	float *t;
+	unsigned char *tie;
+	__device__ __forceinline__ V3 o(int i) const { return mk(orig[i * 3], orig[i * 3 + 1], orig[i * 3 + 2]); }
+	__device__ __forceinline__ V3 d(int i) const { return mk(dir[i * 3], dir[i * 3 + 1], dir[i * 3 + 2]); }
+	__device__ __forceinline__ int when(const DScene &S, int i) const { return time ? time[i] : S.t0; }
+	__device__ __forceinline__ void put(int i, int o, int p, float dist, int tied) const
+	{
+		obj[i] = o;
+		prim[i] = o >= 0 ? p : -1;
+		t[i] = o >= 0 ? dist : 0.0f;
+		tie[i] = (unsigned char)tied;
+	}
+};
+
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRays R, int n, int chunk, DevCounters *ctr, int *fb)
 {
+	__shared__ int next;
+	const int first = blockIdx.x * chunk;
+	if(threadIdx.x == 0) next = first;
+	__syncthreads();
 	int overflow = 0;
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+	walk_stream<CAST_REFILL, false, false, true>(S, &next, min(first + chunk, n),
+			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
+				o = R.o(i);
+				d = R.d(i);
+				time = R.when(S, i);
+				scene = -1;
+				return i;
+			},
+			[&](int i, int sure, const Walk<false, false, true> &w) {
+				if(!sure) fb[1 + atomicAdd(fb, 1)] = i;
+				else R.put(i, w.bobj, w.bprim, w.best, 0);
+			}, nullptr, &overflow);
+	if(overflow) atomicOr(&ctr->overflow, 1);
+}
+
+__global__ void __launch_bounds__(128) k_cast_warp(DScene S, CastRays R, int n, int *fb)
+{
+	__shared__ int s_ref[4][WR_CAP];
+	__shared__ int s_obj[4][WR_CAP];
+	__shared__ float s_te[4][WR_CAP];
+	int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	for(int i = blockIdx.x * 4 + w; i < n; i += gridDim.x * 4) {
+		float best;
+		int bobj, bprim;
+		int res = warp_trace<false>(S, R.o(i), R.d(i), R.when(S, i), s_ref[w], s_obj[w], s_te[w], best, bobj, bprim, -1);
+		if(lane == 0) {
+			if(!res) fb[1 + atomicAdd(fb, 1)] = i;
+			else R.put(i, bobj, bprim, best, 0);
+		}
+		__syncwarp();
+	}
+}
+
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS) k_cast_octree(DScene S, CastRays R, DevCounters *ctr, const int *fb)
+{
+	const int n = fb[0];
+	int overflow = 0;
+	for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+		int i = fb[1 + k];
 		Hit h;
-		trace_closest<false>(S, mk(orig[i * 3], orig[i * 3 + 1], orig[i * 3 + 2]), mk(dir[i * 3], dir[i * 3 + 1], dir[i * 3 + 2]),
-				time ? time[i] : S.t0, h, nullptr, &overflow);
-		obj[i] = h.obj;
-		prim[i] = h.obj >= 0 ? h.prim : -1;
-		t[i] = h.obj >= 0 ? h.t : 0.0f;
-		tie[i] = (unsigned char)h.tie;
+		trace_closest_octree_impl<false>(S, R.o(i), R.d(i), R.when(S, i), h, nullptr, &overflow);
+		R.put(i, h.obj, h.prim, h.t, h.tie);
 	}
 	if(overflow) atomicOr(&ctr->overflow, 1);
 }
@@ -1932,6 +2040,26 @@ __global__ void k_primary_hits(DScene S, RayQueue q, const int4 *hits, int *obj,
 
 /* at most this many gather requests wait for the photon maps across waves */
 #define DEFER_MAX_REQS ((int64_t)1 << 28)
+
+/* Rays per block of a streaming traversal (k_trace, k_shadow, k_cast) of n
+ * rays: about a wave of resident blocks, each taking its lanes' next rays
+ * from its own chunk, up to the limit of the caller's kind of pass.  A larger
+ * chunk has fewer lanes waiting at its end; a smaller one keeps a block's
+ * rays close together (photons leave sorted by direction and origin) and
+ * ends sooner, which frees its SM for the streams beside it.  Measured:
+ * photon maps of 2.5M photons 7.05 ms with 256, 7.25 with 512, 7.5 with
+ * 1024, 7.2 with 128; frame of 1920x1080, 4 samples, 27.2 ms with 512 for
+ * its own passes, 27.7 with 256, 27.8 with 1024; a million random rays alone
+ * 1.19 ms with 1024, 1.27 with 512. */
+#define PHOTON_CHUNK 256
+#define FRAME_CHUNK 512
+#define CAST_CHUNK 1024
+static int stream_chunk(int n, int most)
+{
+	int c = n / (152 * 8);
+	c = (c + SRAY_TRACE_THREADS - 1) / SRAY_TRACE_THREADS * SRAY_TRACE_THREADS;
+	return c < SRAY_TRACE_THREADS ? SRAY_TRACE_THREADS : (c > most ? most : c);
+}
 
 static int grid_for(int n, int block)
 {
@@ -3542,32 +3670,24 @@ int Renderer::queue_overflow(int count, int cap)
  * rays of q into hits: the hierarchy pass, then the octree pass over the
  * rays it listed */
 int Renderer::trace_rays_with(const DScene &D, const RayQueue &qq, int n, const char *name, bool count, cudaStream_t s,
-		int4 *hit_out, DevBuf &fb, DevCounters *c, bool short_blocks, bool coherent)
+		int4 *hit_out, DevBuf &fb, DevCounters *c, bool coherent)
 {
 	CK(fb.ensure(((size_t)n + 1) * sizeof(int)), "fallback list");
 	CK(cudaMemsetAsync(fb.p, 0, sizeof(int), s), "reset fallback list");
-	/* short_blocks (the photon stream's passes): a block per 128 rays
-	 * instead of a capped grid that strides, so that its blocks free their
-	 * SMs for the frame's stream as they finish */
-	int g = short_blocks ? std::max(1, (n + 127) / 128) : grid_for(n, 128);
-	if(!count && coherent && D.nscenes <= 1 && n > tune.warp_rays) {
-		LAUNCH(*this, name, s, k_trace_packet<<<g, SRAY_TRACE_THREADS, 0, s>>>(D, qq, hit_out, c, fb.as<int>()));
-		LAUNCH(*this, "octree_retrace", s, k_trace<false, false><<<retrace_grid(), 128, 0, s>>>(D, qq, hit_out, c, fb.as<int>()));
-		return 0;
-	}
+	int4 *out = hit_out;
+	int *f = fb.as<int>();
 	if(!count && n <= tune.warp_rays) {
 		/* a pass of few rays: one warp per ray */
-		LAUNCH(*this, name, s, k_trace_warp<<<grid_for(n, 4), 128, 0, s>>>(D, qq, hit_out, fb.as<int>()));
-		LAUNCH(*this, "octree_retrace", s, k_trace<false, false><<<retrace_grid(), 128, 0, s>>>(D, qq, hit_out, c, fb.as<int>()));
-		return 0;
-	}
-	if(count) {
-		LAUNCH(*this, name, s, k_trace<true, true><<<g, 128, 0, s>>>(D, qq, hit_out, c, fb.as<int>()));
-		LAUNCH(*this, "octree_retrace", s, k_trace<true, false><<<retrace_grid(), 128, 0, s>>>(D, qq, hit_out, c, fb.as<int>()));
+		LAUNCH(*this, name, s, k_trace_warp<<<grid_for(n, 4), 128, 0, s>>>(D, qq, out, f));
+	} else if(!count && coherent && D.nscenes <= 1) {
+		LAUNCH(*this, name, s, k_trace_packet<<<grid_for(n, 128), SRAY_TRACE_THREADS, 0, s>>>(D, qq, out, c, f));
 	} else {
-		LAUNCH(*this, name, s, k_trace<false, true><<<g, 128, 0, s>>>(D, qq, hit_out, c, fb.as<int>()));
-		LAUNCH(*this, "octree_retrace", s, k_trace<false, false><<<retrace_grid(), 128, 0, s>>>(D, qq, hit_out, c, fb.as<int>()));
+		const int chunk = stream_chunk(n, c == pctr.as<DevCounters>() ? PHOTON_CHUNK : FRAME_CHUNK), g = (n + chunk - 1) / chunk;
+		if(count) LAUNCH(*this, name, s, k_trace<true><<<g, SRAY_TRACE_THREADS, 0, s>>>(D, qq, chunk, out, c, f));
+		else LAUNCH(*this, name, s, k_trace<false><<<g, SRAY_TRACE_THREADS, 0, s>>>(D, qq, chunk, out, c, f));
 	}
+	if(count) LAUNCH(*this, "octree_retrace", s, k_trace_octree<true><<<retrace_grid(), 128, 0, s>>>(D, qq, out, c, f));
+	else LAUNCH(*this, "octree_retrace", s, k_trace_octree<false><<<retrace_grid(), 128, 0, s>>>(D, qq, out, c, f));
 	return 0;
 }
 
@@ -3584,19 +3704,19 @@ int Renderer::shadow_rays_on(const ShadowReq *q, int *count, int cap, DevBuf &fb
 {
 	CK(fb.ensure(((size_t)cap + 1) * sizeof(int)), "fallback list");
 	CK(cudaMemsetAsync(fb.p, 0, sizeof(int), st), "reset fallback list");
-	int g = grid_for(cap, 128);
+	const int chunk = stream_chunk(cap, FRAME_CHUNK), g = (cap + chunk - 1) / chunk;
 	float4 *a = acc.as<float4>();
 	DevCounters *c = ctr.as<DevCounters>();
 	int *f = fb.as<int>();
 	if(prof_flags & 2)   /* counting the traversal work: every pass thread per segment */
-		LAUNCH(*this, "shadow", st, k_shadow<true, true, true><<<g, 128, 0, st>>>(S, q, count, a, c, f));
+		LAUNCH(*this, "shadow", st, k_shadow<true, true><<<g, 128, 0, st>>>(S, q, count, chunk, a, c, f));
 	else if(cap <= tune.warp_segments)
 		LAUNCH(*this, "shadow", st, k_shadow_warp<<<grid_for(cap, 4), 128, 0, st>>>(S, q, count, a, c, f));
 	else if(tune.shadow_order)
-		LAUNCH(*this, "shadow", st, k_shadow<true, false><<<g, 128, 0, st>>>(S, q, count, a, c, f));
+		LAUNCH(*this, "shadow", st, k_shadow<false><<<g, 128, 0, st>>>(S, q, count, chunk, a, c, f));
 	else
-		LAUNCH(*this, "shadow", st, k_shadow<true><<<g, 128, 0, st>>>(S, q, count, a, c, f));
-	LAUNCH(*this, "octree_retrace", st, k_shadow<false><<<retrace_grid(), 128, 0, st>>>(S, q, count, a, c, f));
+		LAUNCH(*this, "shadow", st, k_shadow<true><<<g, 128, 0, st>>>(S, q, count, chunk, a, c, f));
+	LAUNCH(*this, "octree_retrace", st, k_shadow_octree<<<retrace_grid(), 128, 0, st>>>(S, q, a, c, f));
 	return 0;
 }
 
@@ -3625,13 +3745,13 @@ int Renderer::side_stream()
 
 int Renderer::trace_rays(const RayQueue &qq, int n, const char *name, bool count, cudaStream_t s, bool coherent)
 {
-	return trace_rays_with(S, qq, n, name, count, s, hits.as<int4>(), fbl, ctr.as<DevCounters>(), false, coherent);
+	return trace_rays_with(S, qq, n, name, count, s, hits.as<int4>(), fbl, ctr.as<DevCounters>(), coherent);
 }
 
 /* photon passes: the photon buffers and counters */
 int launch_trace(Renderer &R, const DScene &D, const RayQueue &q, int n, const char *name, cudaStream_t s)
 {
-	return R.trace_rays_with(D, q, n, name, false, s, R.phits.as<int4>(), R.pfbl, R.pctr.as<DevCounters>(), true);
+	return R.trace_rays_with(D, q, n, name, false, s, R.phits.as<int4>(), R.pfbl, R.pctr.as<DevCounters>());
 }
 
 int Renderer::photon_stream()
@@ -4289,9 +4409,19 @@ int sray_gpu_cast_rays(int n, const float *orig, const float *dir, const int *ti
 	if(n == 0) return 0;
 	cudaStream_t s = as_stream(stream);
 	cudaError_t e = R.ctr.ensure(sizeof(DevCounters));
+	if(e == cudaSuccess) e = R.fbl.ensure(((size_t)n + 1) * sizeof(int));
 	if(e == cudaSuccess) e = cudaMemsetAsync(R.ctr.p, 0, sizeof(DevCounters), s);
+	if(e == cudaSuccess) e = cudaMemsetAsync(R.fbl.p, 0, sizeof(int), s);
 	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
-	k_cast<<<grid_for(n, 128), 128, 0, s>>>(R.S, n, orig, dir, time, obj, prim, t, tie, R.ctr.as<DevCounters>());
+	const CastRays rays = {orig, dir, time, obj, prim, t, tie};
+	int *fb = R.fbl.as<int>();
+	if(n <= R.tune.warp_rays) {
+		k_cast_warp<<<grid_for(n, 4), 128, 0, s>>>(R.S, rays, n, fb);
+	} else {
+		const int chunk = stream_chunk(n, CAST_CHUNK);
+		k_cast<<<(n + chunk - 1) / chunk, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, n, chunk, R.ctr.as<DevCounters>(), fb);
+	}
+	k_cast_octree<<<grid_for(n, 128) < R.nsm ? grid_for(n, 128) : R.nsm, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, R.ctr.as<DevCounters>(), fb);
 	DevCounters hc;
 	e = cudaMemcpyAsync(&hc, R.ctr.p, sizeof hc, cudaMemcpyDeviceToHost, s);
 	if(e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -311,7 +311,7 @@ struct Renderer {
 	/* coherent: a pass of camera rays (traced as warp packets when it is large) */
 	int trace_rays(const RayQueue &q, int n, const char *name, bool count, cudaStream_t s, bool coherent = false);
 	int trace_rays_with(const DScene &D, const RayQueue &q, int n, const char *name, bool count, cudaStream_t s, int4 *hit_out,
-			DevBuf &fb, DevCounters *c, bool short_blocks = false, bool coherent = false);
+			DevBuf &fb, DevCounters *c, bool coherent = false);
 	int photon_stream();
 	void fill_scene_desc();
 };
