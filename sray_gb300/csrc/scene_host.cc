@@ -439,6 +439,69 @@ Box Object::bounds(const std::vector<Mesh> &meshes, int t) const
 	return b;
 }
 
+/* A mesh's own bounds, or the box of the transformed quadric (the bounds
+ * above ignore its scaling and rotation), widened by 2^-16 of its largest
+ * coordinate: far more than the rounding of transforms, vertices and hit
+ * points to float. */
+Box Object::reach(const Box &vertices, int t) const
+{
+	Box b = vertices;
+	if(type != OBJ_MESH) {
+		double m[4][4];
+		xf.matrix(t, m);
+		Vec3 c0 = m_pt(m, Vec3(0, type == OBJ_CYLINDER ? start : 0.0, 0)), c1 = m_pt(m, Vec3(0, type == OBJ_CYLINDER ? end : 0.0, 0));
+		for(int i = 0; i < 3; i++) {
+			double y = type == OBJ_CYLINDER ? 0.0 : m[i][1];
+			double e = fabs(rad) * sqrt(m[i][0] * m[i][0] + y * y + m[i][2] * m[i][2]);
+			b.mn[i] = std::min(c0[i], c1[i]) - e;
+			b.mx[i] = std::max(c0[i], c1[i]) + e;
+		}
+	}
+	double most = 0.0;
+	for(int i = 0; i < 3; i++) most = std::max(most, std::max(fabs(b.mn[i]), fabs(b.mx[i])));
+	for(int i = 0; i < 3; i++) {
+		b.mn[i] -= most / 65536.0;
+		b.mx[i] += most / 65536.0;
+	}
+	return b;
+}
+
+bool HostScene::object_reach(size_t i, int tlo, int thi, Box &b) const
+{
+	const Object &o = objs[i];
+	if(o.is_static) {
+		b = o.static_reach;
+		return true;
+	}
+	const Track<Vec3> &p = o.xf.pos;
+	if(o.xf.rot.time.size() > 1 || o.xf.scale.time.size() > 1 || p.interp == INTERP_CUBIC || p.extrap == EXTRAP_PINGPONG) return false;
+	/* the object at bt0, moved to every place it takes: between two keys a
+	 * position is between theirs (or one of them), and a repeated track
+	 * stays among its keys */
+	Vec3 at = o.xf.position(bt0);
+	Vec3 e[2] = {o.xf.position(tlo), o.xf.position(thi)};
+	double lo[3], hi[3];
+	for(int k = 0; k < 3; k++) {
+		lo[k] = std::min(e[0][k], e[1][k]);
+		hi[k] = std::max(e[0][k], e[1][k]);
+	}
+	const bool all = p.extrap == EXTRAP_REPEAT && !p.time.empty() && (tlo < p.time.front() || thi > p.time.back());
+	for(size_t j = 0; j < p.time.size(); j++) {
+		if(!all && (p.time[j] < tlo || p.time[j] > thi)) continue;
+		for(int k = 0; k < 3; k++) {
+			lo[k] = std::min(lo[k], p.val[j][k]);
+			hi[k] = std::max(hi[k], p.val[j][k]);
+		}
+	}
+	b = o.reach(object_bounds(i, bt0), bt0);
+	for(int k = 0; k < 3; k++) {
+		double most = std::max(fabs(lo[k]), fabs(hi[k])) / 65536.0;
+		b.mn[k] += lo[k] - at[k] - most;
+		b.mx[k] += hi[k] - at[k] + most;
+	}
+	return true;
+}
+
 static inline bool overlap(const Box &a, const Box &b)
 {
 	for(int i = 0; i < 3; i++) if(a.mn[i] > b.mx[i] || b.mn[i] > a.mx[i]) return false;
@@ -1491,6 +1554,7 @@ void HostScene::finish_load(const sray_opts &opt, bool build_meshes)
 		o.is_static = false;
 		if(o.xf.pos.time.size() <= 1 && o.xf.rot.time.size() <= 1 && o.xf.scale.time.size() <= 1) {
 			o.static_box = o.bounds(meshes, 0);
+			o.static_reach = o.reach(o.static_box, 0);
 			o.is_static = true;
 		}
 	}

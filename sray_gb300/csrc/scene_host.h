@@ -118,7 +118,11 @@ struct Object {
 	int mesh = -1;
 	bool is_static = false;    /* every transform track has at most one key */
 	Box static_box;
+	Box static_reach;          /* of a static object: its reach() */
 	Box bounds(const std::vector<Mesh> &meshes, int t) const;
+	/* a box that holds every point of the object at time t (vertices: a mesh's
+	 * own bounds at that time), float rounding included */
+	Box reach(const Box &vertices, int t) const;
 };
 
 struct ProjMap {
@@ -185,6 +189,10 @@ struct HostScene {
 	std::vector<Box> box_t0, box_t1;   /* object bounds at the frame's t0 / t1 */
 	std::vector<Box> oct_boxes;        /* the boxes the scene octree was built from */
 	Box object_bounds(size_t i, int t) const;
+	/* a box that holds every point of object i at every time in [tlo, thi];
+	 * false where that is not known cheaply (rotating or scaling objects,
+	 * cubic positions) */
+	bool object_reach(size_t i, int tlo, int thi, Box &b) const;
 
 	/* Load an S-ray XML document.  With a side-car path: when the file
 	 * there holds the meshes of this exact document (and their octrees and
