@@ -183,6 +183,251 @@ __device__ bool gen_dir(const uint32_t *bits, sray_rng *s, V3 *out)
 	return false;
 }
 
+/* ---------------- projection maps ----------------
+ * Light::build_proj_intern and ::build_projmap (src/light.cc:151-200,
+ * 392-432): from each sample point of a light, every object's box becomes a
+ * sphere around its centre, and a cell of the 64 x 32 direction grid is set
+ * when a corner of it, taken to the centre's distance, lies in the sphere, or
+ * when it holds the centre's direction; a light inside a box sets the whole
+ * map.  The coverage is the sum of the set cells' shares of the sphere in the
+ * order in which they were set (samples, boxes, the centre's cell, then rows)
+ * -- a sum in double, whose rounding depends on that order.
+ *
+ * k_proj_view takes a thread per (sample, box), k_proj_mark a block: the
+ * corners' tests (33 rows of 65, a warp per row) and, per cell they set, the
+ * smallest (sample, box, place) over all blocks.  k_proj_cover, a block per
+ * map, gives the bits, sorts the set cells by that order and sums.  On the
+ * host, a thread per light, this took 1.9 ms for three lights over 201
+ * objects before the first photon left (1.4 ms for six frames of 25); here
+ * under 80 us (120 us).  What bounds it is the latency of its chains: double
+ * arithmetic, the sort, the ordered sum. */
+struct ProjSample {
+	double lp[3];
+	int box0, nbox;       /* the boxes it sees */
+	int slot;             /* the light of the job */
+	unsigned order;       /* among the light's samples */
+};
+
+struct ProjBox {
+	double mn[3], mx[3];
+	int caustic, pad;     /* also in the caustic map */
+};
+
+#define PROJ_CELLS 2048
+#define PROJ_SLOT (PROJ_CELLS + 1)   /* a map's cells, and 0 when the light is inside a box */
+#define PROJ_NONE 0xffffffffffffffffull
+
+/* one box as one sample sees it */
+struct ProjView {
+	double c[3], dist, rad_sq;    /* the box's centre, its distance, the sphere's squared radius */
+	float u[3];                   /* the centre's direction */
+	float lo, hi;                 /* cosines below / above which a corner is out / in the sphere for certain */
+	float phi, cap;               /* its colatitude; the angle beyond which a row holds no corner in the sphere */
+	int live;                     /* 0: the light is inside the box (or no such box) */
+};
+
+/* a thread per (sample, box): the double arithmetic, of which this GPU does
+ * little at once, with every lane at work; a light inside a box, and the
+ * cell of the centre's direction, go straight into the maps */
+__global__ void __launch_bounds__(128) k_proj_view(const ProjSample *samples, int nsamples, int most, const ProjBox *boxes, ProjView *views,
+		unsigned long long *first)
+{
+	for(long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)nsamples * most; i += (long long)gridDim.x * blockDim.x) {
+		const int si = (int)(i / most), bi = (int)(i - (long long)si * most);
+		const ProjSample &S = samples[si];
+		ProjView &V = views[i];
+		V.live = 0;
+		if(bi >= S.nbox) continue;
+		const ProjBox &B = boxes[S.box0 + bi];
+		unsigned long long *map = first + (size_t)S.slot * 2 * PROJ_SLOT;
+		const double lx = S.lp[0], ly = S.lp[1], lz = S.lp[2];
+		if(lx >= B.mn[0] && ly >= B.mn[1] && lz >= B.mn[2] && lx < B.mx[0] && ly < B.mx[1] && lz < B.mx[2]) {
+			map[PROJ_CELLS] = 0;
+			if(B.caustic) map[PROJ_SLOT + PROJ_CELLS] = 0;
+			continue;
+		}
+		const double cx = (B.mn[0] + B.mx[0]) / 2.0, cy = (B.mn[1] + B.mx[1]) / 2.0, cz = (B.mn[2] + B.mx[2]) / 2.0;
+		const double ex = B.mn[0] - cx, ey = B.mn[1] - cy, ez = B.mn[2] - cz;
+		const double rad_sq = ex * ex + ey * ey + ez * ez;
+		const double vx = cx - lx, vy = cy - ly, vz = cz - lz;
+		const double dist = sqrt(vx * vx + vy * vy + vz * vz);
+		V.c[0] = cx; V.c[1] = cy; V.c[2] = cz;
+		V.dist = dist;
+		V.rad_sq = rad_sq;
+		/* a corner direction c is in the sphere when c . v / dist >= 1 -
+		 * rad_sq / (2 dist^2): decided in float outside a margin of its
+		 * rounding (and of the double test's where the light is far from the
+		 * origin), by the reference's own test in double within it */
+		const float fd = (float)dist, cos_t = (float)(1.0 - rad_sq / (2.0 * dist * dist));
+		const float far = (float)fmax(fmax(fabs(lx), fabs(ly)), fabs(lz)) / fd;
+		const float margin = 4e-6f + 1e-12f * far * (1.0f + far);
+		V.u[0] = (float)vx / fd;
+		V.u[1] = (float)vy / fd;
+		V.u[2] = (float)vz / fd;
+		V.lo = cos_t - margin;
+		V.hi = cos_t + margin;
+		V.phi = acosf(fminf(fmaxf(V.u[1], -1.0f), 1.0f));
+		V.cap = V.lo > -1.0f ? acosf(fminf(V.lo, 1.0f)) + 2e-3f : 4.0f;
+		V.live = 1;
+		double theta = atan2(vz, vx), ph = acos(vy / dist);
+		if(theta < 0.0) theta = 3.14159265358979323846 * 2.0 + theta;
+		double u = theta / (3.14159265358979323846 * 2.0), v = ph / 3.14159265358979323846;
+		int a = (int)(u * 64), b = (int)(v * 32);
+		a = a < 0 ? 0 : (a >= 64 ? 63 : a);
+		b = b < 0 ? 0 : (b >= 32 ? 31 : b);
+		const int cell = b * 64 + a;
+		const unsigned long long key = (((unsigned long long)S.order * (unsigned)S.nbox + bi) * 2ull) * PROJ_CELLS + cell;
+		atomicMin(map + cell, key);
+		if(B.caustic) atomicMin(map + PROJ_SLOT + cell, key);
+	}
+}
+
+__global__ void __launch_bounds__(128) k_proj_mark(const ProjSample *samples, int nsamples, int most, const ProjBox *boxes,
+		const ProjView *views, const ProjTables *tables, unsigned long long *first)
+{
+	__shared__ unsigned in[33][3];      /* the corners in the sphere */
+	const unsigned FULL = 0xffffffffu;
+	const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+	for(int si = blockIdx.y; si < nsamples; si += gridDim.y) {
+		const ProjView &V = views[(size_t)si * most + blockIdx.x];
+		if(!V.live) continue;
+		const ProjSample &S = samples[si];
+		unsigned long long *map = first + (size_t)S.slot * 2 * PROJ_SLOT;
+		const bool caustic = boxes[S.box0 + blockIdx.x].caustic != 0;
+		const float ux = V.u[0], uy = V.u[1], uz = V.u[2], lo = V.lo, hi = V.hi, phi = V.phi, cap = V.cap;
+		__syncthreads();
+		for(int r = w; r < 33; r += 4) {
+			if(fabsf((float)r * (3.14159265f / 32.0f) - phi) > cap) {
+				if(lane < 3) in[r][lane] = 0;
+				continue;
+			}
+			#pragma unroll
+			for(int k = 0; k < 3; k++) {
+				const int u = k * 32 + lane;
+				bool hit = false;
+				if(u < 65) {
+					const float4 c = *reinterpret_cast<const float4 *>(tables->cornerf[r * 65 + u]);
+					const float s = c.x * ux + c.y * uy + c.z * uz;
+					hit = s > hi;
+					if(!hit && !(s < lo)) {
+						const double *cd = tables->corner[r * 65 + u];
+						double px = S.lp[0] + cd[0] * V.dist, py = S.lp[1] + cd[1] * V.dist, pz = S.lp[2] + cd[2] * V.dist;
+						double dx = px - V.c[0], dy = py - V.c[1], dz = pz - V.c[2];
+						hit = dx * dx + dy * dy + dz * dz <= V.rad_sq;
+					}
+				}
+				const unsigned b = __ballot_sync(FULL, hit);
+				if(lane == 0) in[r][k] = b;
+			}
+		}
+		__syncthreads();
+		/* after the centre's own cell, the others by rows */
+		const unsigned long long order = ((unsigned long long)S.order * (unsigned)S.nbox + blockIdx.x) * 2ull + 1ull;
+		for(int cell = tid; cell < PROJ_CELLS; cell += 128) {
+			const int uc = cell & 63, vc = cell >> 6;
+			const unsigned *a = in[vc], *b = in[vc + 1];
+			const int k0 = uc >> 5, k1 = (uc + 1) >> 5;
+			const unsigned m0 = 1u << (uc & 31), m1 = 1u << ((uc + 1) & 31);
+			if(!((a[k0] | b[k0]) & m0) && !((a[k1] | b[k1]) & m1)) continue;
+			const unsigned long long key = order * PROJ_CELLS + cell;
+			if(map[cell] > key) atomicMin(map + cell, key);
+			if(caustic && map[PROJ_SLOT + cell] > key) atomicMin(map + PROJ_SLOT + cell, key);
+		}
+	}
+}
+
+/* v[0] + v[1] + ... in double, each addition rounded, by a warp.  While the
+ * sum stays within one power of two it is a multiple of the same unit, so an
+ * addition adds the term rounded to that unit: 32 terms at a time, as
+ * integers, by a scan.  A term half way between two units rounds to an even
+ * sum; those are taken in their order.  32 terms over which the sum leaves
+ * its power of two are added one by one.  Terms are positive.  (2,048
+ * dependent double additions take 65 us on this GPU.) */
+__device__ __forceinline__ double ordered_sum(const double *v, int n, int lane)
+{
+	const unsigned FULL = 0xffffffffu;
+	double c = 0.0;
+	for(int i0 = 0; i0 < n; i0 += 32) {
+		const double s = i0 + lane < n ? v[i0 + lane] : 0.0;
+		const long long cb = __double_as_longlong(c), sb = __double_as_longlong(s);
+		const int ce = (int)(cb >> 52), se = (int)(sb >> 52);       /* biased exponents (signs are 0) */
+		const long long cm = (cb & 0xfffffffffffffll) | 0x10000000000000ll, sm = (sb & 0xfffffffffffffll) | 0x10000000000000ll;
+		const int shift = ce - se;
+		const bool slow = ce == 0 || (se && shift < 1) || (!se && sb != 0);
+		bool tie = false;
+		long long q = 0;
+		if(!slow && se && shift <= 53) {
+			const long long half = 1ll << (shift - 1), rem = sm & ((1ll << shift) - 1);
+			q = (sm >> shift) + (rem > half ? 1 : 0);
+			tie = rem == half;
+		}
+		long long incl = q;
+		for(int o = 1; o < 32; o <<= 1) {
+			long long u = __shfl_up_sync(FULL, incl, o);
+			if(lane >= o) incl += u;
+		}
+		/* the ties in order: up when the sum so far is odd */
+		int up = 0;
+		for(unsigned m = __ballot_sync(FULL, tie); m; m &= m - 1)
+			up += ((int)cm + __shfl_sync(FULL, (int)incl, __ffs(m) - 1) + up) & 1;
+		const long long total = __shfl_sync(FULL, incl, 31) + up;
+		if(__any_sync(FULL, slow) || cm + total >= 0x20000000000000ll) {
+			for(int k = 0; k < 32; k++) c += __shfl_sync(FULL, s, k);
+		} else {
+			c = __longlong_as_double(((long long)ce << 52) | ((cm + total) & 0xfffffffffffffll));
+		}
+	}
+	return c;
+}
+
+__global__ void __launch_bounds__(1024) k_proj_cover(const unsigned long long *first, const ProjTables *tables, uint32_t *bits, float *cov)
+{
+	__shared__ unsigned long long key[PROJ_CELLS];
+	__shared__ double share[PROJ_CELLS];
+	__shared__ int nset;
+	const int t = threadIdx.x, lane = t & 31;
+	const unsigned long long *map = first + (size_t)blockIdx.x * PROJ_SLOT;
+	const bool whole = map[PROJ_CELLS] == 0;
+	if(t == 0) nset = 0;
+	__syncthreads();
+	for(int k = 0; k < 2; k++) {
+		const int cell = k * 1024 + t;
+		const unsigned long long v = map[cell];
+		const bool set = whole || v != PROJ_NONE;
+		const unsigned b = __ballot_sync(0xffffffffu, set);
+		if(lane == 0) {
+			bits[(size_t)blockIdx.x * 64 + (cell >> 5)] = b;
+			atomicAdd(&nset, __popc(b));
+		}
+		key[cell] = v;
+	}
+	__syncthreads();
+	if(whole || nset == 0) {
+		if(t == 0) cov[blockIdx.x] = whole ? 1.0f : 0.0f;
+		return;
+	}
+	/* bitonic sort of the cells by the order in which they were set (unset
+	 * ones last); a key's low bits are its cell */
+	for(int size = 2; size <= PROJ_CELLS; size <<= 1) {
+		for(int step = size >> 1; step > 0; step >>= 1) {
+			const int i = 2 * t - (t & (step - 1));
+			const bool up = (i & size) == 0;
+			const unsigned long long a = key[i], b = key[i + step];
+			if((a > b) == up) {
+				key[i] = b;
+				key[i + step] = a;
+			}
+			__syncthreads();
+		}
+	}
+	for(int i = t; i < nset; i += 1024) share[i] = tables->share[key[i] & (PROJ_CELLS - 1)];
+	__syncthreads();
+	if(t < 32) {
+		const double c = ordered_sum(share, nset, t);
+		if(t == 0) cov[blockIdx.x] = (float)(c < 0.0 ? 0.0 : (c > 1.0 ? 1.0 : c));
+	}
+}
+
 /* The reference traces one photon to its end with recursive calls, one map
  * after the other.  Here the photons of both maps advance together, one
  * surface interaction per pass, over ray queues that the renderer's
@@ -686,8 +931,83 @@ static int split_photons(const Renderer &R, int light0, int nl, int num, std::ve
 	return prefix[p0 + nl];
 }
 
-/* Both photon maps of every job, traced as one wavefront on stream s: the
- * emission of all jobs' photons in one launch, then passes of closest hits
+/* every job's projection maps on stream s: bits (128 words per light of a
+ * job: 2048 cells of the map, then of the caustic map) in R.pw_bits, the two
+ * coverages in R.pw_cov */
+static int project_jobs(Renderer &R, const std::vector<PhotonJobSpec> &spec, cudaStream_t s)
+{
+	double tp = Renderer::host_now_ms();
+	std::vector<ProjSample> samples;
+	std::vector<ProjBox> boxes;
+	std::vector<Vec3> pts;
+	std::vector<int> times;
+	int slots = 0, most = 0;
+	for(const PhotonJobSpec &J : spec) {
+		/* the job's object boxes at its interval's ends */
+		const int ends[2] = {J.t0, J.t1};
+		size_t box0[2] = {boxes.size(), boxes.size()};
+		for(int e = 0; e < (J.t0 == J.t1 ? 1 : 2); e++) {
+			box0[e] = boxes.size();
+			for(int i = J.obj0; i < J.obj0 + J.nobj; i++) {
+				const Box b = R.sc.object_bounds((size_t)i, ends[e]);
+				const Material &m = R.sc.objs[i].mat >= 0 ? R.sc.mats[R.sc.objs[i].mat] : R.sc.defmat;
+				ProjBox d;
+				for(int k = 0; k < 3; k++) { d.mn[k] = b.mn[k]; d.mx[k] = b.mx[k]; }
+				d.caustic = m.refl > 0.0 || m.refr > 0.0 ? 1 : 0;
+				d.pad = 0;
+				boxes.push_back(d);
+			}
+		}
+		for(int k = 0; k < J.nlights; k++, slots++) {
+			if(J.nobj <= 0) continue;
+			pts.clear();
+			times.clear();
+			R.sc.light_samples((size_t)(J.light0 + k), J.t0, J.t1, R.opt.seed, k, pts, times);
+			for(size_t q = 0; q < pts.size(); q++) {
+				ProjSample d;
+				for(int c = 0; c < 3; c++) d.lp[c] = pts[q][c];
+				d.box0 = (int)box0[times[q] == J.t0 ? 0 : 1];
+				d.nbox = J.nobj;
+				d.slot = slots;
+				d.order = (unsigned)q;
+				samples.push_back(d);
+				most = std::max(most, J.nobj);
+			}
+		}
+	}
+	if(slots == 0) return 0;
+	if(!R.pj_tables_ready) {
+		PCK(R.pj_tables.ensure(sizeof(ProjTables)), "projection tables");
+		PCK(cudaMemcpyAsync(R.pj_tables.p, &proj_tables(), sizeof(ProjTables), cudaMemcpyHostToDevice, s), "projection tables");
+		R.h2d += (int64_t)sizeof(ProjTables);
+		R.pj_tables_ready = true;
+	}
+	PCK(R.pw_bits.ensure((size_t)slots * 128 * sizeof(uint32_t)), "projection maps");
+	PCK(R.pw_cov.ensure((size_t)slots * 2 * sizeof(float)), "coverage");
+	PCK(R.pj_first.ensure((size_t)slots * 2 * PROJ_SLOT * sizeof(unsigned long long)), "projection cells");
+	PCK(cudaMemsetAsync(R.pj_first.p, 0xff, (size_t)slots * 2 * PROJ_SLOT * sizeof(unsigned long long), s), "projection cells");
+	if(!samples.empty()) {
+		PCK(R.pj_samples.upload(samples, s), "light samples");
+		PCK(R.pj_boxes.upload(boxes, s), "object boxes");
+		R.h2d += (int64_t)(samples.size() * sizeof(ProjSample) + boxes.size() * sizeof(ProjBox));
+		PCK(R.pj_views.ensure(samples.size() * most * sizeof(ProjView)), "projections");
+		const int ns = (int)samples.size();
+		LAUNCH(R, "projmaps", s, k_proj_view<<<(unsigned)std::min<size_t>(((size_t)ns * most + 127) / 128, 1 << 20), 128, 0, s>>>(
+				R.pj_samples.as<ProjSample>(), ns, most, R.pj_boxes.as<ProjBox>(), R.pj_views.as<ProjView>(),
+				R.pj_first.as<unsigned long long>()));
+		LAUNCH(R, "projmaps", s, k_proj_mark<<<dim3((unsigned)most, (unsigned)std::min(ns, 65535)), 128, 0, s>>>(
+				R.pj_samples.as<ProjSample>(), ns, most, R.pj_boxes.as<ProjBox>(), R.pj_views.as<ProjView>(), R.pj_tables.as<ProjTables>(),
+				R.pj_first.as<unsigned long long>()));
+	}
+	LAUNCH(R, "projmaps", s, k_proj_cover<<<slots * 2, 1024, 0, s>>>(R.pj_first.as<unsigned long long>(), R.pj_tables.as<ProjTables>(),
+			R.pw_bits.as<uint32_t>(), R.pw_cov.as<float>()));
+	PCK(cudaGetLastError(), "projection maps");
+	R.host_time("host.projmaps", tp);
+	return 0;
+}
+
+/* Both photon maps of every job, traced as one wavefront on stream s: their
+ * projection maps, the emission of all jobs' photons in one launch, then passes of closest hits
  * and interactions over one queue (each photon finds its job, and through
  * it its scene, lights, interval and projection maps), then the tail.  The
  * stored photons and their flags stay in R.pw_out / R.pw_valid by global
@@ -699,9 +1019,9 @@ int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJ
 	out.assign(n, PJobOut());
 	std::vector<PJob> jobs(n);
 	std::vector<int> prefix;
-	std::vector<float> scale, cov;
-	std::vector<uint32_t> bits;
+	std::vector<float> scale;
 	std::vector<DevJob> pj(n);
+	int proj = 0;
 	int64_t all = 0;
 	for(int j = 0; j < n; j++) {
 		const PhotonJobSpec &J = spec[j];
@@ -712,16 +1032,11 @@ int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJ
 		d.nlights = J.nlights;
 		d.prefix0 = (int)prefix.size();
 		d.scale0 = (int)scale.size();
-		d.proj0 = (int)(cov.size() / 2);
+		d.proj0 = proj;
+		proj += J.nlights;
 		d.t0 = J.t0;
 		d.t1 = J.t1;
 		for(int m = 0; m < 2; m++) d.total[m] = split_photons(R, J.light0, J.nlights, J.num[m], prefix, scale);
-		if(J.nlights > 0) {
-			if(!J.bits || !J.cov || J.bits->size() < (size_t)J.nlights * 128 || J.cov->size() < (size_t)J.nlights * 2)
-				return R.fail(SRAY_ESTATE, "photon job without its projection maps");
-			bits.insert(bits.end(), J.bits->begin(), J.bits->begin() + (size_t)J.nlights * 128);
-			cov.insert(cov.end(), J.cov->begin(), J.cov->begin() + (size_t)J.nlights * 2);
-		}
 		memset(&pj[j], 0, sizeof pj[j]);
 		pj[j].pix0 = d.base;
 		pj[j].scene = J.scene;
@@ -732,14 +1047,12 @@ int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJ
 		if(all > INT_MAX / 2) return R.fail(SRAY_EINVAL, "too many photons in one wavefront");
 	}
 	if(all == 0) return 0;
+	if(int r = project_jobs(R, spec, s)) return r;
 	PCK(R.pw_jobs.upload(jobs, s), "photon jobs");
 	PCK(R.pw_prefix.upload(prefix, s), "photon prefix");
 	PCK(R.pw_scale.upload(scale, s), "photon scale");
-	PCK(R.pw_bits.upload(bits, s), "projection maps");
-	PCK(R.pw_cov.upload(cov, s), "coverage");
 	PCK(R.pw_pix.upload(pj, s), "photon job table");
-	R.h2d += (int64_t)(jobs.size() * sizeof(PJob) + prefix.size() * 4 + scale.size() * 4 + bits.size() * 4 + cov.size() * 4 +
-			pj.size() * sizeof(DevJob));
+	R.h2d += (int64_t)(jobs.size() * sizeof(PJob) + prefix.size() * 4 + scale.size() * 4 + pj.size() * sizeof(DevJob));
 	PCK(R.pw_out.ensure((size_t)all * sizeof(DevPhoton)), "photon buffer");
 	PCK(R.pw_valid.ensure((size_t)all * sizeof(int)), "photon flags");
 	PhotonSet PSet;
@@ -851,8 +1164,7 @@ int photon_finalize(Renderer &R, int global, const int *valid, const DevPhoton *
 
 /* both photon maps of the frame (one job): the wavefront, then each map from
  * its segment */
-int photon_shoot_maps(Renderer &R, const DScene &base, const std::vector<uint32_t> &bits, const std::vector<float> &cov,
-		cudaStream_t s, int *nc, int *ng)
+int photon_shoot_maps(Renderer &R, const DScene &base, cudaStream_t s, int *nc, int *ng)
 {
 	*nc = *ng = 0;
 	R.caust.map.n = 0;
@@ -866,8 +1178,7 @@ int photon_shoot_maps(Renderer &R, const DScene &base, const std::vector<uint32_
 	J.t0 = base.t0;
 	J.t1 = base.t1;
 	J.scene = -1;
-	J.bits = &bits;
-	J.cov = &cov;
+	J.nobj = (int)R.sc.objs.size();
 	std::vector<PJobOut> out;
 	int r = photon_trace_jobs(R, base, spec, out, s);
 	if(r) return r;

@@ -2638,60 +2638,6 @@ int Renderer::build_frame(long bt0, long bt1, cudaStream_t s)
 	return 0;
 }
 
-/* a light's projection maps as the photon kernels read them: 2048 cell bits
- * of the map, then of the caustic map; their coverages */
-static void pack_projmaps(const ProjMap &pm, const ProjMap &spm, uint32_t *bits, float *cov)
-{
-	for(int k = 0; k < 128; k++) bits[k] = 0u;
-	for(int k = 0; k < 2048; k++) {
-		if(pm.cells[k]) bits[k >> 5] |= 1u << (k & 31);
-		if(spm.cells[k]) bits[64 + (k >> 5)] |= 1u << (k & 31);
-	}
-	cov[0] = (float)pm.get_coverage();
-	cov[1] = (float)spm.get_coverage();
-}
-
-/* every job's projection maps of a batch, on all host cores: each light of a
- * job is one task (its own random stream, its own output) */
-void Renderer::batch_projmaps(std::vector<std::vector<uint32_t>> &bits, std::vector<std::vector<float>> &cov)
-{
-	size_t n = batch_t0.size();
-	bits.assign(n, std::vector<uint32_t>());
-	cov.assign(n, std::vector<float>());
-	struct Task { size_t job; int light; };
-	std::vector<Task> tasks;
-	std::vector<int> l0(n, 0), o0(n, 0), no(n, (int)sc.objs.size());
-	for(size_t j = 0; j < n; j++) {
-		int nl = (int)sc.lights.size();
-		if(!scene_refs.empty()) {
-			const SceneRange &rg = sc.ranges[batch_scene[j]];
-			l0[j] = rg.light0;
-			nl = rg.nlight;
-			o0[j] = rg.obj0;
-			no[j] = rg.nobj;
-		}
-		bits[j].assign((size_t)nl * 128, 0u);
-		cov[j].assign((size_t)nl * 2, 0.0f);
-		for(int k = 0; k < nl; k++) tasks.push_back(Task{j, k});
-	}
-	std::atomic<size_t> next{0};
-	auto work = [&]() {
-		for(size_t i; (i = next.fetch_add(1)) < tasks.size();) {
-			const Task &T = tasks[i];
-			ProjMap pm, spm;
-			sc.light_projmaps((size_t)(l0[T.job] + T.light), (int)batch_t0[T.job], (int)batch_t1[T.job], opt.seed, T.light, o0[T.job],
-					no[T.job], pm, spm);
-			pack_projmaps(pm, spm, &bits[T.job][(size_t)T.light * 128], &cov[T.job][(size_t)T.light * 2]);
-		}
-	};
-	unsigned hw = std::thread::hardware_concurrency();
-	size_t nth = std::min<size_t>(tasks.size(), hw ? hw : 4);
-	std::vector<std::thread> th;
-	for(size_t t = 1; t < nth; t++) th.push_back(std::thread(work));
-	work();
-	for(auto &t : th) t.join();
-}
-
 /* projection maps and both photon maps on stream s, with the scene view
  * `base` (the projection-map tables are set in a copy of it); the map
  * descriptors land in caust.map / gi.map, which fill_scene_desc() copies
@@ -2701,16 +2647,8 @@ int Renderer::shoot_maps(const DScene &base, cudaStream_t s, int *nc, int *ng)
 	caust.map.n = 0;
 	gi.map.n = 0;
 	*nc = *ng = 0;
-	int nl = (int)sc.lights.size();
-	if(!(opt.caust_photons || opt.gi_photons) || nl == 0) return 0;
-	/* projection maps (src/render.cc:87-103) over the photons' interval */
-	double tp = host_now_ms();
-	sc.build_projmaps(base.t0, base.t1, opt.seed);
-	std::vector<uint32_t> bits((size_t)nl * 128, 0u);
-	std::vector<float> cov((size_t)nl * 2, 0.0f);
-	for(size_t i = 0; i < (size_t)nl; i++) pack_projmaps(sc.lights[i].pm, sc.lights[i].spm, &bits[i * 128], &cov[i * 2]);
-	host_time("host.projmaps", tp);
-	return photon_shoot_maps(*this, base, bits, cov, s, nc, ng);
+	if(!(opt.caust_photons || opt.gi_photons) || sc.lights.empty()) return 0;
+	return photon_shoot_maps(*this, base, s, nc, ng);
 }
 
 int Renderer::photon_job(DScene base)
@@ -2722,11 +2660,6 @@ int Renderer::photon_job(DScene base)
 	 * each map from its segment, and their table */
 	size_t n = batch_t0.size();
 	std::vector<DPhotonMap> hm(2 * n);
-	std::vector<std::vector<uint32_t>> jbits;
-	std::vector<std::vector<float>> jcov;
-	double tp = host_now_ms();
-	batch_projmaps(jbits, jcov);
-	host_time("host.projmaps", tp);
 	std::vector<PhotonJobSpec> spec(n);
 	std::vector<int> o0(n, 0), no(n, (int)sc.objs.size());
 	for(size_t j = 0; j < n; j++) {
@@ -2745,8 +2678,8 @@ int Renderer::photon_job(DScene base)
 		J.num[1] = batch_gi[j] > 0 ? batch_gi[j] : opt.gi_photons;
 		J.t0 = (int)batch_t0[j];
 		J.t1 = (int)batch_t1[j];
-		J.bits = &jbits[j];
-		J.cov = &jcov[j];
+		J.obj0 = o0[j];
+		J.nobj = no[j];
 	}
 	/* the grids of the jobs' own frames: boxes and range radii over their
 	 * own intervals (the batch's tree spans every job's interval) */
@@ -4737,7 +4670,7 @@ void sray_gpu_shutdown(void)
 		&R.xf, &R.light_pos, &R.cam_m, &R.qbuf[0], &R.qbuf[1], &R.hits, &R.gq, &R.sq, &R.acc, &R.hist, &R.sums,
 		&R.active[0], &R.active[1], &R.spp, &R.fbdev, &R.ctr, &R.counts, &R.bnodes, &R.btris, &R.bprim, &R.bhome,
 		&R.fbl, &R.tnodes, &R.ohome, &R.pool_ready, &R.pqbuf[0], &R.pqbuf[1], &R.phits, &R.pfbl, &R.pcounts, &R.pctr,
-		&R.pw_jobs, &R.pw_prefix, &R.pw_scale, &R.pw_bits, &R.pw_cov, &R.pw_pix, &R.pw_out, &R.pw_valid,
+		&R.pw_jobs, &R.pw_prefix, &R.pw_scale, &R.pw_bits, &R.pw_cov, &R.pj_tables, &R.pj_samples, &R.pj_boxes, &R.pj_views, &R.pj_first, &R.pw_pix, &R.pw_out, &R.pw_valid,
 		&R.pw_part, &R.pw_tiles, &R.pw_bounds, &R.pw_offs, &R.pw_ph, &R.pw_sorted, &R.pw_grids, &R.pw_cellbase,
 		&R.pw_keys, &R.pw_lin, &R.pw_starts, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1],
 		&R.pqsbuf, &R.ps_keys, &R.ps_hist, &R.ps_part,

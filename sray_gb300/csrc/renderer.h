@@ -232,11 +232,14 @@ struct Renderer {
 	double map_gather_dist = -1.0;         /* >= 0: the range radius of the maps being built (a batch job's) */
 	bool map_has_box = false;              /* the grid box of the maps being built (a batch job's scene */
 	Box map_box;                           /* over its own interval), else the frame octree's root box */
-	void batch_projmaps(std::vector<std::vector<uint32_t>> &bits, std::vector<std::vector<float>> &cov);
 	/* the photon wavefront's tables (photon.cu): jobs, per-light prefix sums
 	 * and scales, projection maps and coverages, the photons' job table for
 	 * the traversal, stored photons and their flags by global index */
 	DevBuf pw_jobs, pw_prefix, pw_scale, pw_bits, pw_cov, pw_pix, pw_out, pw_valid;
+	/* the projection maps' making: geometry tables (once), light samples,
+	 * object boxes, the first projection that covers each cell */
+	DevBuf pj_tables, pj_samples, pj_boxes, pj_views, pj_first;
+	bool pj_tables_ready = false;
 	/* a batch's maps built together (photon_finalize_jobs): scan scratch,
 	 * segment bounds and offsets, compacted and sorted photons, grids, keys,
 	 * cell tables */
@@ -333,8 +336,7 @@ struct PhotonJobSpec {
 	int light0 = 0, nlights = 0;  /* its scene's lights */
 	int t0 = 0, t1 = 0;           /* its interval */
 	int scene = -1;               /* its scene in a scene set (-1: the view's own) */
-	const std::vector<uint32_t> *bits = nullptr;   /* its projection maps, 128 words per light */
-	const std::vector<float> *cov = nullptr;       /* their coverages, 2 per light */
+	int obj0 = 0, nobj = 0;       /* its scene's objects */
 };
 struct PJobOut { int base = 0; int total[2] = {0, 0}; };   /* a job's photons: first global index, counts per map */
 int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJobSpec> &spec, std::vector<PJobOut> &out,
@@ -344,8 +346,7 @@ int sort_pairs(Renderer &R, unsigned *keys, unsigned *vals, unsigned *keys2, uns
 		DevBuf &part, const char *name, cudaStream_t s, unsigned **keys_out, unsigned **vals_out);
 int photon_finalize_jobs(Renderer &R, const std::vector<PJobOut> &jobs, const std::vector<Box> &boxes,
 		const std::vector<double> &gather_dist, std::vector<DPhotonMap> &maps, cudaStream_t s);
-int photon_shoot_maps(Renderer &R, const DScene &base, const std::vector<uint32_t> &bits, const std::vector<float> &cov,
-		cudaStream_t s, int *caust_stored, int *gi_stored);
+int photon_shoot_maps(Renderer &R, const DScene &base, cudaStream_t s, int *caust_stored, int *gi_stored);
 /* photon.cu: map `global` (0 caustic, 1 global) over the n photons in its buffer / from host photons */
 int photon_map_build(Renderer &R, int global, int n, cudaStream_t s);
 int photon_map_read(Renderer &R, int global, std::vector<DevPhoton> &h, cudaStream_t s);

@@ -678,227 +678,75 @@ void octree_homes(const BuildOctree &oct, const std::vector<double> &posd, const
 /* ------------------------------------------------------------------ */
 /* projection maps                                                       */
 /* ------------------------------------------------------------------ */
-ProjMap::ProjMap()
+/* a cell corner's direction: ProjMap::cell_corner_dir (src/projmap.cc:124-140) */
+static void corner_dir(int uc, int vc, double out[3])
 {
-	cells.assign(udiv * vdiv, 0);
-	cell_area.resize(udiv * vdiv);
-	total_area = 0.0;
-	for(int i = 0; i < udiv * vdiv; i++) {
-		int uc = i % udiv, vc = i / udiv;
-		double c[4][3];
-		for(int j = 0; j < 4; j++) corner_dir(uc, vc, j, c[j]);
-		Vec3 v0(c[0][0], c[0][1], c[0][2]), v1(c[1][0], c[1][1], c[1][2]);
-		Vec3 v2(c[2][0], c[2][1], c[2][2]), v3(c[3][0], c[3][1], c[3][2]);
-		Vec3 e1(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z), e2(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z);
-		Vec3 e3(v3.x - v0.x, v3.y - v0.y, v3.z - v0.z);
-		double area = v_len(v_cross(e1, e2)) * 0.5;
-		area += v_len(v_cross(e2, e3)) * 0.5;
-		cell_area[i] = area;
-		total_area += area;
-	}
-}
-
-/* ProjMap::cell_corner_dir (src/projmap.cc:124-140); the 64x32 grid's corner
- * directions are computed once and reused (same values every call) */
-static void corner_dir_eval(int udiv, int vdiv, int uc, int vc, int corner, double out[3])
-{
-	static const int offs[4][2] = {{0, 0}, {1, 0}, {1, 1}, {0, 1}};
-	double du = 1.0 / udiv, dv = 1.0 / vdiv;
-	double u = (uc + offs[corner][0]) * du, v = (vc + offs[corner][1]) * dv;
+	double du = 1.0 / 64, dv = 1.0 / 32;
+	double u = uc * du, v = vc * dv;
 	double theta = u * M_PI * 2.0, phi = v * M_PI;
 	out[0] = 1.0 * cos(theta) * sin(phi);
 	out[1] = 1.0 * cos(phi);
 	out[2] = 1.0 * sin(theta) * sin(phi);
 }
 
-struct CornerTable {
-	double d[64 * 32][4][3];
-	CornerTable()
-	{
-		for(int i = 0; i < 64 * 32; i++)
-			for(int k = 0; k < 4; k++) corner_dir_eval(64, 32, i % 64, i / 64, k, d[i][k]);
-	}
-};
-
-static const CornerTable &corner_table()
+const ProjTables &proj_tables()
 {
-	static const CornerTable *t = new CornerTable();
-	return *t;
-}
-
-void ProjMap::corner_dir(int uc, int vc, int corner, double out[3]) const
-{
-	if(udiv == 64 && vdiv == 32) {
-		const double *c = corner_table().d[vc * 64 + uc][corner];
-		out[0] = c[0]; out[1] = c[1]; out[2] = c[2];
-		return;
-	}
-	corner_dir_eval(udiv, vdiv, uc, vc, corner, out);
-}
-
-void ProjMap::cell_from_dir(const double d[3], int *uc, int *vc) const
-{
-	double r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-	double theta = atan2(d[2], d[0]);
-	double phi = acos(d[1] / r);
-	if(theta < 0.0) theta = M_PI * 2.0 + theta;
-	double u = theta / (M_PI * 2.0), v = phi / M_PI;
-	int a = (int)(u * udiv), b = (int)(v * vdiv);
-	*uc = a < 0 ? 0 : (a >= udiv ? udiv - 1 : a);
-	*vc = b < 0 ? 0 : (b >= vdiv ? vdiv - 1 : b);
-}
-
-void ProjMap::set_cell(int uc, int vc, bool val)
-{
-	int idx = vc * udiv + uc;
-	if((bool)cells[idx] != val) {
-		double change = cell_area[idx] / total_area;
-		coverage += val ? change : -change;
-	}
-	cells[idx] = val;
-}
-
-void ProjMap::set_all(bool v) { std::fill(cells.begin(), cells.end(), v ? 1 : 0); coverage = v ? 1.0 : 0.0; }
-void ProjMap::clear() { set_all(false); }
-double ProjMap::get_coverage() const { return coverage < 0.0 ? 0.0 : (coverage > 1.0 ? 1.0 : coverage); }
-
-/* Candidate columns/rows of the 64x32 grid for one box: every cell with a
- * corner inside the box's bounding sphere (seen from the light) lies in the
- * spherical cap of angular radius t around the sphere's direction, since the
- * corner test |lpos + c d - ctr|^2 <= r^2 with |c| = 1, d = |ctr - lpos| is
- * c . v^ >= 1 - r^2 / (2 d^2).  The cap is bounded in colatitude by t and in
- * azimuth by asin(sin t / sin phi); one cell and 0.02 rad of margin are added,
- * and the exact corner test of the reference decides inside the candidates. */
-static bool cap_candidates(const double v[3], double objdist, double rad_sq, int *vc0, int *vc1, bool cols[64])
-{
-	double cos_t = 1.0 - rad_sq / (2.0 * objdist * objdist);
-	if(cos_t <= -1.0 + 1e-9) return false;
-	double t = acos(cos_t < 1.0 ? cos_t : 1.0) + 0.02;
-	double phi0 = acos(v[1] / objdist);
-	double theta0 = atan2(v[2], v[0]);
-	if(theta0 < 0.0) theta0 += 2.0 * M_PI;
-	double dv = M_PI / 32.0, du = 2.0 * M_PI / 64.0;
-	double plo = phi0 - t, phi_hi = phi0 + t;
-	int a = (int)floor(plo / dv) - 1, b = (int)floor(phi_hi / dv) + 1;
-	*vc0 = a < 0 ? 0 : a;
-	*vc1 = b > 31 ? 31 : b;
-	if(plo <= 0.0 || phi_hi >= M_PI) {
-		for(int k = 0; k < 64; k++) cols[k] = true;
-		return true;
-	}
-	double smin = sin(plo) < sin(phi_hi) ? sin(plo) : sin(phi_hi);
-	double st = sin(t);
-	if(st >= smin) {
-		for(int k = 0; k < 64; k++) cols[k] = true;
-		return true;
-	}
-	double dmax = asin(st / smin) + 0.02;
-	for(int k = 0; k < 64; k++) cols[k] = false;
-	int u0 = (int)floor((theta0 - dmax) / du) - 1, u1 = (int)floor((theta0 + dmax) / du) + 1;
-	if(u1 - u0 >= 63) {
-		for(int k = 0; k < 64; k++) cols[k] = true;
-		return true;
-	}
-	for(int u = u0; u <= u1; u++) cols[((u % 64) + 64) % 64] = true;
-	return true;
-}
-
-/* ::build_projmap (src/light.cc:392-432) */
-static void project_boxes(ProjMap *map, const Vec3 &lpos, const std::vector<Box> &boxes)
-{
-	for(size_t i = 0; i < boxes.size(); i++) {
-		const Box &b = boxes[i];
-		if(lpos.x >= b.mn[0] && lpos.y >= b.mn[1] && lpos.z >= b.mn[2] && lpos.x < b.mx[0] && lpos.y < b.mx[1] && lpos.z < b.mx[2]) {
-			map->set_all(true);
-			return;
-		}
-		Vec3 ctr((b.mn[0] + b.mx[0]) / 2.0, (b.mn[1] + b.mx[1]) / 2.0, (b.mn[2] + b.mx[2]) / 2.0);
-		Vec3 dm(b.mn[0] - ctr.x, b.mn[1] - ctr.y, b.mn[2] - ctr.z);
-		double rad_sq = dm.x * dm.x + dm.y * dm.y + dm.z * dm.z;
-		double v[3] = {ctr.x - lpos.x, ctr.y - lpos.y, ctr.z - lpos.z};
-		double objdist = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-		int uc, vc;
-		map->cell_from_dir(v, &uc, &vc);
-		map->set_cell(uc, vc, true);
-		int vc0 = 0, vc1 = map->vdiv - 1;
-		bool cols[64];
-		bool limited = map->udiv == 64 && map->vdiv == 32 && objdist > 0.0 && cap_candidates(v, objdist, rad_sq, &vc0, &vc1, cols);
-		for(int row = vc0; row <= vc1; row++) {
-			for(int col = 0; col < map->udiv; col++) {
-				if(limited && !cols[col]) continue;
-				for(int k = 0; k < 4; k++) {
-					double cd[3];
-					map->corner_dir(col, row, k, cd);
-					double px = lpos.x + cd[0] * objdist, py = lpos.y + cd[1] * objdist, pz = lpos.z + cd[2] * objdist;
-					double dx = px - ctr.x, dy = py - ctr.y, dz = pz - ctr.z;
-					if(dx * dx + dy * dy + dz * dz <= rad_sq) {
-						map->set_cell(col, row, true);
-						break;
-					}
-				}
+	static const ProjTables *tables = []() {
+		ProjTables *t = new ProjTables();
+		for(int r = 0; r < 33; r++) {
+			for(int c = 0; c < 65; c++) {
+				const int i = r * 65 + c;
+				corner_dir(c, r, t->corner[i]);
+				for(int k = 0; k < 4; k++) t->cornerf[i][k] = k < 3 ? (float)t->corner[i][k] : 0.0f;
 			}
 		}
-	}
+		double total = 0.0;
+		for(int i = 0; i < 64 * 32; i++) {
+			int uc = i % 64, vc = i / 64;
+			const int at[4] = {vc * 65 + uc, vc * 65 + uc + 1, (vc + 1) * 65 + uc + 1, (vc + 1) * 65 + uc};
+			Vec3 v[4];
+			for(int j = 0; j < 4; j++) v[j] = Vec3(t->corner[at[j]][0], t->corner[at[j]][1], t->corner[at[j]][2]);
+			Vec3 e1(v[1].x - v[0].x, v[1].y - v[0].y, v[1].z - v[0].z), e2(v[2].x - v[0].x, v[2].y - v[0].y, v[2].z - v[0].z);
+			Vec3 e3(v[3].x - v[0].x, v[3].y - v[0].y, v[3].z - v[0].z);
+			double area = v_len(v_cross(e1, e2)) * 0.5;
+			area += v_len(v_cross(e2, e3)) * 0.5;
+			t->share[i] = area;
+			total += area;
+		}
+		for(int i = 0; i < 64 * 32; i++) t->share[i] = t->share[i] / total;
+		return t;
+	}();
+	return *tables;
 }
 
-/* Light::build_proj_intern (src/light.cc:151-200); light samples on the
- * projection-map stream of the light */
-void HostScene::build_projmaps(int t0, int t1, uint64_t seed, int light0, int nlight, int obj0, int nobj)
+void HostScene::light_samples(size_t li, int t0, int t1, uint64_t seed, int key, std::vector<Vec3> &pts, std::vector<int> &times) const
 {
-	if(nlight < 0) nlight = (int)lights.size() - light0;
-	if(nobj < 0) nobj = (int)objs.size() - obj0;
-	/* each light's maps depend only on its own random stream: one thread per light */
-	std::vector<std::thread> th;
-	for(int k = 0; k < nlight; k++)
-		th.push_back(std::thread([this, light0, k, t0, t1, seed, obj0, nobj]() { build_light_projmaps(light0 + k, t0, t1, seed, k, obj0, nobj); }));
-	for(auto &t : th) t.join();
-}
-
-void HostScene::build_light_projmaps(size_t li, int t0, int t1, uint64_t seed, int key, int obj0, int nobj)
-{
-	light_projmaps(li, t0, t1, seed, key, obj0, nobj, lights[li].pm, lights[li].spm);
-}
-
-void HostScene::light_projmaps(size_t li, int t0, int t1, uint64_t seed, int key, int obj0, int nobj, ProjMap &pm, ProjMap &spm) const
-{
-	{
-		const Light &L = lights[li];
-		pm.clear();
-		spm.clear();
-		if(nobj <= 0) return;
-		int tm[3] = {t0, t1, -1};
-		if(t0 == t1) tm[1] = -1;
-		int samples = L.type == LT_SPHERE ? 8 : 1;
-		/* one stream per light, drawn in order over both shutter ends */
-		sray_rng s;
-		sray_rng_init(&s, seed, SRAY_DOM_PROJMAP, (uint32_t)key, 0);
-		for(int ti = 0; ti < 2 && tm[ti] != -1; ti++) {
-			std::vector<Box> boxes((size_t)nobj), cboxes;
-			for(int j = 0; j < nobj; j++) {
-				size_t i = (size_t)(obj0 + j);
-				const Material &m = objs[i].mat >= 0 ? mats[objs[i].mat] : defmat;
-				boxes[j] = object_bounds(i, tm[ti]);
-				if(m.refl > 0.0 || m.refr > 0.0) cboxes.push_back(boxes[j]);
+	const Light &L = lights[li];
+	int tm[3] = {t0, t1, -1};
+	if(t0 == t1) tm[1] = -1;
+	int samples = L.type == LT_SPHERE ? 8 : 1;
+	/* one stream per light, drawn in order over both shutter ends */
+	sray_rng s;
+	sray_rng_init(&s, seed, SRAY_DOM_PROJMAP, (uint32_t)key, 0);
+	for(int ti = 0; ti < 2 && tm[ti] != -1; ti++) {
+		for(int k = 0; k < samples; k++) {
+			Vec3 lp = L.xf.position(tm[ti]);
+			if(L.type == LT_SPHERE) {
+				double u0 = sray_rng_uniform_d(&s), u1 = sray_rng_uniform_d(&s);
+				double z = 2.0 * u1 - 1.0, sxy = sqrt(1.0 - z * z), ang = 2.0 * M_PI * u0;
+				double r = (double)L.radius;
+				lp = Vec3(lp.x + r * cos(ang) * sxy, lp.y + r * sin(ang) * sxy, lp.z + r * z);
+			} else if(L.type == LT_BOX) {
+				double m0[4][4];
+				L.xf.matrix(0, m0);
+				Vec3 v;
+				v.x = L.dim.x * sray_rng_uniform_d(&s) - 0.5 * L.dim.x;
+				v.y = L.dim.y * sray_rng_uniform_d(&s) - 0.5 * L.dim.y;
+				v.z = L.dim.z * sray_rng_uniform_d(&s) - 0.5 * L.dim.z;
+				lp = m_pt(m0, v);
 			}
-			for(int k = 0; k < samples; k++) {
-				Vec3 lp = L.xf.position(tm[ti]);
-				if(L.type == LT_SPHERE) {
-					double u0 = sray_rng_uniform_d(&s), u1 = sray_rng_uniform_d(&s);
-					double z = 2.0 * u1 - 1.0, sxy = sqrt(1.0 - z * z), ang = 2.0 * M_PI * u0;
-					double r = (double)L.radius;
-					lp = Vec3(lp.x + r * cos(ang) * sxy, lp.y + r * sin(ang) * sxy, lp.z + r * z);
-				} else if(L.type == LT_BOX) {
-					double m0[4][4];
-					L.xf.matrix(0, m0);
-					Vec3 v;
-					v.x = L.dim.x * sray_rng_uniform_d(&s) - 0.5 * L.dim.x;
-					v.y = L.dim.y * sray_rng_uniform_d(&s) - 0.5 * L.dim.y;
-					v.z = L.dim.z * sray_rng_uniform_d(&s) - 0.5 * L.dim.z;
-					lp = m_pt(m0, v);
-				}
-				project_boxes(&pm, lp, boxes);
-				project_boxes(&spm, lp, cboxes);
-			}
+			pts.push_back(lp);
+			times.push_back(tm[ti]);
 		}
 	}
 }

@@ -11,6 +11,7 @@
 #define SRAY_SCENE_HOST_H_
 
 #include <stdint.h>
+#include <stddef.h>
 #include <string>
 #include <vector>
 #include "sray_gpu.h"
@@ -125,19 +126,16 @@ struct Object {
 	Box reach(const Box &vertices, int t) const;
 };
 
-struct ProjMap {
-	int udiv = 64, vdiv = 32;
-	std::vector<char> cells;
-	std::vector<double> cell_area;
-	double total_area = 0.0, coverage = 0.0;
-	ProjMap();
-	void corner_dir(int uc, int vc, int corner, double out[3]) const;
-	void cell_from_dir(const double d[3], int *uc, int *vc) const;
-	void set_cell(int uc, int vc, bool v);
-	void set_all(bool v);
-	void clear();
-	double get_coverage() const;
+/* The 64 x 32 projection maps' geometry (src/projmap.cc:60-140), the same
+ * for every map: the directions of the 65 x 33 cell corners (and
+ * the same in float), and each cell's share of the sphere. */
+struct ProjTables {
+	alignas(16) float cornerf[33 * 65][4];   /* read as float4 */
+	double corner[33 * 65][3];
+	double share[64 * 32];
 };
+static_assert(offsetof(ProjTables, cornerf) % 16 == 0 && sizeof(float[4]) == 16, "float4 reads of the corners");
+const ProjTables &proj_tables();
 
 struct Light {
 	int type = LT_POINT;
@@ -145,7 +143,6 @@ struct Light {
 	XForm xf;
 	float radius = 1.0f;
 	Vec3 dim = Vec3(1, 1, 1);
-	ProjMap pm, spm;
 };
 
 struct Camera {
@@ -213,13 +210,11 @@ struct HostScene {
 	 * objects obj0 .. obj0 + nobj, without building */
 	Box box_at(int t0, int t1, int obj0 = 0, int nobj = -1) const;
 	double gather_dist_at(int t0, int t1, const sray_opts &opt, int obj0 = 0, int nobj = -1) const;
-	/* the projection maps of lights [light0, light0 + nlight) over objects
-	 * [obj0, obj0 + nobj) (all by default); a light's stream is keyed by its
-	 * index within that range */
-	void build_projmaps(int t0, int t1, uint64_t seed, int light0 = 0, int nlight = -1, int obj0 = 0, int nobj = -1);
-	void build_light_projmaps(size_t li, int t0, int t1, uint64_t seed, int key, int obj0, int nobj);
-	/* the same maps of light li into pm / spm (the light's own are untouched) */
-	void light_projmaps(size_t li, int t0, int t1, uint64_t seed, int key, int obj0, int nobj, ProjMap &pm, ProjMap &spm) const;
+	/* the points of light li from which its projection maps see the objects:
+	 * Light::build_proj_intern's samples (src/light.cc:151-200) at time t0 and,
+	 * where it differs, t1, drawn from the stream of the light's key; their
+	 * times beside them */
+	void light_samples(size_t li, int t0, int t1, uint64_t seed, int key, std::vector<Vec3> &pts, std::vector<int> &times) const;
 };
 
 /* general 4x4 inverse by the adjugate */
