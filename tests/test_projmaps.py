@@ -69,3 +69,23 @@ def test_photons_of_projection_maps(gpu_lib, oracle_lib, name):
         stored += len(a)
     g.close()
     assert stored > 0
+
+
+@pytest.mark.parametrize("n", [1, 31, 5000, 20001, 60000, 320000])
+def test_emission_by_count(gpu_lib, oracle_lib, n):
+    """The emission gives a photon a lane of its own, or several, by the number
+    of photons (2 to 32 photons per warp): the same photons at every count."""
+    objects, lights, moving = _cases()["many"]
+    xml = _scene(objects, lights, moving)
+    opts = dict(width=32, height=32, caust_photons=n, gi_photons=max(1, n // 4), caust_k=8, gi_k=8, iter=4)
+    g = gpu_lib.GpuRenderer(**opts)
+    g.load_xml(xml)
+    o = oracle_lib.Oracle(fp64=False, rng_mode=1, **opts)
+    o.load_xml(xml)
+    o.prepare(0)
+    g.shoot_photons(0, 0)
+    for which in (0, 1):
+        a, b = g.photons(which)[:, :12], o.photons(which)[:, :12]
+        assert len(a) == len(b)
+        assert np.array_equal(a[np.lexsort(a.T[::-1])], b[np.lexsort(b.T[::-1])])
+    g.close()
