@@ -276,19 +276,12 @@ int sray_gpu_photon_gather(int which, int n, const float *pos, const float *norm
  * device memory while they run: an application that hands all device memory
  * to its own pooling allocator (a cudaMalloc from inside the frame can fail
  * or fragment that pool), or an interactive loop that cannot afford the
- * device-wide synchronisation a cudaMalloc or cudaFree implies.  The request
- * staging that sray_gpu_photon_gather allocates lives instead in a fixed
- * array compiled into the library: SRAY_NOALLOC_MAX_POINTS requests (3 MiB,
- * held on every GPU that loads the library until the process exits).
+ * device-wide synchronisation a cudaMalloc or cudaFree implies.  It reads the
+ * caller's arrays and writes its output in one launch and holds no memory of
+ * its own.
  *  - n > SRAY_NOALLOC_MAX_POINTS is rejected with SRAY_EINVAL.
- *  - The first call on a device looks up the array's device address on that
- *    device (the renderer's, which must be current).  No call may be made
- *    while a stream is being captured into a graph: every call waits for its
- *    stream (below).
- *  - All calls share the one array and it keeps the previous call's
- *    requests; each call writes all the requests it reads, so nothing needs
- *    clearing, but calls that overlap on the GPU (several host threads or
- *    streams at once) race on it.
+ *  - No call may be made while a stream is being captured into a graph: every
+ *    call waits for its stream (below).
  * Arguments, results and errors are those of sray_gpu_photon_gather.  Like
  * it, the call waits for `stream` to finish its work (cudaStreamSynchronize)
  * before it returns, so `out` is written on return. */

@@ -1659,6 +1659,69 @@ __device__ __noinline__ unsigned gather_unlisted(const DPhotonMap &M, const Gath
 	return __reduce_max_sync(FULL, kmax);
 }
 
+/* The map a request's kind names: the frame's caustic (0) or global (1) map,
+ * in a batch its job's */
+__device__ __forceinline__ const DPhotonMap &gather_map(const DScene &S, int kind)
+{
+	return S.maps ? S.maps[kind] : (kind == 0 ? S.caust : S.gi);
+}
+
+/* Estimate of one query by one thread, for queries that see few photons: at
+ * most GATHER_FEW in at most FEW_RUNS runs of the rows their sphere reaches,
+ * and no more than k, so that all those in range count.  Returns false
+ * (nothing computed) where there are more.  runs: the thread's column of
+ * FEW_RUNS (first, end) pairs in shared memory, `stride` apart. */
+#define GATHER_FEW 64
+#define FEW_RUNS 20
+__device__ __forceinline__ bool gather_few(const DScene &S, int kind, V3 pos, V3 n, uint2 *runs, int stride, float (&est)[3],
+		int &tested, int &cnt)
+{
+	const DPhotonMap &M = gather_map(S, kind);
+	kind &= 1;
+	est[0] = est[1] = est[2] = 0.0f;
+	tested = cnt = 0;
+	if(M.n == 0) return true;
+	const unsigned most = M.k > 0 && M.k < GATHER_FEW ? (unsigned)M.k : (unsigned)GATHER_FEW;
+	GatherCells gc;
+	gather_cells(M, pos, gc);
+	unsigned seen = 0;
+	int nrun = 0;
+	for(int r = 0; r < gc.nrow; r++) {
+		const uint2 run = gather_row(M, gc, r);
+		if(run.x == run.y) continue;
+		seen += run.y - run.x;
+		if(seen > most || nrun == FEW_RUNS) return false;
+		runs[nrun++ * stride] = run;
+	}
+	tested = (int)seen;
+	const float thr = M.screen, sure = gather_below(M.r2_hi);
+	float sum[3] = {0.0f, 0.0f, 0.0f}, far = 0.0f;
+	unsigned kth = 0, j = 0, end = 0;
+	for(int i = 0; seen > 0; seen--, j++) {
+		if(j == end) {
+			j = runs[i * stride].x;
+			end = runs[i++ * stride].y;
+		}
+		float4 p = __ldg(reinterpret_cast<const float4 *>(M.ph + j));
+		float dx = p.x - pos.x, dy = p.y - pos.y, dz = p.z - pos.z;
+		float d = dx * dx + dy * dy + dz * dz;
+		if(!(d <= thr)) continue;
+		if(!(d < sure) || (M.k > 0 && d >= gather_below(far))) {
+			/* near the range, or perhaps the farthest so far: the exact key */
+			unsigned key;
+			if(!gather_exact(M, p, pos, key)) continue;
+			kth = key > kth ? key : kth;
+			far = fmaxf(far, d);
+		}
+		cnt++;
+		photon_term(M, (int)j, p, kind, n, S.max_cos, sum);
+	}
+	if(cnt < (kind == 0 ? 8 : 1)) return true;
+	const float inv_area = M.k > 0 ? 1.0f / (3.14159265358979323846f * __uint_as_float(kth)) : M.inv_area;
+	for(int c = 0; c < 3; c++) est[c] = sum[c] * inv_area;
+	return true;
+}
+
 /* Estimate of one query by one full warp: the sums over the photons in
  * range, or over the k nearest of them, times the reciprocal of their disc's
  * area.  Component 0 returns in lane 0, component 1 in lane 16, component 2
@@ -1676,8 +1739,7 @@ __device__ __noinline__ unsigned gather_unlisted(const DPhotonMap &M, const Gath
 __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V3 n, GatherMem &gm, GatherWork &gw)
 {
 	const unsigned FULL = 0xffffffffu;
-	/* in a batch the request's kind is the index of its job's map */
-	const DPhotonMap &M = S.maps ? S.maps[kind] : (kind == 0 ? S.caust : S.gi);
+	const DPhotonMap &M = gather_map(S, kind);
 	kind &= 1;
 	const int lane = threadIdx.x & 31;
 	const unsigned lt_mask = (1u << lane) - 1u;
@@ -1840,60 +1902,116 @@ __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V
 /* the component of an estimate that a lane holds (lanes 0, 16, 8), -1 in the others */
 __device__ __forceinline__ int gather_comp(int lane) { return (lane & 7) || lane == 24 ? -1 : (lane == 16 ? 1 : lane >> 2); }
 
-__global__ void __launch_bounds__(GATHER_WARPS * 32, 4) k_gather(DScene S, const GatherReq *gq, const int *gq_count,
-		float4 *acc, DevCounters *ctr)
+/* a frame's queries: requests, their estimates weighted into accumulators */
+struct FrameQueries {
+	const GatherReq *gq;
+	float4 *acc;
+	__device__ __forceinline__ void get(int i, int &kind, V3 &pos, V3 &n) const
+	{
+		float4 a = gq[i].a, b = gq[i].b;
+		kind = __float_as_int(a.w);
+		pos = mk(a.x, a.y, a.z);
+		n = mk(b.x, b.y, b.z);
+	}
+	__device__ __forceinline__ void put(int i, const float (&est)[3]) const
+	{
+		float4 w = gq[i].w;
+		float c[3] = {w.x * est[0], w.y * est[1], w.z * est[2]};
+		/* (not so where the weight makes it no number) */
+		if(c[0] == 0.0f && c[1] == 0.0f && c[2] == 0.0f) return;
+		acc_add(acc, __float_as_int(gq[i].b.w), c[0], c[1], c[2]);
+	}
+	__device__ __forceinline__ void put(int i, int comp, float est) const
+	{
+		float4 w = gq[i].w;
+		atomicAdd(reinterpret_cast<float *>(acc + __float_as_int(gq[i].b.w)) + comp, (comp == 0 ? w.x : (comp == 1 ? w.y : w.z)) * est);
+	}
+};
+
+/* a program's queries: points and normals, three floats each, to three floats each */
+struct PointQueries {
+	int which;
+	const float *pos, *norm;
+	float *out;
+	__device__ __forceinline__ void get(int i, int &kind, V3 &p, V3 &n) const
+	{
+		kind = which;
+		p = mk(pos[i * 3], pos[i * 3 + 1], pos[i * 3 + 2]);
+		n = mk(norm[i * 3], norm[i * 3 + 1], norm[i * 3 + 2]);
+	}
+	__device__ __forceinline__ void put(int i, const float (&est)[3]) const { for(int c = 0; c < 3; c++) out[i * 3 + c] = est[c]; }
+	__device__ __forceinline__ void put(int i, int comp, float est) const { out[i * 3 + comp] = est; }
+};
+
+/* Queries that see few photons, a thread each; the others are listed for
+ * k_gather (list[0] of them, from list + 1).  In a frame's sparse maps a query
+ * meets a fraction of a photon to a few, and what a warp spends on it (about
+ * 780 instructions) is the walk, not the photons: the 5.8M gathers of a
+ * 1920x1080 frame at 4 samples and its 0.28M photons cost 4 ms of its 20.0
+ * that way and next to nothing this way (15.9 ms; 16.4 with at most 16
+ * photons here, 16.0 with 32), six frames' 0.85M gathers 0.5 ms of 3.0.  In
+ * a dense map a thread finds out after a few rows (500,009 points of a
+ * 500k-photon map: 1.17 ms with and without).  Calls of at least
+ * GATHER_FEW_MIN queries come here first: below, they would not fill the GPU
+ * a thread each (no difference measured between 8,192 and 131,072 but for a
+ * 320x240 preview's 54,000 gathers, 635 against 649 us). */
+template <class Q>
+__global__ void __launch_bounds__(128) k_gather_few(DScene S, Q q, const int *count, int most, int *list, DevCounters *ctr)
+{
+	__shared__ uint2 runs[FEW_RUNS * 128];
+	const int n = count ? min(*count, most) : most;
+	int tested = 0, cand = 0;
+	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+		int kind, t, c;
+		V3 pos, nrm;
+		q.get(i, kind, pos, nrm);
+		float est[3];
+		if(gather_few(S, kind, pos, nrm, runs + threadIdx.x, 128, est, t, c)) {
+			q.put(i, est);
+			tested += t;
+			cand += c;
+		} else {
+			list[1 + warp_alloc(list, 1)] = i;
+		}
+	}
+	if(ctr) {
+		__syncwarp();
+		tested = __reduce_add_sync(0xffffffffu, tested);
+		cand = __reduce_add_sync(0xffffffffu, cand);
+		if((threadIdx.x & 31) == 0 && tested) {
+			atomicAdd(&ctr->g_tested, (unsigned long long)tested);
+			atomicAdd(&ctr->g_cand, (unsigned long long)cand);
+		}
+		if(blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->rays[3], (unsigned long long)n);
+	}
+}
+
+/* a warp per query: the listed ones, or (list null) all of them */
+template <class Q>
+__global__ void __launch_bounds__(GATHER_WARPS * 32, 4) k_gather(DScene S, Q q, const int *count, int most, const int *list, DevCounters *ctr)
 {
 	__shared__ __align__(16) GatherMem mem[GATHER_WARPS];
-	int n = *gq_count;
+	const int n = list ? list[0] : (count ? min(*count, most) : most);
 	int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	int gw = blockIdx.x * GATHER_WARPS + w, nw = gridDim.x * GATHER_WARPS;
 	const int comp = gather_comp(lane);
 	GatherWork work = {0, 0, 0, 0};
 	for(int r = gw; r < n; r += nw) {
-		GatherReq g = gq[r];
-		int kind = __float_as_int(g.a.w);
-		int pixel = __float_as_int(g.b.w);
-		float est = gather_one(S, kind, mk(g.a.x, g.a.y, g.a.z), mk(g.b.x, g.b.y, g.b.z), mem[w], work);
-		if(comp >= 0) atomicAdd(reinterpret_cast<float *>(acc + pixel) + comp, (comp == 0 ? g.w.x : (comp == 1 ? g.w.y : g.w.z)) * est);
+		const int i = list ? list[1 + r] : r;
+		int kind;
+		V3 pos, nrm;
+		q.get(i, kind, pos, nrm);
+		float est = gather_one(S, kind, pos, nrm, mem[w], work);
+		if(comp >= 0) q.put(i, comp, est);
 		__syncwarp();
 	}
-	if(lane == 0 && work.tested) {
+	if(ctr && lane == 0 && work.tested) {
 		atomicAdd(&ctr->g_tested, work.tested);
 		atomicAdd(&ctr->g_cand, work.cand);
 		atomicAdd(&ctr->g_select, work.select);
 		atomicAdd(&ctr->g_spill, work.spill);
 	}
-	if(blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->rays[3], (unsigned long long)n);
-}
-
-/* gathers at caller-given points: requests packed from the caller's arrays,
- * one warp per request, the estimate written to out[3 * i] */
-__global__ void k_pack_gather(int kind, int n, const float *pos, const float *norm, GatherReq *gq)
-{
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		GatherReq g;
-		g.a = make_float4(pos[i * 3], pos[i * 3 + 1], pos[i * 3 + 2], __int_as_float(kind));
-		g.b = make_float4(norm[i * 3], norm[i * 3 + 1], norm[i * 3 + 2], __int_as_float(i));
-		g.w = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-		gq[i] = g;
-	}
-}
-
-__global__ void __launch_bounds__(GATHER_WARPS * 32, 4) k_gather_points(DScene S, const GatherReq *gq, int n, float *out)
-{
-	__shared__ __align__(16) GatherMem mem[GATHER_WARPS];
-	int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	int gw = blockIdx.x * GATHER_WARPS + w, nw = gridDim.x * GATHER_WARPS;
-	const int comp = gather_comp(lane);
-	GatherWork work = {0, 0, 0, 0};
-	for(int r = gw; r < n; r += nw) {
-		GatherReq g = gq[r];
-		int kind = __float_as_int(g.a.w);
-		int pt = __float_as_int(g.b.w);
-		float est = gather_one(S, kind, mk(g.a.x, g.a.y, g.a.z), mk(g.b.x, g.b.y, g.b.z), mem[w], work);
-		if(comp >= 0) out[pt * 3 + comp] = est;
-		__syncwarp();
-	}
+	if(ctr && !list && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->rays[3], (unsigned long long)n);
 }
 
 /* end of a sample batch: the reference's stop rule applied sample by sample
@@ -3250,13 +3368,11 @@ int Renderer::render_pixels(long msec, float *fb, int fb_is_device, cudaStream_t
 			CK(cudaMemcpyAsync(cnt + 24, cnt + 2, sizeof(int), cudaMemcpyDeviceToDevice, s), "side gather count");
 			CK(cudaEventRecord(gs_fork, s), "side gather fork");
 			CK(cudaStreamWaitEvent(gs, gs_fork, 0), "side gather fork");
-			LAUNCH(*this, "gather", gs, k_gather<<<grid_for((int)gq_upper, GATHER_WARPS), GATHER_WARPS * 32, 0, gs>>>(S,
-					gq_side.as<GatherReq>(), cnt + 24, acc.as<float4>(), ctr.as<DevCounters>()));
+			if(int r2 = gathers(gq_side.as<GatherReq>(), cnt + 24, (int)gq_upper, glist[1], gs)) return r2;
 			CK(cudaEventRecord(gs_done, gs), "side gather done");
 			side_pending = true;
 		} else if(gq_upper > 0) {
-			LAUNCH(*this, "gather", s, k_gather<<<grid_for((int)gq_upper, GATHER_WARPS), GATHER_WARPS * 32, 0, s>>>(S,
-					gq.as<GatherReq>(), cnt + 2, acc.as<float4>(), ctr.as<DevCounters>()));
+			if(int r2 = gathers(gq.as<GatherReq>(), cnt + 2, (int)gq_upper, glist[0], s)) return r2;
 		}
 		gq_upper = 0;
 		CK(cudaMemsetAsync(cnt + 2, 0, sizeof(int), s), "reset gather queue");
@@ -3412,8 +3528,7 @@ int Renderer::render_pixels(long msec, float *fb, int fb_is_device, cudaStream_t
 						pool_ready.as<int>(), ctl, so,
 						acc.as<float4>(), ctr.as<DevCounters>(), g_faults.spin_limit.load() > 0 ? g_faults.spin_limit.load() : POOL_SPIN_LIMIT));
 				if(int r = shadow_rays(so.sq_cap, s)) return r;
-				LAUNCH(*this, "gather", s, k_gather<<<grid_for(so.gq_cap, GATHER_WARPS), GATHER_WARPS * 32, 0, s>>>(S,
-						gq.as<GatherReq>(), cnt + 2, acc.as<float4>(), ctr.as<DevCounters>()));
+				if(int r = gathers(gq.as<GatherReq>(), cnt + 2, so.gq_cap, glist[0], s)) return r;
 				CK(cudaMemcpyAsync(pin, q[cur ^ 1].count, sizeof(int), cudaMemcpyDeviceToHost, s), "read queue count");
 				CK(cudaMemcpyAsync(pin + 1, ctl + 3, sizeof(int), cudaMemcpyDeviceToHost, s), "read pool error");
 				CK(cudaStreamSynchronize(s), "shading tail");
@@ -3477,8 +3592,7 @@ int Renderer::render_pixels(long msec, float *fb, int fb_is_device, cudaStream_t
 				CK(cudaStreamWaitEvent(xs, xs_fork, 0), "light-sample fork");
 				if(int r = shadow_rays_on(sqb.as<ShadowReq>(), sqc, n_rays * shadow_per_ray, fbs[par], xs)) return r;
 				if(!deferring)
-					LAUNCH(*this, "gather", xs, k_gather<<<grid_for(n_rays, GATHER_WARPS), GATHER_WARPS * 32, 0, xs>>>(S,
-							gqb.as<GatherReq>(), gqc, acc.as<float4>(), ctr.as<DevCounters>()));
+					if(int r = gathers(gqb.as<GatherReq>(), gqc, n_rays, glist[2], xs)) return r;
 				CK(cudaEventRecord(xs_done[par], xs), "light-sample done");
 				side_busy[par] = true;
 			} else if(int r = shadow_rays(n_rays * shadow_per_ray, s)) {
@@ -3486,9 +3600,8 @@ int Renderer::render_pixels(long msec, float *fb, int fb_is_device, cudaStream_t
 			}
 			if(deferring)
 				gq_upper += n_rays;
-			else if(!sides)
-				LAUNCH(*this, "gather", s, k_gather<<<grid_for(n_rays, GATHER_WARPS), GATHER_WARPS * 32, 0, s>>>(S, gq.as<GatherReq>(),
-						cnt + 2, acc.as<float4>(), ctr.as<DevCounters>()));
+			else if(!sides && (r = gathers(gq.as<GatherReq>(), cnt + 2, n_rays, glist[0], s)))
+				return r;
 			stats.secondary_rays += depth ? n_rays : 0;
 			CK(cudaMemcpyAsync(pin, q[cur ^ 1].count, sizeof(int), cudaMemcpyDeviceToHost, s), "read queue count");
 			double tw = host_now_ms();
@@ -3604,6 +3717,24 @@ int Renderer::trace_rays_with(const DScene &D, const RayQueue &qq, int n, const 
 	}
 	if(count) LAUNCH(*this, "octree_retrace", s, k_trace_octree<true><<<retrace_grid(), 128, 0, s>>>(D, qq, out, c, f));
 	else LAUNCH(*this, "octree_retrace", s, k_trace_octree<false><<<retrace_grid(), 128, 0, s>>>(D, qq, out, c, f));
+	return 0;
+}
+
+/* the gathers q (count at *count, at most cap) on stream st: from
+ * GATHER_FEW_MIN on a thread each first, the dense ones (list) a warp each */
+#define GATHER_FEW_MIN 32768
+int Renderer::gathers(const GatherReq *q, const int *count, int cap, DevBuf &list, cudaStream_t st)
+{
+	const FrameQueries Q = {q, acc.as<float4>()};
+	DevCounters *c = ctr.as<DevCounters>();
+	int *l = nullptr;
+	if(cap >= GATHER_FEW_MIN) {
+		CK(list.ensure(((size_t)cap + 1) * sizeof(int)), "gather list");
+		l = list.as<int>();
+		CK(cudaMemsetAsync(l, 0, sizeof(int), st), "reset gather list");
+		LAUNCH(*this, "gather", st, k_gather_few<<<grid_for(cap, 128), 128, 0, st>>>(S, Q, count, cap, l, c));
+	}
+	LAUNCH(*this, "gather", st, k_gather<<<grid_for(cap, GATHER_WARPS), GATHER_WARPS * 32, 0, st>>>(S, Q, count, cap, l, c));
 	return 0;
 }
 
@@ -4391,39 +4522,20 @@ int sray_gpu_photon_gather(int which, int n, const float *pos, const float *norm
 	if((which != 0 && which != 1) || n < 0 || (n > 0 && (!pos || !norm || !out))) { g_err = "bad arguments"; return SRAY_EINVAL; }
 	if(n == 0) return 0;
 	cudaStream_t s = as_stream(stream);
-	cudaError_t e = R.gq.ensure((size_t)n * sizeof(GatherReq));
-	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
-	k_pack_gather<<<grid_for(n, 256), 256, 0, s>>>(which, n, pos, norm, R.gq.as<GatherReq>());
-	k_gather_points<<<grid_for(n, GATHER_WARPS), GATHER_WARPS * 32, 0, s>>>(R.S, R.gq.as<GatherReq>(), n, out);
+	const PointQueries q = {which, pos, norm, out};
+	cudaError_t e = cudaSuccess;
+	int *list = nullptr;
+	if(n >= GATHER_FEW_MIN) {
+		e = R.glist[0].ensure(((size_t)n + 1) * sizeof(int));
+		if(e == cudaSuccess) e = cudaMemsetAsync(R.glist[0].p, 0, sizeof(int), s);
+		if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
+		list = R.glist[0].as<int>();
+		k_gather_few<<<grid_for(n, 128), 128, 0, s>>>(R.S, q, nullptr, n, list, nullptr);
+	}
+	k_gather<<<grid_for(n, GATHER_WARPS), GATHER_WARPS * 32, 0, s>>>(R.S, q, nullptr, n, list, nullptr);
 	e = cudaStreamSynchronize(s);
 	if(e == cudaSuccess) e = cudaGetLastError();
 	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
-	return 0;
-}
-
-/* Fixed staging for sray_gpu_photon_gather_noalloc.  Host code must not
- * take this symbol as a device address: the device address is looked up
- * once per device with cudaGetSymbolAddress while that device is current. */
-static __device__ __align__(256) GatherReq g_noalloc_req[SRAY_NOALLOC_MAX_POINTS];
-static GatherReq *g_noalloc_addr[64];
-static std::mutex g_noalloc_mu;
-
-/* the staging's address on the renderer's device (which the caller has
- * made current: NEED_CTX refuses calls from another device) */
-static int noalloc_requests(int dev, GatherReq **out)
-{
-	if(dev < 0 || dev >= 64) { g_err = "device index out of range for the fixed gather staging"; return SRAY_EINVAL; }
-	std::lock_guard<std::mutex> lk(g_noalloc_mu);
-	if(!g_noalloc_addr[dev]) {
-		void *p = nullptr;
-		cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_req);
-		if(e != cudaSuccess || !p) {
-			g_err = std::string("cudaGetSymbolAddress of the gather staging: ") + cudaGetErrorString(e);
-			return SRAY_ECUDA;
-		}
-		g_noalloc_addr[dev] = (GatherReq *)p;
-	}
-	*out = g_noalloc_addr[dev];
 	return 0;
 }
 
@@ -4441,12 +4553,9 @@ int sray_gpu_photon_gather_noalloc(int which, int n, const float *pos, const flo
 		return SRAY_EINVAL;
 	}
 	if(n == 0) return 0;
-	GatherReq *req = nullptr;
-	int r = noalloc_requests(R.device, &req);
-	if(r) return r;
 	cudaStream_t s = as_stream(stream);
-	k_pack_gather<<<grid_for(n, 256), 256, 0, s>>>(which, n, pos, norm, req);
-	k_gather_points<<<grid_for(n, GATHER_WARPS), GATHER_WARPS * 32, 0, s>>>(R.S, req, n, out);
+	/* a warp per point: no list to hold */
+	k_gather<<<grid_for(n, GATHER_WARPS), GATHER_WARPS * 32, 0, s>>>(R.S, PointQueries{which, pos, norm, out}, nullptr, n, nullptr, nullptr);
 	cudaError_t e = cudaStreamSynchronize(s);
 	if(e == cudaSuccess) e = cudaGetLastError();
 	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
@@ -4672,7 +4781,7 @@ void sray_gpu_shutdown(void)
 		&R.fbl, &R.tnodes, &R.ohome, &R.pool_ready, &R.pqbuf[0], &R.pqbuf[1], &R.phits, &R.pfbl, &R.pcounts, &R.pctr,
 		&R.pw_jobs, &R.pw_prefix, &R.pw_scale, &R.pw_bits, &R.pw_cov, &R.pj_tables, &R.pj_samples, &R.pj_boxes, &R.pj_views, &R.pj_first, &R.pw_pix, &R.pw_out, &R.pw_valid,
 		&R.pw_part, &R.pw_tiles, &R.pw_bounds, &R.pw_offs, &R.pw_ph, &R.pw_sorted, &R.pw_grids, &R.pw_cellbase,
-		&R.pw_keys, &R.pw_lin, &R.pw_starts, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1],
+		&R.pw_keys, &R.pw_lin, &R.pw_starts, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1], &R.glist[0], &R.glist[1], &R.glist[2],
 		&R.pqsbuf, &R.ps_keys, &R.ps_hist, &R.ps_part,
 		&R.nrc_qx, &R.nrc_qw, &R.nrc_rx, &R.nrc_rt, &R.nrc_ry, &R.nrc_regions};
 	if(R.ps) cudaStreamSynchronize(R.ps);

@@ -196,6 +196,8 @@ struct Renderer {
 	cudaEvent_t hs_fork = nullptr, hs_join = nullptr;
 	int priority_stream();
 	int shadow_rays(int cap, cudaStream_t s);
+	DevBuf glist[3];           /* dense gathers: the frame's stream, the gather stream, the light-sample stream */
+	int gathers(const GatherReq *q, const int *count, int cap, DevBuf &list, cudaStream_t st);
 
 	cudaEvent_t ps_done = nullptr;
 	sray_stats stats;

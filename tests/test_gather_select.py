@@ -179,3 +179,37 @@ def test_gather_grid(gpu_lib, tmp_path, n, k):
     c = np.clip(np.floor((pos.astype(np.float64) - lo) / cell).astype(np.int64), 0, dims - 1)
     order = np.argsort(_spread3(c[:, 0]) | _spread3(c[:, 1]) << 1 | _spread3(c[:, 2]) << 2, kind="stable")
     assert np.array_equal(ph[:, 0:3], pos[order]) and np.array_equal(ph[:, 9:12], power[order])
+
+
+@pytest.mark.parametrize("which", [0, 1])
+@pytest.mark.parametrize("k", [0, 1, 8, 50, 100])
+def test_gather_of_many_points(gpu_lib, dump, which, k):
+    """The same selections asked for 32,768 and more times in one call, where
+    a thread answers the queries that see few photons and lists the others:
+    every copy of a query gets the same answer."""
+    lay, path, pos, power = dump
+    frac = np.float32(0.5 / np.sqrt(40.0 ** 2 + 4.0 ** 2 + 40.0 ** 2))
+    rad = np.sqrt(40.0 ** 2 + 4.0 ** 2 + 40.0 ** 2) * float(frac) if k == 0 else 0.5
+    rng = np.random.default_rng(9)
+    q = np.stack([c for c, _ in lay.values()]).astype(np.float32)
+    # off the centres too: the edges of the discs, between layouts, outside the box
+    q = np.concatenate([q, q + rng.uniform(-0.6, 0.6, q.shape).astype(np.float32), rng.uniform((-21, -1, -21), (21, 5, 21), (40, 3)).astype(np.float32)])
+    copies = 32768 // len(q) + 2
+    g = gpu_lib.GpuRenderer(width=64, height=64, caust_k=k, gi_k=k, gather_rcap=0.5, gather_dist=float(frac), caust_photons=1000,
+                            gi_photons=1000)
+    g.load_xml(SCENE)
+    g.build(0, 0)
+    g.restore_photons(which, path)
+    qd = torch.tensor(np.tile(q, (copies, 1)), device="cuda")
+    nd = torch.tensor([[0.0, 1.0, 0.0]], device="cuda").repeat(len(qd), 1).contiguous()
+    out = torch.full((len(qd), 3), -1.0, device="cuda")
+    g.photon_gather(which, qd, nd, out)
+    got = out.cpu().numpy().astype(np.float64).reshape(copies, len(q), 3)
+    g.close()
+    assert np.array_equal(got, np.broadcast_to(got[0], got.shape), equal_nan=True)
+    for i in range(len(q)):
+        want = _expected(pos, power, q[i], k, which, rad)
+        if not np.isfinite(want).all():
+            assert not np.isfinite(got[0, i]).any()
+            continue
+        assert (np.abs(got[0, i] - want) <= BOUND * np.maximum(np.abs(want), 1e-9)).all(), (i, got[0, i], want)
