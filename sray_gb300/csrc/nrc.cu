@@ -10,22 +10,19 @@
  * Adam master copy) and used as BF16 with FP32 accumulation: inference and
  * queries on the 5th-generation tensor cores (tcgen05.mma, a 128-sample tile
  * per MMA); the training step by warp-level MMAs (mma.sync m16n8k16: a warp
- * carries 16 samples through all five layers with the activations in
- * registers, the accumulator tile of one layer becoming the operand tile of
- * the next).
+ * carries 16 samples through all five layers and back, the accumulator tile
+ * of one layer becoming the operand tile of the next, and a share of the
+ * block's weight gradients).
  *
  *   k_nrc_forward_tc<FWD_INFER>  inference: encode + 5 layers on the
  *                         5th-generation tensor cores (TMEM accumulators
  *                         and hidden operands, three tiles in flight per SM)
  *   k_nrc_forward_tc<FWD_QUERY>  the renderer's queries: the same, the output
  *                         weighted into the pixel's accumulator
- *   k_nrc_forward<FWD_TRAIN>  training forward (warp-level MMA): also stores
- *                         the layer inputs (BF16) and the loss gradient of
- *                         the outputs
- *   k_nrc_backward        dZ of layers 4..1 through the transposed weights,
- *                         bias gradients
- *   k_nrc_wgrad<L>        weight gradients dW = dZ^T H over the batch (MMA,
- *                         samples split over blocks, FP32 atomics)
+ *   k_nrc_gradient        the training step's gradient: forward, loss, backward
+ *                         and weight gradients of 128-sample tiles in one
+ *                         kernel (warp-level MMA), activations in shared
+ *                         memory, weight gradients in registers
  *   k_nrc_adam            Adam on the FP32 master, BF16 copies refreshed
  *
  * The CPU restatement (checker of these kernels) is oracle/nrc.py.
@@ -63,20 +60,18 @@ enum {
 };
 static_assert(NRC_NPARAM == SRAY_NRC_PARAMS, "parameter count");
 
-/* shared-memory row strides (bf16 elements), padded against bank conflicts */
-enum { LD1 = 232, LDH = 72, LD5T = 24 };
-#define NRC_FWD_THREADS 256   /* forward blocks: 8 warps share one copy of the weights in shared memory */
+/* row strides (bf16 elements) of the weight images and of the training
+ * step's shared memory, padded against bank conflicts */
+enum { LD1 = 232, LDH = 72, LD5 = 24 };
 
-/* BF16 weight images in global memory, in the shared-memory layout:
+/* BF16 weight images in global memory, in the training step's shared-memory
+ * layout:
  *   w1  [64][LD1]      (in 0..215, zero up to 231)
  *   w2-4 [64][LDH]     (out rows, in columns)
  *   w5  [8][LDH]       (rows 3..7 zero)
- *   w2t-w4t [64][LDH]  transposed (in rows, out columns), for the backward pass
- *   w5t [64][LD5T]     transposed, out columns 3..23 zero
  * plus the FP32 biases b1-b4 [64], b5 [8]. */
 struct NrcDev {
 	const __nv_bfloat16 *w1, *w2, *w3, *w4, *w5;
-	const __nv_bfloat16 *w2t, *w3t, *w4t, *w5t;
 	const float *bias;            /* 4 x 64 + 8 */
 };
 
@@ -86,13 +81,7 @@ enum {
 	IMG_W3 = IMG_W2 + 64 * LDH,
 	IMG_W4 = IMG_W3 + 64 * LDH,
 	IMG_W5 = IMG_W4 + 64 * LDH,
-	IMG_W2T = IMG_W5 + 8 * LDH,
-	IMG_W3T = IMG_W2T + 64 * LDH,
-	IMG_W4T = IMG_W3T + 64 * LDH,
-	IMG_W5T = IMG_W4T + 64 * LDH,
-	IMG_END = IMG_W5T + 64 * LD5T,
-	FWD_SMEM_BF16 = IMG_W2T,                /* w1..w5 */
-	BWD_SMEM_BF16 = IMG_END - IMG_W2T,      /* w2t..w5t */
+	IMG_END = IMG_W5 + 8 * LDH,
 	NRC_NBIAS = 4 * 64 + 8
 };
 
@@ -113,14 +102,39 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
-/* B operand of a k16 x n8 tile whose element (k, n) is M[n0 + n][k0 + k] of
- * a row-major shared matrix with row stride ld: two adjacent k per register */
-__device__ __forceinline__ void load_b(const __nv_bfloat16 *M, int ld, int n0, int k0, int lane, uint32_t &b0, uint32_t &b1)
+/* Four 8 x 8 BF16 blocks of a row-major shared matrix, one register each; the
+ * lanes of eight give a block's row addresses.  T: each block transposed. */
+template <bool T>
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t saddr)
 {
-	int g = lane >> 2, t = lane & 3;
-	const __nv_bfloat16 *p = M + (size_t)(n0 + g) * ld + k0 + 2 * t;
-	b0 = *reinterpret_cast<const uint32_t *>(p);
-	b1 = *reinterpret_cast<const uint32_t *>(p + 8);
+	if(T)
+		asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+				: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
+	else
+		asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+				: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
+}
+
+/* B operands of two k16 x n8 tiles (columns n0 and n0 + 8): r[0], r[1] and
+ * r[2], r[3].  Element (k, n) is M[n0 + n][k0 + k]. */
+__device__ __forceinline__ void load_b2(uint32_t (&r)[4], uint32_t M, int ld, int n0, int k0, int lane)
+{
+	int i = lane >> 3, row = n0 + (lane & 7) + (i >> 1) * 8, col = k0 + (i & 1) * 8;
+	ldsm4<false>(r, M + (uint32_t)(row * ld + col) * 2);
+}
+
+/* the same where element (k, n) is M[k0 + k][n0 + n] */
+__device__ __forceinline__ void load_bt2(uint32_t (&r)[4], uint32_t M, int ld, int n0, int k0, int lane)
+{
+	int i = lane >> 3, row = k0 + (lane & 7) + (i & 1) * 8, col = n0 + (i >> 1) * 8;
+	ldsm4<true>(r, M + (uint32_t)(row * ld + col) * 2);
+}
+
+/* A operand of an m16 x k16 tile whose element (m, k) is M[k0 + k][m0 + m] */
+__device__ __forceinline__ void load_at(uint32_t (&r)[4], uint32_t M, int ld, int m0, int k0, int lane)
+{
+	int i = lane >> 3, row = k0 + (lane & 7) + (i >> 1) * 8, col = m0 + (i & 1) * 8;
+	ldsm4<true>(r, M + (uint32_t)(row * ld + col) * 2);
 }
 
 /* a 16 x 64 activation block as accumulators: 8 n-tiles x 4 floats */
@@ -147,23 +161,6 @@ __device__ __forceinline__ void acc_to_a(const Acc64 &z, uint32_t (&a)[4][4], bo
 	}
 }
 
-/* 16 x 64 = A(16 x 64) W^T: W [64][LDH] (out, in) */
-__device__ __forceinline__ void layer64(const uint32_t (&a)[4][4], const __nv_bfloat16 *W, const float *bias, int lane, Acc64 &z)
-{
-	int t = lane & 3;
-	#pragma unroll
-	for(int nt = 0; nt < 8; nt++) {
-		float b0 = bias[nt * 8 + 2 * t], b1 = bias[nt * 8 + 2 * t + 1];
-		z.d[nt][0] = b0; z.d[nt][1] = b1; z.d[nt][2] = b0; z.d[nt][3] = b1;
-		#pragma unroll
-		for(int kt = 0; kt < 4; kt++) {
-			uint32_t w0, w1;
-			load_b(W, LDH, nt * 8, kt * 16, lane, w0, w1);
-			mma16816(z.d[nt], a[kt], w0, w1);
-		}
-	}
-}
-
 /* one encoded feature pair (sin, cos of pi 2^b x_v) for pair index p, 0 for padding */
 __device__ __forceinline__ uint32_t feature_pair(const float *x, int p)
 {
@@ -185,24 +182,6 @@ __device__ __forceinline__ void encode_a(const float *xg, const float *xg8, int 
 	a[3] = feature_pair(xg8, p1);
 }
 
-__device__ __forceinline__ void copy_to_shared(__nv_bfloat16 *dst, const __nv_bfloat16 *src, int n)
-{
-	const uint4 *s = reinterpret_cast<const uint4 *>(src);
-	uint4 *d = reinterpret_cast<uint4 *>(dst);
-	for(int i = threadIdx.x; i < n / 8; i += blockDim.x) d[i] = s[i];
-}
-
-/* Forward pass, a warp per 16 samples.  x: [n][9]; y: [n][3] (inference) or
- * unused.  TRAIN: t [n][3] targets; stores h0 [n16][NRC_FP] (encoded, BF16),
- * h1..h4 [n16][64] (BF16), dz5 [n16][16] (BF16 loss gradient of the
- * outputs), db5 partial sums and the loss. */
-struct TrainBufs {
-	__nv_bfloat16 *h[5];          /* h[0] encoded inputs, h[1..4] hidden */
-	__nv_bfloat16 *dz[6];         /* dz[1..4] hidden, dz[5] outputs (16 wide) */
-	float *grad;                  /* packed FP32 gradient */
-	float *loss;
-};
-
 /* queries of the renderer: inputs x [n][9]; w[i] = weight rgb and the
  * accumulator slot; acc[slot] += w * max(y, 0); the count is read on the
  * device (n is the capacity) */
@@ -212,151 +191,338 @@ struct QueryOut {
 	float4 *acc;
 };
 
-enum { FWD_INFER = 0, FWD_TRAIN = 1, FWD_QUERY = 2 };
+enum { FWD_INFER = 0, FWD_QUERY = 2 };
 
-template <int MODE>
-__global__ void __launch_bounds__(NRC_FWD_THREADS) k_nrc_forward(NrcDev net, int n, const float *x, float *y, const float *tgt, TrainBufs tb,
-		QueryOut qo)
+/* ---- The gradient of a batch ----
+ * A block of eight warps takes tiles of 128 samples, 16 per warp.  Forward as
+ * a chain of MMAs in registers, each layer's BF16 input also stored in shared
+ * memory; loss and its gradient; backward through the same weights (read
+ * transposed by ldmatrix).  After each layer's dZ the block's warps form its
+ * weight gradient dW = dZ^T H over the tile's samples (both operands read
+ * transposed), each warp a fixed part of it in registers -- 108 floats per
+ * thread for all layers -- which go to the packed gradient once, after the
+ * block's last tile, by vector atomics.  Weights and everything a sample needs
+ * stay on the SM: the batch's inputs are read once, and nothing but the
+ * gradient is written.
+ *
+ * Bound by the latency of its chain (weights, encoding, ten MMA layers with a
+ * barrier each) up to a tile per SM, then by the warp-level tensor pipe.
+ * As five kernels through global memory (forward, backward, a weight-gradient
+ * kernel per layer whose operands were transposed element by element) a step
+ * of 16,384 samples took 107 us on the device and 144 us per call; this way a
+ * call takes 41 us (262,144 samples: 872 and 267 us, 155 TFLOP/s). */
+#define GR_THREADS 256
+#define GR_TILE 128
+enum {
+	GR_W = 0,                                   /* the images; w5 padded to 16 rows */
+	GR_W5 = GR_W + IMG_W5 * 2,
+	GR_BIAS = GR_W5 + 16 * LDH * 2,
+	GR_DB = GR_BIAS + NRC_NBIAS * 4,            /* bias gradients: 4 x 64, then 3 */
+	GR_H0 = GR_DB + NRC_NBIAS * 4,              /* encoded inputs [128][LD1] */
+	GR_H1 = GR_H0 + GR_TILE * LD1 * 2,          /* hidden activations, four of [128][LDH] */
+	GR_HSIZE = GR_TILE * LDH * 2,
+	GR_DZ = GR_H1 + 4 * GR_HSIZE,               /* dZ of layers 4 and 2 (3 and 1: in place of h4) */
+	GR_DZ5 = GR_DZ + GR_HSIZE,                  /* dZ of the outputs [128][LD5], 16 columns used */
+	GR_SMEM = GR_DZ5 + GR_TILE * LD5 * 2
+};
+static_assert(GR_SMEM <= 232448, "shared memory of the gradient");
+static_assert(GR_W5 % 16 == 0 && GR_BIAS % 16 == 0 && GR_H0 % 16 == 0 && GR_H1 % 16 == 0 && GR_DZ % 16 == 0 && GR_DZ5 % 16 == 0 &&
+		LD1 * 2 % 16 == 0 && LDH * 2 % 16 == 0 && LD5 * 2 % 16 == 0 && IMG_END * 2 % 16 == 0, "16-byte rows for ldmatrix and cp.async");
+
+__device__ __forceinline__ void red_add2(float *p, float a, float b)
 {
-	constexpr bool TRAIN = MODE == FWD_TRAIN;
-	if(MODE == FWD_QUERY) {
-		int c = *qo.count;
-		n = c < n ? c : n;
+	asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" :: "l"(p), "f"(a), "f"(b) : "memory");
+}
+
+/* 16 x 64 = A(16 x 64) W^T + bias: W [64][LDH] (out, in) at M */
+__device__ __forceinline__ void layer64(const uint32_t (&a)[4][4], uint32_t M, const float *bias, int lane, Acc64 &z)
+{
+	int t = lane & 3;
+	#pragma unroll
+	for(int nt = 0; nt < 8; nt += 2) {
+		#pragma unroll
+		for(int h = 0; h < 2; h++) {
+			float b0 = bias[(nt + h) * 8 + 2 * t], b1 = bias[(nt + h) * 8 + 2 * t + 1];
+			z.d[nt + h][0] = b0; z.d[nt + h][1] = b1; z.d[nt + h][2] = b0; z.d[nt + h][3] = b1;
+		}
+		#pragma unroll
+		for(int kt = 0; kt < 4; kt++) {
+			uint32_t w[4];
+			load_b2(w, M, LDH, nt * 8, kt * 16, lane);
+			mma16816(z.d[nt], a[kt], w[0], w[1]);
+			mma16816(z.d[nt + 1], a[kt], w[2], w[3]);
+		}
 	}
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	__nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(smem_raw);
-	float *sb = reinterpret_cast<float *>(sw + FWD_SMEM_BF16);
-	copy_to_shared(sw, net.w1, FWD_SMEM_BF16);
-	for(int i = threadIdx.x; i < NRC_NBIAS; i += blockDim.x) sb[i] = net.bias[i];
-	__syncthreads();
-	const __nv_bfloat16 *W1 = sw + IMG_W1, *W2 = sw + IMG_W2, *W3 = sw + IMG_W3, *W4 = sw + IMG_W4, *W5 = sw + IMG_W5;
-	int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	int g = lane >> 2, t = lane & 3;
-	int ntiles = (n + 15) >> 4;
-	float loss = 0.0f;
-	float db5[2] = {0.0f, 0.0f};
-	const int wpb = NRC_FWD_THREADS / 32;
-	for(int tile = blockIdx.x * wpb + warp; tile < ntiles; tile += gridDim.x * wpb) {
-		int r0 = tile * 16 + g, r1 = r0 + 8;
+}
+
+/* this warp's part of a 64 x 64 weight gradient over the tile: rows 16 mt ..,
+ * columns 32 nh .. */
+__device__ __forceinline__ void wgrad64(float (&g)[4][4], uint32_t dz, uint32_t h, int mt, int nh, int lane)
+{
+	#pragma unroll
+	for(int k = 0; k < GR_TILE; k += 16) {
+		uint32_t a[4], b[4];
+		load_at(a, dz, LDH, mt * 16, k, lane);
+		#pragma unroll
+		for(int j = 0; j < 4; j += 2) {
+			load_bt2(b, h, LDH, nh * 32 + j * 8, k, lane);
+			mma16816(g[j], a, b[0], b[1]);
+			mma16816(g[j + 1], a, b[2], b[3]);
+		}
+	}
+}
+
+__global__ void __launch_bounds__(GR_THREADS, 1) k_nrc_gradient(NrcDev net, int n, const float *x, const float *tgt, float *grad, float *loss_out)
+{
+	extern __shared__ __align__(16) unsigned char gsm[];
+	const uint32_t sb = (uint32_t)__cvta_generic_to_shared(gsm);
+	float *bias = reinterpret_cast<float *>(gsm + GR_BIAS), *sdb = reinterpret_cast<float *>(gsm + GR_DB);
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int g = lane >> 2, t = lane & 3;
+	/* the weights arrive while the first tile is encoded */
+	for(int i = threadIdx.x; i < IMG_END / 8; i += GR_THREADS)
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(sb + GR_W + i * 16), "l"(reinterpret_cast<const uint4 *>(net.w1) + i) : "memory");
+	asm volatile("cp.async.commit_group;" ::: "memory");
+	for(int i = threadIdx.x; i < 8 * LDH / 8; i += GR_THREADS)
+		*reinterpret_cast<uint4 *>(gsm + GR_W5 + 8 * LDH * 2 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+	for(int i = threadIdx.x; i < NRC_NBIAS; i += GR_THREADS) {
+		bias[i] = net.bias[i];
+		sdb[i] = 0.0f;
+	}
+	const uint32_t sW1 = sb + GR_W + IMG_W1 * 2, sW5 = sb + GR_W5, sH0 = sb + GR_H0, sDZ5 = sb + GR_DZ5;
+	const int mt = warp & 3, nh = warp >> 2;       /* this warp's part of the weight gradients */
+	float g1[14][4], gh[3][4][4], g5[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+	#pragma unroll
+	for(int j = 0; j < 14; j++) g1[j][0] = g1[j][1] = g1[j][2] = g1[j][3] = 0.0f;
+	#pragma unroll
+	for(int l = 0; l < 3; l++)
+		#pragma unroll
+		for(int j = 0; j < 4; j++) gh[l][j][0] = gh[l][j][1] = gh[l][j][2] = gh[l][j][3] = 0.0f;
+	float loss = 0.0f, db5[2] = {0.0f, 0.0f};
+	const int ntiles = (n + GR_TILE - 1) / GR_TILE;
+	const int lr = warp * 16 + g;                  /* this lane's rows in the tile: lr and lr + 8 */
+	for(int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+		const int r0 = tile * GR_TILE + lr, r1 = r0 + 8;
 		float xg[9], xg8[9];
 		#pragma unroll
 		for(int k = 0; k < 9; k++) {
 			xg[k] = r0 < n ? x[(size_t)r0 * 9 + k] : 0.0f;
 			xg8[k] = r1 < n ? x[(size_t)r1 * 9 + k] : 0.0f;
 		}
-		/* layer 1: 14 k-tiles of encoded features */
-		Acc64 z;
-		#pragma unroll
-		for(int nt = 0; nt < 8; nt++) {
-			float b0 = sb[nt * 8 + 2 * t], b1 = sb[nt * 8 + 2 * t + 1];
-			z.d[nt][0] = b0; z.d[nt][1] = b1; z.d[nt][2] = b0; z.d[nt][3] = b1;
-		}
+		/* the encoded inputs, in the layout of the A operand */
+		uint32_t *h0 = reinterpret_cast<uint32_t *>(gsm + GR_H0) + lr * (LD1 / 2) + t;
+		#pragma unroll 2
 		for(int kt = 0; kt < NRC_FP / 16; kt++) {
 			uint32_t a[4];
 			encode_a(xg, xg8, kt, lane, a);
-			if(TRAIN) {
-				__nv_bfloat16 *h0 = tb.h[0];
-				uint32_t *p0 = reinterpret_cast<uint32_t *>(h0 + (size_t)r0 * NRC_FP + kt * 16 + 2 * t);
-				uint32_t *p1 = reinterpret_cast<uint32_t *>(h0 + (size_t)r1 * NRC_FP + kt * 16 + 2 * t);
-				p0[0] = a[0]; p1[0] = a[1]; p0[4] = a[2]; p1[4] = a[3];
-			}
-			#pragma unroll
-			for(int nt = 0; nt < 8; nt++) {
-				uint32_t w0, w1;
-				load_b(W1, LD1, nt * 8, kt * 16, lane, w0, w1);
-				mma16816(z.d[nt], a, w0, w1);
-			}
+			uint32_t *q = h0 + kt * 8;
+			q[0] = a[0];
+			q[8 * (LD1 / 2)] = a[1];
+			q[4] = a[2];
+			q[8 * (LD1 / 2) + 4] = a[3];
 		}
-		uint32_t a[4][4];
-		const __nv_bfloat16 *Ws[3] = {W2, W3, W4};
+		if(tile == (int)blockIdx.x) {
+			asm volatile("cp.async.wait_group 0;" ::: "memory");
+			__syncthreads();
+		} else {
+			__syncwarp();
+		}
+		/* layer 1 */
+		Acc64 z;
 		#pragma unroll
-		for(int l = 0; l < 3; l++) {
-			acc_to_a(z, a, true);
-			if(TRAIN) {
-				/* h_{l+1}: the BF16 input of layer l + 2 */
-				__nv_bfloat16 *h = tb.h[l + 1];
-				#pragma unroll
-				for(int kt = 0; kt < 4; kt++) {
-					uint32_t *p0 = reinterpret_cast<uint32_t *>(h + (size_t)r0 * 64 + kt * 16 + 2 * t);
-					uint32_t *p1 = reinterpret_cast<uint32_t *>(h + (size_t)r1 * 64 + kt * 16 + 2 * t);
-					p0[0] = a[kt][0]; p1[0] = a[kt][1]; p0[4] = a[kt][2]; p1[4] = a[kt][3];
-				}
-			}
-			layer64(a, Ws[l], sb + 64 * (l + 1), lane, z);
+		for(int nt = 0; nt < 8; nt++) {
+			float b0 = bias[nt * 8 + 2 * t], b1 = bias[nt * 8 + 2 * t + 1];
+			z.d[nt][0] = b0; z.d[nt][1] = b1; z.d[nt][2] = b0; z.d[nt][3] = b1;
 		}
-		acc_to_a(z, a, true);
-		if(TRAIN) {
-			__nv_bfloat16 *h = tb.h[4];
+		#pragma unroll 2
+		for(int kt = 0; kt < NRC_FP / 16; kt++) {
+			const uint32_t *q = h0 + kt * 8;
+			const uint32_t a[4] = {q[0], q[8 * (LD1 / 2)], q[4], q[8 * (LD1 / 2) + 4]};
+			#pragma unroll
+			for(int nt = 0; nt < 8; nt += 2) {
+				uint32_t w[4];
+				load_b2(w, sW1, LD1, nt * 8, kt * 16, lane);
+				mma16816(z.d[nt], a, w[0], w[1]);
+				mma16816(z.d[nt + 1], a, w[2], w[3]);
+			}
+		}
+		/* layers 2-4 and the inputs of the output layer; which activations
+		 * are positive, a bit each */
+		uint32_t a[4][4], on[4];
+		#pragma unroll
+		for(int l = 0; l < 4; l++) {
+			acc_to_a(z, a, true);
+			uint32_t *h = reinterpret_cast<uint32_t *>(gsm + GR_H1 + l * GR_HSIZE) + lr * (LDH / 2) + t;
+			on[l] = 0;
 			#pragma unroll
 			for(int kt = 0; kt < 4; kt++) {
-				uint32_t *p0 = reinterpret_cast<uint32_t *>(h + (size_t)r0 * 64 + kt * 16 + 2 * t);
-				uint32_t *p1 = reinterpret_cast<uint32_t *>(h + (size_t)r1 * 64 + kt * 16 + 2 * t);
-				p0[0] = a[kt][0]; p1[0] = a[kt][1]; p0[4] = a[kt][2]; p1[4] = a[kt][3];
+				h[kt * 8] = a[kt][0];
+				h[kt * 8 + 8 * (LDH / 2)] = a[kt][1];
+				h[kt * 8 + 4] = a[kt][2];
+				h[kt * 8 + 4 + 8 * (LDH / 2)] = a[kt][3];
+				#pragma unroll
+				for(int i = 0; i < 4; i++)
+					on[l] |= ((bf16_lo(a[kt][i]) > 0.0f ? 1u : 0u) | (bf16_hi(a[kt][i]) > 0.0f ? 2u : 0u)) << (kt * 8 + i * 2);
 			}
+			if(l < 3) layer64(a, sb + GR_W + (l == 0 ? IMG_W2 : (l == 1 ? IMG_W3 : IMG_W4)) * 2, bias + 64 * (l + 1), lane, z);
 		}
 		/* output layer: one n-tile (outputs 0..7, 3 used) */
 		float o[4];
-		o[0] = sb[256 + 2 * t]; o[1] = sb[256 + 2 * t + 1]; o[2] = o[0]; o[3] = o[1];
+		o[0] = bias[256 + 2 * t]; o[1] = bias[256 + 2 * t + 1]; o[2] = o[0]; o[3] = o[1];
 		#pragma unroll
 		for(int kt = 0; kt < 4; kt++) {
-			uint32_t w0, w1;
-			load_b(W5, LDH, 0, kt * 16, lane, w0, w1);
-			mma16816(o, a[kt], w0, w1);
+			uint32_t w[4];
+			load_b2(w, sW5, LDH, 0, kt * 16, lane);
+			mma16816(o, a[kt], w[0], w[1]);
 		}
-		/* lane (g, t) holds outputs 2t, 2t+1 of rows g and g + 8 */
+		/* lane (g, t) holds outputs 2t, 2t+1 of rows g and g + 8: the loss and
+		 * its gradient */
+		uint32_t a5[4] = {0u, 0u, 0u, 0u};
 		#pragma unroll
 		for(int half = 0; half < 2; half++) {
-			int r = half ? r1 : r0;
+			const int r = half ? r1 : r0;
+			float dy[2];
 			#pragma unroll
 			for(int c = 0; c < 2; c++) {
-				int col = 2 * t + c;
-				float yv = o[2 * half + c];
-				if(MODE == FWD_QUERY) {
-					if(r < n && col < NRC_O) {
-						float4 wv = qo.w[r];
-						float wc = col == 0 ? wv.x : (col == 1 ? wv.y : wv.z);
-						atomicAdd(reinterpret_cast<float *>(qo.acc + __float_as_int(wv.w)) + col, wc * fmaxf(yv, 0.0f));
+				const int col = 2 * t + c;
+				dy[c] = 0.0f;
+				if(r < n && col < NRC_O) {
+					float yv = o[2 * half + c], tv = tgt[(size_t)r * 3 + col];
+					float den = yv * yv + 0.01f;
+					float e = yv - tv;
+					loss += e * e / den;
+					dy[c] = 2.0f * e / den / (float)(3 * n);
+				}
+				db5[c] += dy[c];
+			}
+			a5[half] = pack_bf16(dy[0], dy[1]);
+			uint32_t *q = reinterpret_cast<uint32_t *>(gsm + GR_DZ5) + (lr + 8 * half) * (LD5 / 2) + t;
+			q[0] = a5[half];
+			q[4] = 0u;
+		}
+		/* dZ of layer 4 from the outputs' */
+		#pragma unroll
+		for(int nt = 0; nt < 8; nt += 2) {
+			uint32_t w[4];
+			#pragma unroll
+			for(int h = 0; h < 2; h++) z.d[nt + h][0] = z.d[nt + h][1] = z.d[nt + h][2] = z.d[nt + h][3] = 0.0f;
+			load_bt2(w, sW5, LDH, nt * 8, 0, lane);
+			mma16816(z.d[nt], a5, w[0], w[1]);
+			mma16816(z.d[nt + 1], a5, w[2], w[3]);
+		}
+		__syncthreads();
+		/* the output layer's weight gradient: columns 8 warp .. of h4 */
+		#pragma unroll
+		for(int k = 0; k < GR_TILE; k += 16) {
+			uint32_t am[4], b[4];
+			load_at(am, sDZ5, LD5, 0, k, lane);
+			load_bt2(b, sb + GR_H1 + 3 * GR_HSIZE, LDH, (warp >> 1) * 16, k, lane);
+			if(warp & 1) mma16816(g5, am, b[2], b[3]);
+			else mma16816(g5, am, b[0], b[1]);
+		}
+		#pragma unroll
+		for(int l = 4; l >= 1; l--) {
+			/* dZ_l: masked by h_l > 0; bias sums, BF16 for the products.  The
+			 * buffer it goes to was last read before the barrier of the layer
+			 * after next (dZ_3 and dZ_1 in place of h4) */
+			const uint32_t off = (l & 1) ? GR_H1 + 3 * GR_HSIZE : GR_DZ;
+			uint32_t *dz = reinterpret_cast<uint32_t *>(gsm + off) + lr * (LDH / 2) + t;
+			#pragma unroll
+			for(int nt = 0; nt < 8; nt++) {
+				const int kt = nt >> 1, i0 = (nt & 1) * 2;     /* this tile in the forward's A operand: registers i0 and i0 + 1 */
+				const uint32_t m = on[l - 1] >> (kt * 8 + i0 * 2);
+				if(!(m & 1u)) z.d[nt][0] = 0.0f;
+				if(!(m & 2u)) z.d[nt][1] = 0.0f;
+				if(!(m & 4u)) z.d[nt][2] = 0.0f;
+				if(!(m & 8u)) z.d[nt][3] = 0.0f;
+				float s0 = z.d[nt][0] + z.d[nt][2], s1 = z.d[nt][1] + z.d[nt][3];
+				#pragma unroll
+				for(int q = 4; q < 32; q <<= 1) {
+					s0 += __shfl_xor_sync(0xffffffffu, s0, q);
+					s1 += __shfl_xor_sync(0xffffffffu, s1, q);
+				}
+				if(g == 0) {
+					atomicAdd(&sdb[(l - 1) * 64 + nt * 8 + 2 * t], s0);
+					atomicAdd(&sdb[(l - 1) * 64 + nt * 8 + 2 * t + 1], s1);
+				}
+			}
+			acc_to_a(z, a, false);
+			#pragma unroll
+			for(int kt = 0; kt < 4; kt++) {
+				dz[kt * 8] = a[kt][0];
+				dz[kt * 8 + 8 * (LDH / 2)] = a[kt][1];
+				dz[kt * 8 + 4] = a[kt][2];
+				dz[kt * 8 + 4 + 8 * (LDH / 2)] = a[kt][3];
+			}
+			if(l > 1) {
+				/* dH_{l-1} = dZ_l W_l */
+				const uint32_t W = sb + GR_W + (l == 4 ? IMG_W4 : (l == 3 ? IMG_W3 : IMG_W2)) * 2;
+				#pragma unroll
+				for(int nt = 0; nt < 8; nt += 2) {
+					#pragma unroll
+					for(int h = 0; h < 2; h++) z.d[nt + h][0] = z.d[nt + h][1] = z.d[nt + h][2] = z.d[nt + h][3] = 0.0f;
+					#pragma unroll
+					for(int kt = 0; kt < 4; kt++) {
+						uint32_t w[4];
+						load_bt2(w, W, LDH, nt * 8, kt * 16, lane);
+						mma16816(z.d[nt], a[kt], w[0], w[1]);
+						mma16816(z.d[nt + 1], a[kt], w[2], w[3]);
 					}
-				} else if(!TRAIN) {
-					if(r < n && col < NRC_O) y[(size_t)r * 3 + col] = yv;
-				} else {
-					float dy = 0.0f;
-					if(r < n && col < NRC_O) {
-						float tv = tgt[(size_t)r * 3 + col];
-						float den = yv * yv + 0.01f;
-						float e = yv - tv;
-						loss += e * e / den;
-						dy = 2.0f * e / den / (float)(3 * n);
+				}
+			}
+			__syncthreads();
+			if(l > 1) {
+				wgrad64(gh[l - 2], sb + off, sb + GR_H1 + (l - 2) * GR_HSIZE, mt, nh, lane);
+			} else {
+				#pragma unroll 2
+				for(int k = 0; k < GR_TILE; k += 16) {
+					uint32_t am[4];
+					load_at(am, sb + off, LDH, mt * 16, k, lane);
+					#pragma unroll
+					for(int j = 0; j < 14; j += 2) {
+						uint32_t b[4];
+						load_bt2(b, sH0, LD1, nh * 112 + j * 8, k, lane);
+						mma16816(g1[j], am, b[0], b[1]);
+						mma16816(g1[j + 1], am, b[2], b[3]);
 					}
-					/* dz5 row r, columns 0..15 (BF16); db5 from the FP32 value */
-					tb.dz[5][(size_t)r * 16 + col] = __float2bfloat16_rn(dy);
-					db5[c] += dy;
-					if(y && r < n && col < NRC_O) y[(size_t)r * 3 + col] = yv;
 				}
 			}
 		}
-		if(TRAIN && t < 4) {
-			/* columns 8..15 of dz5 are zero padding for the backward MMA k-tile */
-			tb.dz[5][(size_t)r0 * 16 + 8 + 2 * t] = __float2bfloat16_rn(0.0f);
-			tb.dz[5][(size_t)r0 * 16 + 9 + 2 * t] = __float2bfloat16_rn(0.0f);
-			tb.dz[5][(size_t)r1 * 16 + 8 + 2 * t] = __float2bfloat16_rn(0.0f);
-			tb.dz[5][(size_t)r1 * 16 + 9 + 2 * t] = __float2bfloat16_rn(0.0f);
+		__syncthreads();      /* the next tile overwrites the activations */
+	}
+	/* the block's sums */
+	for(int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+	if(lane == 0 && loss != 0.0f) atomicAdd(loss_out, loss / (float)(3 * n));
+	for(int o = 4; o < 32; o <<= 1) {
+		db5[0] += __shfl_xor_sync(0xffffffffu, db5[0], o);
+		db5[1] += __shfl_xor_sync(0xffffffffu, db5[1], o);
+	}
+	if(g == 0) {
+		if(2 * t < NRC_O) atomicAdd(&sdb[256 + 2 * t], db5[0]);
+		if(2 * t + 1 < NRC_O) atomicAdd(&sdb[256 + 2 * t + 1], db5[1]);
+	}
+	#pragma unroll
+	for(int half = 0; half < 2; half++) {
+		const int row = mt * 16 + g + 8 * half;
+		#pragma unroll
+		for(int j = 0; j < 14; j++) {
+			const int col = nh * 112 + j * 8 + 2 * t;
+			if(col < NRC_F) red_add2(grad + OFF_W1 + row * NRC_F + col, g1[j][2 * half], g1[j][2 * half + 1]);
+		}
+		#pragma unroll
+		for(int l = 0; l < 3; l++) {
+			const int off = l == 0 ? OFF_W2 : (l == 1 ? OFF_W3 : OFF_W4);
+			#pragma unroll
+			for(int j = 0; j < 4; j++) red_add2(grad + off + row * 64 + nh * 32 + j * 8 + 2 * t, gh[l][j][2 * half], gh[l][j][2 * half + 1]);
 		}
 	}
-	if(TRAIN) {
-		for(int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-		if(lane == 0 && loss != 0.0f) atomicAdd(tb.loss, loss / (float)(3 * n));
-		/* output-bias gradient: lanes with the same t hold the same columns */
-		for(int o = 4; o < 32; o <<= 1) {
-			db5[0] += __shfl_xor_sync(0xffffffffu, db5[0], o);
-			db5[1] += __shfl_xor_sync(0xffffffffu, db5[1], o);
-		}
-		if(g == 0) {
-			if(2 * t < NRC_O && db5[0] != 0.0f) atomicAdd(&tb.grad[OFF_B5 + 2 * t], db5[0]);
-			if(2 * t + 1 < NRC_O && db5[1] != 0.0f) atomicAdd(&tb.grad[OFF_B5 + 2 * t + 1], db5[1]);
-		}
-	}
+	if(g < NRC_O) red_add2(grad + OFF_W5 + g * 64 + warp * 8 + 2 * t, g5[0], g5[1]);
+	__syncthreads();
+	const int boff[5] = {OFF_B1, OFF_B2, OFF_B3, OFF_B4, OFF_B5};
+	for(int i = threadIdx.x; i < 256 + NRC_O; i += GR_THREADS) atomicAdd(&grad[boff[i >> 6] + (i & 63)], sdb[i]);
 }
+static_assert(OFF_W1 % 2 == 0 && OFF_W2 % 2 == 0 && OFF_W3 % 2 == 0 && OFF_W4 % 2 == 0 && OFF_W5 % 2 == 0 && NRC_F % 2 == 0,
+		"pairs of the packed gradient for vector atomics");
 
 /* ---- The inference and query forward on the 5th-generation tensor cores ----
  * tcgen05.mma with the accumulators in tensor memory (TMEM).  A CTA of 768
@@ -787,161 +953,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_forward_tc(NrcDev net, in
 	if(warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"((uint32_t)TC_TMEM_COLS) : "memory");
 }
 
-/* Backward pass, a warp per 16 samples: dH_{l-1} = dZ_l W_l, dZ_{l-1} =
- * dH_{l-1} where h_{l-1} > 0; stores dz[4..1] (BF16) and adds the bias
- * gradients (from the FP32 values) to the packed gradient. */
-__global__ void __launch_bounds__(128) k_nrc_backward(NrcDev net, int n, TrainBufs tb)
-{
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	__nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(smem_raw);
-	float *sdb = reinterpret_cast<float *>(sw + BWD_SMEM_BF16);   /* 4 x 64 bias sums of the block */
-	copy_to_shared(sw, net.w2t, BWD_SMEM_BF16);
-	for(int i = threadIdx.x; i < 256; i += blockDim.x) sdb[i] = 0.0f;
-	__syncthreads();
-	const __nv_bfloat16 *W2T = sw, *W3T = sw + (IMG_W3T - IMG_W2T), *W4T = sw + (IMG_W4T - IMG_W2T), *W5T = sw + (IMG_W5T - IMG_W2T);
-	int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	int g = lane >> 2, t = lane & 3;
-	int ntiles = (n + 15) >> 4;
-	for(int tile = blockIdx.x * 4 + warp; tile < ntiles; tile += gridDim.x * 4) {
-		int r0 = tile * 16 + g, r1 = r0 + 8;
-		/* dz5 as an A tile (k = outputs, 16 wide) */
-		uint32_t a5[4];
-		const __nv_bfloat16 *d5 = tb.dz[5];
-		a5[0] = *reinterpret_cast<const uint32_t *>(d5 + (size_t)r0 * 16 + 2 * t);
-		a5[1] = *reinterpret_cast<const uint32_t *>(d5 + (size_t)r1 * 16 + 2 * t);
-		a5[2] = *reinterpret_cast<const uint32_t *>(d5 + (size_t)r0 * 16 + 8 + 2 * t);
-		a5[3] = *reinterpret_cast<const uint32_t *>(d5 + (size_t)r1 * 16 + 8 + 2 * t);
-		Acc64 dz;
-		#pragma unroll
-		for(int nt = 0; nt < 8; nt++) {
-			dz.d[nt][0] = dz.d[nt][1] = dz.d[nt][2] = dz.d[nt][3] = 0.0f;
-			uint32_t w0, w1;
-			load_b(W5T, LD5T, nt * 8, 0, lane, w0, w1);
-			mma16816(dz.d[nt], a5, w0, w1);
-		}
-		const __nv_bfloat16 *WT[3] = {W4T, W3T, W2T};
-		for(int l = 4; l >= 1; l--) {
-			/* mask by h_l > 0, bias sums, BF16 store of dz_l */
-			const __nv_bfloat16 *h = tb.h[l];
-			__nv_bfloat16 *dzo = tb.dz[l];
-			#pragma unroll
-			for(int nt = 0; nt < 8; nt++) {
-				int col = nt * 8 + 2 * t;
-				uint32_t hv0 = *reinterpret_cast<const uint32_t *>(h + (size_t)r0 * 64 + col);
-				uint32_t hv1 = *reinterpret_cast<const uint32_t *>(h + (size_t)r1 * 64 + col);
-				if(!(bf16_lo(hv0) > 0.0f)) dz.d[nt][0] = 0.0f;
-				if(!(bf16_hi(hv0) > 0.0f)) dz.d[nt][1] = 0.0f;
-				if(!(bf16_lo(hv1) > 0.0f)) dz.d[nt][2] = 0.0f;
-				if(!(bf16_hi(hv1) > 0.0f)) dz.d[nt][3] = 0.0f;
-				*reinterpret_cast<uint32_t *>(dzo + (size_t)r0 * 64 + col) = pack_bf16(dz.d[nt][0], dz.d[nt][1]);
-				*reinterpret_cast<uint32_t *>(dzo + (size_t)r1 * 64 + col) = pack_bf16(dz.d[nt][2], dz.d[nt][3]);
-				float s0 = dz.d[nt][0] + dz.d[nt][2], s1 = dz.d[nt][1] + dz.d[nt][3];
-				for(int o = 4; o < 32; o <<= 1) {
-					s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-					s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-				}
-				if(g == 0) {
-					atomicAdd(&sdb[(l - 1) * 64 + col], s0);
-					atomicAdd(&sdb[(l - 1) * 64 + col + 1], s1);
-				}
-			}
-			if(l == 1) break;
-			uint32_t a[4][4];
-			acc_to_a(dz, a, false);
-			const __nv_bfloat16 *W = WT[4 - l];
-			#pragma unroll
-			for(int nt = 0; nt < 8; nt++) {
-				dz.d[nt][0] = dz.d[nt][1] = dz.d[nt][2] = dz.d[nt][3] = 0.0f;
-				#pragma unroll
-				for(int kt = 0; kt < 4; kt++) {
-					uint32_t w0, w1;
-					load_b(W, LDH, nt * 8, kt * 16, lane, w0, w1);
-					mma16816(dz.d[nt], a[kt], w0, w1);
-				}
-			}
-		}
-	}
-	__syncthreads();
-	const int boff[4] = {OFF_B1, OFF_B2, OFF_B3, OFF_B4};
-	for(int i = threadIdx.x; i < 256; i += blockDim.x) {
-		float v = sdb[i];
-		if(v != 0.0f) atomicAdd(&tb.grad[boff[i >> 6] + (i & 63)], v);
-	}
-}
-
-/* Weight gradient of one layer over the batch: dW[o][i] = sum_s dz[s][o] h[s][i],
- * M outputs (rows of dz, 16-wide storage stride DZS), N inputs (h stride HS).
- * Samples are split over blocks; each block stages 32 samples at a time,
- * transposed, in shared memory and its 8 warps hold TPW 16x8 output tiles
- * each; the block's sums are added to the packed gradient at OFF (only
- * o < MO, i < NI are real). */
-template <int MT, int NT, int TPW, int DZS, int HS>
-__global__ void __launch_bounds__(256) k_nrc_wgrad(int n, const __nv_bfloat16 *dz, const __nv_bfloat16 *h, float *grad, int off,
-		int MO, int NI, int per_block)
-{
-	enum { M = MT * 16, N = NT * 8, LDS = 40 };
-	__shared__ __align__(16) __nv_bfloat16 sdz[M * LDS];
-	__shared__ __align__(16) __nv_bfloat16 sh[N * LDS];
-	int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	int g = lane >> 2, t = lane & 3;
-	float acc[TPW][4];
-	#pragma unroll
-	for(int k = 0; k < TPW; k++) acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.0f;
-	int s_begin = blockIdx.x * per_block, s_end = min(n, s_begin + per_block);
-	for(int s0 = s_begin; s0 < s_end; s0 += 32) {
-		__syncthreads();
-		/* stage dz^T [M][32] and h^T [N][32] */
-		for(int i = threadIdx.x; i < 32 * M; i += blockDim.x) {
-			int s = i / M, o = i - s * M;
-			__nv_bfloat16 v = __float2bfloat16_rn(0.0f);
-			if(s0 + s < s_end && o < DZS) v = dz[(size_t)(s0 + s) * DZS + o];
-			sdz[o * LDS + s] = v;
-		}
-		for(int i = threadIdx.x; i < 32 * N; i += blockDim.x) {
-			int s = i / N, c = i - s * N;
-			__nv_bfloat16 v = __float2bfloat16_rn(0.0f);
-			if(s0 + s < s_end && c < HS) v = h[(size_t)(s0 + s) * HS + c];
-			sh[c * LDS + s] = v;
-		}
-		__syncthreads();
-		#pragma unroll
-		for(int k = 0; k < TPW; k++) {
-			int tile = warp * TPW + k;
-			if(tile >= MT * NT) break;
-			int mt = tile / NT, nt = tile - mt * NT;
-			#pragma unroll
-			for(int ks = 0; ks < 2; ks++) {
-				uint32_t a[4];
-				const __nv_bfloat16 *pa = sdz + (mt * 16 + g) * LDS + ks * 16 + 2 * t;
-				a[0] = *reinterpret_cast<const uint32_t *>(pa);
-				a[1] = *reinterpret_cast<const uint32_t *>(pa + 8 * LDS);
-				a[2] = *reinterpret_cast<const uint32_t *>(pa + 8);
-				a[3] = *reinterpret_cast<const uint32_t *>(pa + 8 * LDS + 8);
-				uint32_t b0, b1;
-				load_b(sh, LDS, nt * 8, ks * 16, lane, b0, b1);
-				mma16816(acc[k], a, b0, b1);
-			}
-		}
-	}
-	#pragma unroll
-	for(int k = 0; k < TPW; k++) {
-		int tile = warp * TPW + k;
-		if(tile >= MT * NT) break;
-		int mt = tile / NT, nt = tile - mt * NT;
-		int rows[2] = {mt * 16 + g, mt * 16 + g + 8};
-		#pragma unroll
-		for(int half = 0; half < 2; half++) {
-			int o = rows[half];
-			#pragma unroll
-			for(int c = 0; c < 2; c++) {
-				int i = nt * 8 + 2 * t + c;
-				float v = acc[k][2 * half + c];
-				if(o < MO && i < NI && v != 0.0f) atomicAdd(&grad[off + o * NI + i], v);
-			}
-		}
-	}
-}
-
 /* Adam on the FP32 master; the BF16 images are rewritten from it */
 __global__ void k_nrc_adam(float *p, float *m, float *v, float *grad, const int *step_dev, float lr)
 {
@@ -975,17 +986,9 @@ __global__ void k_nrc_images(const float *p, __nv_bfloat16 *img, float *bias, in
 			int o = r / LDH, c = r - o * LDH;
 			const int offs[3] = {OFF_W2, OFF_W3, OFF_W4};
 			if(c < 64) v = p[offs[l] + o * 64 + c];
-		} else if(i < IMG_W2T) {
+		} else {
 			int r = i - IMG_W5, o = r / LDH, c = r - o * LDH;
 			if(o < NRC_O && c < 64) v = p[OFF_W5 + o * 64 + c];
-		} else if(i < IMG_W5T) {
-			int l = (i - IMG_W2T) / (64 * LDH), r = i - IMG_W2T - l * 64 * LDH;
-			int in = r / LDH, o = r - in * LDH;
-			const int offs[3] = {OFF_W2, OFF_W3, OFF_W4};
-			if(o < 64) v = p[offs[l] + o * 64 + in];
-		} else {
-			int r = i - IMG_W5T, in = r / LD5T, o = r - in * LD5T;
-			if(o < NRC_O) v = p[OFF_W5 + o * 64 + in];
 		}
 		img[i] = __float2bfloat16_rn(v);
 	}
@@ -1017,8 +1020,6 @@ struct NrcState {
 	const float *g_x = nullptr, *g_t = nullptr;
 	float g_lr = 0.0f;
 	__nv_bfloat16 *img = nullptr;
-	__nv_bfloat16 *hbuf = nullptr;   /* training activations */
-	int hcap = 0;                    /* samples the training buffers hold */
 	int step = 0;
 	bool ready = false;
 	std::string err;
@@ -1040,7 +1041,6 @@ static NrcDev nrc_dev()
 	NrcDev d;
 	const __nv_bfloat16 *b = g_nrc.img;
 	d.w1 = b + IMG_W1; d.w2 = b + IMG_W2; d.w3 = b + IMG_W3; d.w4 = b + IMG_W4; d.w5 = b + IMG_W5;
-	d.w2t = b + IMG_W2T; d.w3t = b + IMG_W3T; d.w4t = b + IMG_W4T; d.w5t = b + IMG_W5T;
 	d.bias = g_nrc.bias;
 	return d;
 }
@@ -1063,9 +1063,7 @@ static int nrc_alloc()
 	NCK(cudaDeviceGetAttribute(&g_nrc.nsm, cudaDevAttrMultiProcessorCount, dev), "multiprocessors");
 	NCK(cudaFuncSetAttribute(k_nrc_forward_tc<FWD_INFER>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM), "smem");
 	NCK(cudaFuncSetAttribute(k_nrc_forward_tc<FWD_QUERY>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM), "smem");
-	NCK(cudaFuncSetAttribute(k_nrc_forward<FWD_TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			FWD_SMEM_BF16 * 2 + NRC_NBIAS * 4), "smem");
-	NCK(cudaFuncSetAttribute(k_nrc_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM_BF16 * 2 + 256 * 4), "smem");
+	NCK(cudaFuncSetAttribute(k_nrc_gradient, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM), "smem");
 	g_nrc.device = dev;
 	g_nrc.ready = true;
 	return 0;
@@ -1097,63 +1095,13 @@ static void nrc_init_host(uint64_t seed, std::vector<float> &p)
 	}
 }
 
-static int nrc_train_bufs(int n, TrainBufs &tb, cudaStream_t s)
+/* gradient of the loss over a batch, added into grad (8-byte aligned); the
+ * loss into *loss */
+static int nrc_gradient(int n, const float *x, const float *t, float *grad, float *loss, cudaStream_t s)
 {
-	int n16 = (n + 15) & ~15;
-	if(n16 > g_nrc.hcap) {
-		if(g_nrc.hbuf) cudaFree(g_nrc.hbuf);
-		g_nrc.hbuf = nullptr;
-		g_nrc.hcap = 0;
-		size_t per = NRC_FP + 4 * 64 + 4 * 64 + 16;
-		NCK(cudaMalloc(&g_nrc.hbuf, (size_t)n16 * per * sizeof(__nv_bfloat16)), "radiance cache training buffers");
-		g_nrc.hcap = n16;
-	}
-	__nv_bfloat16 *b = g_nrc.hbuf;
-	size_t cap = (size_t)g_nrc.hcap;
-	tb.h[0] = b; b += cap * NRC_FP;
-	for(int l = 1; l <= 4; l++) { tb.h[l] = b; b += cap * 64; }
-	tb.dz[0] = nullptr;
-	for(int l = 1; l <= 4; l++) { tb.dz[l] = b; b += cap * 64; }
-	tb.dz[5] = b;
-	tb.grad = g_nrc.grad;
-	tb.loss = g_nrc.loss;
-	(void)s;
-	return 0;
-}
-
-/* blocks for n samples at wpb warps per block (16 samples per warp); at
- * most a few resident waves, the kernels loop over the rest */
-static int nrc_grid(int n, int wpb)
-{
-	int tiles = (n + 15) / 16;
-	int blocks = (tiles + wpb - 1) / wpb;
-	int cap = 152 * 32 / wpb;
-	if(blocks > cap) blocks = cap;
-	return blocks < 1 ? 1 : blocks;
-}
-
-/* gradient of the loss over a batch into g_nrc.grad (which must hold zeros) */
-static int nrc_gradient(int n, const float *x, const float *t, float *y, cudaStream_t s)
-{
-	TrainBufs tb;
-	int r = nrc_train_bufs(n, tb, s);
-	if(r) return r;
-	NCK(cudaMemsetAsync(g_nrc.loss, 0, sizeof(float), s), "reset loss");
-	NrcDev d = nrc_dev();
-	k_nrc_forward<FWD_TRAIN><<<nrc_grid(n, NRC_FWD_THREADS / 32), NRC_FWD_THREADS, FWD_SMEM_BF16 * 2 + NRC_NBIAS * 4, s>>>(d, n, x, y, t,
-			tb, QueryOut());
-	k_nrc_backward<<<nrc_grid(n, 4), 128, BWD_SMEM_BF16 * 2 + 256 * 4, s>>>(d, n, tb);
-	/* samples per weight-gradient block: about two blocks per SM, at least
-	 * 128 (each block adds its partial dW with atomics) */
-	int per = (n + 2 * 152 - 1) / (2 * 152);
-	per = per < 128 ? 128 : (per + 31) & ~31;
-	int blocks = (n + per - 1) / per;
-	/* layer 1: 64 x 224 (216 real), layers 2-4: 64 x 64, layer 5: 16 x 64 (3 real) */
-	k_nrc_wgrad<4, 28, 14, 64, NRC_FP><<<blocks, 256, 0, s>>>(n, tb.dz[1], tb.h[0], g_nrc.grad, OFF_W1, 64, NRC_F, per);
-	k_nrc_wgrad<4, 8, 4, 64, 64><<<blocks, 256, 0, s>>>(n, tb.dz[2], tb.h[1], g_nrc.grad, OFF_W2, 64, 64, per);
-	k_nrc_wgrad<4, 8, 4, 64, 64><<<blocks, 256, 0, s>>>(n, tb.dz[3], tb.h[2], g_nrc.grad, OFF_W3, 64, 64, per);
-	k_nrc_wgrad<4, 8, 4, 64, 64><<<blocks, 256, 0, s>>>(n, tb.dz[4], tb.h[3], g_nrc.grad, OFF_W4, 64, 64, per);
-	k_nrc_wgrad<1, 8, 1, 16, 64><<<blocks, 256, 0, s>>>(n, tb.dz[5], tb.h[4], g_nrc.grad, OFF_W5, NRC_O, 64, per);
+	NCK(cudaMemsetAsync(loss, 0, sizeof(float), s), "reset loss");
+	int tiles = (n + GR_TILE - 1) / GR_TILE, cap = g_nrc.nsm > 0 ? g_nrc.nsm : 152;
+	k_nrc_gradient<<<tiles < cap ? tiles : cap, GR_THREADS, GR_SMEM, s>>>(nrc_dev(), n, x, t, grad, loss);
 	NCK(cudaGetLastError(), "radiance cache gradient");
 	return 0;
 }
@@ -1220,7 +1168,7 @@ int nrc_query(const int *count, int cap, const float *x, const float4 *w, float4
 int nrc_train(int n, const float *x, const float *t, float lr, cudaStream_t s)
 {
 	if(n <= 0) return 0;
-	int r = nrc_gradient(n, x, t, nullptr, s);
+	int r = nrc_gradient(n, x, t, g_nrc.grad, g_nrc.loss, s);
 	if(r) return r;
 	g_nrc.step++;
 	k_nrc_adam<<<64, 256, 0, s>>>(g_nrc.p, g_nrc.m, g_nrc.v, g_nrc.grad, g_nrc.step_dev, lr);
@@ -1230,8 +1178,8 @@ int nrc_train(int n, const float *x, const float *t, float lr, cudaStream_t s)
 }
 
 /* `steps` Adam steps over consecutive batches of `per` samples: captured
- * once as a CUDA graph (forward, backward, weight gradients, Adam and weight
- * images of every step: steps * NRC_TRAIN_KERNELS kernels) and replayed
+ * once as a CUDA graph (gradient, Adam and weight images of every step: steps *
+ * NRC_TRAIN_KERNELS kernels) and replayed
  * while the shape, buffers and rate stay the same */
 int nrc_train_steps(int steps, int per, const float *x, const float *t, float lr, cudaStream_t s)
 {
@@ -1242,9 +1190,7 @@ int nrc_train_steps(int steps, int per, const float *x, const float *t, float lr
 			cudaGraphExecDestroy(G.graph);
 			G.graph = nullptr;
 		}
-		TrainBufs tb;
-		int r = nrc_train_bufs(per, tb, s);   /* allocate before the capture */
-		if(r) return r;
+		int r = 0;
 		if(!G.cap) NCK(cudaStreamCreateWithFlags(&G.cap, cudaStreamNonBlocking), "capture stream");
 		cudaGraph_t g = nullptr;
 		NCK(cudaStreamBeginCapture(G.cap, cudaStreamCaptureModeThreadLocal), "capture training steps");
@@ -1361,13 +1307,18 @@ int sray_nrc_gradients(int n, const float *x, const float *t, float *grad, float
 	if(n <= 0 || !x || !t || !grad || !loss) { g_nrc.err = "bad arguments"; return nrc_err_ret(SRAY_EINVAL); }
 	if(!g_nrc.ready) { g_nrc.err = "radiance cache not initialised"; return nrc_err_ret(SRAY_ESTATE); }
 	cudaStream_t s = (cudaStream_t)stream;
+	/* straight into the caller's buffers (the gradient by way of the cache's
+	 * own where its pairs are not aligned) */
+	float *gr = (uintptr_t)grad % 8 ? g_nrc.grad : grad;
 	int r = 0;
-	cudaError_t e = cudaMemsetAsync(g_nrc.grad, 0, NRC_NPARAM * sizeof(float), s);
+	cudaError_t e = cudaMemsetAsync(gr, 0, NRC_NPARAM * sizeof(float), s);
 	if(e != cudaSuccess) r = nrc_fail(e, "reset gradient");
-	if(!r) r = nrc_gradient(n, x, t, nullptr, s);
-	if(!r) { e = cudaMemcpyAsync(grad, g_nrc.grad, NRC_NPARAM * sizeof(float), cudaMemcpyDeviceToDevice, s); if(e != cudaSuccess) r = nrc_fail(e, "copy gradient"); }
-	if(!r) { e = cudaMemcpyAsync(loss, g_nrc.loss, sizeof(float), cudaMemcpyDeviceToDevice, s); if(e != cudaSuccess) r = nrc_fail(e, "copy loss"); }
-	if(!r) { e = cudaMemsetAsync(g_nrc.grad, 0, NRC_NPARAM * sizeof(float), s); if(e != cudaSuccess) r = nrc_fail(e, "reset gradient"); }
+	if(!r) r = nrc_gradient(n, x, t, gr, loss, s);
+	if(!r && gr != grad) {
+		e = cudaMemcpyAsync(grad, gr, NRC_NPARAM * sizeof(float), cudaMemcpyDeviceToDevice, s);
+		if(e == cudaSuccess) e = cudaMemsetAsync(gr, 0, NRC_NPARAM * sizeof(float), s);
+		if(e != cudaSuccess) r = nrc_fail(e, "copy gradient");
+	}
 	if(!r) { e = cudaStreamSynchronize(s); if(e != cudaSuccess) r = nrc_fail(e, "gradients"); }
 	return nrc_err_ret(r);
 }

@@ -16,7 +16,7 @@ int nrc_infer(int n, const float *x, float *y, cudaStream_t s);
  * i < *count (at most cap), slot = the int in w[i].w */
 int nrc_query(const int *count, int cap, const float *x, const float4 *w, float4 *acc, cudaStream_t s);
 /* one Adam step on the batch (x[n][9], targets t[n][3]): NRC_TRAIN_KERNELS launches */
-#define NRC_TRAIN_KERNELS 9
+#define NRC_TRAIN_KERNELS 3
 int nrc_train(int n, const float *x, const float *t, float lr, cudaStream_t s);
 /* `steps` Adam steps over consecutive batches of `per` samples of (x, t),
  * replayed from a CUDA graph while the arguments stay the same */
