@@ -2155,6 +2155,18 @@ __global__ void k_primary_hits(DScene S, RayQueue q, const int4 *hits, int *obj,
 /* at most this many gather requests wait for the photon maps across waves */
 #define DEFER_MAX_REQS ((int64_t)1 << 28)
 
+/* Whether a frame's camera rays are traced as packets: where its image is
+ * large enough for the 8 x 4 pixels of a warp to see the same part of the
+ * scene.  A warp's packet walks everything any of its rays meets, in one
+ * chain: on small images that chain is the pass.  Object ids of moving scenes
+ * (100,000 / 400,000 triangles), packets against rays that each walk alone:
+ * 480x270 281 / 385 against 199 / 221 us, 640x360 256 / 433 against 259 /
+ * 310, 960x540 296 / 477 against 383 / 481, 1280x720 300 / 442 against 407 /
+ * 493, 1920x1080 473 / 664 against 486 / 590; frames of the small scene 817
+ * against 910 us at 960x540 and no difference at 480x270. */
+#define PACKET_MIN_PIXELS 400000
+static bool packet_image(int npix, int njobs) { return npix / (njobs > 1 ? njobs : 1) >= PACKET_MIN_PIXELS; }
+
 /* Rays per block of a streaming traversal (k_trace, k_shadow, k_cast) of n
  * rays: about a wave of resident blocks, each taking its lanes' next rays
  * from its own chunk, up to the limit of the caller's kind of pass.  A larger
@@ -3569,7 +3581,7 @@ int Renderer::render_pixels(long msec, float *fb, int fb_is_device, cudaStream_t
 			CK(cudaMemsetAsync(sqc, 0, sizeof(int), s), "reset shadow queue");
 			CK(sqb.ensure((size_t)n_rays * shadow_per_ray * sizeof(ShadowReq)), "shadow queue");
 			if(depth >= 1 && tune.sort_rays > 0 && n_rays >= tune.sort_rays && (r = sort_pass(cur, n_rays, s))) return r;
-			r = trace_rays(q[cur], n_rays, "trace", (prof_flags & 2) != 0, s, depth == 0);
+			r = trace_rays(q[cur], n_rays, "trace", (prof_flags & 2) != 0, s, depth == 0 && packet_image(npix, S.njobs));
 			if(r) return r;
 			ShadeOut so;
 			so.qo = q[cur ^ 1];
@@ -4500,7 +4512,7 @@ int sray_gpu_primary_hits(long msec, int *obj, int *prim, float *t, unsigned cha
 	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
 	R.q[0].count = cnt + 0;
 	k_camera<<<grid_for(npix, 256), 256, 0, s>>>(R.S, nullptr, 0, npix, 0, 1, R.q[0], R.acc.as<float4>(), R.ctr.as<DevCounters>());
-	if(R.trace_rays(R.q[0], npix, "trace", false, s, true)) { g_err = R.err; return SRAY_ECUDA; }
+	if(R.trace_rays(R.q[0], npix, "trace", false, s, packet_image(npix, 0))) { g_err = R.err; return SRAY_ECUDA; }
 	k_primary_hits<<<grid_for(npix, 256), 256, 0, s>>>(R.S, R.q[0], R.hits.as<int4>(), obj, prim, t, tie);
 	DevCounters hc;
 	e = cudaMemcpyAsync(&hc, R.ctr.p, sizeof hc, cudaMemcpyDeviceToHost, s);
