@@ -2622,6 +2622,23 @@ static void object_hierarchy(const BuildOctree &oct, const HostScene &sc, size_t
 	tn.insert(tn.end(), part.begin(), part.end());
 }
 
+/* object transforms and light positions for every time the frame can touch,
+ * evaluated from the keyframe tracks on the device while the host builds the
+ * frame's hierarchies (tlo and nt are set) */
+int Renderer::launch_xforms(cudaStream_t s)
+{
+	size_t nobj = sc.objs.size(), nlt = sc.lights.size();
+	CK(xf.ensure(nobj * nt * XF_STRIDE * sizeof(float) + 16), "transform table");
+	CK(light_pos.ensure(nlt * nt * 4 * sizeof(float) + 16), "light positions");
+	size_t nthr = (nobj + nlt) * (size_t)nt;
+	if(nthr) {
+		LAUNCH(*this, "xforms", s, k_xforms<<<(unsigned)((nthr + 127) / 128), 128, 0, s>>>(anims.as<DevAnim>(), key_t.as<int>(),
+				key_v.as<double>(), (int)nobj, (int)nlt, tlo, nt, xf.as<float>(), light_pos.as<float>()));
+		CK(cudaGetLastError(), "transform table");
+	}
+	return 0;
+}
+
 /* A scene set's frame: every scene's octree over its own objects (the
  * reference's Scene::build_tree, src/scene.cc:353-390, per scene) and object
  * hierarchy, side by side in one node table; their roots, lights and
@@ -2630,17 +2647,18 @@ int Renderer::build_frame_set(long bt0, long bt1, cudaStream_t s)
 {
 	t0 = (int)bt0;
 	t1 = (int)bt1;
+	int shutter = 0;
+	for(const SceneRange &rg : sc.ranges) shutter = std::max(shutter, rg.cam.shutter);
+	tlo = t0 - shutter - 2;
+	const int thi = t1 + shutter + 2;
+	nt = thi - tlo + 1;
+	if(int r = launch_xforms(s)) return r;
 	sc.bound_objects(t0, t1, opt);   /* the object bounds cache and the union's box; the scenes' octrees follow */
 	int ns = (int)sc.ranges.size();
 	std::vector<DevNode> nodes;
 	std::vector<int> slots, ohome_h(sc.objs.size(), 0);
 	std::vector<DevBvh4> tn;
 	scene_refs.assign(ns, DevSceneRef());
-	int shutter = 0;
-	for(int k = 0; k < ns; k++) shutter = std::max(shutter, sc.ranges[k].cam.shutter);
-	tlo = t0 - shutter - 2;
-	const int thi = t1 + shutter + 2;
-	nt = thi - tlo + 1;
 	for(int k = 0; k < ns; k++) {
 		const SceneRange &rg = sc.ranges[k];
 		DevSceneRef &R = scene_refs[k];
@@ -2671,15 +2689,6 @@ int Renderer::build_frame_set(long bt0, long bt1, cudaStream_t s)
 		for(int i = 0; i < rg.nobj; i++) ohome_h[rg.obj0 + i] = hm[i];
 	}
 	scene_root = ns > 0 ? scene_refs[0].sroot : 0;
-	size_t nobj = sc.objs.size(), nlt = sc.lights.size();
-	CK(xf.ensure(nobj * nt * XF_STRIDE * sizeof(float) + 16), "transform table");
-	CK(light_pos.ensure(nlt * nt * 4 * sizeof(float) + 16), "light positions");
-	size_t nthr = (nobj + nlt) * (size_t)nt;
-	if(nthr) {
-		LAUNCH(*this, "xforms", s, k_xforms<<<(unsigned)((nthr + 127) / 128), 128, 0, s>>>(anims.as<DevAnim>(), key_t.as<int>(),
-				key_v.as<double>(), (int)nobj, (int)nlt, tlo, nt, xf.as<float>(), light_pos.as<float>()));
-		CK(cudaGetLastError(), "transform table");
-	}
 	std::vector<float> cm((size_t)ns * nt * 12);
 	for(int k = 0; k < ns; k++) {
 		for(int t = 0; t < nt; t++) {
@@ -2715,32 +2724,22 @@ int Renderer::build_frame(long bt0, long bt1, cudaStream_t s)
 	scene_refs.clear();
 	t0 = (int)bt0;
 	t1 = (int)bt1;
+	const int shutter = sc.cam.shutter;
+	tlo = t0 - shutter - 2;
+	const int thi = t1 + shutter + 2;
+	nt = thi - tlo + 1;
+	if(int r = launch_xforms(s)) return r;
 	sc.build_tree(t0, t1, opt);
 	std::vector<DevNode> nodes;
 	std::vector<int> slots;
 	std::vector<int> index_of;
 	flatten_octree(sc.oct, nodes, slots, &index_of);
 	scene_root = sc.oct.nodes.empty() ? 0 : (int)(nodes.size() - sc.oct.nodes.size());
-	const int shutter = sc.cam.shutter;
-	tlo = t0 - shutter - 2;
-	const int thi = t1 + shutter + 2;
-	nt = thi - tlo + 1;
 	std::vector<DevBvh4> tn;
 	std::vector<int> ohome_h;
 	if(!sc.oct.nodes.empty() && !sc.objs.empty()) {
 		object_hierarchy(sc.oct, sc, sc.objs.size(), 0, tlo, thi, 0, tn);
 		octree_homes_boxes(sc.oct, sc.oct_boxes, index_of, ohome_h);
-	}
-	/* object transforms and light positions for every time the frame can
-	 * touch, evaluated from the keyframe tracks on the device */
-	size_t nobj = sc.objs.size(), nlt = sc.lights.size();
-	CK(xf.ensure(nobj * nt * XF_STRIDE * sizeof(float) + 16), "transform table");
-	CK(light_pos.ensure(nlt * nt * 4 * sizeof(float) + 16), "light positions");
-	size_t nthr = (nobj + nlt) * (size_t)nt;
-	if(nthr) {
-		LAUNCH(*this, "xforms", s, k_xforms<<<(unsigned)((nthr + 127) / 128), 128, 0, s>>>(anims.as<DevAnim>(), key_t.as<int>(),
-				key_v.as<double>(), (int)nobj, (int)nlt, tlo, nt, xf.as<float>(), light_pos.as<float>()));
-		CK(cudaGetLastError(), "transform table");
 	}
 	std::vector<float> cm((size_t)nt * 12);
 	for(int t = 0; t < nt; t++) {

@@ -303,6 +303,7 @@ struct Renderer {
 
 	int upload_scene(cudaStream_t s);
 	int build_frame(long t0, long t1, cudaStream_t s);
+	int launch_xforms(cudaStream_t s);
 	int shoot(cudaStream_t s, int *nc, int *ng);
 	/* overlap_photons: shoot the photon maps on the photon stream while the
 	 * first bounce's closest hits, shading and shadow rays run, the gathers
