@@ -252,11 +252,9 @@ __device__ __forceinline__ bool gen_dirs(bool need, const uint32_t *bits, sray_r
  * k_proj_view takes a thread per (sample, box), k_proj_mark a block: the
  * corners' tests (33 rows of 65, a warp per row) and, per cell they set, the
  * smallest (sample, box, place) over all blocks.  k_proj_cover, a block per
- * map, gives the bits, sorts the set cells by that order and sums.  On the
- * host, a thread per light, this took 1.9 ms for three lights over 201
- * objects before the first photon left (1.4 ms for six frames of 25); here
- * under 80 us (120 us).  What bounds it is the latency of its chains: double
- * arithmetic, the sort, the ordered sum. */
+ * map, gives the bits and the sum.  On the host, a thread per light, this
+ * took 1.9 ms for three lights over 201 objects before the first photon left
+ * (1.4 ms for six frames of 25 objects); here under 50 us (80 us). */
 struct ProjSample {
 	double lp[3];
 	int box0, nbox;       /* the boxes it sees */
@@ -392,78 +390,52 @@ __global__ void __launch_bounds__(128) k_proj_mark(const ProjSample *samples, in
 	}
 }
 
-/* v[0] + v[1] + ... in double, each addition rounded, by a warp.  While the
- * sum stays within one power of two it is a multiple of the same unit, so an
- * addition adds the term rounded to that unit: 32 terms at a time, as
- * integers, by a scan.  A term half way between two units rounds to an even
- * sum; those are taken in their order.  32 terms over which the sum leaves
- * its power of two are added one by one.  Terms are positive.  (2,048
- * dependent double additions take 65 us on this GPU.) */
-__device__ __forceinline__ double ordered_sum(const double *v, int n, int lane)
-{
-	const unsigned FULL = 0xffffffffu;
-	double c = 0.0;
-	for(int i0 = 0; i0 < n; i0 += 32) {
-		const double s = i0 + lane < n ? v[i0 + lane] : 0.0;
-		const long long cb = __double_as_longlong(c), sb = __double_as_longlong(s);
-		const int ce = (int)(cb >> 52), se = (int)(sb >> 52);       /* biased exponents (signs are 0) */
-		const long long cm = (cb & 0xfffffffffffffll) | 0x10000000000000ll, sm = (sb & 0xfffffffffffffll) | 0x10000000000000ll;
-		const int shift = ce - se;
-		const bool slow = ce == 0 || (se && shift < 1) || (!se && sb != 0);
-		bool tie = false;
-		long long q = 0;
-		if(!slow && se && shift <= 53) {
-			const long long half = 1ll << (shift - 1), rem = sm & ((1ll << shift) - 1);
-			q = (sm >> shift) + (rem > half ? 1 : 0);
-			tie = rem == half;
-		}
-		long long incl = q;
-		for(int o = 1; o < 32; o <<= 1) {
-			long long u = __shfl_up_sync(FULL, incl, o);
-			if(lane >= o) incl += u;
-		}
-		/* the ties in order: up when the sum so far is odd */
-		int up = 0;
-		for(unsigned m = __ballot_sync(FULL, tie); m; m &= m - 1)
-			up += ((int)cm + __shfl_sync(FULL, (int)incl, __ffs(m) - 1) + up) & 1;
-		const long long total = __shfl_sync(FULL, incl, 31) + up;
-		if(__any_sync(FULL, slow) || cm + total >= 0x20000000000000ll) {
-			for(int k = 0; k < 32; k++) c += __shfl_sync(FULL, s, k);
-		} else {
-			c = __longlong_as_double(((long long)ce << 52) | ((cm + total) & 0xfffffffffffffll));
-		}
-	}
-	return c;
-}
-
+/* A block per map: its bits and its coverage.  The coverage that counts is the
+ * ordered double sum rounded to float.  Any order of summation is within
+ * 2^-41 of it (2,048 terms, each addition within 2^-53), so a sum in parallel
+ * gives that float unless it lies within 2^-40 of where floats round; then
+ * (once in some 30,000 maps) the cells are sorted by the order in which they
+ * were set and added one by one, 2,048 dependent additions taking 65 us. */
 __global__ void __launch_bounds__(1024) k_proj_cover(const unsigned long long *first, const ProjTables *tables, uint32_t *bits, float *cov)
 {
 	__shared__ unsigned long long key[PROJ_CELLS];
-	__shared__ double share[PROJ_CELLS];
-	__shared__ int nset;
+	__shared__ double part[32];
+	__shared__ int nset, unsure;
+	const unsigned FULL = 0xffffffffu;
 	const int t = threadIdx.x, lane = t & 31;
 	const unsigned long long *map = first + (size_t)blockIdx.x * PROJ_SLOT;
 	const bool whole = map[PROJ_CELLS] == 0;
 	if(t == 0) nset = 0;
 	__syncthreads();
+	double c = 0.0;
 	for(int k = 0; k < 2; k++) {
 		const int cell = k * 1024 + t;
 		const unsigned long long v = map[cell];
 		const bool set = whole || v != PROJ_NONE;
-		const unsigned b = __ballot_sync(0xffffffffu, set);
+		const unsigned b = __ballot_sync(FULL, set);
 		if(lane == 0) {
 			bits[(size_t)blockIdx.x * 64 + (cell >> 5)] = b;
 			atomicAdd(&nset, __popc(b));
 		}
 		key[cell] = v;
+		if(set) c += tables->share[cell];
+	}
+	for(int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
+	if(lane == 0) part[t >> 5] = c;
+	__syncthreads();
+	if(t < 32) {
+		c = part[lane];
+		for(int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
+		if(t == 0) {
+			const float f = whole ? 1.0f : (nset == 0 ? 0.0f : (float)fmin(c, 1.0));
+			const double lo = c * (1.0 - 1.0 / 1099511627776.0), hi = c * (1.0 + 1.0 / 1099511627776.0);
+			unsure = !whole && nset > 0 && ((float)fmin(lo, 1.0) != f || (float)fmin(hi, 1.0) != f);
+			cov[blockIdx.x] = f;
+		}
 	}
 	__syncthreads();
-	if(whole || nset == 0) {
-		if(t == 0) cov[blockIdx.x] = whole ? 1.0f : 0.0f;
-		return;
-	}
-	/* bitonic sort of the cells by the order in which they were set (unset
-	 * ones last); a key's low bits are its cell */
+	if(!unsure) return;
+	/* bitonic sort (unset cells last); a key's low bits are its cell */
 	for(int size = 2; size <= PROJ_CELLS; size <<= 1) {
 		for(int step = size >> 1; step > 0; step >>= 1) {
 			const int i = 2 * t - (t & (step - 1));
@@ -476,11 +448,10 @@ __global__ void __launch_bounds__(1024) k_proj_cover(const unsigned long long *f
 			__syncthreads();
 		}
 	}
-	for(int i = t; i < nset; i += 1024) share[i] = tables->share[key[i] & (PROJ_CELLS - 1)];
-	__syncthreads();
-	if(t < 32) {
-		const double c = ordered_sum(share, nset, t);
-		if(t == 0) cov[blockIdx.x] = (float)(c < 0.0 ? 0.0 : (c > 1.0 ? 1.0 : c));
+	if(t == 0) {
+		c = 0.0;
+		for(int i = 0; i < nset; i++) c += tables->share[key[i] & (PROJ_CELLS - 1)];
+		cov[blockIdx.x] = (float)(c < 0.0 ? 0.0 : (c > 1.0 ? 1.0 : c));
 	}
 }
 
