@@ -396,6 +396,15 @@ struct TStack {
 	float te[SRAY_STACK];
 };
 
+/* the hierarchy walk's stack: an entry and its distance in one 8-byte word,
+ * so that a push or a pop is one access to local memory (stacks of a warp's
+ * lanes stand at different heights: each access is its own sector) */
+struct WStack {
+	uint2 e[SRAY_STACK];
+	__device__ __forceinline__ void put(int k, int node, float te) { e[k] = make_uint2((unsigned)node, __float_as_uint(te)); }
+	__device__ __forceinline__ uint2 get(int k) const { return e[k]; }
+};
+
 /* test the children of an inner node and push the hit ones far to near.
  * A child's box is one octant of the node's box split at `mid`, so its slab
  * parameters are three of the nine plane parameters (mn, mid, mx per axis)
@@ -872,11 +881,62 @@ __device__ __forceinline__ RayT object_ray(const DScene &S, int o, int ti, V3 wo
 enum { WALK_GOES = 0, WALK_HIT = 1, WALK_UNDECIDED = 2, WALK_OVERFLOW = 3 };
 enum { WALK_NODE = 0, WALK_LEAF = 1, WALK_OBJECT = 2, WALK_END = 3 };
 
-template <bool COUNT, bool ANY, bool SORT = true>
+/* The ray in world space and its box constants: needed where an object is
+ * entered or left and at the end, not by the steps between.  In registers, or
+ * (SharedWorld) in the thread's column of a block's shared memory: the stream
+ * kernels are held to 64 registers for 8 blocks per SM, and spilled 150-220
+ * bytes of theirs with these 15 values in them (60-110 without).  With the
+ * stack's 8-byte entries: 1,000,003 incoherent rays over the 1.26M-triangle
+ * terrain 652 -> 625 us, 1080p frames of it 15.75 -> 15.47 ms.  (The stack's
+ * top 4 or 8 entries in shared memory too: 614 us, but the frames 15.63.) */
+struct RegWorld {
+	V3 o_, d_;
+	RayC c_;
+	__device__ __forceinline__ void put(V3 o, V3 d, const RayC &c) { o_ = o; d_ = d; c_ = c; }
+	__device__ __forceinline__ V3 o() const { return o_; }
+	__device__ __forceinline__ V3 d() const { return d_; }
+	__device__ __forceinline__ RayC c() const { return c_; }
+};
+
+#define WORLD_WORDS 15
+struct SharedWorld {
+	float *p;             /* [WORLD_WORDS][SRAY_TRACE_THREADS], this thread's column */
+	__device__ __forceinline__ V3 at(int k) const
+	{
+		return mk(p[k * SRAY_TRACE_THREADS], p[(k + 1) * SRAY_TRACE_THREADS], p[(k + 2) * SRAY_TRACE_THREADS]);
+	}
+	__device__ __forceinline__ void set(int k, V3 v)
+	{
+		p[k * SRAY_TRACE_THREADS] = v.x;
+		p[(k + 1) * SRAY_TRACE_THREADS] = v.y;
+		p[(k + 2) * SRAY_TRACE_THREADS] = v.z;
+	}
+	__device__ __forceinline__ void put(V3 o, V3 d, const RayC &c)
+	{
+		set(0, o);
+		set(3, d);
+		set(6, c.inv);
+		set(9, c.cn);
+		set(12, c.cf);
+	}
+	__device__ __forceinline__ V3 o() const { return at(0); }
+	__device__ __forceinline__ V3 d() const { return at(3); }
+	__device__ __forceinline__ RayC c() const
+	{
+		RayC c;
+		c.inv = at(6);
+		c.cn = at(9);
+		c.cf = at(12);
+		c.neg = (c.inv.x < 0.0f ? 1u : 0u) | (c.inv.y < 0.0f ? 2u : 0u) | (c.inv.z < 0.0f ? 4u : 0u);
+		return c;
+	}
+};
+
+template <bool COUNT, bool ANY, bool SORT = true, class World = RegWorld>
 struct Walk {
-	V3 wo, wd;            /* the ray */
-	RayT r, wr;           /* in the current space, in world space */
-	RayC rc, wc;
+	World world;
+	V3 ro, rd;            /* the ray in the current space */
+	RayC rc;
 	float best;
 	int ti;
 	int bobj, bprim, bslot;
@@ -885,14 +945,12 @@ struct Walk {
 
 	__device__ __forceinline__ void start(const DScene &S, V3 o, V3 d, int time, int2 roots)
 	{
-		wo = o;
-		wd = d;
 		ti = time_index(S, time);
-		wr = make_ray(wo, wd);
 		const DevNode &sroot = S.snodes[roots.x];
-		wc = make_rayc(wr, box_bound(sroot.mn, sroot.mx));
-		r = wr;
-		rc = wc;
+		rc = make_rayc(make_ray(o, d), box_bound(sroot.mn, sroot.mx));
+		world.put(o, d, rc);
+		ro = o;
+		rd = d;
 		best = ANY ? 1.0f : FLT_MAX;
 		bobj = bprim = bslot = -1;
 		eq = false;
@@ -906,7 +964,7 @@ struct Walk {
 	__device__ __forceinline__ int kind() const { return cur == BVH_NONE ? WALK_END : (cur >= 0 ? WALK_NODE : (inst ? WALK_LEAF : WALK_OBJECT)); }
 
 	/* the next entry that can hold a closer hit */
-	__device__ __forceinline__ void pop(const TStack &st)
+	__device__ __forceinline__ void pop(const WStack &st)
 	{
 		cur = BVH_NONE;
 		while(sp > 0) {
@@ -914,12 +972,12 @@ struct Walk {
 			if(inst && k < inst_base) {   /* the instance's entries are done */
 				inst = false;
 				iobj = -1;
-				r = wr;
-				rc = wc;
+				rc = world.c();
 			}
 			sp = k;
-			if(ANY || st.te[k] <= best) {
-				cur = st.node[k];
+			const uint2 e = st.get(k);
+			if(ANY || __uint_as_float(e.y) <= best) {
+				cur = (int)e.x;
 				break;
 			}
 		}
@@ -940,11 +998,11 @@ struct Walk {
 	}
 
 	/* enter object ~cur, or test it where it is a quadric */
-	__device__ __forceinline__ int step_object(const DScene &S, const TStack &st, TraceCounters *tc)
+	__device__ __forceinline__ int step_object(const DScene &S, const WStack &st, TraceCounters *tc)
 	{
 		int o = ~cur;
 		const DevObj ob = S.objs[o];
-		RayT orr = object_ray(S, o, ti, wo, wd);
+		RayT orr = object_ray(S, o, ti, world.o(), world.d());
 		if(ob.type != 2) {
 			if(COUNT) tc->prims++;
 			float t;
@@ -960,7 +1018,8 @@ struct Walk {
 			float te;
 			const DevNode &rn = S.mnodes[ob.mesh_root];
 			if(box_hit(rn.mn, rn.mx, orr, te) && (ANY || !SRAY_PRUNE(te, best))) {
-				r = orr;
+				ro = orr.o;
+				rd = orr.d;
 				rc = make_rayc(orr, box_bound(rn.mn, rn.mx));
 				inst = true;
 				inst_base = sp;
@@ -974,11 +1033,14 @@ struct Walk {
 	}
 
 	/* a leaf of the mesh hierarchy: its faces */
-	__device__ __forceinline__ int step_leaf(const DScene &S, const TStack &st, TraceCounters *tc)
+	__device__ __forceinline__ int step_leaf(const DScene &S, const WStack &st, TraceCounters *tc)
 	{
 		unsigned v = ~(unsigned)cur;
 		int start = (int)(v >> 4), cnt = (int)(v & 15u);
 		const float4 *tp = reinterpret_cast<const float4 *>(S.btris + start);
+		RayT r;
+		r.o = ro;
+		r.d = rd;
 		for(int k = 0; k < cnt; k++) {
 			float4 a = __ldg(tp + 3 * k), b = __ldg(tp + 3 * k + 1), c = __ldg(tp + 3 * k + 2);
 			if(COUNT) tc->prims++;
@@ -995,7 +1057,7 @@ struct Walk {
 	 * four children in one 128-byte line; the hit ones (nodes, leaves, or
 	 * objects) are visited nearest first, each leaf and object in a step of
 	 * its own so that the lanes of a warp stay together */
-	__device__ __forceinline__ int step_node(const DScene &S, TStack &st, TraceCounters *tc)
+	__device__ __forceinline__ int step_node(const DScene &S, WStack &st, TraceCounters *tc)
 	{
 		const float4 *np = reinterpret_cast<const float4 *>((inst ? S.bnodes : S.tnodes) + cur);
 		const NodePlanes pl = node_planes(np, rc);
@@ -1019,7 +1081,7 @@ struct Walk {
 				if(key[k] == INFINITY) continue;
 				if(nxt != BVH_NONE) {
 					if(sp >= SRAY_STACK) return WALK_OVERFLOW;
-					st.node[sp++] = nxt;
+					st.put(sp++, nxt, 0.0f);
 				}
 				nxt = ref[k];
 			}
@@ -1042,9 +1104,7 @@ struct Walk {
 		for(int k = 3; k >= 1; k--) {
 			if(key[k] == INFINITY) continue;
 			if(sp >= SRAY_STACK) return WALK_OVERFLOW;
-			st.node[sp] = ref[k];
-			if(!ANY) st.te[sp] = key[k];   /* any hit visits every entry */
-			sp++;
+			st.put(sp++, ref[k], key[k]);
 		}
 		cur = ref[0];
 		return WALK_GOES;
@@ -1056,6 +1116,7 @@ struct Walk {
 	{
 		if(bobj < 0) return true;
 		if(!ANY && eq) return false;
+		const V3 wo = world.o(), wd = world.d();
 		if(bslot >= 0 && !octree_reaches(S.mnodes, S.mprim, __ldg(S.bhome + bslot), object_ray(S, bobj, ti, wo, wd), bprim, best, !ANY))
 			return false;
 		return octree_reaches(S.snodes, S.sslots, __ldg(S.ohome + bobj), make_ray(wo, wd), bobj, best, !ANY);
@@ -1078,7 +1139,7 @@ __device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, in
 	if(roots.x < 0) return ANY ? 0 : 1;
 	if(roots.y < 0) return ANY ? 2 : 0;
 	Walk<COUNT, ANY, SORT> w;
-	TStack st;
+	WStack st;
 	w.start(S, wo, wd, time, roots);
 	while(w.cur != BVH_NONE) {
 		int res;
@@ -1112,12 +1173,13 @@ __device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, in
  * directions over the 1.26M-triangle terrain: 1.19 ms, against 1.89 with a
  * ray per thread. */
 template <int REFILL, bool COUNT, bool ANY, bool SORT, class Load, class Done>
-__device__ __forceinline__ void walk_stream(const DScene &S, int *next, int end, Load load, Done done, TraceCounters *tc, int *overflow)
+__device__ __forceinline__ void walk_stream(const DScene &S, float *world, int *next, int end, Load load, Done done, TraceCounters *tc, int *overflow)
 {
 	const unsigned FULL = 0xffffffffu;
 	const int lane = threadIdx.x & 31;
-	Walk<COUNT, ANY, SORT> w;
-	TStack st;
+	Walk<COUNT, ANY, SORT, SharedWorld> w;
+	WStack st;
+	w.world.p = world;
 	w.cur = BVH_NONE;
 	int ri = -1;                 /* the lane's ray */
 	int res = WALK_GOES;

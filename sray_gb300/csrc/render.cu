@@ -156,6 +156,7 @@ __global__ void k_ray_permute(RayQueue in, const unsigned *vals, int n, RayQueue
 template <bool COUNT>
 __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQueue q, int chunk, int4 *hits, DevCounters *ctr, int *fb)
 {
+	__shared__ float world[WORLD_WORDS * SRAY_TRACE_THREADS];
 	__shared__ int next;
 	const int n = *q.count;
 	const int first = blockIdx.x * chunk;
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQu
 	__syncthreads();
 	TraceCounters tc = {0, 0};
 	int overflow = 0;
-	walk_stream<TRACE_REFILL, COUNT, false, true>(S, &next, min(first + chunk, n),
+	walk_stream<TRACE_REFILL, COUNT, false, true>(S, world + threadIdx.x, &next, min(first + chunk, n),
 			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
 				float4 o4 = q.o[i], d4 = q.d[i];
 				o = mk(o4.x, o4.y, o4.z);
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQu
 				scene = S.nscenes > 1 ? pixel_scene(S, __float_as_int(q.w[i].w)) : -1;
 				return i;
 			},
-			[&](int i, int sure, const Walk<COUNT, false, true> &w) {
+			[&](int i, int sure, const Walk<COUNT, false, true, SharedWorld> &w) {
 				if(!sure) fb[1 + atomicAdd(fb, 1)] = i;
 				else hits[i] = w.bobj >= 0 ? make_int4(__float_as_int(w.best), w.bobj, w.bprim, 0) : make_int4(__float_as_int(FLT_MAX), -1, -1, 0);
 			}, &tc, &overflow);
@@ -1222,6 +1223,7 @@ template <bool SORT = true, bool COUNT = false>
 __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow(DScene S, const ShadowReq *sq, const int *sq_count, int chunk, float4 *acc,
 		DevCounters *ctr, int *fb)
 {
+	__shared__ float world[WORLD_WORDS * SRAY_TRACE_THREADS];
 	__shared__ int next;
 	const int n = *sq_count;
 	if(blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->rays[2], (unsigned long long)n);
@@ -1231,7 +1233,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow(DScene S, cons
 	__syncthreads();
 	TraceCounters tc = {0, 0};
 	int overflow = 0;
-	walk_stream<SHADOW_REFILL, COUNT, true, SORT>(S, &next, min(first + chunk, n),
+	walk_stream<SHADOW_REFILL, COUNT, true, SORT>(S, world + threadIdx.x, &next, min(first + chunk, n),
 			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
 				float4 a = sq[i].a, b = sq[i].b;
 				o = mk(a.x, a.y, a.z);
@@ -1240,7 +1242,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow(DScene S, cons
 				scene = S.nscenes > 1 ? __float_as_int(sq[i].w.w) : -1;
 				return i;
 			},
-			[&](int i, int res, const Walk<COUNT, true, SORT> &) {
+			[&](int i, int res, const Walk<COUNT, true, SORT, SharedWorld> &) {
 				if(res == 2) {
 					fb[1 + atomicAdd(fb, 1)] = i;
 				} else if(res == 0) {
@@ -2082,12 +2084,13 @@ struct CastRays {
 
 __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRays R, int n, int chunk, DevCounters *ctr, int *fb)
 {
+	__shared__ float world[WORLD_WORDS * SRAY_TRACE_THREADS];
 	__shared__ int next;
 	const int first = blockIdx.x * chunk;
 	if(threadIdx.x == 0) next = first;
 	__syncthreads();
 	int overflow = 0;
-	walk_stream<CAST_REFILL, false, false, true>(S, &next, min(first + chunk, n),
+	walk_stream<CAST_REFILL, false, false, true>(S, world + threadIdx.x, &next, min(first + chunk, n),
 			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
 				o = R.o(i);
 				d = R.d(i);
@@ -2095,7 +2098,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRa
 				scene = -1;
 				return i;
 			},
-			[&](int i, int sure, const Walk<false, false, true> &w) {
+			[&](int i, int sure, const Walk<false, false, true, SharedWorld> &w) {
 				if(!sure) fb[1 + atomicAdd(fb, 1)] = i;
 				else R.put(i, w.bobj, w.bprim, w.best, 0);
 			}, nullptr, &overflow);
