@@ -539,8 +539,11 @@ static_assert(OFF_W1 % 2 == 0 && OFF_W2 % 2 == 0 && OFF_W3 % 2 == 0 && OFF_W4 % 
  * there, two BF16 per column); the biases come with the products (a BF16 pair
  * per row of each weight tile against a constant pair in the operand).  The
  * features are read only by the first layer, so a group encodes its next
- * tile while the MMAs of the current one's layers 2-5 run (a quarter of the
- * encoding after each of their issues), and the three groups interleave.
+ * tile while the MMAs of the current one's layers 2-4 run (a third of the
+ * encoding after each of their issues), and issues that tile's first layer
+ * together with the current one's fifth: four waits per tile (the chain of
+ * round trips is what bounds a tile; five waits took 362 us for a call of
+ * 4,194,304 samples, four 340).  The three groups interleave.
  *
  * Shared memory, canonical K-major layouts without swizzle (8-row x 16-byte
  * core matrices; a descriptor's leading byte offset steps along K, its
@@ -867,58 +870,48 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_forward_tc(NrcDev net, in
 	uint32_t phase = 0;
 	bool ok = true;        /* this thread's waits so far */
 	bool agreed = true;    /* the group's, at its last barrier */
+	/* A round of a group: layer 5 of its tile and layer 1 of its next one in
+	 * one issue (they share no operand), then layers 2, 3 and 4 of that one,
+	 * under whose MMAs (which read the hidden operand, not the features) the
+	 * features of the one after it are encoded.  xv holds the inputs of the
+	 * tile to encode next. */
 	const int ntiles = (n + 127) >> 7, stride = gridDim.x * TC_NG;
-	/* The encoding of a group's next tile runs under the MMAs of the
-	 * current tile's layers 2-5 (which read the hidden operand, not the
-	 * features): a quarter of it after each of their issues.  xv holds the
-	 * inputs of the tile to encode next. */
-	int tile = blockIdx.x * TC_NG + g;
+	int next = blockIdx.x * TC_NG + g;
+	int row = -1;          /* this thread's sample in the tile before next, -1 none */
 	float xv[TC_XH];
-	tc_inputs(xv, x, n, tile * 128 + tid, hf);
-	if(tile < ntiles) tc_encode_part<0, 7>(hf, A1, tid, xv);
-	for(; tile < ntiles; tile += stride) {
-		const int row = tile * 128 + tid;
-		const bool more = tile + stride < ntiles;
-		tc_inputs(xv, x, n, row + stride * 128, hf);
-		#pragma unroll
-		for(int l = 0; l < 5; l++) {
-			proxy_fence();
-			tc_fence_before();
-			agreed = group_all(g, ok);
-			if(!agreed) break;
-			if(leader) {
-				tc_fence_after();
-				if(l == 0) {
-					for(int j = 0; j < NRC_FP / 16 - 1; j++)
-						tc_mma(tD, tc_desc(sA1 + 2 * j * TC_CHUNK, TC_CHUNK, 128), tc_desc(sW1 + j * 256, 128, (NRC_FP / 8) * 128), id64, j);
-					/* the last K step: chunk 26, then the constant block's bias pairs */
-					const uint32_t a = sA1 + (NRC_F / 8 - 1) * TC_CHUNK;
-					tc_mma(tD, tc_desc(a, sK - a, 128), tc_desc(sW1 + (NRC_FP / 16 - 1) * 256, 128, (NRC_FP / 8) * 128), id64, 1);
-				} else {
-					const uint32_t sW = l < 4 ? sbase + TC_W2 + (uint32_t)(l - 1) * (TC_W3 - TC_W2) : sW5;   /* W2, W3, W4 back to back */
-					const uint32_t td = l < 4 ? tD : tO, id = l < 4 ? id64 : id16;
-					for(int j = 0; j < TC_KH / 16; j++)
-						tc_mma_ta(td, tA + (uint32_t)(8 * j), tc_desc(sW + j * 256, 128, TC_KH / 8 * 128), id, j);
-				}
-				tc_commit(mbar);
-			}
+	tc_inputs(xv, x, n, next * 128 + tid, hf);
+	if(next < ntiles) tc_encode_part<0, 7>(hf, A1, tid, xv);
+	while(next < ntiles || row >= 0) {
+		const bool more = next < ntiles;
+		proxy_fence();
+		tc_fence_before();
+		agreed = group_all(g, ok);
+		if(!agreed) break;
+		if(leader) {
+			tc_fence_after();
+			if(row >= 0)
+				for(int j = 0; j < TC_KH / 16; j++)
+					tc_mma_ta(tO, tA + (uint32_t)(8 * j), tc_desc(sW5 + j * 256, 128, TC_KH / 8 * 128), id16, j);
 			if(more) {
-				if(l == 1) tc_encode_part<0, 2>(hf, A1, tid, xv);
-				else if(l == 2) tc_encode_part<2, 4>(hf, A1, tid, xv);
-				else if(l == 3) tc_encode_part<4, 6>(hf, A1, tid, xv);
-				else if(l == 4) tc_encode_part<6, 7>(hf, A1, tid, xv);
+				for(int j = 0; j < NRC_FP / 16 - 1; j++)
+					tc_mma(tD, tc_desc(sA1 + 2 * j * TC_CHUNK, TC_CHUNK, 128), tc_desc(sW1 + j * 256, 128, (NRC_FP / 8) * 128), id64, j);
+				/* the last K step: chunk 26, then the constant block's bias pairs */
+				const uint32_t a = sA1 + (NRC_F / 8 - 1) * TC_CHUNK;
+				tc_mma(tD, tc_desc(a, sK - a, 128), tc_desc(sW1 + (NRC_FP / 16 - 1) * 256, 128, (NRC_FP / 8) * 128), id64, 1);
 			}
-			if(!tc_wait(mbar, phase)) {
-				ok = false;     /* phase stays the one still outstanding */
-				continue;
-			}
+			tc_commit(mbar);
+		}
+		const int after = next + stride;
+		if(after < ntiles) tc_inputs(xv, x, n, after * 128 + tid, hf);
+		if(tc_wait(mbar, phase)) {
 			phase ^= 1u;
 			tc_fence_after();
-			if(l < 4) {
+			if(more) {
 				float v[32];
 				tc_ld32(tD + lane_off + (uint32_t)(hf * 32), v);
 				tc_hidden(tA + lane_off, hf, v);
-			} else if(hf == 0) {
+			}
+			if(row >= 0 && hf == 0) {
 				float v[16];
 				tc_ld16(tO + lane_off, v);
 				if(row < n) {
@@ -935,6 +928,39 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_forward_tc(NrcDev net, in
 						y[(size_t)row * 3 + 2] = o[2];
 					}
 				}
+			}
+		} else {
+			ok = false;        /* phase stays the one still outstanding */
+		}
+		if(!more) break;
+		row = next * 128 + tid;
+		next = after;
+		#pragma unroll
+		for(int l = 1; l < 4; l++) {
+			proxy_fence();
+			tc_fence_before();
+			agreed = group_all(g, ok);
+			if(!agreed) break;
+			if(leader) {
+				tc_fence_after();
+				const uint32_t sW = sbase + TC_W2 + (uint32_t)(l - 1) * (TC_W3 - TC_W2);   /* W2, W3, W4 back to back */
+				for(int j = 0; j < TC_KH / 16; j++)
+					tc_mma_ta(tD, tA + (uint32_t)(8 * j), tc_desc(sW + j * 256, 128, TC_KH / 8 * 128), id64, j);
+				tc_commit(mbar);
+			}
+			if(next < ntiles) {
+				if(l == 1) tc_encode_part<0, 3>(hf, A1, tid, xv);
+				else if(l == 2) tc_encode_part<3, 5>(hf, A1, tid, xv);
+				else tc_encode_part<5, 7>(hf, A1, tid, xv);
+			}
+			if(tc_wait(mbar, phase)) {
+				phase ^= 1u;
+				tc_fence_after();
+				float v[32];
+				tc_ld32(tD + lane_off + (uint32_t)(hf * 32), v);
+				tc_hidden(tA + lane_off, hf, v);
+			} else {
+				ok = false;
 			}
 		}
 		if(!agreed) break;
