@@ -525,25 +525,35 @@ static_assert(OFF_W1 % 2 == 0 && OFF_W2 % 2 == 0 && OFF_W3 % 2 == 0 && OFF_W4 % 
 		"pairs of the packed gradient for vector atomics");
 
 /* ---- The inference and query forward on the 5th-generation tensor cores ----
- * tcgen05.mma with the accumulators in tensor memory (TMEM).  A CTA of 768
- * threads is three groups of eight warps; each group carries a tile of 128
- * samples through the five layers, two threads per sample (row): its threads
- * write the tile's encoded inputs (half of a row's features each) into
- * shared memory, one elected thread issues the layer's MMAs (M = 128, N = 64,
- * K = 16 each; 14 for the 224-wide first layer, 5 for the 80-wide others,
- * N = 16 for the output layer) and commits them to the group's mbarrier, and
- * the threads read their rows of the accumulator back from TMEM (tcgen05.ld,
+ * tcgen05.mma with the accumulators in tensor memory (TMEM).  A CTA is
+ * three groups of eight warps and a warp per group that issues its MMAs;
+ * each group carries a tile of 128 samples through the five layers, two
+ * threads per sample (row): its threads write the tile's encoded inputs (half
+ * of a row's features each) into shared memory and arrive on the group's
+ * "full" mbarrier, the issuing warp's elected thread issues the layer's MMAs
+ * (M = 128, N = 64, K = 16 each; 14 for the 224-wide first layer, 5 for the
+ * 80-wide others, N = 16 for the output layer) and commits them to the
+ * group's other mbarrier, and the threads read their rows of the accumulator back from TMEM (tcgen05.ld,
  * 32x32b: warp w its lanes 32 (w mod 4) on; the two warps of a lane quarter
  * take 32 columns each) for the ReLU and BF16 rounding that make the next
  * layer's operand, which stays in TMEM (tcgen05.st; the MMA's A operand
  * there, two BF16 per column); the biases come with the products (a BF16 pair
  * per row of each weight tile against a constant pair in the operand).  The
  * features are read only by the first layer, so a group encodes its next
- * tile while the MMAs of the current one's layers 2-4 run (a third of the
- * encoding after each of their issues), and issues that tile's first layer
- * together with the current one's fifth: four waits per tile (the chain of
- * round trips is what bounds a tile; five waits took 362 us for a call of
- * 4,194,304 samples, four 340).  The three groups interleave.
+ * tile while the MMAs of the current one's layers 2-4 run (three, three and
+ * one seventh of it after each of their issues), and that tile's first layer
+ * is issued together with the current one's fifth: four waits per tile.  The
+ * three groups interleave.
+ *
+ * The chain of round trips bounds a tile, then the encoding's instructions.
+ * A call of 4,194,304 samples, host work (27 us) included: 362 us with five
+ * waits per tile, 340 with four.  There a warp of each group issued the MMAs
+ * from a branch that one lane took, every operand passing from vector to
+ * uniform registers first: 299 us with elect.sync and operands that the
+ * whole warp computes.  One issuing warp that polls all three groups 305,
+ * one per group 260: no warp waits for the others of its group before it
+ * encodes.  257 with the encoding split 3/3/1 over the windows (3/2/2 260,
+ * 2/2/3 266, 4/2/1 278, 3/4 288).
  *
  * Shared memory, canonical K-major layouts without swizzle (8-row x 16-byte
  * core matrices; a descriptor's leading byte offset steps along K, its
@@ -557,13 +567,13 @@ static_assert(OFF_W1 % 2 == 0 && OFF_W2 % 2 == 0 && OFF_W3 % 2 == 0 && OFF_W4 % 
  *   constant  2 KB of rows (1, 1, 0 ...), the features' bias pair (chunk 27),
  *             reached by the first layer's last K step through its leading
  *             byte offset
- * 228,648 bytes.  TMEM: 128 columns per group (the hidden accumulator, the
+ * 228,672 bytes.  TMEM: 128 columns per group (the hidden accumulator, the
  * hidden operand, the output accumulator).  Every wait on an mbarrier is
- * bounded; one that runs out sets the error word and the group stops at its
- * next barrier (TMEM is released as usual). */
+ * bounded; one that runs out sets the error word and its warp stops, whereupon
+ * the waits of the group's others run out (TMEM is released as usual). */
 #define TC_NG 3                 /* groups (tiles in flight) per CTA */
 #define TC_GROUP_THREADS 256
-#define TC_THREADS (TC_NG * TC_GROUP_THREADS)
+#define TC_THREADS (TC_NG * (TC_GROUP_THREADS + 32))   /* and a warp per group that issues its MMAs */
 #define TC_WAIT_LIMIT (1 << 20)
 #define TC_XH 5                 /* inputs a half of the encoding reads: 0-4 or 4-8 */
 
@@ -579,7 +589,8 @@ enum {
 	TC_GROUP_BYTES = (NRC_F / 8) * TC_CHUNK,        /* the 27 feature chunks */
 	TC_CONST = TC_GROUP0 + TC_NG * TC_GROUP_BYTES,
 	TC_MBAR = TC_CONST + TC_CHUNK,
-	TC_TMEM_SLOT = TC_MBAR + 8 * TC_NG,
+	TC_FULL = TC_MBAR + 8 * TC_NG,      /* per group: its operands are written */
+	TC_TMEM_SLOT = TC_FULL + 8 * TC_NG,
 	TC_SMEM = TC_TMEM_SLOT + 16,
 	TC_TMEM_COLS = 512,                 /* a power of two >= 128 per group */
 	/* a group's TMEM columns, from 128 g: the hidden layers' accumulator,
@@ -638,18 +649,31 @@ __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity)
 	return false;
 }
 
+/* one lane of a converged warp, the same one each time */
+__device__ __forceinline__ bool tc_elect()
+{
+	uint32_t r;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(r) :: "memory");
+	return r != 0;
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-/* true when v holds in every thread of group g (its named barrier): a wait
- * that ran out in one thread stops the whole group together */
-__device__ __forceinline__ bool group_all(int g, bool v)
+/* the same for a whole warp, which stays together */
+__device__ __forceinline__ bool tc_wait_warp(uint32_t mbar, uint32_t parity)
 {
-	uint32_t r;
-	asm volatile("{\n\t.reg .pred q, p;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, %2, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-			: "=r"(r) : "r"((uint32_t)v), "r"(1 + g), "n"(TC_GROUP_THREADS) : "memory");
-	return r != 0;
+	return __all_sync(0xffffffffu, tc_wait(mbar, parity));
+}
+
+/* the calling warp's part of its group's operands is written, and what it
+ * reads of the accumulators has been read */
+__device__ __forceinline__ void tc_arrive(uint32_t full, int lane)
+{
+	tc_fence_before();
+	__syncwarp();
+	if(lane == 0) asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}\n" :: "r"(full) : "memory");
 }
 
 /* 32 columns of the calling thread's accumulator row (its warp's 32 lanes) */
@@ -821,6 +845,63 @@ __device__ __forceinline__ void tc_hidden(uint32_t ta, int hf, const float (&v)[
 	tc_st16(ta + (uint32_t)(hf * 16), q);
 }
 
+/* The issuing warp of group g: the MMAs of the group's next step once its
+ * eight warps have arrived.  A group's steps are those of its warps: layer 5
+ * of a tile with layer 1 of the next, then layers 2, 3 and 4 of that one. */
+__device__ __forceinline__ void tc_issue(uint32_t sbase, uint32_t tmem, int g, int ntiles, int stride, unsigned *err)
+{
+	const uint32_t id64 = tc_idesc(128, 64), id16 = tc_idesc(128, 16);
+	const uint32_t full = sbase + TC_FULL + 8 * g, mbar = sbase + TC_MBAR + 8 * g;
+	const uint32_t tD = tmem + (uint32_t)(g * 128) + TC_TD, tA = tmem + (uint32_t)(g * 128) + TC_TA, tO = tmem + (uint32_t)(g * 128) + TC_TO;
+	const uint32_t sA1 = sbase + TC_GROUP0 + g * TC_GROUP_BYTES, sA26 = sA1 + (NRC_F / 8 - 1) * TC_CHUNK;
+	const uint64_t dA1 = tc_desc(sA1, TC_CHUNK, 128), dA26 = tc_desc(sA26, sbase + TC_CONST - sA26, 128);
+	const uint64_t dW1 = tc_desc(sbase + TC_W1, 128, (NRC_FP / 8) * 128), dW2 = tc_desc(sbase + TC_W2, 128, TC_KH / 8 * 128);
+	const uint64_t dW5 = tc_desc(sbase + TC_W5, 128, TC_KH / 8 * 128);
+	uint32_t phase = 0;
+	bool ok = true, have = false;
+	int next = blockIdx.x * TC_NG + g;
+	while(next < ntiles || have) {
+		const bool more = next < ntiles;
+		ok = tc_wait_warp(full, phase);
+		if(!ok) break;
+		phase ^= 1u;
+		tc_fence_after();
+		if(tc_elect()) {
+			if(have) {
+				#pragma unroll
+				for(int j = 0; j < TC_KH / 16; j++) tc_mma_ta(tO, tA + (uint32_t)(8 * j), dW5 + j * 16, id16, j);
+			}
+			if(more) {
+				#pragma unroll
+				for(int j = 0; j < NRC_FP / 16 - 1; j++) tc_mma(tD, dA1 + j * (2 * TC_CHUNK >> 4), dW1 + j * 16, id64, j);
+				/* the last K step: chunk 26, then the constant block's bias pairs */
+				tc_mma(tD, dA26, dW1 + (NRC_FP / 16 - 1) * 16, id64, 1);
+			}
+			tc_commit(mbar);
+		}
+		__syncwarp();
+		if(!more) break;
+		have = true;
+		next += stride;
+		#pragma unroll
+		for(int l = 1; l < 4; l++) {
+			ok = tc_wait_warp(full, phase);
+			if(!ok) break;
+			phase ^= 1u;
+			tc_fence_after();
+			if(tc_elect()) {
+				#pragma unroll
+				for(int j = 0; j < TC_KH / 16; j++)
+					tc_mma_ta(tD, tA + (uint32_t)(8 * j), dW2 + (l - 1) * ((TC_W3 - TC_W2) >> 4) + j * 16, id64, j);   /* W2, W3, W4 back to back */
+				tc_commit(mbar);
+			}
+			__syncwarp();
+		}
+		if(!ok) break;
+	}
+	if(!ok && tc_elect()) atomicOr(err, 1u);
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_forward_tc(NrcDev net, int n, const float *x, float *y, QueryOut qo,
 		unsigned *err)
@@ -840,13 +921,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_forward_tc(NrcDev net, in
 		*reinterpret_cast<uint4 *>(tsm + TC_CONST + i * 16) = make_uint4(pack_bf16(1.0f, 1.0f), 0u, 0u, 0u);
 	/* group g: warps 8g .. 8g + 7; a warp's lane quarter (warp mod 4) gives
 	 * its rows, its half (hf) the features and accumulator columns it takes */
-	const int warp = threadIdx.x >> 5, g = warp >> 3, hf = (warp >> 2) & 1;
-	const int tid = ((warp & 3) << 5) | (threadIdx.x & 31);
-	const bool leader = (threadIdx.x & (TC_GROUP_THREADS - 1)) == 0;
-	unsigned char *A1 = tsm + TC_GROUP0 + g * TC_GROUP_BYTES;
-	const uint32_t sA1 = sbase + TC_GROUP0 + g * TC_GROUP_BYTES;
-	const uint32_t mbar = sbase + TC_MBAR + 8 * g;
-	if(leader) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(mbar) : "memory");
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = warp >> 3, hf = (warp >> 2) & 1;
+	const int tid = ((warp & 3) << 5) | lane;
+	if(threadIdx.x == 0) {
+		for(int k = 0; k < TC_NG; k++) {
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(sbase + TC_MBAR + 8 * k) : "memory");
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(sbase + TC_FULL + 8 * k), "n"(TC_GROUP_THREADS / 32) : "memory");
+		}
+	}
 	if(warp == 0) {
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
 				:: "r"(sbase + TC_TMEM_SLOT), "r"((uint32_t)TC_TMEM_COLS) : "memory");
@@ -858,62 +940,47 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_forward_tc(NrcDev net, in
 	__syncthreads();
 	tc_fence_after();
 	const uint32_t tmem = *reinterpret_cast<const uint32_t *>(tsm + TC_TMEM_SLOT);
-	const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-	const uint32_t tD = tmem + (uint32_t)(g * 128) + TC_TD, tA = tmem + (uint32_t)(g * 128) + TC_TA, tO = tmem + (uint32_t)(g * 128) + TC_TO;
-	const uint32_t sW1 = sbase + TC_W1, sW5 = sbase + TC_W5, sK = sbase + TC_CONST;
-	const uint32_t id64 = tc_idesc(128, 64), id16 = tc_idesc(128, 16);
-	if(hf == 0) {
-		/* the hidden operand's last K step: the bias pair (1, 1), then zeros */
-		uint32_t q[16] = {pack_bf16(1.0f, 1.0f)};
-		tc_st16(tA + lane_off + 32, q);
-	}
-	uint32_t phase = 0;
-	bool ok = true;        /* this thread's waits so far */
-	bool agreed = true;    /* the group's, at its last barrier */
-	/* A round of a group: layer 5 of its tile and layer 1 of its next one in
-	 * one issue (they share no operand), then layers 2, 3 and 4 of that one,
-	 * under whose MMAs (which read the hidden operand, not the features) the
-	 * features of the one after it are encoded.  xv holds the inputs of the
-	 * tile to encode next. */
 	const int ntiles = (n + 127) >> 7, stride = gridDim.x * TC_NG;
-	int next = blockIdx.x * TC_NG + g;
-	int row = -1;          /* this thread's sample in the tile before next, -1 none */
-	float xv[TC_XH];
-	tc_inputs(xv, x, n, next * 128 + tid, hf);
-	if(next < ntiles) tc_encode_part<0, 7>(hf, A1, tid, xv);
-	while(next < ntiles || row >= 0) {
-		const bool more = next < ntiles;
-		proxy_fence();
-		tc_fence_before();
-		agreed = group_all(g, ok);
-		if(!agreed) break;
-		if(leader) {
-			tc_fence_after();
-			if(row >= 0)
-				for(int j = 0; j < TC_KH / 16; j++)
-					tc_mma_ta(tO, tA + (uint32_t)(8 * j), tc_desc(sW5 + j * 256, 128, TC_KH / 8 * 128), id16, j);
-			if(more) {
-				for(int j = 0; j < NRC_FP / 16 - 1; j++)
-					tc_mma(tD, tc_desc(sA1 + 2 * j * TC_CHUNK, TC_CHUNK, 128), tc_desc(sW1 + j * 256, 128, (NRC_FP / 8) * 128), id64, j);
-				/* the last K step: chunk 26, then the constant block's bias pairs */
-				const uint32_t a = sA1 + (NRC_F / 8 - 1) * TC_CHUNK;
-				tc_mma(tD, tc_desc(a, sK - a, 128), tc_desc(sW1 + (NRC_FP / 16 - 1) * 256, 128, (NRC_FP / 8) * 128), id64, 1);
-			}
-			tc_commit(mbar);
+	if(g >= TC_NG) {
+		tc_issue(sbase, __shfl_sync(0xffffffffu, tmem, 0), __shfl_sync(0xffffffffu, warp, 0) - TC_NG * TC_GROUP_THREADS / 32, ntiles, stride, err);
+	} else {
+		unsigned char *A1 = tsm + TC_GROUP0 + g * TC_GROUP_BYTES;
+		const uint32_t mbar = sbase + TC_MBAR + 8 * g, full = sbase + TC_FULL + 8 * g;
+		const uint32_t mine = tmem + (uint32_t)(g * 128) + ((uint32_t)((warp & 3) * 32) << 16);   /* the warp's lanes of the group's columns */
+		if(hf == 0) {
+			/* the hidden operand's last K step: the bias pair (1, 1), then zeros */
+			uint32_t q[16] = {pack_bf16(1.0f, 1.0f)};
+			tc_st16(mine + TC_TA + 32, q);
 		}
-		const int after = next + stride;
-		if(after < ntiles) tc_inputs(xv, x, n, after * 128 + tid, hf);
-		if(tc_wait(mbar, phase)) {
+		uint32_t phase = 0;
+		/* A round of a group: layer 5 of its tile and layer 1 of its next one,
+		 * then layers 2, 3 and 4 of that one, under whose MMAs (which read the
+		 * hidden operand, not the features) the features of the one after it
+		 * are encoded.  xv holds the inputs of the tile to encode next. */
+		int next = blockIdx.x * TC_NG + g;
+		int row = -1;          /* this thread's sample in the tile before next, -1 none */
+		bool ok = true;        /* the warp's waits so far */
+		float xv[TC_XH];
+		tc_inputs(xv, x, n, next * 128 + tid, hf);
+		if(next < ntiles) tc_encode_part<0, 7>(hf, A1, tid, xv);
+		while(next < ntiles || row >= 0) {
+			const bool more = next < ntiles;
+			proxy_fence();     /* the features are read by the tensor cores (async proxy) */
+			tc_arrive(full, lane);
+			const int after = next + stride;
+			if(after < ntiles) tc_inputs(xv, x, n, after * 128 + tid, hf);
+			ok = tc_wait_warp(mbar, phase);
+			if(!ok) break;
 			phase ^= 1u;
 			tc_fence_after();
 			if(more) {
 				float v[32];
-				tc_ld32(tD + lane_off + (uint32_t)(hf * 32), v);
-				tc_hidden(tA + lane_off, hf, v);
+				tc_ld32(mine + TC_TD + (uint32_t)(hf * 32), v);
+				tc_hidden(mine + TC_TA, hf, v);
 			}
 			if(row >= 0 && hf == 0) {
 				float v[16];
-				tc_ld16(tO + lane_off, v);
+				tc_ld16(mine + TC_TO, v);
 				if(row < n) {
 					const float *o = v;   /* the bias came with the product */
 					if(MODE == FWD_QUERY) {
@@ -929,50 +996,34 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_forward_tc(NrcDev net, in
 					}
 				}
 			}
-		} else {
-			ok = false;        /* phase stays the one still outstanding */
-		}
-		if(!more) break;
-		row = next * 128 + tid;
-		next = after;
-		#pragma unroll
-		for(int l = 1; l < 4; l++) {
-			proxy_fence();
-			tc_fence_before();
-			agreed = group_all(g, ok);
-			if(!agreed) break;
-			if(leader) {
-				tc_fence_after();
-				const uint32_t sW = sbase + TC_W2 + (uint32_t)(l - 1) * (TC_W3 - TC_W2);   /* W2, W3, W4 back to back */
-				for(int j = 0; j < TC_KH / 16; j++)
-					tc_mma_ta(tD, tA + (uint32_t)(8 * j), tc_desc(sW + j * 256, 128, TC_KH / 8 * 128), id64, j);
-				tc_commit(mbar);
-			}
-			if(next < ntiles) {
-				if(l == 1) tc_encode_part<0, 3>(hf, A1, tid, xv);
-				else if(l == 2) tc_encode_part<3, 5>(hf, A1, tid, xv);
-				else tc_encode_part<5, 7>(hf, A1, tid, xv);
-			}
-			if(tc_wait(mbar, phase)) {
+			if(!more) break;
+			row = next * 128 + tid;
+			next = after;
+			#pragma unroll
+			for(int l = 1; l < 4; l++) {
+				tc_arrive(full, lane);
+				if(next < ntiles) {
+					if(l == 1) tc_encode_part<0, 3>(hf, A1, tid, xv);
+					else if(l == 2) tc_encode_part<3, 6>(hf, A1, tid, xv);
+					else tc_encode_part<6, 7>(hf, A1, tid, xv);
+				}
+				ok = tc_wait_warp(mbar, phase);
+				if(!ok) break;
 				phase ^= 1u;
 				tc_fence_after();
 				float v[32];
-				tc_ld32(tD + lane_off + (uint32_t)(hf * 32), v);
-				tc_hidden(tA + lane_off, hf, v);
-			} else {
-				ok = false;
+				tc_ld32(mine + TC_TD + (uint32_t)(hf * 32), v);
+				tc_hidden(mine + TC_TA, hf, v);
 			}
+			if(!ok) break;
 		}
-		if(!agreed) break;
+		if(!ok) {
+			/* what was committed may still be running: a last bounded wait */
+			if(lane == 0) atomicOr(err, 1u);
+			tc_wait(mbar, phase);
+		}
 	}
-	/* the waits of the group's last layer */
-	if(agreed) agreed = group_all(g, ok);
-	if(!agreed) {
-		if(leader) atomicOr(err, 1u);
-		/* what was committed may still be running: a last bounded wait by
-		 * the threads whose wait ran out (they hold its phase) */
-		if(!ok) tc_wait(mbar, phase);
-	}
+	__syncwarp();
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
