@@ -4791,7 +4791,7 @@ void sray_gpu_shutdown(void)
 		&R.fbl, &R.tnodes, &R.ohome, &R.pool_ready, &R.pqbuf[0], &R.pqbuf[1], &R.phits, &R.pfbl, &R.pcounts, &R.pctr,
 		&R.pw_jobs, &R.pw_prefix, &R.pw_scale, &R.pw_bits, &R.pw_cov, &R.pj_tables, &R.pj_samples, &R.pj_boxes, &R.pj_views, &R.pj_first, &R.pw_pix, &R.pw_out, &R.pw_valid,
 		&R.pw_part, &R.pw_tiles, &R.pw_bounds, &R.pw_offs, &R.pw_ph, &R.pw_sorted, &R.pw_grids, &R.pw_cellbase,
-		&R.pw_keys, &R.pw_lin, &R.pw_starts, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1], &R.glist[0], &R.glist[1], &R.glist[2],
+		&R.pw_keys, &R.pw_starts, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1], &R.glist[0], &R.glist[1], &R.glist[2],
 		&R.pqsbuf, &R.ps_keys, &R.ps_hist, &R.ps_part,
 		&R.nrc_qx, &R.nrc_qw, &R.nrc_rx, &R.nrc_rt, &R.nrc_ry, &R.nrc_regions};
 	if(R.ps) cudaStreamSynchronize(R.ps);

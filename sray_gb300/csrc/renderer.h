@@ -245,7 +245,7 @@ struct Renderer {
 	/* a batch's maps built together (photon_finalize_jobs): scan scratch,
 	 * segment bounds and offsets, compacted and sorted photons, grids, keys,
 	 * cell tables */
-	DevBuf pw_part, pw_tiles, pw_bounds, pw_offs, pw_ph, pw_sorted, pw_grids, pw_cellbase, pw_keys, pw_lin, pw_starts, pw_hist;
+	DevBuf pw_part, pw_tiles, pw_bounds, pw_offs, pw_ph, pw_sorted, pw_grids, pw_cellbase, pw_keys, pw_starts, pw_hist;
 	std::vector<int> batch_scene, batch_caust, batch_gi;   /* jobs' scenes and photon counts (0: the options') */
 	/* a scene set: its scene descriptors on the device */
 	DevBuf dscenes;
@@ -348,7 +348,7 @@ int photon_finalize(Renderer &R, int global, const int *valid, const DevPhoton *
 int sort_pairs(Renderer &R, unsigned *keys, unsigned *vals, unsigned *keys2, unsigned *vals2, int n, int bits, DevBuf &hist,
 		DevBuf &part, const char *name, cudaStream_t s, unsigned **keys_out, unsigned **vals_out);
 int photon_finalize_jobs(Renderer &R, const std::vector<PJobOut> &jobs, const std::vector<Box> &boxes,
-		const std::vector<double> &gather_dist, std::vector<DPhotonMap> &maps, cudaStream_t s);
+		const std::vector<double> &gather_dist, std::vector<DPhotonMap> &maps, cudaStream_t s, bool own = false);
 int photon_shoot_maps(Renderer &R, const DScene &base, cudaStream_t s, int *caust_stored, int *gi_stored);
 /* photon.cu: map `global` (0 caustic, 1 global) over the n photons in its buffer / from host photons */
 int photon_map_build(Renderer &R, int global, int n, cudaStream_t s);
