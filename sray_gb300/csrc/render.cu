@@ -1403,16 +1403,26 @@ __device__ __forceinline__ float gather_below(float d) { return d * (1.0f - GATH
 __device__ __forceinline__ float gather_above(float d) { return d * (1.0f + GATHER_EPS) + 1e-37f; }
 
 /* the reference's key of a photon: its squared distance in double, rounded
- * to float; and whether it is in range */
+ * to float; the sign bit set where it is out of range (out of line: see
+ * gather_one) */
+static __device__ __noinline__ unsigned gather_exact_key(float px, float py, float pz, float qx, float qy, float qz, float r2_hi, float r2_lo,
+		double range)
+{
+	int inr = 0;
+	uint32_t k = 0;
+	if(!sray_range_ff(px, py, pz, qx, qy, qz, r2_hi, r2_lo, &inr, &k)) {
+		double d2 = dist2(make_float4(px, py, pz, 0.0f), mk(qx, qy, qz));
+		inr = d2 <= range * range;
+		k = __float_as_uint((float)d2);
+	}
+	return inr ? k : k | 0x80000000u;
+}
+
 __device__ __forceinline__ bool gather_exact(const DPhotonMap &M, const float4 &p, V3 q, unsigned &key)
 {
-	bool in;
-	if(!range_ff(M, p, q, in, key)) {
-		double d2 = dist2(p, q);
-		in = d2 <= M.range * M.range;
-		key = __float_as_uint((float)d2);
-	}
-	return in;
+	unsigned k = gather_exact_key(p.x, p.y, p.z, q.x, q.y, q.z, M.r2_hi, M.r2_lo, M.range);
+	key = k & 0x7fffffffu;
+	return k == key;
 }
 
 /* The rows of cells that the query's sphere reaches (25 where the cells are
@@ -1657,6 +1667,48 @@ __device__ __noinline__ unsigned gather_unlisted(const DPhotonMap &M, const Gath
 	return __reduce_max_sync(FULL, kmax);
 }
 
+/* many photons at one distance: the exact keys of those between lo and hi
+ * in the list, the others around them; the k nearest into the sums */
+__device__ __noinline__ int gather_edge(const DPhotonMap &M, V3 pos, int lane, int ncand, float lo, float hi, GatherMem &gm, int kind,
+		V3 n, float max_cos, float *sum, unsigned &kth)
+{
+	int cnt = 0;
+	for(int c = lane; c < ncand; c += 32) {
+		float d = __uint_as_float(gm.keys[c]);
+		unsigned key = d < lo ? 0u : 0xffffffffu;
+		if(d >= lo && d <= hi) {
+			float4 p = __ldg(reinterpret_cast<const float4 *>(M.ph + gm.idx[c]));
+			gather_exact(M, p, pos, key);
+			key = key < 1u ? 1u : key;
+		}
+		gm.keys[c] = key;
+	}
+	__syncwarp();
+	kth = gather_kth_bitwise(gm.keys, ncand, lane, M.k);
+	for(int c = lane; c < ncand; c += 32) {
+		unsigned key = gm.keys[c];
+		if(key == 0u || key > kth) continue;
+		cnt++;
+		float4 p = __ldg(reinterpret_cast<const float4 *>(M.ph + gm.idx[c]));
+		photon_term(M, gm.idx[c], p, kind, n, max_cos, sum);
+	}
+	return cnt;
+}
+
+/* the photons in range into the sums; their number */
+__device__ __noinline__ int gather_all(const DPhotonMap &M, const GatherCells &gc, V3 pos, int lane, GatherMem &gm, int kind, V3 n,
+		float max_cos, float *sums)
+{
+	float sum[3] = {0.0f, 0.0f, 0.0f};
+	int cnt = 0;
+	for_range(M, gc, pos, lane, gm, [&](bool in, int j, const float4 &p, float) {
+		cnt += __popc(__ballot_sync(0xffffffffu, in));
+		if(in) photon_term(M, j, p, kind, n, max_cos, sum);
+	});
+	for(int c = 0; c < 3; c++) sums[c] = sum[c];
+	return cnt;
+}
+
 /* The map a request's kind names: the frame's caustic (0) or global (1) map,
  * in a batch its job's */
 __device__ __forceinline__ const DPhotonMap &gather_map(const DScene &S, int kind)
@@ -1729,11 +1781,16 @@ __device__ __forceinline__ bool gather_few(const DScene &S, int kind, V3 pos, V3
  * margin of GATHER_EPS; the k-th of them (a 256-bin histogram, then the rank
  * within its bin) splits the list into photons that are surely among the k
  * nearest, photons that surely are not, and the few within the margin, for
- * which the exact keys decide.  The kernel is bound by instruction issue:
- * 1.15 ms for 500,009 points of a map of 500k emitted photons (k = 100)
- * against 2.33 ms with the exact key of every photon, a 32-step search over
- * all of them and cells of twice the radius (1.51 ms with those cells
- * alone). */
+ * which the exact keys decide.  The kernel is bound by instruction issue and
+ * by fetching instructions (warps are at many places of a long program): what
+ * is rare -- exact keys, more candidates than the list holds, many at one
+ * distance, the range gather beside the k nearest -- is out of line, and what
+ * such a call writes goes through copies, so that the sums of the others stay
+ * in registers.  500,009 points of a map of 500k emitted photons (k = 100),
+ * those with few photons by a thread each: 1.01 ms, against 1.17 with all of
+ * it in line and 2.37 with the exact key of every photon, a 32-step search
+ * over all of them and cells of twice the radius.  (80 registers instead of
+ * 64: 1.07.) */
 __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V3 n, GatherMem &gm, GatherWork &gw)
 {
 	const unsigned FULL = 0xffffffffu;
@@ -1748,10 +1805,10 @@ __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V
 	int cnt = 0;
 	float inv_area = M.inv_area;
 	if(M.k <= 0) {
-		for_range(M, gc, pos, lane, gm, [&](bool in, int j, const float4 &p, float) {
-			cnt += __popc(__ballot_sync(FULL, in));
-			if(in) photon_term(M, j, p, kind, n, S.max_cos, sum);
-		});
+		GatherCells cells = gc;
+		float part[3];
+		cnt = gather_all(M, cells, pos, lane, gm, kind, n, S.max_cos, part);
+		for(int c = 0; c < 3; c++) sum[c] = part[c];
 	} else {
 		unsigned maxkey = 0;
 		int ncand = 0;
@@ -1775,7 +1832,10 @@ __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V
 		bool listed = ncand <= KEY_CAP;
 		gw.spill += listed ? 0u : 1u;
 		if(!listed && select) {
-			int nl = gather_narrow(M, gc, pos, lane, maxkey, gm);
+			GatherCells cells = gc;
+			unsigned top = maxkey;
+			int nl = gather_narrow(M, cells, pos, lane, top, gm);
+			maxkey = top;
 			if(nl >= 0) {
 				ncand = nl;
 				listed = true;
@@ -1783,7 +1843,12 @@ __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V
 		}
 		unsigned kth = 0;
 		if(!listed) {
-			kth = gather_unlisted(M, gc, pos, lane, ncand, gm, kind, n, S.max_cos, sum, cnt);
+			GatherCells cells = gc;
+			float part[3] = {0.0f, 0.0f, 0.0f};
+			int got = 0;
+			kth = gather_unlisted(M, cells, pos, lane, ncand, gm, kind, n, S.max_cos, part, got);
+			for(int c = 0; c < 3; c++) sum[c] = part[c];
+			cnt = got;
 		} else if(!select) {
 			/* every candidate; the farthest's exact key gives the disc */
 			const float far = gather_below(__uint_as_float(maxkey));
@@ -1853,26 +1918,11 @@ __device__ __forceinline__ float gather_one(const DScene &S, int kind, V3 pos, V
 				if(take) photon_term(M, gm.hist[lane], p, kind, n, S.max_cos, sum);
 				cnt = near + __popc(__ballot_sync(FULL, take));
 			} else {
-				/* many photons at one distance: exact keys for them in the list, the others around them */
-				for(int c = lane; c < ncand; c += 32) {
-					float d = __uint_as_float(gm.keys[c]);
-					unsigned key = d < lo ? 0u : 0xffffffffu;
-					if(d >= lo && d <= hi) {
-						float4 p = __ldg(reinterpret_cast<const float4 *>(M.ph + gm.idx[c]));
-						gather_exact(M, p, pos, key);
-						key = key < 1u ? 1u : key;
-					}
-					gm.keys[c] = key;
-				}
-				__syncwarp();
-				kth = gather_kth_bitwise(gm.keys, ncand, lane, M.k);
-				for(int c = lane; c < ncand; c += 32) {
-					unsigned key = gm.keys[c];
-					if(key == 0u || key > kth) continue;
-					cnt++;
-					float4 p = __ldg(reinterpret_cast<const float4 *>(M.ph + gm.idx[c]));
-					photon_term(M, gm.idx[c], p, kind, n, S.max_cos, sum);
-				}
+				float part[3] = {sum[0], sum[1], sum[2]};
+				unsigned far = 0;
+				cnt = gather_edge(M, pos, lane, ncand, lo, hi, gm, kind, n, S.max_cos, part, far);
+				for(int c = 0; c < 3; c++) sum[c] = part[c];
+				kth = far;
 				cnt = near + __reduce_add_sync(FULL, cnt);
 			}
 		}
@@ -1986,7 +2036,7 @@ __global__ void __launch_bounds__(128) k_gather_few(DScene S, Q q, const int *co
 
 /* a warp per query: the listed ones, or (list null) all of them */
 template <class Q>
-__global__ void __launch_bounds__(GATHER_WARPS * 32, 4) k_gather(DScene S, Q q, const int *count, int most, const int *list, DevCounters *ctr)
+__global__ void __launch_bounds__(GATHER_WARPS * 32, 4) k_gather(const __grid_constant__ DScene S, Q q, const int *count, int most, const int *list, DevCounters *ctr)
 {
 	__shared__ __align__(16) GatherMem mem[GATHER_WARPS];
 	const int n = list ? list[0] : (count ? min(*count, most) : most);
