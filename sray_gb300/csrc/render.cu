@@ -7,7 +7,8 @@
  *                                        camera rays by k_trace_packet, a warp per 8 x 4 patch
  *   k_shade     Phong + shadows + spawn shade_phong / calc_lighting / shade_undef
  *                                        (src/shader.cc:36-283)
- *   k_gather    photon-map estimates    PhotonMap::irradiance_est / radiance_est (src/pmap.cc:109-178)
+ *   k_gather    photon-map estimates    PhotonMap::irradiance_est / radiance_est (src/pmap.cc:109-178);
+ *                                        those with few photons by k_gather_few
  *   k_finish    adaptive supersampling  render_block / variance (src/render.cc:194-270)
  * The recursion of trace_ray is unrolled into bounces over SoA ray queues:
  * every ray carries the product of the weights that the reference's nested
@@ -1050,7 +1051,7 @@ struct QueueEmitter {
 /* Bound by latency (the hit's surface, its material and light tables, one
  * after the other; 5 of 11 stall cycles per issue), so by warps in flight: 6
  * blocks of 128 per SM (80 registers, some spilled) instead of the 4 that 124
- * registers leave.  Batches of three 960x540 frames 2.38 -> 2.32 ms, 1080p
+ * registers leave.  Batches of six 480x270 frames 2.38 -> 2.32 ms, 1080p
  * frames 15.50 -> 15.45; 5 blocks 2.36, 8 blocks 2.36. */
 __global__ void __launch_bounds__(128, 6) k_shade(DScene S, RayQueue qi, const int4 *hits, ShadeOut out, float4 *acc, int depth,
 		DevCounters *ctr)
@@ -2117,8 +2118,10 @@ __global__ void k_finish(const int *active, int tw, int th, const int *n_active_
 }
 
 /* closest hits of caller-supplied world rays (sray_gpu_cast_rays), as the
- * frame's passes: chunks of rays per block, or one warp per ray; then the
- * listed rays by the octrees */
+ * frame's passes: chunks of rays per block, then the listed rays by the
+ * octrees; or one warp per ray, whose first lane follows the octrees itself
+ * where they must decide (64 rays 45.4 us per call with a list, its clearing
+ * and a second launch for the few such rays, 41.9 without) */
 struct CastRays {
 	const float *orig, *dir;
 	const int *time;          /* may be null: the frame's */
@@ -2160,7 +2163,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRa
 	if(overflow) atomicOr(&ctr->overflow, 1);
 }
 
-__global__ void __launch_bounds__(128) k_cast_warp(DScene S, CastRays R, int n, int *fb)
+__global__ void __launch_bounds__(128) k_cast_warp(const __grid_constant__ DScene S, CastRays R, int n, DevCounters *ctr)
 {
 	__shared__ int s_ref[4][WR_CAP];
 	__shared__ int s_obj[4][WR_CAP];
@@ -2171,8 +2174,15 @@ __global__ void __launch_bounds__(128) k_cast_warp(DScene S, CastRays R, int n, 
 		int bobj, bprim;
 		int res = warp_trace<false>(S, R.o(i), R.d(i), R.when(S, i), s_ref[w], s_obj[w], s_te[w], best, bobj, bprim, -1);
 		if(lane == 0) {
-			if(!res) fb[1 + atomicAdd(fb, 1)] = i;
-			else R.put(i, bobj, bprim, best, 0);
+			if(!res) {
+				Hit h;
+				int overflow = 0;
+				trace_closest_octree<false>(S, R.o(i), R.d(i), R.when(S, i), h, nullptr, &overflow);
+				R.put(i, h.obj, h.prim, h.t, h.tie);
+				if(overflow) atomicOr(&ctr->overflow, 1);
+			} else {
+				R.put(i, bobj, bprim, best, 0);
+			}
 		}
 		__syncwarp();
 	}
@@ -4521,19 +4531,20 @@ int sray_gpu_cast_rays(int n, const float *orig, const float *dir, const int *ti
 	if(n == 0) return 0;
 	cudaStream_t s = as_stream(stream);
 	cudaError_t e = R.ctr.ensure(sizeof(DevCounters));
-	if(e == cudaSuccess) e = R.fbl.ensure(((size_t)n + 1) * sizeof(int));
+	const bool listed = n > R.tune.warp_rays;
+	if(e == cudaSuccess && listed) e = R.fbl.ensure(((size_t)n + 1) * sizeof(int));
 	if(e == cudaSuccess) e = cudaMemsetAsync(R.ctr.p, 0, sizeof(DevCounters), s);
-	if(e == cudaSuccess) e = cudaMemsetAsync(R.fbl.p, 0, sizeof(int), s);
+	if(e == cudaSuccess && listed) e = cudaMemsetAsync(R.fbl.p, 0, sizeof(int), s);
 	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
 	const CastRays rays = {orig, dir, time, obj, prim, t, tie};
-	int *fb = R.fbl.as<int>();
-	if(n <= R.tune.warp_rays) {
-		k_cast_warp<<<grid_for(n, 4), 128, 0, s>>>(R.S, rays, n, fb);
+	if(!listed) {
+		k_cast_warp<<<grid_for(n, 4), 128, 0, s>>>(R.S, rays, n, R.ctr.as<DevCounters>());
 	} else {
+		int *fb = R.fbl.as<int>();
 		const int chunk = stream_chunk(n, CAST_CHUNK);
 		k_cast<<<(n + chunk - 1) / chunk, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, n, chunk, R.ctr.as<DevCounters>(), fb);
+		k_cast_octree<<<grid_for(n, 128) < R.nsm ? grid_for(n, 128) : R.nsm, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, R.ctr.as<DevCounters>(), fb);
 	}
-	k_cast_octree<<<grid_for(n, 128) < R.nsm ? grid_for(n, 128) : R.nsm, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, R.ctr.as<DevCounters>(), fb);
 	DevCounters hc;
 	e = cudaMemcpyAsync(&hc, R.ctr.p, sizeof hc, cudaMemcpyDeviceToHost, s);
 	if(e == cudaSuccess) e = cudaStreamSynchronize(s);

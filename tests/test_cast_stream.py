@@ -60,3 +60,33 @@ def test_cast_rays_by_size(gpu_lib, cast_pair, n, warp_rays):
     assert (got[1][~hit] == -1).all() and (got[2][~hit] == 0).all()
     if n == N:
         assert hit.any() and (~hit).any()
+
+
+@pytest.mark.parametrize("n", [1, 64, 5000, 16384])
+def test_octree_decided_rays(gpu_lib, n):
+    """Two coincident meshes: every hit is a tie that the octrees decide, by the
+    ray's own warp in a small call, by a second launch in a large one."""
+    quad = ('<object type="mesh" name="%s"><matref name="d"/><mesh>'
+            + "".join('<vertex id="%d" val="%s"/>' % (i, v) for i, v in enumerate(["-20 0 -20", "20 0 -20", "20 0 20", "-20 0 20"]))
+            + '<face><vref vertex="0"/><vref vertex="2"/><vref vertex="1"/></face>'
+              '<face><vref vertex="0"/><vref vertex="3"/><vref vertex="2"/></face></mesh></object>\n')
+    xml = ('<?xml version="1.0"?>\n<scene>\n<material name="d" shader="phong"><mattr name="diffuse" value="0.5 0.5 0.4"/></material>\n'
+           + quad % "a" + quad % "b" + '<light type="point" color="1.0"><xform pos="0 9 0"/></light>\n'
+           '<camera type="target" fov="50.0"><xform pos="0 7 16"/><target><xform pos="0 0 0"/></target></camera></scene>\n')
+    rng = np.random.default_rng(n)
+    o = torch.tensor(rng.uniform((-15, 2, -15), (15, 9, 15), (n, 3)).astype(np.float32), device="cuda")
+    d = torch.tensor((rng.normal(size=(n, 3)) * (1, 0.3, 1) - (0, 1, 0)).astype(np.float32) * 60.0, device="cuda")
+    got = []
+    for warp_rays in (16384, 0):
+        g = gpu_lib.GpuRenderer(width=32, height=32)
+        g.load_xml(xml)
+        g.set_tuning(warp_rays=warp_rays)
+        g.build(0, 0)
+        out = [torch.full((n,), 7, dtype=torch.int32, device="cuda") for _ in range(2)]
+        out += [torch.full((n,), 7.0, device="cuda"), torch.full((n,), 7, dtype=torch.uint8, device="cuda")]
+        g.cast_rays(o, d, None, *out)
+        got.append([x.cpu().numpy() for x in out])
+        g.close()
+    assert (got[0][0] >= 0).any() or n == 1
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
