@@ -1,5 +1,5 @@
 /* anim_eval.h -- keyframe tracks and node transforms, one implementation for
- * the host (scene loading, per-frame object bounds, projection maps, the
+ * the host (scene loading, per-frame object bounds, light samples, the
  * camera) and the device (the per-frame table of object transforms and
  * light positions, k_xforms in render.cu).
  *

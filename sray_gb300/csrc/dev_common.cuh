@@ -1171,7 +1171,8 @@ __device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, in
  * number for done), done(i, result, walk) takes its result as
  * trace_two_level returns it.  1,000,003 rays from random points in random
  * directions over the 1.26M-triangle terrain: 1.19 ms, against 1.89 with a
- * ray per thread. */
+ * ray per thread (0.62 with the objects' own boxes and the ray and stack laid
+ * out as above). */
 template <int REFILL, bool COUNT, bool ANY, bool SORT, class Load, class Done>
 __device__ __forceinline__ void walk_stream(const DScene &S, float *world, int *next, int end, Load load, Done done, TraceCounters *tc, int *overflow)
 {

@@ -3,7 +3,7 @@
  * builds and their flattening into the device layouts.
  *
  * Everything here runs once per scene load (meshes) or once per frame
- * (top-level octree, per-time matrices, projection maps) in double
+ * (top-level octree, light samples, the camera) in double
  * precision, exactly as the reference computes it, and is rounded to float
  * only when written into the device tables.
  */
