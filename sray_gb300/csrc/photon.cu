@@ -662,7 +662,8 @@ __device__ __forceinline__ int photon_interact(const DScene &S, const PhotonSet 
 __global__ void __launch_bounds__(128) k_photon_bounce(DScene S, PhotonSet P, RayQueue qi, const int4 *hits, RayQueue qo)
 {
 	int n = *qi.count;
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+	for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+		const int i = qi.order ? (int)qi.order[k] : k;
 		int4 hv = hits[i];
 		if(hv.y < 0) continue;                       /* photon left the scene */
 		Hit h;
@@ -1109,6 +1110,7 @@ int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJ
 	int *cnt = R.pcounts.as<int>();
 	R.pq[0].count = cnt + 0;
 	R.pq[1].count = cnt + 1;
+	R.pq[0].order = R.pq[1].order = nullptr;
 	if(R.ensure_pqueue(0, (int)all) || R.ensure_pqueue(1, (int)all)) return SRAY_ECUDA;
 	PCK(R.phits.ensure((size_t)all * 16), "photon hits");
 	/* the scene as the photon kernels see it: their counters, and in a scene
@@ -1159,6 +1161,7 @@ int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJ
 		if(launch_trace(R, PS, R.pq[cur], n_live, "photon_trace", s)) return SRAY_ECUDA;
 		LAUNCH(R, "photon_bounce", s, k_photon_bounce<<<grid_n(n_live, 128), 128, 0, s>>>(PS, PSet, R.pq[cur], R.phits.as<int4>(),
 				R.pq[cur ^ 1]));
+		R.pq[cur].order = nullptr;
 		PCK(cudaMemcpyAsync(R.pin + 8, R.pq[cur ^ 1].count, sizeof(int), cudaMemcpyDeviceToHost, s), "photon queue count");
 		PCK(cudaStreamSynchronize(s), "photon pass");
 		n_live = R.pin[8];

@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQu
 	int overflow = 0;
 	walk_stream<TRACE_REFILL, COUNT, false, true>(S, world + threadIdx.x, &next, min(first + chunk, n),
 			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
+				if(q.order) i = (int)q.order[i];
 				float4 o4 = q.o[i], d4 = q.d[i];
 				o = mk(o4.x, o4.y, o4.z);
 				d = mk(d4.x, d4.y, d4.z);
@@ -3087,11 +3088,9 @@ int Renderer::ensure_pqueue(int which, int cap)
 /* the n rays of q[cur], sorted by direction octant and origin cell into the
  * spare queue, which then becomes q[cur] (the pass's queue and its
  * allocation swapped with the spare's) */
-int Renderer::sort_queue(RayQueue &Q, DevBuf &Qbuf, int &Qcap, RayQueue &T, DevBuf &Tbuf, int &Tcap, DevBuf &keysb, DevBuf &hist,
-		DevBuf &part, int n, int bits, const char *name, cudaStream_t s)
+int Renderer::sort_queue(const RayQueue &Q, DevBuf &keysb, DevBuf &hist, DevBuf &part, int n, int bits, const char *name, cudaStream_t s,
+		unsigned **sorted)
 {
-	if(n < 2 || sc.oct.nodes.empty()) return 0;
-	if(int r = queue_alloc(Tbuf, T, Tcap, Q.cap)) return r;
 	CK(keysb.ensure((size_t)n * 16), "ray sort keys");
 	unsigned *keys = keysb.as<unsigned>(), *vals = keys + n, *keys2 = keys + 2 * (size_t)n, *vals2 = keys + 3 * (size_t)n;
 	const Box &b = sc.oct.nodes[0].box;
@@ -3103,27 +3102,35 @@ int Renderer::sort_queue(RayQueue &Q, DevBuf &Qbuf, int &Qcap, RayQueue &T, DevB
 	}
 	LAUNCH(*this, name, s, k_ray_keys<<<grid_for(n, 256), 256, 0, s>>>(Q, n, lo[0], lo[1], lo[2], ext[0], ext[1], ext[2],
 			24 - bits, keys, vals));
-	unsigned *sorted = nullptr;
-	if(int r = sort_pairs(*this, keys, vals, keys2, vals2, n, bits, hist, part, name, s, &keys, &sorted)) return r;
-	LAUNCH(*this, name, s, k_ray_permute<<<grid_for(n, 256), 256, 0, s>>>(Q, sorted, n, T));
-	int *count = Q.count;
-	std::swap(Q, T);
-	std::swap(Qbuf, Tbuf);
-	std::swap(Qcap, Tcap);
-	Q.count = count;
-	return 0;
+	return sort_pairs(*this, keys, vals, keys2, vals2, n, bits, hist, part, name, s, &keys, sorted);
 }
 
 int Renderer::sort_pass(int cur, int n, cudaStream_t s)
 {
-	return sort_queue(q[cur], qbuf[cur], qcap[cur], qs, qsbuf, qscap, rs_keys, rs_hist, rs_part, n, 24, "ray_sort", s);
+	if(n < 2 || sc.oct.nodes.empty()) return 0;
+	if(int r = queue_alloc(qsbuf, qs, qscap, q[cur].cap)) return r;
+	unsigned *sorted = nullptr;
+	if(int r = sort_queue(q[cur], rs_keys, rs_hist, rs_part, n, 24, "ray_sort", s, &sorted)) return r;
+	LAUNCH(*this, "ray_sort", s, k_ray_permute<<<grid_for(n, 256), 256, 0, s>>>(q[cur], sorted, n, qs));
+	int *count = q[cur].count;
+	std::swap(q[cur], qs);
+	std::swap(qbuf[cur], qsbuf);
+	std::swap(qcap[cur], qscap);
+	q[cur].count = count;
+	return 0;
 }
 
 int Renderer::sort_photon_pass(int cur, int n, cudaStream_t s)
 {
 	/* one radix pass: the direction octant and the origin's cell in a coarse
-	 * grid (the first pass's photons leave from the lights) */
-	return sort_queue(pq[cur], pqbuf[cur], pqcap[cur], pqs, pqsbuf, pqscap, ps_keys, ps_hist, ps_part, n, 8, "photon_ray_sort", s);
+	 * grid (the first pass's photons leave from the lights).  The pass takes
+	 * the photons in that order where they are: bakes with 2.5M photons 3.40
+	 * ms, 3.50 with the 88 bytes of each moved into it first. */
+	if(n < 2 || sc.oct.nodes.empty()) return 0;
+	unsigned *sorted = nullptr;
+	if(int r = sort_queue(pq[cur], ps_keys, ps_hist, ps_part, n, 8, "photon_ray_sort", s, &sorted)) return r;
+	pq[cur].order = sorted;
+	return 0;
 }
 
 /* ---------------------------------------------------------------- */
@@ -4916,7 +4923,7 @@ void sray_gpu_shutdown(void)
 		&R.pw_jobs, &R.pw_prefix, &R.pw_scale, &R.pw_bits, &R.pw_cov, &R.pj_tables, &R.pj_samples, &R.pj_boxes, &R.pj_views, &R.pj_first, &R.pw_pix, &R.pw_out, &R.pw_valid,
 		&R.pw_part, &R.pw_tiles, &R.pw_bounds, &R.pw_offs, &R.pw_ph, &R.pw_sorted, &R.pw_grids, &R.pw_cellbase,
 		&R.pw_keys, &R.pw_starts, &R.pw_hist, &R.qsbuf, &R.rs_keys, &R.rs_hist, &R.rs_part, &R.sq2, &R.gq2, &R.fbs[0], &R.fbs[1], &R.glist[0], &R.glist[1], &R.glist[2],
-		&R.pqsbuf, &R.ps_keys, &R.ps_hist, &R.ps_part,
+		&R.ps_keys, &R.ps_hist, &R.ps_part,
 		&R.nrc_qx, &R.nrc_qw, &R.nrc_rx, &R.nrc_rt, &R.nrc_ry, &R.nrc_regions};
 	if(R.ps) cudaStreamSynchronize(R.ps);
 	if(R.xs) cudaStreamSynchronize(R.xs);

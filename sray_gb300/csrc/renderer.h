@@ -75,6 +75,7 @@ struct RayQueue {
 	int2 *ext;      /* sample | diffuse index << 16, stack depth */
 	int *count;
 	int cap;
+	const unsigned *order = nullptr;   /* the order to take the entries in; null: as they are */
 };
 
 /* a pending photon-map gather: pos + kind, normal + pixel, weight */
@@ -158,12 +159,11 @@ struct Renderer {
 	RayQueue qs = {};
 	int qscap = 0;
 	int sort_pass(int cur, int n, cudaStream_t s);
-	/* queue Q's first n entries in the order of the top `bits` of their
-	 * 24-bit keys (direction octant over the Morton code of the origin's cell
-	 * in a 128^3 grid), through the scratch queue T (swapped with Q) and the
-	 * key, histogram and partial-sum buffers */
-	int sort_queue(RayQueue &Q, DevBuf &Qbuf, int &Qcap, RayQueue &T, DevBuf &Tbuf, int &Tcap, DevBuf &keysb, DevBuf &hist,
-			DevBuf &part, int n, int bits, const char *name, cudaStream_t s);
+	/* the order of queue Q's first n entries by the top `bits` of their 24-bit
+	 * keys (direction octant over the Morton code of the origin's cell in a
+	 * 128^3 grid): their indices, in the key buffer until its next sort */
+	int sort_queue(const RayQueue &Q, DevBuf &keysb, DevBuf &hist, DevBuf &part, int n, int bits, const char *name, cudaStream_t s,
+			unsigned **sorted);
 	/* photon tracing has buffers and a stream of its own, so that it can run
 	 * beside the first bounce of a frame */
 	DevBuf pqbuf[2], phits, pfbl, pcounts, pctr;
@@ -172,9 +172,7 @@ struct Renderer {
 	/* an emission pass of at least PHOTON_SORT_MIN photons is sorted before
 	 * it is traced, with scratch of its own (the photon stream runs beside
 	 * the frame's) */
-	DevBuf pqsbuf, ps_keys, ps_hist, ps_part;
-	RayQueue pqs = {};
-	int pqscap = 0;
+	DevBuf ps_keys, ps_hist, ps_part;
 	int sort_photon_pass(int cur, int n, cudaStream_t s);
 	cudaStream_t ps = nullptr;
 	int ps_priority = -1;      /* 1 when ps has the greatest priority */
