@@ -281,11 +281,37 @@ struct ProjView {
 	int live;                     /* 0: the light is inside the box (or no such box) */
 };
 
+/* The angles of a direction (x, y, z), as the cell it lies in needs them:
+ * |atan2(z, x)|, and acos of c = y / length, correctly rounded where a cell
+ * ends.  There the last bit decides the cell: the host's functions round
+ * correctly but for a few per cent of the last place, the device's are up to
+ * two places off (acos put 72 of the 117,648 directions of integers up to 24,
+ * all at 45 degrees' elevation, into the row before theirs).  Near an edge B
+ * the angle is B plus the small rest sin(a - B) = (z cos B - x sin B) / r,
+ * taken without cancellation from B's sine and cosine in two doubles. */
+__device__ __forceinline__ double proj_theta(const ProjAngle *edge, double x, double z)
+{
+	const double a = atan2(fabs(z), x);
+	const ProjAngle &e = edge[(int)rint(a * (32.0 / 3.14159265358979323846))];
+	if(!(fabs(a - e.hi) < 1e-13) || e.hi == 0.0) return a;
+	const double w = fabs(z), p = w * e.cos_hi, q = x * e.sin_hi;
+	const double s = (p - q) + ((fma(w, e.cos_hi, -p) - fma(x, e.sin_hi, -q)) + (w * e.cos_lo - x * e.sin_lo));
+	return e.hi + (e.lo + s / sqrt(x * x + z * z));
+}
+
+__device__ __forceinline__ double proj_phi(const ProjAngle *edge, double c)
+{
+	const double a = acos(c);
+	const ProjAngle &e = edge[(int)rint(a * (32.0 / 3.14159265358979323846))];
+	if(!(fabs(a - e.hi) < 1e-13) || e.sin_hi == 0.0) return a;
+	return e.hi + (e.lo + ((e.cos_hi - c) + e.cos_lo) / e.sin_hi);
+}
+
 /* a thread per (sample, box): the double arithmetic, of which this GPU does
  * little at once, with every lane at work; a light inside a box, and the
  * cell of the centre's direction, go straight into the maps */
 __global__ void __launch_bounds__(128) k_proj_view(const ProjSample *samples, int nsamples, int most, const ProjBox *boxes, ProjView *views,
-		unsigned long long *first)
+		const ProjTables *tables, unsigned long long *first)
 {
 	for(long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)nsamples * most; i += (long long)gridDim.x * blockDim.x) {
 		const int si = (int)(i / most), bi = (int)(i - (long long)si * most);
@@ -324,8 +350,9 @@ __global__ void __launch_bounds__(128) k_proj_view(const ProjSample *samples, in
 		V.phi = acosf(fminf(fmaxf(V.u[1], -1.0f), 1.0f));
 		V.cap = V.lo > -1.0f ? acosf(fminf(V.lo, 1.0f)) + 2e-3f : 4.0f;
 		V.live = 1;
-		double theta = atan2(vz, vx), ph = acos(vy / dist);
-		if(theta < 0.0) theta = 3.14159265358979323846 * 2.0 + theta;
+		double theta = proj_theta(tables->edge, vx, vz);
+		const double ph = proj_phi(tables->edge, vy / dist);
+		if(vz < 0.0) theta = 3.14159265358979323846 * 2.0 - theta;
 		double u = theta / (3.14159265358979323846 * 2.0), v = ph / 3.14159265358979323846;
 		int a = (int)(u * 64), b = (int)(v * 32);
 		a = a < 0 ? 0 : (a >= 64 ? 63 : a);
@@ -1031,7 +1058,7 @@ static int project_jobs(Renderer &R, const std::vector<PhotonJobSpec> &spec, cud
 		PCK(R.pj_views.ensure(samples.size() * most * sizeof(ProjView)), "projections");
 		const int ns = (int)samples.size();
 		LAUNCH(R, "projmaps", s, k_proj_view<<<(unsigned)std::min<size_t>(((size_t)ns * most + 127) / 128, 1 << 20), 128, 0, s>>>(
-				R.pj_samples.as<ProjSample>(), ns, most, R.pj_boxes.as<ProjBox>(), R.pj_views.as<ProjView>(),
+				R.pj_samples.as<ProjSample>(), ns, most, R.pj_boxes.as<ProjBox>(), R.pj_views.as<ProjView>(), R.pj_tables.as<ProjTables>(),
 				R.pj_first.as<unsigned long long>()));
 		LAUNCH(R, "projmaps", s, k_proj_mark<<<dim3((unsigned)most, (unsigned)std::min(ns, 65535)), 128, 0, s>>>(
 				R.pj_samples.as<ProjSample>(), ns, most, R.pj_boxes.as<ProjBox>(), R.pj_views.as<ProjView>(), R.pj_tables.as<ProjTables>(),

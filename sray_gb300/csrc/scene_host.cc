@@ -714,6 +714,19 @@ const ProjTables &proj_tables()
 			total += area;
 		}
 		for(int i = 0; i < 64 * 32; i++) t->share[i] = t->share[i] / total;
+		for(int k = 0; k < 33; k++) {
+			const long double a = 3.14159265358979323846264338327950288L * k / 32, d = sqrtl(0.5L);
+			long double c = cosl(a), s = sinl(a);
+			if(k % 16 == 0) { c = k == 0 ? 1 : (k == 16 ? 0 : -1); s = k == 16 ? 1 : 0; }
+			if(k % 16 == 8) { c = k == 8 ? d : -d; s = d; }
+			ProjAngle &e = t->edge[k];
+			e.hi = (double)a;
+			e.lo = (double)(a - e.hi);
+			e.cos_hi = (double)c;
+			e.cos_lo = (double)(c - e.cos_hi);
+			e.sin_hi = (double)s;
+			e.sin_lo = (double)(s - e.sin_hi);
+		}
 		return t;
 	}();
 	return *tables;

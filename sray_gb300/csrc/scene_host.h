@@ -128,11 +128,17 @@ struct Object {
 
 /* The 64 x 32 projection maps' geometry (src/projmap.cc:60-140), the same
  * for every map: the directions of the 65 x 33 cell corners (and
- * the same in float), and each cell's share of the sphere. */
+ * the same in float), each cell's share of the sphere, and the angles where
+ * a cell ends (both ways multiples of pi / 32): the angle, its cosine and
+ * its sine, each the sum of two doubles. */
+struct ProjAngle {
+	double hi, lo, cos_hi, cos_lo, sin_hi, sin_lo;
+};
 struct ProjTables {
 	alignas(16) float cornerf[33 * 65][4];   /* read as float4 */
 	double corner[33 * 65][3];
 	double share[64 * 32];
+	ProjAngle edge[33];
 };
 static_assert(offsetof(ProjTables, cornerf) % 16 == 0 && sizeof(float[4]) == 16, "float4 reads of the corners");
 const ProjTables &proj_tables();
