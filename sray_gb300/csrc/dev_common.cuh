@@ -742,12 +742,13 @@ __device__ __forceinline__ bool trace_any_octree_impl(const DScene &S, V3 wo, V3
  * closest among the faces listed in the mesh-octree leaves the ray reaches
  * (a leaf is reached when its box test and every ancestor's pass).
  *
- * Two binary hierarchies find the same hit faster: one over the objects,
- * each boxed by the union of the top-level leaves that list it, and one per
- * unique mesh over its faces.  Their boxes are widened per ray, so neither
- * skips an object the octree would test or a face the triangle test accepts;
- * the hit found is therefore the closest over a superset of the octrees'
- * candidates.  If it is unique at its distance and both octrees reach it
+ * Two binary hierarchies find the same hit faster: one over the objects and
+ * one per unique mesh over its faces.  An object is boxed by the union of the
+ * top-level leaves that list it, outside which the octree never tests it, or
+ * by its own reach where that is smaller, outside which it has no hit.  The
+ * boxes are widened per ray, so neither hierarchy skips a face or an object
+ * with a hit that the octrees would find; the hit found is therefore the
+ * closest over a superset of the octrees' candidates.  If it is unique at its distance and both octrees reach it
  * (the hit point's leaf lists the face, resp. the object, and that leaf's
  * box test passes), the octrees return it too.  Otherwise -- a second hit at
  * the same distance, or a hit an octree would not reach, both confined to
@@ -766,7 +767,12 @@ __device__ __forceinline__ bool trace_any_octree_impl(const DScene &S, V3 wo, V3
  * by at most 3 * 2^-24 of |x - o|.  Every point and plane involved lies in
  * the hierarchy's bounds, so all of this is below 2^-20.5 (|o| + R), where
  * R is the largest coordinate of those bounds.  The widening is 2^-17 of that
- * (a factor of 11 over it).  It does not grow with the segment's length, which
+ * (a factor of 11 over it).  An object's box is tested in world space, its
+ * hit found in the object's: there the transformed origin and direction are
+ * each off by 5 roundings of the sums' terms per component (the matrix's
+ * entries, three products' sums), which in world space is 2^-20.1 (|o| + R)
+ * for a rotation and scales -- together 2^-19.1, a quarter of the widening.
+ * It does not grow with the segment's length, which
  * is RAY_MAGNITUDE times the unit direction (src/opt.h:21), while the scene is
  * a few hundred units across. */
 struct RayC {

@@ -2676,8 +2676,9 @@ int Renderer::upload_scene(cudaStream_t s)
  * leaf; node references offset by tbase.  Two boxes are safe: the union of
  * the octree leaves that list the object (a ray outside it is never tested
  * against the object by the octree) and, where it is known, the object's
- * reach over [tlo, thi] (a ray outside it has no hit on the object, whatever
- * the octree tests).  Their common part is not: an object may reach beyond
+ * reach over [tlo, thi] (a segment that does not enter it has no hit on the
+ * object, whatever the octree tests; cylinders have none: they report hits
+ * beyond the segment's end).  Their common part is not: an object may reach beyond
  * the leaves that list it, and a ray that crosses such a leaf may hit it
  * outside.  The smaller of the two is taken.  Leaves are far larger
  * than most objects, and each object entered in vain costs a transform and

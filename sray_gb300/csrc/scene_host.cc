@@ -439,22 +439,22 @@ Box Object::bounds(const std::vector<Mesh> &meshes, int t) const
 	return b;
 }
 
-/* A mesh's own bounds, or the box of the transformed quadric (the bounds
+/* A mesh's own bounds, or the box of the transformed sphere (the bounds
  * above ignore its scaling and rotation), widened by 2^-16 of its largest
- * coordinate: far more than the rounding of transforms, vertices and hit
- * points to float. */
+ * coordinate for the rounding of vertices and matrices to float.  (The
+ * rounding of a ray's transform and hit point grows with its origin: the
+ * traversal's widening per ray covers that.) */
 Box Object::reach(const Box &vertices, int t) const
 {
 	Box b = vertices;
-	if(type != OBJ_MESH) {
+	if(type == OBJ_SPHERE) {
 		double m[4][4];
 		xf.matrix(t, m);
-		Vec3 c0 = m_pt(m, Vec3(0, type == OBJ_CYLINDER ? start : 0.0, 0)), c1 = m_pt(m, Vec3(0, type == OBJ_CYLINDER ? end : 0.0, 0));
+		Vec3 c = m_pt(m, Vec3(0, 0, 0));
 		for(int i = 0; i < 3; i++) {
-			double y = type == OBJ_CYLINDER ? 0.0 : m[i][1];
-			double e = fabs(rad) * sqrt(m[i][0] * m[i][0] + y * y + m[i][2] * m[i][2]);
-			b.mn[i] = std::min(c0[i], c1[i]) - e;
-			b.mx[i] = std::max(c0[i], c1[i]) + e;
+			double e = fabs(rad) * sqrt(m[i][0] * m[i][0] + m[i][1] * m[i][1] + m[i][2] * m[i][2]);
+			b.mn[i] = c[i] - e;
+			b.mx[i] = c[i] + e;
 		}
 	}
 	double most = 0.0;
@@ -469,6 +469,10 @@ Box Object::reach(const Box &vertices, int t) const
 bool HostScene::object_reach(size_t i, int tlo, int thi, Box &b) const
 {
 	const Object &o = objs[i];
+	/* a segment may end before the hit that a cylinder reports: the far root
+	 * (Cylinder::intersect, src/cylinder.cc:125-185) counts beyond the end
+	 * where the near one is behind the origin or beside the cylinder */
+	if(o.type == OBJ_CYLINDER) return false;
 	if(o.is_static) {
 		b = o.static_reach;
 		return true;

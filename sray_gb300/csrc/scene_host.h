@@ -121,8 +121,8 @@ struct Object {
 	Box static_box;
 	Box static_reach;          /* of a static object: its reach() */
 	Box bounds(const std::vector<Mesh> &meshes, int t) const;
-	/* a box that holds every point of the object at time t (vertices: a mesh's
-	 * own bounds at that time), float rounding included */
+	/* a box that holds every point of a sphere or mesh at time t (vertices: a
+	 * mesh's own bounds at that time), widened for the rounding of its data */
 	Box reach(const Box &vertices, int t) const;
 };
 
@@ -192,8 +192,9 @@ struct HostScene {
 	std::vector<Box> box_t0, box_t1;   /* object bounds at the frame's t0 / t1 */
 	std::vector<Box> oct_boxes;        /* the boxes the scene octree was built from */
 	Box object_bounds(size_t i, int t) const;
-	/* a box that holds every point of object i at every time in [tlo, thi];
-	 * false where that is not known cheaply (rotating or scaling objects,
+	/* a box that a segment must enter within its length to hit object i at any
+	 * time in [tlo, thi]; false where there is none but the octree's leaves
+	 * (cylinders) or it is not known cheaply (rotating or scaling objects,
 	 * cubic positions) */
 	bool object_reach(size_t i, int tlo, int thi, Box &b) const;
 
