@@ -289,10 +289,17 @@ struct ProjView {
  * all at 45 degrees' elevation, into the row before theirs).  Near an edge B
  * the angle is B plus the small rest sin(a - B) = (z cos B - x sin B) / r,
  * taken without cancellation from B's sine and cosine in two doubles. */
+__device__ __forceinline__ const ProjAngle &proj_edge(const ProjAngle *edge, double a)
+{
+	/* (no number, of a light at the very centre of a flat box, becomes INT_MIN) */
+	const int k = (int)rint(a * (32.0 / 3.14159265358979323846));
+	return edge[k < 0 ? 0 : (k > 32 ? 32 : k)];
+}
+
 __device__ __forceinline__ double proj_theta(const ProjAngle *edge, double x, double z)
 {
 	const double a = atan2(fabs(z), x);
-	const ProjAngle &e = edge[(int)rint(a * (32.0 / 3.14159265358979323846))];
+	const ProjAngle &e = proj_edge(edge, a);
 	if(!(fabs(a - e.hi) < 1e-13) || e.hi == 0.0) return a;
 	const double w = fabs(z), p = w * e.cos_hi, q = x * e.sin_hi;
 	const double s = (p - q) + ((fma(w, e.cos_hi, -p) - fma(x, e.sin_hi, -q)) + (w * e.cos_lo - x * e.sin_lo));
@@ -302,7 +309,7 @@ __device__ __forceinline__ double proj_theta(const ProjAngle *edge, double x, do
 __device__ __forceinline__ double proj_phi(const ProjAngle *edge, double c)
 {
 	const double a = acos(c);
-	const ProjAngle &e = edge[(int)rint(a * (32.0 / 3.14159265358979323846))];
+	const ProjAngle &e = proj_edge(edge, a);
 	if(!(fabs(a - e.hi) < 1e-13) || e.sin_hi == 0.0) return a;
 	return e.hi + (e.lo + ((e.cos_hi - c) + e.cos_lo) / e.sin_hi);
 }

@@ -50,3 +50,23 @@ def test_photons_at_cell_ends(gpu_lib, oracle_lib, name):
             stored += len(a)
         g.close()
     assert stored > 0
+
+
+@pytest.mark.parametrize("light", ["point", "sphere", "box"])
+def test_light_at_a_flat_objects_centre(gpu_lib, oracle_lib, light):
+    """The direction from the light to the floor's centre has no length, so
+    its angles are no numbers (the floor's box is flat: the light is not inside)."""
+    xml = _scene([((3, 1.5, 2), 0.7, True)], [(light, "0 0 0")], False).replace("-0.5 -0.25 -1", "0 0 0").replace("0.5 0.25 1", "0 0 0")
+    xml = xml.replace('<sphere rad="0.6"/>', '<sphere rad="0"/>')
+    opts = dict(width=32, height=32, caust_photons=3000, gi_photons=3000, caust_k=8, gi_k=8, iter=5)
+    g = gpu_lib.GpuRenderer(**opts)
+    g.load_xml(xml)
+    o = oracle_lib.Oracle(fp64=False, rng_mode=1, **opts)
+    o.load_xml(xml)
+    o.prepare(0)
+    g.shoot_photons(0, 0)
+    for which in (0, 1):
+        a, b = g.photons(which)[:, :12], o.photons(which)[:, :12]
+        assert len(a) == len(b) > 0
+        assert np.array_equal(a[np.lexsort(a.T[::-1])], b[np.lexsort(b.T[::-1])])
+    g.close()
