@@ -453,9 +453,10 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, SRAY_PACKET_BLOCKS) k_trac
  * was a chain of 15 exchanges: 64 rays took 57.6 us per call with it, 45.1
  * without; a 321x181 draft 1502 and 1395).  The result is the thread-per-ray
  * traversal's: the closest candidate over every entry whose box is reached
- * within the best distance so far, with a tie where two different faces or
- * objects share it (the candidates at the final distance are reached in any
- * order), confirmed against the octrees; a ray it cannot decide (a tie, an
+ * within the best distance so far (an instance, by the exact box test with
+ * the pruning's slack), with a tie where two different faces or objects share
+ * it (the candidates at the final distance are reached in any order),
+ * confirmed against the octrees; a ray it cannot decide (a tie, an
  * unconfirmed hit, a full stack) goes to the octree retrace. */
 #define WR_CAP 512
 #define WR_POP 8
@@ -528,10 +529,12 @@ __device__ __forceinline__ int warp_trace(const DScene &S, V3 wo, V3 wd, int tim
 							float te;
 							const DevNode &rn = S.mnodes[ob.mesh_root];
 							if(box_hit(rn.mn, rn.mx, orr, te) && (ANY || !SRAY_PRUNE(te, best))) {
+								/* stacked with the pruning's slack: the exact entry
+								 * distance of a flat box can round past a hit in it */
 								push = true;
 								pref = ob.bvh_root;
 								pobj = o;
-								pte = te;
+								pte = fminf(te, te * 0.99998f);
 							}
 						}
 					}
