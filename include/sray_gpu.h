@@ -465,8 +465,10 @@ int sray_gpu_autotune(long msec, float *fb, int frames, void *stream, sray_tunin
  *    SRAY_EDEVICE.
  *  - photon_group > 0: a batch's photon maps are traced in wavefronts of
  *    at most about that many photons (whole jobs; default 2^26), each
- *    group's maps copied out of the wavefront's buffers before the next;
- *    the images do not change. */
+ *    group's maps copied out of the wavefront's buffers before the next,
+ *    and the lights' projection maps are made for two lights, and from about
+ *    that many pairs of a light sample and an object, at a time (default
+ *    1,024 and 2^20); the images do not change. */
 typedef struct sray_faults {
 	int fail_alloc_after;
 	int queue_cap;

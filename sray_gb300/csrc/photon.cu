@@ -1003,90 +1003,145 @@ static int split_photons(const Renderer &R, int light0, int nl, int num, std::ve
 	return prefix[p0 + nl];
 }
 
+/* the projection maps' inputs on the host: kept until the stream that copies
+ * them has been waited for */
+struct ProjHost {
+	std::vector<ProjSample> samples;
+	std::vector<ProjBox> boxes;
+};
+
+/* What is made at a time, so that the workspace does not grow with lights,
+ * objects and jobs: pairs of a light sample and a box (72 bytes each),
+ * lights (33 kB each), boxes (56 bytes each).  What a frame or a batch of
+ * some hundred objects needs is one group. */
+#define PROJ_VIEWS (1 << 20)
+#define PROJ_LIGHTS 1024
+#define PROJ_BOXES (1 << 20)
+
 /* every job's projection maps on stream s: bits (128 words per light of a
  * job: 2048 cells of the map, then of the caustic map) in R.pw_bits, the two
  * coverages in R.pw_cov */
-static int project_jobs(Renderer &R, const std::vector<PhotonJobSpec> &spec, cudaStream_t s)
+static int project_jobs(Renderer &R, const std::vector<PhotonJobSpec> &spec, ProjHost &host, cudaStream_t s)
 {
 	double tp = Renderer::host_now_ms();
-	std::vector<ProjSample> samples;
-	std::vector<ProjBox> boxes;
+	const int small = g_faults.photon_group.load();
+	const size_t max_views = small > 0 ? small : PROJ_VIEWS, max_boxes = small > 0 ? small : PROJ_BOXES;
+	const int max_lights = small > 0 ? 2 : PROJ_LIGHTS;
+	int slots = 0;
+	for(const PhotonJobSpec &J : spec) slots += J.nlights;
+	if(slots > 0) {
+		if(!R.pj_tables_ready) {
+			PCK(R.pj_tables.ensure(sizeof(ProjTables)), "projection tables");
+			PCK(cudaMemcpyAsync(R.pj_tables.p, &proj_tables(), sizeof(ProjTables), cudaMemcpyHostToDevice, s), "projection tables");
+			R.h2d += (int64_t)sizeof(ProjTables);
+			R.pj_tables_ready = true;
+		}
+		PCK(R.pw_bits.ensure((size_t)slots * 128 * sizeof(uint32_t)), "projection maps");
+		PCK(R.pw_cov.ensure((size_t)slots * 2 * sizeof(float)), "coverage");
+	}
+	int done = 0, lights = 0, most = 0;   /* lights of earlier groups and of this one; its samples' largest box count */
+	auto send = [&]() -> int {
+		if(lights == 0) return 0;
+		const size_t bytes = (size_t)lights * 2 * PROJ_SLOT * sizeof(unsigned long long);
+		PCK(R.pj_first.ensure(bytes), "projection cells");
+		PCK(cudaMemsetAsync(R.pj_first.p, 0xff, bytes, s), "projection cells");
+		const int ns = (int)host.samples.size();
+		if(ns > 0) {
+			PCK(R.pj_samples.upload(host.samples, s), "light samples");
+			PCK(R.pj_boxes.upload(host.boxes, s), "object boxes");
+			R.h2d += (int64_t)(ns * sizeof(ProjSample) + host.boxes.size() * sizeof(ProjBox));
+			const int per = (int)std::max<size_t>(1, std::min<size_t>(max_views / most, ns));
+			PCK(R.pj_views.ensure((size_t)per * most * sizeof(ProjView)), "projections");
+			const ProjBox *boxes = R.pj_boxes.as<ProjBox>();
+			ProjView *views = R.pj_views.as<ProjView>();
+			const ProjTables *tables = R.pj_tables.as<ProjTables>();
+			unsigned long long *first = R.pj_first.as<unsigned long long>();
+			for(int q = 0; q < ns; q += per) {
+				const ProjSample *smp = R.pj_samples.as<ProjSample>() + q;
+				const int m = std::min(per, ns - q);
+				LAUNCH(R, "projmaps", s, k_proj_view<<<(unsigned)std::min<size_t>(((size_t)m * most + 127) / 128, 1 << 20), 128, 0, s>>>(smp,
+						m, most, boxes, views, tables, first));
+				LAUNCH(R, "projmaps", s, k_proj_mark<<<dim3((unsigned)most, (unsigned)std::min(m, 65535)), 128, 0, s>>>(smp, m, most, boxes,
+						views, tables, first));
+			}
+		}
+		LAUNCH(R, "projmaps", s, k_proj_cover<<<lights * 2, 1024, 0, s>>>(R.pj_first.as<unsigned long long>(), R.pj_tables.as<ProjTables>(),
+				R.pw_bits.as<uint32_t>() + (size_t)done * 128, R.pw_cov.as<float>() + (size_t)done * 2));
+		PCK(cudaGetLastError(), "projection maps");
+		return 0;
+	};
+	/* the next group, whose inputs take the place of the last one's */
+	auto next = [&]() -> int {
+		if(int r = send()) return r;
+		PCK(cudaStreamSynchronize(s), "projection maps");
+		done += lights;
+		lights = most = 0;
+		host.samples.clear();
+		host.boxes.clear();
+		return 0;
+	};
+	std::vector<ProjBox> ends[2];
 	std::vector<Vec3> pts;
 	std::vector<int> times;
-	int slots = 0, most = 0;
 	for(const PhotonJobSpec &J : spec) {
 		/* the job's object boxes at its interval's ends */
-		const int ends[2] = {J.t0, J.t1};
-		size_t box0[2] = {boxes.size(), boxes.size()};
-		for(int e = 0; e < (J.t0 == J.t1 ? 1 : 2); e++) {
-			box0[e] = boxes.size();
+		const int at[2] = {J.t0, J.t1}, nend = J.t0 == J.t1 ? 1 : 2;
+		for(int e = 0; e < nend; e++) {
+			ends[e].clear();
 			for(int i = J.obj0; i < J.obj0 + J.nobj; i++) {
-				const Box b = R.sc.object_bounds((size_t)i, ends[e]);
+				const Box b = R.sc.object_bounds((size_t)i, at[e]);
 				const Material &m = R.sc.objs[i].mat >= 0 ? R.sc.mats[R.sc.objs[i].mat] : R.sc.defmat;
 				ProjBox d;
 				for(int k = 0; k < 3; k++) { d.mn[k] = b.mn[k]; d.mx[k] = b.mx[k]; }
 				d.caustic = m.refl > 0.0 || m.refr > 0.0 ? 1 : 0;
 				d.pad = 0;
-				boxes.push_back(d);
+				ends[e].push_back(d);
 			}
 		}
-		for(int k = 0; k < J.nlights; k++, slots++) {
+		int box0[2] = {-1, -1};
+		for(int k = 0; k < J.nlights; k++) {
+			if(lights >= max_lights || (box0[0] < 0 && lights > 0 && host.boxes.size() + nend * ends[0].size() > max_boxes)) {
+				if(int r = next()) return r;
+				box0[0] = -1;
+			}
+			const int slot = lights++;
 			if(J.nobj <= 0) continue;
+			if(box0[0] < 0) {
+				for(int e = 0; e < nend; e++) {
+					box0[e] = (int)host.boxes.size();
+					host.boxes.insert(host.boxes.end(), ends[e].begin(), ends[e].end());
+				}
+			}
 			pts.clear();
 			times.clear();
 			R.sc.light_samples((size_t)(J.light0 + k), J.t0, J.t1, R.opt.seed, k, pts, times);
 			for(size_t q = 0; q < pts.size(); q++) {
 				ProjSample d;
 				for(int c = 0; c < 3; c++) d.lp[c] = pts[q][c];
-				d.box0 = (int)box0[times[q] == J.t0 ? 0 : 1];
+				d.box0 = box0[times[q] == J.t0 ? 0 : 1];
 				d.nbox = J.nobj;
-				d.slot = slots;
+				d.slot = slot;
 				d.order = (unsigned)q;
-				samples.push_back(d);
+				host.samples.push_back(d);
 				most = std::max(most, J.nobj);
 			}
 		}
 	}
-	if(slots == 0) return 0;
-	if(!R.pj_tables_ready) {
-		PCK(R.pj_tables.ensure(sizeof(ProjTables)), "projection tables");
-		PCK(cudaMemcpyAsync(R.pj_tables.p, &proj_tables(), sizeof(ProjTables), cudaMemcpyHostToDevice, s), "projection tables");
-		R.h2d += (int64_t)sizeof(ProjTables);
-		R.pj_tables_ready = true;
-	}
-	PCK(R.pw_bits.ensure((size_t)slots * 128 * sizeof(uint32_t)), "projection maps");
-	PCK(R.pw_cov.ensure((size_t)slots * 2 * sizeof(float)), "coverage");
-	PCK(R.pj_first.ensure((size_t)slots * 2 * PROJ_SLOT * sizeof(unsigned long long)), "projection cells");
-	PCK(cudaMemsetAsync(R.pj_first.p, 0xff, (size_t)slots * 2 * PROJ_SLOT * sizeof(unsigned long long), s), "projection cells");
-	if(!samples.empty()) {
-		PCK(R.pj_samples.upload(samples, s), "light samples");
-		PCK(R.pj_boxes.upload(boxes, s), "object boxes");
-		R.h2d += (int64_t)(samples.size() * sizeof(ProjSample) + boxes.size() * sizeof(ProjBox));
-		PCK(R.pj_views.ensure(samples.size() * most * sizeof(ProjView)), "projections");
-		const int ns = (int)samples.size();
-		LAUNCH(R, "projmaps", s, k_proj_view<<<(unsigned)std::min<size_t>(((size_t)ns * most + 127) / 128, 1 << 20), 128, 0, s>>>(
-				R.pj_samples.as<ProjSample>(), ns, most, R.pj_boxes.as<ProjBox>(), R.pj_views.as<ProjView>(), R.pj_tables.as<ProjTables>(),
-				R.pj_first.as<unsigned long long>()));
-		LAUNCH(R, "projmaps", s, k_proj_mark<<<dim3((unsigned)most, (unsigned)std::min(ns, 65535)), 128, 0, s>>>(
-				R.pj_samples.as<ProjSample>(), ns, most, R.pj_boxes.as<ProjBox>(), R.pj_views.as<ProjView>(), R.pj_tables.as<ProjTables>(),
-				R.pj_first.as<unsigned long long>()));
-	}
-	LAUNCH(R, "projmaps", s, k_proj_cover<<<slots * 2, 1024, 0, s>>>(R.pj_first.as<unsigned long long>(), R.pj_tables.as<ProjTables>(),
-			R.pw_bits.as<uint32_t>(), R.pw_cov.as<float>()));
-	PCK(cudaGetLastError(), "projection maps");
+	if(int r = send()) return r;
 	R.host_time("host.projmaps", tp);
 	return 0;
 }
 
 /* Both photon maps of every job, traced as one wavefront on stream s: their
- * projection maps, the emission of all jobs' photons in one launch, then passes of closest hits
- * and interactions over one queue (each photon finds its job, and through
+ * projection maps, the emission of all jobs' photons in one launch, then
+ * passes of closest hits and interactions over one queue (each photon finds its job, and through
  * it its scene, lights, interval and projection maps), then the tail.  The
  * stored photons and their flags stay in R.pw_out / R.pw_valid by global
  * index; jobs[j].base and total[] locate each job's two segments. */
 int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJobSpec> &spec, std::vector<PJobOut> &out,
 		cudaStream_t s)
 {
+	ProjHost proj_host;
 	int n = (int)spec.size();
 	out.assign(n, PJobOut());
 	std::vector<PJob> jobs(n);
@@ -1119,7 +1174,7 @@ int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJ
 		if(all > INT_MAX / 2) return R.fail(SRAY_EINVAL, "too many photons in one wavefront");
 	}
 	if(all == 0) return 0;
-	if(int r = project_jobs(R, spec, s)) return r;
+	if(int r = project_jobs(R, spec, proj_host, s)) return r;
 	PCK(R.pw_jobs.upload(jobs, s), "photon jobs");
 	PCK(R.pw_prefix.upload(prefix, s), "photon prefix");
 	PCK(R.pw_scale.upload(scale, s), "photon scale");
