@@ -1020,8 +1020,8 @@ struct ProjHost {
 
 /* every job's projection maps on stream s: bits (128 words per light of a
  * job: 2048 cells of the map, then of the caustic map) in R.pw_bits, the two
- * coverages in R.pw_cov */
-static int project_jobs(Renderer &R, const std::vector<PhotonJobSpec> &spec, ProjHost &host, cudaStream_t s)
+ * coverages in R.pw_cov; and the jobs' boxes, of the same bounds */
+static int project_jobs(Renderer &R, std::vector<PhotonJobSpec> &spec, ProjHost &host, cudaStream_t s)
 {
 	double tp = Renderer::host_now_ms();
 	const int small = g_faults.photon_group.load();
@@ -1083,16 +1083,22 @@ static int project_jobs(Renderer &R, const std::vector<PhotonJobSpec> &spec, Pro
 	std::vector<ProjBox> ends[2];
 	std::vector<Vec3> pts;
 	std::vector<int> times;
-	for(const PhotonJobSpec &J : spec) {
-		/* the job's object boxes at its interval's ends */
+	for(PhotonJobSpec &J : spec) {
+		/* the job's object boxes at its interval's ends, and their union */
 		const int at[2] = {J.t0, J.t1}, nend = J.t0 == J.t1 ? 1 : 2;
+		for(int k = 0; k < 3; k++) { J.box.mn[k] = FLT_MAX; J.box.mx[k] = -FLT_MAX; }
 		for(int e = 0; e < nend; e++) {
 			ends[e].clear();
 			for(int i = J.obj0; i < J.obj0 + J.nobj; i++) {
 				const Box b = R.sc.object_bounds((size_t)i, at[e]);
 				const Material &m = R.sc.objs[i].mat >= 0 ? R.sc.mats[R.sc.objs[i].mat] : R.sc.defmat;
 				ProjBox d;
-				for(int k = 0; k < 3; k++) { d.mn[k] = b.mn[k]; d.mx[k] = b.mx[k]; }
+				for(int k = 0; k < 3; k++) {
+					d.mn[k] = b.mn[k];
+					d.mx[k] = b.mx[k];
+					J.box.mn[k] = std::min(J.box.mn[k], b.mn[k]);
+					J.box.mx[k] = std::max(J.box.mx[k], b.mx[k]);
+				}
 				d.caustic = m.refl > 0.0 || m.refr > 0.0 ? 1 : 0;
 				d.pad = 0;
 				ends[e].push_back(d);
@@ -1138,8 +1144,7 @@ static int project_jobs(Renderer &R, const std::vector<PhotonJobSpec> &spec, Pro
  * it its scene, lights, interval and projection maps), then the tail.  The
  * stored photons and their flags stay in R.pw_out / R.pw_valid by global
  * index; jobs[j].base and total[] locate each job's two segments. */
-int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJobSpec> &spec, std::vector<PJobOut> &out,
-		cudaStream_t s)
+int photon_trace_jobs(Renderer &R, const DScene &base, std::vector<PhotonJobSpec> &spec, std::vector<PJobOut> &out, cudaStream_t s)
 {
 	ProjHost proj_host;
 	int n = (int)spec.size();

@@ -2906,33 +2906,23 @@ int Renderer::photon_job(DScene base)
 	size_t n = batch_t0.size();
 	std::vector<DPhotonMap> hm(2 * n);
 	std::vector<PhotonJobSpec> spec(n);
-	std::vector<int> o0(n, 0), no(n, (int)sc.objs.size());
 	for(size_t j = 0; j < n; j++) {
 		PhotonJobSpec &J = spec[j];
 		J.light0 = 0;
 		J.nlights = (int)sc.lights.size();
+		J.nobj = (int)sc.objs.size();
 		if(!scene_refs.empty()) {
 			const SceneRange &rg = sc.ranges[batch_scene[j]];
 			J.light0 = rg.light0;
 			J.nlights = rg.nlight;
 			J.scene = batch_scene[j];
-			o0[j] = rg.obj0;
-			no[j] = rg.nobj;
+			J.obj0 = rg.obj0;
+			J.nobj = rg.nobj;
 		}
 		J.num[0] = batch_caust[j] > 0 ? batch_caust[j] : opt.caust_photons;
 		J.num[1] = batch_gi[j] > 0 ? batch_gi[j] : opt.gi_photons;
 		J.t0 = (int)batch_t0[j];
 		J.t1 = (int)batch_t1[j];
-		J.obj0 = o0[j];
-		J.nobj = no[j];
-	}
-	/* the grids of the jobs' own frames: boxes and range radii over their
-	 * own intervals (the batch's tree spans every job's interval) */
-	std::vector<Box> boxes(n);
-	std::vector<double> gdist(n);
-	for(size_t j = 0; j < n; j++) {
-		boxes[j] = sc.box_at(batch_t0[j], batch_t1[j], o0[j], no[j]);
-		gdist[j] = sc.gather_dist_at(batch_t0[j], batch_t1[j], opt, o0[j], no[j]);
 	}
 	/* jobs in groups of at most PW_MAX_PHOTONS photons per wavefront, so that
 	 * the wavefront's memory follows the group and not the batch; when the
@@ -2954,11 +2944,17 @@ int Renderer::photon_job(DScene base)
 	for(size_t gi0 = 0; gi0 + 1 < group0.size(); gi0++) {
 		size_t a = group0[gi0], b = group0[gi0 + 1];
 		std::vector<PhotonJobSpec> gspec(spec.begin() + a, spec.begin() + b);
-		std::vector<Box> gbox(boxes.begin() + a, boxes.begin() + b);
-		std::vector<double> gd(gdist.begin() + a, gdist.begin() + b);
 		std::vector<PJobOut> out;
 		int r = photon_trace_jobs(*this, base, gspec, out, ps);
 		if(r) return r;
+		/* the grids of the jobs' own frames: boxes and range radii over their
+		 * own intervals (the batch's tree spans every job's interval) */
+		std::vector<Box> gbox;
+		std::vector<double> gd;
+		for(const PhotonJobSpec &J : gspec) {
+			gbox.push_back(J.box);
+			gd.push_back(sc.gather_dist_of(J.box, opt));
+		}
 		std::vector<DPhotonMap> gm;
 		r = photon_finalize_jobs(*this, out, gbox, gd, gm, ps);
 		if(r == 0) {
@@ -2985,8 +2981,8 @@ int Renderer::photon_job(DScene base)
 		const DevPhoton *ph = pw_out.as<DevPhoton>();
 		const int *valid = pw_valid.as<int>();
 		for(size_t j = a; j < b; j++) {
-			map_gather_dist = gdist[j];
-			map_box = boxes[j];
+			map_gather_dist = gd[j - a];
+			map_box = gbox[j - a];
 			map_has_box = true;
 			std::swap(caust, job_maps[j].caust);
 			std::swap(gi, job_maps[j].gi);

@@ -338,10 +338,10 @@ struct PhotonJobSpec {
 	int t0 = 0, t1 = 0;           /* its interval */
 	int scene = -1;               /* its scene in a scene set (-1: the view's own) */
 	int obj0 = 0, nobj = 0;       /* its scene's objects */
+	Box box;                      /* the union of their bounds at t0 and t1: set by photon_trace_jobs, where it has photons */
 };
 struct PJobOut { int base = 0; int total[2] = {0, 0}; };   /* a job's photons: first global index, counts per map */
-int photon_trace_jobs(Renderer &R, const DScene &base, const std::vector<PhotonJobSpec> &spec, std::vector<PJobOut> &out,
-		cudaStream_t s);
+int photon_trace_jobs(Renderer &R, const DScene &base, std::vector<PhotonJobSpec> &spec, std::vector<PJobOut> &out, cudaStream_t s);
 int photon_finalize(Renderer &R, int global, const int *valid, const DevPhoton *in, int total, cudaStream_t s, int *stored);
 int sort_pairs(Renderer &R, unsigned *keys, unsigned *vals, unsigned *keys2, unsigned *vals2, int n, int bits, DevBuf &hist,
 		DevBuf &part, const char *name, cudaStream_t s, unsigned **keys_out, unsigned **vals_out);

@@ -796,9 +796,7 @@ void HostScene::build_tree(int t0, int t1, const sray_opts &opt)
 	}
 	oct.build(boxes, opt.scnoct_max_depth, opt.scnoct_max_items);
 	oct_boxes = boxes;
-	const Box &rb = oct.nodes[0].box;
-	double dx = rb.mx[0] - rb.mn[0], dy = rb.mx[1] - rb.mn[1], dz = rb.mx[2] - rb.mn[2];
-	gather_dist = sqrt(dx * dx + dy * dy + dz * dz) * opt.gather_dist;
+	gather_dist = gather_dist_of(oct.nodes[0].box, opt);
 }
 
 void HostScene::bound_objects(int t0, int t1, const sray_opts &opt)
@@ -817,35 +815,21 @@ void HostScene::bound_objects(int t0, int t1, const sray_opts &opt)
 		}
 	}
 	oct.nodes.assign(1, BuildOctree::Node());
-	oct.nodes[0].box = box_at(t0, t1);
-	const Box &rb = oct.nodes[0].box;
-	double dx = rb.mx[0] - rb.mn[0], dy = rb.mx[1] - rb.mn[1], dz = rb.mx[2] - rb.mn[2];
-	gather_dist = sqrt(dx * dx + dy * dy + dz * dz) * opt.gather_dist;
-}
-
-/* the root box of Scene::build_tree(t0, t1) (src/scene.cc:353-390): the
- * union of every object's bounds at t0 and t1 */
-Box HostScene::box_at(int t0, int t1, int obj0, int nobj) const
-{
-	if(nobj < 0) nobj = (int)objs.size() - obj0;
-	Box u;
-	for(int k = 0; k < 3; k++) { u.mn[k] = FLT_MAX; u.mx[k] = -FLT_MAX; }
-	for(size_t i = (size_t)obj0; i < (size_t)(obj0 + nobj); i++) {
-		Box b[2] = {object_bounds(i, t0), t1 == t0 ? object_bounds(i, t0) : object_bounds(i, t1)};
-		for(int j = 0; j < 2; j++)
-			for(int k = 0; k < 3; k++) {
-				if(b[j].mn[k] < u.mn[k]) u.mn[k] = b[j].mn[k];
-				if(b[j].mx[k] > u.mx[k]) u.mx[k] = b[j].mx[k];
-			}
+	Box &rb = oct.nodes[0].box;
+	for(int k = 0; k < 3; k++) { rb.mn[k] = FLT_MAX; rb.mx[k] = -FLT_MAX; }
+	for(const Box &b : oct_boxes) {
+		for(int k = 0; k < 3; k++) {
+			rb.mn[k] = std::min(rb.mn[k], b.mn[k]);
+			rb.mx[k] = std::max(rb.mx[k], b.mx[k]);
+		}
 	}
-	return u;
+	gather_dist = gather_dist_of(oct.nodes[0].box, opt);
 }
 
-/* gather_dist of Scene::build_tree(t0, t1) (src/scene.cc:384-387): the
- * diagonal of the root box times the option */
-double HostScene::gather_dist_at(int t0, int t1, const sray_opts &opt, int obj0, int nobj) const
+/* gather_dist of Scene::build_tree (src/scene.cc:384-387): the diagonal of
+ * the root box times the option */
+double HostScene::gather_dist_of(const Box &b, const sray_opts &opt) const
 {
-	Box b = box_at(t0, t1, obj0, nobj);
 	double dx = b.mx[0] - b.mn[0], dy = b.mx[1] - b.mn[1], dz = b.mx[2] - b.mn[2];
 	return sqrt(dx * dx + dy * dy + dz * dz) * opt.gather_dist;
 }

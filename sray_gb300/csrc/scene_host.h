@@ -213,10 +213,8 @@ struct HostScene {
 	 * the octree (a scene set's scenes have octrees of their own): oct keeps
 	 * its root node only */
 	void bound_objects(int t0, int t1, const sray_opts &opt);
-	/* the root box and gather radius build_tree(t0, t1) would give the
-	 * objects obj0 .. obj0 + nobj, without building */
-	Box box_at(int t0, int t1, int obj0 = 0, int nobj = -1) const;
-	double gather_dist_at(int t0, int t1, const sray_opts &opt, int obj0 = 0, int nobj = -1) const;
+	/* the gather radius of a tree with root box b */
+	double gather_dist_of(const Box &b, const sray_opts &opt) const;
 	/* the points of light li from which its projection maps see the objects:
 	 * Light::build_proj_intern's samples (src/light.cc:151-200) at time t0 and,
 	 * where it differs, t1, drawn from the stream of the light's key; their
