@@ -254,7 +254,8 @@ int sray_gpu_render_pixels(long msec, float *fb, int fb_is_device, void *stream)
  * Scene::cast_ray (src/scene.cc:764-794).  All arrays are device pointers.
  * Outputs: object index (-1 = miss), primitive index (triangle index of the
  * object's mesh, 0 for spheres/cylinders), the hit parameter t, and a flag
- * byte that is 1 when another primitive was found at exactly the same t. */
+ * byte that is 1 when another primitive was found at exactly the same t.
+ * After the first call of a context no call allocates device memory. */
 int sray_gpu_cast_rays(int n, const float *orig, const float *dir, const int *time,
 		int *obj, int *prim, float *t, unsigned char *tie, void *stream);
 
@@ -410,7 +411,9 @@ typedef struct sray_tuning {
 	                             render work (on an internal stream ordered after and
 	                             before the caller's) (2) */
 	int warp_rays;            /* closest-hit passes of at most this many rays trace one
-	                             ray per warp instead of one per thread (0: never) (16384) */
+	                             ray per warp instead of one per thread (0: never); calls
+	                             of sray_gpu_cast_rays in scenes of a few objects at most
+	                             4,096 (16384) */
 	int warp_segments;        /* the same for light-sample passes of at most this many
 	                             segments (16384) */
 	int queue_depth;          /* primary rays per wave: a sample batch's pixels go through

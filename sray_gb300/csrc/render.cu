@@ -2129,11 +2129,18 @@ __global__ void k_finish(const int *active, int tw, int th, const int *n_active_
 	}
 }
 
-/* closest hits of caller-supplied world rays (sray_gpu_cast_rays), as the
- * frame's passes: chunks of rays per block, then the listed rays by the
- * octrees; or one warp per ray, whose first lane follows the octrees itself
- * where they must decide (64 rays 45.4 us per call with a list, its clearing
- * and a second launch for the few such rays, 41.9 without) */
+/* Closest hits of caller-supplied world rays (sray_gpu_cast_rays), which
+ * allocates nothing: one warp per ray, whose first lane follows the octrees
+ * where they must decide; or chunks of rays per block, as the frame's passes.
+ * Up to a ray per lane of the GPU a block's threads follow the octrees for
+ * its undecided rays (FUSED; a list in shared memory); above, such rays are
+ * marked in their output and k_cast_octree takes them in a second launch: the
+ * octree's code costs the walk registers (1,000,003 rays over the terrain
+ * 653 us with it, 624 without), the launch 4 us (100,000 rays
+ * over two triangles 42 and 38 us).  A list of all undecided rays in device
+ * memory, a block per SM for it and its clearing took a million rays that all
+ * end on two coincident meshes 277 us, 175 this way (163 with a ray per
+ * thread to its end, octrees included, which took the terrain's 1,900). */
 struct CastRays {
 	const float *orig, *dir;
 	const int *time;          /* may be null: the frame's */
@@ -2152,12 +2159,30 @@ struct CastRays {
 	}
 };
 
-__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRays R, int n, int chunk, DevCounters *ctr, int *fb)
+/* ray i by the octrees alone */
+__device__ __forceinline__ void cast_octree(const DScene &S, const CastRays &R, int i, DevCounters *ctr)
+{
+	Hit h;
+	int overflow = 0;
+	trace_closest_octree<false>(S, R.o(i), R.d(i), R.when(S, i), h, nullptr, &overflow);
+	R.put(i, h.obj, h.prim, h.t, h.tie);
+	if(overflow) atomicOr(&ctr->overflow, 1);
+}
+
+#define CAST_UNDECIDED -2
+#define CAST_OCTREE_RAYS 512     /* per block of k_cast_octree */
+
+template <bool FUSED>
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRays R, int n, int chunk, DevCounters *ctr)
 {
 	__shared__ float world[WORLD_WORDS * SRAY_TRACE_THREADS];
-	__shared__ int next;
+	__shared__ int list[FUSED ? SRAY_TRACE_THREADS : 1];     /* FUSED: chunk is SRAY_TRACE_THREADS */
+	__shared__ int next, listed;
 	const int first = blockIdx.x * chunk;
-	if(threadIdx.x == 0) next = first;
+	if(threadIdx.x == 0) {
+		next = first;
+		listed = 0;
+	}
 	__syncthreads();
 	int overflow = 0;
 	walk_stream<CAST_REFILL, false, false, true>(S, world + threadIdx.x, &next, min(first + chunk, n),
@@ -2169,10 +2194,29 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRa
 				return i;
 			},
 			[&](int i, int sure, const Walk<false, false, true, SharedWorld> &w) {
-				if(!sure) fb[1 + atomicAdd(fb, 1)] = i;
-				else R.put(i, w.bobj, w.bprim, w.best, 0);
+				if(FUSED && !sure) list[atomicAdd(&listed, 1)] = i;
+				R.put(i, sure ? w.bobj : CAST_UNDECIDED, w.bprim, w.best, 0);
 			}, nullptr, &overflow);
 	if(overflow) atomicOr(&ctr->overflow, 1);
+	if(FUSED) {
+		__syncthreads();
+		if(threadIdx.x < listed) cast_octree(S, R, list[threadIdx.x], ctr);
+	}
+}
+
+/* the marked rays by the octrees, gathered from CAST_OCTREE_RAYS per block so
+ * that a warp has more than one of them */
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS) k_cast_octree(DScene S, CastRays R, int n, DevCounters *ctr)
+{
+	__shared__ int list[CAST_OCTREE_RAYS];
+	__shared__ int listed;
+	const int first = blockIdx.x * CAST_OCTREE_RAYS;
+	if(threadIdx.x == 0) listed = 0;
+	__syncthreads();
+	for(int k = threadIdx.x; k < CAST_OCTREE_RAYS && first + k < n; k += SRAY_TRACE_THREADS)
+		if(R.obj[first + k] == CAST_UNDECIDED) list[atomicAdd(&listed, 1)] = first + k;
+	__syncthreads();
+	for(int k = threadIdx.x; k < listed; k += SRAY_TRACE_THREADS) cast_octree(S, R, list[k], ctr);
 }
 
 __global__ void __launch_bounds__(128) k_cast_warp(const __grid_constant__ DScene S, CastRays R, int n, DevCounters *ctr)
@@ -2186,31 +2230,11 @@ __global__ void __launch_bounds__(128) k_cast_warp(const __grid_constant__ DScen
 		int bobj, bprim;
 		int res = warp_trace<false>(S, R.o(i), R.d(i), R.when(S, i), s_ref[w], s_obj[w], s_te[w], best, bobj, bprim, -1);
 		if(lane == 0) {
-			if(!res) {
-				Hit h;
-				int overflow = 0;
-				trace_closest_octree<false>(S, R.o(i), R.d(i), R.when(S, i), h, nullptr, &overflow);
-				R.put(i, h.obj, h.prim, h.t, h.tie);
-				if(overflow) atomicOr(&ctr->overflow, 1);
-			} else {
-				R.put(i, bobj, bprim, best, 0);
-			}
+			if(!res) cast_octree(S, R, i, ctr);
+			else R.put(i, bobj, bprim, best, 0);
 		}
 		__syncwarp();
 	}
-}
-
-__global__ void __launch_bounds__(SRAY_TRACE_THREADS) k_cast_octree(DScene S, CastRays R, DevCounters *ctr, const int *fb)
-{
-	const int n = fb[0];
-	int overflow = 0;
-	for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-		int i = fb[1 + k];
-		Hit h;
-		trace_closest_octree_impl<false>(S, R.o(i), R.d(i), R.when(S, i), h, nullptr, &overflow);
-		R.put(i, h.obj, h.prim, h.t, h.tie);
-	}
-	if(overflow) atomicOr(&ctr->overflow, 1);
 }
 
 /* The primary hits of a whole image (sray_gpu_primary_hits) by the warps that
@@ -2667,6 +2691,7 @@ int Renderer::upload_scene(cudaStream_t s)
 	CK(key_t.upload(kt, s), "upload key times");
 	CK(key_v.upload(kv, s), "upload key values");
 	CK(bnodes.upload(bn, s), "upload mesh hierarchies");
+	mesh_nodes = (int)bn.size();
 	CK(btris.upload(bt, s), "upload hierarchy triangles");
 	CK(bprim.upload(bp, s), "upload hierarchy face ids");
 	CK(bhome.upload(bh, s), "upload hierarchy home nodes");
@@ -2872,6 +2897,7 @@ int Renderer::build_frame(long bt0, long bt1, cudaStream_t s)
 	CK(tnodes.upload(tn, s), "upload object hierarchy");
 	CK(ohome.upload(ohome_h, s), "upload object home nodes");
 	has_tlas = !tn.empty();
+	object_nodes = (int)tn.size();
 	CK(cam_m.upload(cm, s), "upload camera");
 	h2d += (int64_t)(nodes.size() * sizeof(DevNode) + slots.size() * 4 + cm.size() * 4);
 	CK(cudaStreamSynchronize(s), "build frame");
@@ -4574,6 +4600,7 @@ int sray_gpu_render_batch(const sray_job *jobs, int n, void *stream)
 	return r;
 }
 
+#define CAST_FEW_NODES 64
 int sray_gpu_cast_rays(int n, const float *orig, const float *dir, const int *time, int *obj, int *prim, float *t,
 		unsigned char *tie, void *stream)
 {
@@ -4585,19 +4612,26 @@ int sray_gpu_cast_rays(int n, const float *orig, const float *dir, const int *ti
 	if(n == 0) return 0;
 	cudaStream_t s = as_stream(stream);
 	cudaError_t e = R.ctr.ensure(sizeof(DevCounters));
-	const bool listed = n > R.tune.warp_rays;
-	if(e == cudaSuccess && listed) e = R.fbl.ensure(((size_t)n + 1) * sizeof(int));
 	if(e == cudaSuccess) e = cudaMemsetAsync(R.ctr.p, 0, sizeof(DevCounters), s);
-	if(e == cudaSuccess && listed) e = cudaMemsetAsync(R.fbl.p, 0, sizeof(int), s);
 	if(e != cudaSuccess) { g_err = cudaGetErrorString(e); return SRAY_ECUDA; }
 	const CastRays rays = {orig, dir, time, obj, prim, t, tie};
-	if(!listed) {
-		k_cast_warp<<<grid_for(n, 4), 128, 0, s>>>(R.S, rays, n, R.ctr.as<DevCounters>());
+	DevCounters *c = R.ctr.as<DevCounters>();
+	/* A warp per ray shortens a long walk's chain of steps and takes 32 lanes
+	 * for it.  16,384 rays over the 1.26M-triangle terrain 123 us by warps,
+	 * 139 by streams; over 2,000 spheres 64 and 64; but over two triangles 48
+	 * and 37, over 100 spheres 51 and 41 (4,096 rays: 37 and 38, 35 and 40):
+	 * in scenes of few nodes there is no chain to shorten. */
+	const int by_warps = R.object_nodes + R.mesh_nodes < CAST_FEW_NODES ? std::min(R.tune.warp_rays, 4096) : R.tune.warp_rays;
+	if(n <= by_warps) {
+		k_cast_warp<<<grid_for(n, 4), 128, 0, s>>>(R.S, rays, n, c);
 	} else {
-		int *fb = R.fbl.as<int>();
-		const int chunk = stream_chunk(n, CAST_CHUNK);
-		k_cast<<<(n + chunk - 1) / chunk, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, n, chunk, R.ctr.as<DevCounters>(), fb);
-		k_cast_octree<<<grid_for(n, 128) < R.nsm ? grid_for(n, 128) : R.nsm, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, R.ctr.as<DevCounters>(), fb);
+		const int chunk = stream_chunk(n, CAST_CHUNK), blocks = (n + chunk - 1) / chunk;
+		if(chunk == SRAY_TRACE_THREADS) {
+			k_cast<true><<<blocks, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, n, chunk, c);
+		} else {
+			k_cast<false><<<blocks, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, n, chunk, c);
+			k_cast_octree<<<(n + CAST_OCTREE_RAYS - 1) / CAST_OCTREE_RAYS, SRAY_TRACE_THREADS, 0, s>>>(R.S, rays, n, c);
+		}
 	}
 	DevCounters hc;
 	e = cudaMemcpyAsync(&hc, R.ctr.p, sizeof hc, cudaMemcpyDeviceToHost, s);

@@ -138,6 +138,7 @@ struct Renderer {
 	DevBuf snodes, sslots, xf, light_pos, cam_m, tnodes, ohome;
 	bool built = false;
 	bool has_tlas = false;
+	int object_nodes = 0, mesh_nodes = 0;   /* of the object hierarchy, of the meshes' */
 	int t0 = 0, t1 = 0, tlo = 0, nt = 1;
 	int scene_root = 0;
 	long frame_msec = 0;
