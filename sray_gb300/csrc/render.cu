@@ -4747,7 +4747,7 @@ int sray_gpu_get_photons(int which, float *out, int cap, int *n_out)
 	if(!out || cap <= 0 || n == 0) return 0;
 	int m = n < cap ? n : cap;
 	std::vector<DevPhoton> h;
-	if(int r = photon_map_read(R, which ? 1 : 0, h, 0)) { g_err = R.err; return r; }
+	if(int r = photon_map_read(R, which ? 1 : 0, m, h, 0)) { g_err = R.err; return r; }
 	for(int i = 0; i < m; i++) {
 		float *f = out + (size_t)i * 16;
 		f[0] = h[i].p[0]; f[1] = h[i].p[1]; f[2] = h[i].p[2];
@@ -4767,7 +4767,7 @@ int sray_gpu_dump_photons(int which, const char *path)
 	Renderer &R = *g_R;
 	if(!path || (which != 0 && which != 1)) { g_err = "bad arguments"; return SRAY_EINVAL; }
 	std::vector<DevPhoton> h;
-	if(int r = photon_map_read(R, which, h, 0)) { g_err = R.err; return r; }
+	if(int r = photon_map_read(R, which, (which ? R.gi : R.caust).map.n, h, 0)) { g_err = R.err; return r; }
 	FILE *fp = fopen(path, "w");
 	if(!fp) { g_err = std::string("failed to dump photon map: ") + path; return SRAY_EIO; }
 	fprintf(fp, "energy %f\n", R.opt.photon_energy);
@@ -4942,7 +4942,7 @@ void sray_gpu_shutdown(void)
 	for(Renderer::JobMaps &jm : R.job_maps) {
 		PhotonBufs *jp[] = {&jm.caust, &jm.gi};
 		for(PhotonBufs *p : jp) {
-			DevBuf *pbufs[] = {&p->ph, &p->starts, &p->tmp_ph, &p->keys, &p->keys2, &p->vals, &p->vals2, &p->hist, &p->scan};
+			DevBuf *pbufs[] = {&p->ph, &p->starts, &p->tmp_ph};
 			for(DevBuf *b : pbufs) b->release();
 		}
 	}
@@ -4964,7 +4964,7 @@ void sray_gpu_shutdown(void)
 	for(DevBuf *b : bufs) b->release();
 	PhotonBufs *pb[] = {&R.caust, &R.gi};
 	for(PhotonBufs *p : pb) {
-		DevBuf *pbufs[] = {&p->ph, &p->starts, &p->tmp_ph, &p->keys, &p->keys2, &p->vals, &p->vals2, &p->hist, &p->scan};
+		DevBuf *pbufs[] = {&p->ph, &p->starts, &p->tmp_ph};
 		for(DevBuf *b : pbufs) b->release();
 	}
 	if(R.pin) cudaFreeHost(R.pin);

@@ -118,7 +118,7 @@ struct NrcRegionStats {
 };
 
 struct PhotonBufs {
-	DevBuf ph, starts, tmp_ph, keys, keys2, vals, vals2, hist, scan;
+	DevBuf ph, starts, tmp_ph;
 	DPhotonMap map = DPhotonMap();
 	DPhotonMap order = DPhotonMap();   /* the grid of the order programs see the photons in */
 	int n = 0;
@@ -351,7 +351,7 @@ int photon_finalize_jobs(Renderer &R, const std::vector<PJobOut> &jobs, const st
 int photon_shoot_maps(Renderer &R, const DScene &base, cudaStream_t s, int *caust_stored, int *gi_stored);
 /* photon.cu: map `global` (0 caustic, 1 global) over the n photons in its buffer / from host photons */
 int photon_map_build(Renderer &R, int global, int n, cudaStream_t s);
-int photon_map_read(Renderer &R, int global, std::vector<DevPhoton> &h, cudaStream_t s);
+int photon_map_read(Renderer &R, int global, int m, std::vector<DevPhoton> &h, cudaStream_t s);
 int photon_map_restore(Renderer &R, int global, const std::vector<DevPhoton> &h, cudaStream_t s);
 
 }  // namespace sray
