@@ -1060,12 +1060,11 @@ struct QueueEmitter {
 	}
 };
 
-/* Bound by latency (the hit's surface, its material and light tables, one
- * after the other; 5 of 11 stall cycles per issue), so by warps in flight: 6
- * blocks of 128 per SM (80 registers, some spilled) instead of the 4 that 124
- * registers leave.  Batches of six 480x270 frames 2.38 -> 2.32 ms, 1080p
- * frames 15.50 -> 15.45; 5 blocks 2.36, 8 blocks 2.36. */
-__global__ void __launch_bounds__(128, 6) k_shade(DScene S, RayQueue qi, const int4 *hits, ShadeOut out, float4 *acc, int depth,
+/* 124 registers, 4 blocks per SM.  (6 blocks of 80 registers, some spilled,
+ * gained where boxes were wide and rays long; now six 480x270 frames take
+ * 2.35 ms that way and 2.29 this way, 1080p frames 15.41 and 15.34, and
+ * frames of a floor alone, whose queues' bandwidth counts, 1.50 and 1.46.) */
+__global__ void __launch_bounds__(128) k_shade(DScene S, RayQueue qi, const int4 *hits, ShadeOut out, float4 *acc, int depth,
 		DevCounters *ctr)
 {
 	int n = *qi.count;
