@@ -3882,7 +3882,7 @@ int Renderer::gathers(const GatherReq *q, const int *count, int cap, DevBuf &lis
 	const FrameQueries Q = {q, acc.as<float4>()};
 	DevCounters *c = ctr.as<DevCounters>();
 	int *l = nullptr;
-	if(cap >= GATHER_FEW_MIN) {
+	if(cap >= GATHER_FEW_MIN && (S.maps || S.caust.n > 0 || S.gi.n > 0)) {   /* (no photons, no requests) */
 		CK(list.ensure(((size_t)cap + 1) * sizeof(int)), "gather list");
 		l = list.as<int>();
 		CK(cudaMemsetAsync(l, 0, sizeof(int), st), "reset gather list");
