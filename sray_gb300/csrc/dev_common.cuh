@@ -1174,17 +1174,17 @@ __device__ __forceinline__ int trace_two_level(const DScene &S, V3 wo, V3 wd, in
  * once REFILL lanes have finished, writes their results and takes new rays
  * for them.  Each ray's own sequence of steps is that of trace_two_level, so
  * the results are the same.  load(i, o, d, time, scene) gives ray i (and its
- * number for done), done(i, result, walk) takes its result as
- * trace_two_level returns it.  1,000,003 rays from random points in random
+ * number for done), done(i, sure, walk) takes the walk's closest hit, or sure =
+ * 0 where the octrees must decide.  1,000,003 rays from random points in random
  * directions over the 1.26M-triangle terrain: 1.19 ms, against 1.89 with a
  * ray per thread (0.62 with the objects' own boxes and the ray and stack laid
  * out as above). */
-template <int REFILL, bool COUNT, bool ANY, bool SORT, class Load, class Done>
+template <int REFILL, bool COUNT, class Load, class Done>
 __device__ __forceinline__ void walk_stream(const DScene &S, float *world, int *next, int end, Load load, Done done, TraceCounters *tc, int *overflow)
 {
 	const unsigned FULL = 0xffffffffu;
 	const int lane = threadIdx.x & 31;
-	Walk<COUNT, ANY, SORT, SharedWorld> w;
+	Walk<COUNT, false, true, SharedWorld> w;
 	WStack st;
 	w.world.p = world;
 	w.cur = BVH_NONE;
@@ -1201,11 +1201,10 @@ __device__ __forceinline__ void walk_stream(const DScene &S, float *world, int *
 		if(idle == 32 || (more && idle >= REFILL)) {
 			/* the finished rays' results, then new rays for the idle lanes */
 			if(kind == WALK_END && ri >= 0) {
-				int out;
-				if(res == WALK_OVERFLOW) { *overflow = 1; out = ANY ? 0 : 1; w.bobj = -1; }
-				else if(res == WALK_UNDECIDED || !w.confirmed(S)) out = ANY ? 2 : 0;
-				else out = ANY ? (w.bobj >= 0 ? 1 : 0) : 1;
-				done(ri, out, w);
+				int sure = 1;
+				if(res == WALK_OVERFLOW) { *overflow = 1; w.bobj = -1; }
+				else if(res == WALK_UNDECIDED || !w.confirmed(S)) sure = 0;
+				done(ri, sure, w);
 				ri = -1;
 			}
 			if(!more) break;

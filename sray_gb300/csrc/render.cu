@@ -147,14 +147,12 @@ __global__ void k_ray_permute(RayQueue in, const unsigned *vals, int n, RayQueue
 	}
 }
 
-/* idle lanes at which a warp takes new rays: light samples and secondary
- * rays stay in the order of the pixels they come from, and a refill mixes
- * early and late ones, so that they wait longer than a program's own rays
- * (frame of 1920x1080, 4 samples: 27.8 ms at 16 / 24, 28.5 at 12 / 32 and
- * at 24 / 32, 29.0 at 32 / 32, 30.1 at 4 / 4; a million random rays: 1.19 ms
- * at 8 to 12, 1.25 at 20) */
+/* idle lanes at which a warp takes new rays: secondary rays stay in the order
+ * of the pixels they come from, and a refill mixes early and late ones, so
+ * that they wait longer than a program's own rays (frame of 1920x1080, 4
+ * samples: 15.18 ms at 16, 15.57 at 8, 15.35 at 24; bakes with 2.5M photons
+ * 3.41, 3.39, 3.46; a million random rays: 635 us at 10, 650 at 4, 652 at 20) */
 #define TRACE_REFILL 16
-#define SHADOW_REFILL 24
 #define CAST_REFILL 10
 /* Closest hits through the hierarchies, a chunk of the pass's rays per
  * block (walk_stream); the rays whose result the octrees must decide are
@@ -174,7 +172,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_trace(DScene S, RayQu
 	__syncthreads();
 	TraceCounters tc = {0, 0};
 	int overflow = 0;
-	walk_stream<TRACE_REFILL, COUNT, false, true>(S, world + threadIdx.x, &next, min(first + chunk, n),
+	walk_stream<TRACE_REFILL, COUNT>(S, world + threadIdx.x, &next, min(first + chunk, n),
 			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
 				if(q.order) i = (int)q.order[i];
 				float4 o4 = q.o[i], d4 = q.d[i];
@@ -1235,43 +1233,33 @@ __global__ void __launch_bounds__(128) k_render_pool(DScene S, RayQueue pool, in
 
 /* shadow rays: the reference tests visibility with cast_ray(shadow_ray)
  * (src/shader.cc:266), a hit anywhere on the segment [eps, 1] blocks */
-/* shadow rays; chunks and fb as for k_trace */
+/* A ray per thread, fb as for k_trace.  The light samples of neighbouring
+ * pixels walk alike and end at the first hit, so the streamed walk only adds
+ * its votes: floor and 0 / 10 / 100 / 400 spheres under four lights at
+ * 1920x1080, 4 samples, 481 / 662 / 1,175 / 1,670 us this way, 620 / 851 /
+ * 1,350 / 1,773 streamed; the 1.26M-triangle terrain's frames 15.36 ms and
+ * 15.41. */
 template <bool SORT = true, bool COUNT = false>
-__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow(DScene S, const ShadowReq *sq, const int *sq_count, int chunk, float4 *acc,
+__global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_shadow(DScene S, const ShadowReq *sq, const int *sq_count, float4 *acc,
 		DevCounters *ctr, int *fb)
 {
-	__shared__ float world[WORLD_WORDS * SRAY_TRACE_THREADS];
-	__shared__ int next;
 	const int n = *sq_count;
-	if(blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->rays[2], (unsigned long long)n);
-	const int first = blockIdx.x * chunk;
-	if(first >= n) return;
-	if(threadIdx.x == 0) next = first;
-	__syncthreads();
-	TraceCounters tc = {0, 0};
 	int overflow = 0;
-	walk_stream<SHADOW_REFILL, COUNT, true, SORT>(S, world + threadIdx.x, &next, min(first + chunk, n),
-			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
-				float4 a = sq[i].a, b = sq[i].b;
-				o = mk(a.x, a.y, a.z);
-				d = mk(b.x, b.y, b.z);
-				time = __float_as_int(a.w);
-				scene = S.nscenes > 1 ? __float_as_int(sq[i].w.w) : -1;
-				return i;
-			},
-			[&](int i, int res, const Walk<COUNT, true, SORT, SharedWorld> &) {
-				if(res == 2) {
-					fb[1 + atomicAdd(fb, 1)] = i;
-				} else if(res == 0) {
-					float4 w = sq[i].w;
-					acc_add(acc, __float_as_int(sq[i].b.w), w.x, w.y, w.z);
-				}
-			}, &tc, &overflow);
+	TraceCounters tc = {0, 0};
+	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+		ShadowReq r = sq[i];
+		Hit h;
+		int res = trace_two_level<COUNT, true, SORT>(S, mk(r.a.x, r.a.y, r.a.z), mk(r.b.x, r.b.y, r.b.z), __float_as_int(r.a.w), h, &tc,
+				&overflow, S.nscenes > 1 ? __float_as_int(r.w.w) : -1);
+		if(res == 2) fb[1 + atomicAdd(fb, 1)] = i;
+		else if(res == 0) acc_add(acc, __float_as_int(r.b.w), r.w.x, r.w.y, r.w.z);
+	}
 	if(overflow) atomicOr(&ctr->overflow, 1);
 	if(COUNT) {
 		atomicAdd(&ctr->snodes, tc.nodes);
 		atomicAdd(&ctr->sprims, tc.prims);
 	}
+	if(blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr->rays[2], (unsigned long long)n);
 }
 
 /* the listed segments, octrees only */
@@ -2184,7 +2172,7 @@ __global__ void __launch_bounds__(SRAY_TRACE_THREADS, 8) k_cast(DScene S, CastRa
 	}
 	__syncthreads();
 	int overflow = 0;
-	walk_stream<CAST_REFILL, false, false, true>(S, world + threadIdx.x, &next, min(first + chunk, n),
+	walk_stream<CAST_REFILL, false>(S, world + threadIdx.x, &next, min(first + chunk, n),
 			[&](int i, V3 &o, V3 &d, int &time, int &scene) {
 				o = R.o(i);
 				d = R.d(i);
@@ -2309,16 +2297,16 @@ __global__ void k_primary_hits(DScene S, RayQueue q, const int4 *hits, int *obj,
 #define PACKET_MIN_PIXELS 400000
 static bool packet_image(int npix, int njobs) { return npix / (njobs > 1 ? njobs : 1) >= PACKET_MIN_PIXELS; }
 
-/* Rays per block of a streaming traversal (k_trace, k_shadow, k_cast) of n
+/* Rays per block of a streaming traversal (k_trace, k_cast) of n
  * rays: about a wave of resident blocks, each taking its lanes' next rays
  * from its own chunk, up to the limit of the caller's kind of pass.  A larger
  * chunk has fewer lanes waiting at its end; a smaller one keeps a block's
  * rays close together (photons leave sorted by direction and origin) and
- * ends sooner, which frees its SM for the streams beside it.  Measured:
- * photon maps of 2.5M photons 7.05 ms with 256, 7.25 with 512, 7.5 with
- * 1024, 7.2 with 128; frame of 1920x1080, 4 samples, 27.2 ms with 512 for
- * its own passes, 27.7 with 256, 27.8 with 1024; a million random rays alone
- * 1.19 ms with 1024, 1.27 with 512. */
+ * ends sooner, which frees its SM for the streams beside it.  Measured: bakes
+ * with 2.5M photons 3.41 ms with 256 for the photons' passes, 3.52 with 128,
+ * 3.48 with 512; frame of 1920x1080, 4 samples, 15.18 ms with 512 for its own
+ * passes, 15.40 with 256 and with 1024; a million random rays 636 us with
+ * 1024, 673 with 512. */
 #define PHOTON_CHUNK 256
 #define FRAME_CHUNK 512
 #define CAST_CHUNK 1024
@@ -3905,18 +3893,18 @@ int Renderer::shadow_rays_on(const ShadowReq *q, int *count, int cap, DevBuf &fb
 {
 	CK(fb.ensure(((size_t)cap + 1) * sizeof(int)), "fallback list");
 	CK(cudaMemsetAsync(fb.p, 0, sizeof(int), st), "reset fallback list");
-	const int chunk = stream_chunk(cap, FRAME_CHUNK), g = (cap + chunk - 1) / chunk;
+	const int g = grid_for(cap, 128);
 	float4 *a = acc.as<float4>();
 	DevCounters *c = ctr.as<DevCounters>();
 	int *f = fb.as<int>();
 	if(prof_flags & 2)   /* counting the traversal work: every pass thread per segment */
-		LAUNCH(*this, "shadow", st, k_shadow<true, true><<<g, 128, 0, st>>>(S, q, count, chunk, a, c, f));
+		LAUNCH(*this, "shadow", st, k_shadow<true, true><<<g, 128, 0, st>>>(S, q, count, a, c, f));
 	else if(cap <= tune.warp_segments)
 		LAUNCH(*this, "shadow", st, k_shadow_warp<<<grid_for(cap, 4), 128, 0, st>>>(S, q, count, a, c, f));
 	else if(tune.shadow_order)
-		LAUNCH(*this, "shadow", st, k_shadow<false><<<g, 128, 0, st>>>(S, q, count, chunk, a, c, f));
+		LAUNCH(*this, "shadow", st, k_shadow<false><<<g, 128, 0, st>>>(S, q, count, a, c, f));
 	else
-		LAUNCH(*this, "shadow", st, k_shadow<true><<<g, 128, 0, st>>>(S, q, count, chunk, a, c, f));
+		LAUNCH(*this, "shadow", st, k_shadow<true><<<g, 128, 0, st>>>(S, q, count, a, c, f));
 	LAUNCH(*this, "octree_retrace", st, k_shadow_octree<<<retrace_grid(), 128, 0, st>>>(S, q, a, c, f));
 	return 0;
 }
