@@ -66,8 +66,20 @@ struct Builder {
 
 	static int leaf_ref(int b, int e) { return ~((b << 4) | (e - b)); }
 
-	/* reference to a subtree over order[b, e) */
-	int build(int b, int e, int depth)
+	int bin_of(int f, int a, float from, double scale) const
+	{
+		const int k = (int)(((double)(*cen)[(size_t)f * 3 + a] - (double)from) * scale);
+		return k < 0 ? 0 : (k >= NBINS ? NBINS - 1 : k);
+	}
+
+	/* reference to a subtree over order[b, e), whose boxes' bounds are pb.
+	 * A node reads its items three times: the centroids' bounds, the bins of
+	 * all three axes, and the partition by the best split, whose sides'
+	 * bounds are those of its bins.  (2,000 objects with boxes of their own
+	 * 1.6 ms with a pass per axis, all bins cleared and the bounds taken
+	 * anew, 1.2 this way, 20,000 18.3 and 13.9; over the octree leaves'
+	 * unions, many of which coincide and need no bins, 1.1 and 13.8 before.) */
+	int build(int b, int e, int depth, const Bounds &pb)
 	{
 		max_depth = std::max(max_depth, depth);
 		int n = e - b;
@@ -83,63 +95,73 @@ struct Builder {
 		}
 		int axis = -1, split = -1;
 		double best = DBL_MAX;
+		Bounds lb, rbx;
 		if(depth < MEDIAN_DEPTH) {
-			Bounds pb = range_bounds(b, e);
-			double parea = pb.area();
+			/* only bins with items are cleared and looked at: a split after an
+			 * empty bin is the one before it */
+			const double parea = pb.area();
+			Bounds bin[3][NBINS];
+			int cnt[3][NBINS];
+			unsigned used[3] = {0, 0, 0};
+			double sc[3];
 			for(int a = 0; a < 3; a++) {
-				double ext = (double)cb.mx[a] - (double)cb.mn[a];
-				if(!(ext > 0.0)) continue;
-				Bounds bin[NBINS];
-				int cnt[NBINS] = {0};
-				for(int k = 0; k < NBINS; k++) bin[k].clear();
-				double sc = NBINS / ext;
-				for(int i = b; i < e; i++) {
-					int f = (*order)[i];
-					int k = (int)(((double)(*cen)[(size_t)f * 3 + a] - (double)cb.mn[a]) * sc);
-					k = k < 0 ? 0 : (k >= NBINS ? NBINS - 1 : k);
-					cnt[k]++;
-					bin[k].grow((*tb)[f]);
+				const double ext = (double)cb.mx[a] - (double)cb.mn[a];
+				sc[a] = ext > 0.0 ? NBINS / ext : 0.0;
+			}
+			for(int i = b; i < e; i++) {
+				const int f = (*order)[i];
+				const Bounds &fb = (*tb)[f];
+				for(int a = 0; a < 3; a++) {
+					if(sc[a] == 0.0) continue;
+					const int k = bin_of(f, a, cb.mn[a], sc[a]);
+					if((used[a] >> k) & 1u) {
+						cnt[a][k]++;
+						bin[a][k].grow(fb);
+					} else {
+						used[a] |= 1u << k;
+						cnt[a][k] = 1;
+						bin[a][k] = fb;
+					}
 				}
-				double ra[NBINS];
+			}
+			for(int a = 0; a < 3; a++) {
+				if(sc[a] == 0.0) continue;
+				int at[NBINS], m = 0;
+				for(int k = 0; k < NBINS; k++) if((used[a] >> k) & 1u) at[m++] = k;
+				if(m < 2) continue;
+				Bounds right[NBINS];
 				int rn[NBINS];
-				Bounds acc;
-				acc.clear();
-				int accn = 0;
-				for(int k = NBINS - 1; k > 0; k--) {
-					acc.grow(bin[k]);
-					accn += cnt[k];
-					ra[k] = acc.area();
-					rn[k] = accn;
+				right[m - 1] = bin[a][at[m - 1]];
+				rn[m - 1] = cnt[a][at[m - 1]];
+				for(int j = m - 2; j > 0; j--) {
+					right[j] = right[j + 1];
+					right[j].grow(bin[a][at[j]]);
+					rn[j] = rn[j + 1] + cnt[a][at[j]];
 				}
-				acc.clear();
-				accn = 0;
-				for(int k = 0; k < NBINS - 1; k++) {
-					acc.grow(bin[k]);
-					accn += cnt[k];
-					if(accn == 0 || rn[k + 1] == 0) continue;
-					double cost = 1.0 + (acc.area() * accn + ra[k + 1] * rn[k + 1]) / (parea > 0.0 ? parea : 1.0);
+				Bounds acc = bin[a][at[0]];
+				int accn = cnt[a][at[0]];
+				for(int j = 0; j < m - 1; j++) {
+					if(j > 0) {
+						acc.grow(bin[a][at[j]]);
+						accn += cnt[a][at[j]];
+					}
+					double cost = 1.0 + (acc.area() * accn + right[j + 1].area() * rn[j + 1]) / (parea > 0.0 ? parea : 1.0);
 					if(cost < best) {
 						best = cost;
 						axis = a;
-						split = k;
+						split = at[j];
+						lb = acc;
+						rbx = right[j + 1];
 					}
 				}
 			}
 			if(n <= leaf_max && (axis < 0 || best >= (double)n)) return leaf_ref(b, e);
 		}
-		int mid;
+		int mid = b;
 		if(axis >= 0) {
-			double ext = (double)cb.mx[axis] - (double)cb.mn[axis];
-			double sc = NBINS / ext;
-			int *beg = order->data() + b, *end = order->data() + e;
-			int *m = std::partition(beg, end, [&](int f) {
-				int k = (int)(((double)(*cen)[(size_t)f * 3 + axis] - (double)cb.mn[axis]) * sc);
-				k = k < 0 ? 0 : (k >= NBINS ? NBINS - 1 : k);
-				return k <= split;
-			});
+			const double sc = NBINS / ((double)cb.mx[axis] - (double)cb.mn[axis]);
+			int *m = std::partition(order->data() + b, order->data() + e, [&](int f) { return bin_of(f, axis, cb.mn[axis], sc) <= split; });
 			mid = (int)(m - order->data());
-		} else {
-			mid = b;
 		}
 		if(mid <= b || mid >= e) {
 			/* no useful split (coincident centroids or the depth cap): halve
@@ -149,12 +171,13 @@ struct Builder {
 			mid = b + n / 2;
 			std::nth_element(order->begin() + b, order->begin() + mid, order->begin() + e,
 					[&](int x, int y) { return (*cen)[(size_t)x * 3 + a] < (*cen)[(size_t)y * 3 + a]; });
+			lb = range_bounds(b, mid);
+			rbx = range_bounds(mid, e);
 		}
 		int id = (int)nodes->size();
 		nodes->push_back(DevBvhNode());
-		int l = build(b, mid, depth + 1);
-		int r = build(mid, e, depth + 1);
-		Bounds lb = range_bounds(b, mid), rbx = range_bounds(mid, e);
+		int l = build(b, mid, depth + 1, lb);
+		int r = build(mid, e, depth + 1, rbx);
 		DevBvhNode &nd = (*nodes)[id];
 		memset(&nd, 0, sizeof nd);
 		for(int a = 0; a < 3; a++) {
@@ -196,8 +219,8 @@ void MeshBvh::build_items(const float *mn, const float *mx, size_t n, int leaf_m
 	B.nodes = &nodes;
 	B.leaf_min = leaf_max < LEAF_MIN ? leaf_max : LEAF_MIN;
 	B.leaf_max = leaf_max;
-	nodes.reserve(n / 2 + 1);
-	int ref = B.build(0, (int)n, 1);
+	nodes.reserve(leaf_max < 2 ? n : n / 2 + 1);
+	int ref = B.build(0, (int)n, 1, B.range_bounds(0, (int)n));
 	if(ref < 0) {
 		/* at most leaf_min items: a root node with one leaf */
 		DevBvhNode nd;

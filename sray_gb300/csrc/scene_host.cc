@@ -517,6 +517,7 @@ struct OctBuilder {
 	BuildOctree *o;
 	const std::vector<Box> *boxes;
 	int max_depth, max_items;
+	std::vector<int> taken;      /* a child's items, while they are counted */
 
 	void subdivide(int ni, int lvl)
 	{
@@ -536,9 +537,9 @@ struct OctBuilder {
 				ch.box.mx[i] = hi[k][i] ? b.mx[i] : c[i];
 			}
 			const std::vector<int> &pit = o->nodes[ni].items;
-			std::vector<int> it;
-			for(size_t j = 0; j < pit.size(); j++) if(overlap((*boxes)[pit[j]], ch.box)) it.push_back(pit[j]);
-			o->nodes[first + k].items.swap(it);
+			taken.clear();
+			for(int j : pit) if(overlap((*boxes)[j], ch.box)) taken.push_back(j);
+			ch.items.assign(taken.begin(), taken.end());
 			subdivide(first + k, lvl + 1);
 		}
 		std::vector<int>().swap(o->nodes[ni].items);
