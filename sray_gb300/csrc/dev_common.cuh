@@ -99,7 +99,6 @@ struct DScene {
 	const int *bhome;         /* their home nodes in the mesh octrees */
 	const DevBvh4 *tnodes;    /* object hierarchy, 4-wide (world space), null if none */
 	const int *ohome;         /* per object: its home node in the scene octree */
-	unsigned long long *bvh_fallbacks;   /* hits the octree did not confirm */
 	const DevObj *objs;
 	int nobj;
 	const float *xf;          /* per object per time, XF_STRIDE floats */
@@ -1250,30 +1249,6 @@ template <bool COUNT>
 static __device__ __noinline__ void trace_closest_octree(const DScene &S, V3 wo, V3 wd, int time, Hit &h, TraceCounters *tc, int *overflow)
 {
 	trace_closest_octree_impl<COUNT>(S, wo, wd, time, h, tc, overflow);
-}
-
-static __device__ __noinline__ bool trace_any_octree(const DScene &S, V3 wo, V3 wd, int time, int *overflow)
-{
-	return trace_any_octree_impl(S, wo, wd, time, overflow);
-}
-
-/* closest hit, the octrees deciding when the hierarchies cannot */
-template <bool COUNT>
-__device__ inline void trace_closest(const DScene &S, V3 wo, V3 wd, int time, Hit &h, TraceCounters *tc, int *overflow)
-{
-	if(!trace_two_level<COUNT, false>(S, wo, wd, time, h, tc, overflow)) {
-		atomicAdd(S.bvh_fallbacks, 1ull);
-		trace_closest_octree<COUNT>(S, wo, wd, time, h, tc, overflow);
-	}
-}
-
-__device__ inline bool trace_any(const DScene &S, V3 wo, V3 wd, int time, int *overflow)
-{
-	Hit h;
-	int res = trace_two_level<false, true>(S, wo, wd, time, h, nullptr, overflow);
-	if(res != 2) return res == 1;
-	atomicAdd(S.bvh_fallbacks, 1ull);
-	return trace_any_octree(S, wo, wd, time, overflow);
 }
 
 /* ---------------- surface point ---------------- */

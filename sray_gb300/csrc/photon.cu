@@ -1207,11 +1207,10 @@ int photon_trace_jobs(Renderer &R, const DScene &base, std::vector<PhotonJobSpec
 	R.pq[0].order = R.pq[1].order = nullptr;
 	if(R.ensure_pqueue(0, (int)all) || R.ensure_pqueue(1, (int)all)) return SRAY_ECUDA;
 	PCK(R.phits.ensure((size_t)all * 16), "photon hits");
-	/* the scene as the photon kernels see it: their counters, and in a scene
-	 * set the photon job table, through which a photon's global index finds
-	 * its scene (the render's pixel table is not theirs) */
+	/* the scene as the photon kernels see it: in a scene set with the photon
+	 * job table, through which a photon's global index finds its scene (the
+	 * render's pixel table is not theirs) */
 	DScene PS = base;
-	PS.bvh_fallbacks = &R.pctr.as<DevCounters>()->bvh_fallbacks;
 	PS.jobs = PS.nscenes > 1 ? R.pw_pix.as<DevJob>() : nullptr;
 	PS.njobs = PS.nscenes > 1 ? n : 0;
 	DevCounters *pctr = R.pctr.as<DevCounters>();

@@ -677,20 +677,6 @@ struct ShadeOut {
 	int sq_cap;
 };
 
-__device__ __forceinline__ void push_child(ShadeOut &out, V3 o, V3 d, float energy, int iter, int path, int dsub,
-		const IorStack &st, float wr, float wg, float wb, int pixel, int aslot, int sample, int time, int *overflow)
-{
-	int slot = warp_alloc(out.qo.count, 1);
-	if(slot >= out.qo.cap) { *overflow = 1; return; }
-	RayQueue &q = out.qo;
-	q.o[slot] = make_float4(o.x, o.y, o.z, energy);
-	q.d[slot] = make_float4(d.x, d.y, d.z, st.ior);
-	q.w[slot] = make_float4(wr, wg, wb, __int_as_float(pixel));
-	q.meta[slot] = make_int4(aslot, iter, path, time);
-	q.stk[slot] = make_float4(st.stk[0], st.stk[1], st.stk[2], st.stk[3]);
-	q.ext[slot] = make_int2(sample | (dsub << 16), st.sp);
-}
-
 __device__ __forceinline__ void push_gather(ShadeOut &out, V3 pos, V3 n, int kind, int pixel, float wr, float wg, float wb,
 		int *overflow)
 {
@@ -1372,17 +1358,6 @@ __device__ __forceinline__ double dist2(const float4 &p, V3 q)
 {
 	double dx = (double)p.x - (double)q.x, dy = (double)p.y - (double)q.y, dz = (double)p.z - (double)q.z;
 	return dx * dx + dy * dy + dz * dz;
-}
-
-/* exact range decisions without double arithmetic (range_ff.h) */
-__device__ __forceinline__ bool range_ff(const DPhotonMap &M, float4 p, V3 q, bool &in, unsigned &key)
-{
-	int inr = 0;
-	uint32_t k = 0;
-	if(!sray_range_ff(p.x, p.y, p.z, q.x, q.y, q.z, M.r2_hi, M.r2_lo, &inr, &k)) return false;
-	in = inr != 0;
-	key = k;
-	return true;
 }
 
 /* a warp's shared memory: the candidates of its query (squared distances'
@@ -2438,7 +2413,6 @@ void Renderer::fill_scene_desc()
 	D.bhome = bhome.as<int>();
 	D.tnodes = has_tlas ? tnodes.as<DevBvh4>() : nullptr;
 	D.ohome = ohome.as<int>();
-	D.bvh_fallbacks = ctr.p ? &ctr.as<DevCounters>()->bvh_fallbacks : nullptr;
 	D.objs = objs.as<DevObj>();
 	D.nobj = (int)sc.objs.size();
 	D.xf = xf.as<float>();
