@@ -473,7 +473,8 @@ int sray_gpu_autotune(long msec, float *fb, int frames, void *stream, sray_tunin
  *    group's maps copied out of the wavefront's buffers before the next,
  *    and the lights' projection maps are made for two lights, and from about
  *    that many pairs of a light sample and an object, at a time (default
- *    1,024 and 2^20); the images do not change. */
+ *    1,024 and 2^20), every map's coverage by the ordered sum that few maps
+ *    need otherwise; the images do not change. */
 typedef struct sray_faults {
 	int fail_alloc_after;
 	int queue_cap;

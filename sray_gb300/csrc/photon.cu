@@ -428,10 +428,11 @@ __global__ void __launch_bounds__(128) k_proj_mark(const ProjSample *samples, in
 /* A block per map: its bits and its coverage.  The coverage that counts is the
  * ordered double sum rounded to float.  Any order of summation is within
  * 2^-41 of it (2,048 terms, each addition within 2^-53), so a sum in parallel
- * gives that float unless it lies within 2^-40 of where floats round; then
- * (once in some 30,000 maps) the cells are sorted by the order in which they
+ * gives that float unless it lies within margin = 2^-40 of where floats round;
+ * then (once in some 30,000 maps) the cells are sorted by the order in which they
  * were set and added one by one, 2,048 dependent additions taking 65 us. */
-__global__ void __launch_bounds__(1024) k_proj_cover(const unsigned long long *first, const ProjTables *tables, uint32_t *bits, float *cov)
+__global__ void __launch_bounds__(1024) k_proj_cover(const unsigned long long *first, const ProjTables *tables, double margin,
+		uint32_t *bits, float *cov)
 {
 	__shared__ unsigned long long key[PROJ_CELLS];
 	__shared__ double part[32];
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(1024) k_proj_cover(const unsigned long long *f
 		for(int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
 		if(t == 0) {
 			const float f = whole ? 1.0f : (nset == 0 ? 0.0f : (float)fmin(c, 1.0));
-			const double lo = c * (1.0 - 1.0 / 1099511627776.0), hi = c * (1.0 + 1.0 / 1099511627776.0);
+			const double lo = c * (1.0 - margin), hi = c * (1.0 + margin);
 			unsure = !whole && nset > 0 && ((float)fmin(lo, 1.0) != f || (float)fmin(hi, 1.0) != f);
 			cov[blockIdx.x] = f;
 		}
@@ -1066,7 +1067,7 @@ static int project_jobs(Renderer &R, std::vector<PhotonJobSpec> &spec, ProjHost 
 			}
 		}
 		LAUNCH(R, "projmaps", s, k_proj_cover<<<lights * 2, 1024, 0, s>>>(R.pj_first.as<unsigned long long>(), R.pj_tables.as<ProjTables>(),
-				R.pw_bits.as<uint32_t>() + (size_t)done * 128, R.pw_cov.as<float>() + (size_t)done * 2));
+				small > 0 ? 1.0 : 1.0 / 1099511627776.0, R.pw_bits.as<uint32_t>() + (size_t)done * 128, R.pw_cov.as<float>() + (size_t)done * 2));
 		PCK(cudaGetLastError(), "projection maps");
 		return 0;
 	};
