@@ -206,9 +206,9 @@ def algorithmic_bytes(st):
         "shadow": (st["shadow_rays"] * (48 + 16) + st["shadow_node_visits"] * 128 + st["shadow_prim_tests"] * 48,
                    st["shadow_rays"], "segments",
                    "48 B request + 16 B accumulator per light-sample segment, 128 B per node read, 48 B per triangle tested"),
-        "gather": (st["gathers"] * (48 + 16 + 64) + st["gather_tested"] * 16 + st["gather_candidates"] * 32,
+        "gather": (st["gathers"] * (48 + 16 + 176) + st["gather_tested"] * 16 + st["gather_candidates"] * 32,
                    st["gathers"], "queries",
-                   "48 B request + 16 B accumulator + 8 cells x 8 B per query, 16 B position per photon tested, "
+                   "48 B request + 16 B accumulator + 22 rows of cells x 8 B per query, 16 B position per photon tested, "
                    "32 B more per photon within range"),
     }
 

@@ -474,8 +474,8 @@ __device__ __forceinline__ float4 load_split(const DevNode *nodes, int ni)
  * last triangle seen per slot of a 16-way direct-mapped table, cleared
  * whenever the ray enters a mesh, and skips repeats.  The table is the
  * thread's own (local memory), not shared memory: the octree-only kernels
- * run between the hierarchy kernels, which use no shared memory, and a
- * kernel that needs shared memory waits for SMs to drain the other
+ * run between the hierarchy kernels, which use little or none, and a kernel
+ * that needs much of it (24 KB per block) waits for SMs to drain the other
  * stream's blocks before it can start. */
 #define SRAY_TRACE_THREADS 128
 #define SRAY_TRI_MBOX 16

@@ -2265,15 +2265,15 @@ __global__ void k_primary_hits(DScene S, RayQueue q, const int4 *hits, int *obj,
  * scene.  A warp's packet walks everything any of its rays meets, in one
  * chain: on small images that chain is the pass.  Object ids of moving scenes
  * (100,000 / 400,000 triangles), packets against rays that each walk alone:
- * 480x270 281 / 385 against 199 / 221 us, 640x360 256 / 433 against 259 /
- * 310, 960x540 296 / 477 against 383 / 481, 1280x720 300 / 442 against 407 /
- * 493, 1920x1080 473 / 664 against 486 / 590; frames of the small scene 817
- * against 910 us at 960x540 and no difference at 480x270. */
+ * 480x270 244 / 346 against 186 / 209 us, 640x360 223 / 380 against 234 /
+ * 271, 960x540 235 / 384 against 369 / 471, 1280x720 237 / 366 against 373 /
+ * 453, 1920x1080 381 / 584 against 499 / 604; frames of the small scene 443
+ * against 430 us at 480x270, 538 against 588 at 960x540. */
 #define PACKET_MIN_PIXELS 400000
 static bool packet_image(int npix, int njobs) { return npix / (njobs > 1 ? njobs : 1) >= PACKET_MIN_PIXELS; }
 
-/* Rays per block of a streaming traversal (k_trace, k_cast) of n
- * rays: about a wave of resident blocks, each taking its lanes' next rays
+/* Rays per block of a streaming traversal (k_trace, k_cast) of n rays:
+ * about a wave of resident blocks, each taking its lanes' next rays
  * from its own chunk, up to the limit of the caller's kind of pass.  A larger
  * chunk has fewer lanes waiting at its end; a smaller one keeps a block's
  * rays close together (photons leave sorted by direction and origin) and
@@ -2871,9 +2871,8 @@ int Renderer::build_frame(long bt0, long bt1, cudaStream_t s)
 }
 
 /* projection maps and both photon maps on stream s, with the scene view
- * `base` (the projection-map tables are set in a copy of it); the map
- * descriptors land in caust.map / gi.map, which fill_scene_desc() copies
- * into S */
+ * `base`; the map descriptors land in caust.map / gi.map, which
+ * fill_scene_desc() copies into S */
 int Renderer::shoot_maps(const DScene &base, cudaStream_t s, int *nc, int *ng)
 {
 	caust.map.n = 0;
@@ -3072,9 +3071,8 @@ int Renderer::ensure_pqueue(int which, int cap)
 	return queue_alloc(pqbuf[which], pq[which], pqcap[which], cap);
 }
 
-/* the n rays of q[cur], sorted by direction octant and origin cell into the
- * spare queue, which then becomes q[cur] (the pass's queue and its
- * allocation swapped with the spare's) */
+/* the order of Q's first n rays by direction octant and origin cell: their
+ * indices, in keysb until its next use */
 int Renderer::sort_queue(const RayQueue &Q, DevBuf &keysb, DevBuf &hist, DevBuf &part, int n, int bits, const char *name, cudaStream_t s,
 		unsigned **sorted)
 {
@@ -3092,6 +3090,8 @@ int Renderer::sort_queue(const RayQueue &Q, DevBuf &keysb, DevBuf &hist, DevBuf 
 	return sort_pairs(*this, keys, vals, keys2, vals2, n, bits, hist, part, name, s, &keys, sorted);
 }
 
+/* the n rays of q[cur] moved in that order into the spare queue, which then
+ * becomes q[cur] (the queues and their allocations swapped) */
 int Renderer::sort_pass(int cur, int n, cudaStream_t s)
 {
 	if(n < 2 || sc.oct.nodes.empty()) return 0;
