@@ -255,6 +255,8 @@ int sray_gpu_render_pixels(long msec, float *fb, int fb_is_device, void *stream)
  * Outputs: object index (-1 = miss), primitive index (triangle index of the
  * object's mesh, 0 for spheres/cylinders), the hit parameter t, and a flag
  * byte that is 1 when another primitive was found at exactly the same t.
+ * (A cylinder reports its far root, also beyond t = 1, where the near one is
+ * behind the origin or beside the cylinder: src/cylinder.cc:125-185.)
  * After the first call of a context no call allocates device memory. */
 int sray_gpu_cast_rays(int n, const float *orig, const float *dir, const int *time,
 		int *obj, int *prim, float *t, unsigned char *tie, void *stream);
